@@ -98,40 +98,57 @@ __device__ __forceinline__ void load_wtile(WTile<Q>& w, const uint4* qbase, cons
     if (Q != BF16) w.s = ldg_stream(sbase + (size_t)tile * 8 + (lane >> 2));
 }
 
+// The constants of the unpacking, pinned in registers: as literals they are materialised anew at every use
+// once registers are short, ~45 extra instructions per 16 x 128 tile.
+struct UnpackConst {
+    uint32_t or_a, or_b, sub_a, sub_b;
+};
+template <int Q>
+__device__ __forceinline__ UnpackConst unpack_const() {
+    // Q4_0: 1024 + n and 64 + n as f16 with their offsets 1032 and 72; Q8_0: 0x64xx = 1024 + xx, offset 1152
+    return (Q == Q4_0) ? UnpackConst{0x64006400u, 0x54005400u, 0x64086408u, 0x54805480u}
+                       : UnpackConst{0x64646464u, 0x80808080u, 0x64806480u, 0u};
+}
+template <int Q>
+__device__ __forceinline__ UnpackConst unpack_const_pinned() {
+    UnpackConst c = unpack_const<Q>();
+    asm volatile("" : "+r"(c.or_a), "+r"(c.or_b), "+r"(c.sub_a), "+r"(c.sub_b));
+    return c;
+}
+
 // A fragments of the two MMAs of block b of the tile: a_lo covers elements 0..15,
 // a_hi elements 16..31. Values are the exact integers (q - 8) / q as f16, or the
 // bf16 weights themselves.
 template <int Q>
 __device__ __forceinline__ void unpack_block(const WTile<Q>& w, int b, uint32_t (&a_lo)[4],
-                                             uint32_t (&a_hi)[4]) {
+                                             uint32_t (&a_hi)[4], const UnpackConst& k = unpack_const<Q>()) {
     if (Q == Q4_0) {
         const uint4 v = w.q[b >> 1];
         const uint32_t wg = (b & 1) ? v.z : v.x;   // row g
         const uint32_t wg8 = (b & 1) ? v.w : v.y;  // row g+8
-        const uint32_t sub_lo = 0x64086408u;       // 1032 = 1024 + 8
-        const uint32_t sub_hi = 0x54805480u;       // 72   = 64 + 8
-        a_lo[0] = hsub2_u32(lop_and_or(wg, 0x000F000Fu, 0x64006400u), sub_lo);
-        a_lo[1] = hsub2_u32(lop_and_or(wg8, 0x000F000Fu, 0x64006400u), sub_lo);
-        a_lo[2] = hsub2_u32(lop_and_or(wg >> 8, 0x000F000Fu, 0x64006400u), sub_lo);
-        a_lo[3] = hsub2_u32(lop_and_or(wg8 >> 8, 0x000F000Fu, 0x64006400u), sub_lo);
-        a_hi[0] = hsub2_u32(lop_and_or(wg, 0x00F000F0u, 0x54005400u), sub_hi);
-        a_hi[1] = hsub2_u32(lop_and_or(wg8, 0x00F000F0u, 0x54005400u), sub_hi);
-        a_hi[2] = hsub2_u32(lop_and_or(wg >> 8, 0x00F000F0u, 0x54005400u), sub_hi);
-        a_hi[3] = hsub2_u32(lop_and_or(wg8 >> 8, 0x00F000F0u, 0x54005400u), sub_hi);
+        const uint32_t sub_lo = k.sub_a, sub_hi = k.sub_b;
+        a_lo[0] = hsub2_u32(lop_and_or(wg, 0x000F000Fu, k.or_a), sub_lo);
+        a_lo[1] = hsub2_u32(lop_and_or(wg8, 0x000F000Fu, k.or_a), sub_lo);
+        a_lo[2] = hsub2_u32(lop_and_or(wg >> 8, 0x000F000Fu, k.or_a), sub_lo);
+        a_lo[3] = hsub2_u32(lop_and_or(wg8 >> 8, 0x000F000Fu, k.or_a), sub_lo);
+        a_hi[0] = hsub2_u32(lop_and_or(wg, 0x00F000F0u, k.or_b), sub_hi);
+        a_hi[1] = hsub2_u32(lop_and_or(wg8, 0x00F000F0u, k.or_b), sub_hi);
+        a_hi[2] = hsub2_u32(lop_and_or(wg >> 8, 0x00F000F0u, k.or_b), sub_hi);
+        a_hi[3] = hsub2_u32(lop_and_or(wg8 >> 8, 0x00F000F0u, k.or_b), sub_hi);
     } else if (Q == Q8_0) {
         const uint4 v = w.q[b];
         // bytes biased by 128 -> unsigned; 0x64xx = 1024 + xx; subtract 1152.
-        const uint32_t sub = 0x64806480u;
-        const uint32_t x0 = v.x ^ 0x80808080u, x1 = v.y ^ 0x80808080u;
-        const uint32_t y0 = v.z ^ 0x80808080u, y1 = v.w ^ 0x80808080u;
-        a_lo[0] = hsub2_u32(prmt(x0, 0x64646464u, 0x4240u), sub);
-        a_lo[1] = hsub2_u32(prmt(y0, 0x64646464u, 0x4240u), sub);
-        a_lo[2] = hsub2_u32(prmt(x0, 0x64646464u, 0x4341u), sub);
-        a_lo[3] = hsub2_u32(prmt(y0, 0x64646464u, 0x4341u), sub);
-        a_hi[0] = hsub2_u32(prmt(x1, 0x64646464u, 0x4240u), sub);
-        a_hi[1] = hsub2_u32(prmt(y1, 0x64646464u, 0x4240u), sub);
-        a_hi[2] = hsub2_u32(prmt(x1, 0x64646464u, 0x4341u), sub);
-        a_hi[3] = hsub2_u32(prmt(y1, 0x64646464u, 0x4341u), sub);
+        const uint32_t sub = k.sub_a;
+        const uint32_t x0 = v.x ^ k.or_b, x1 = v.y ^ k.or_b;
+        const uint32_t y0 = v.z ^ k.or_b, y1 = v.w ^ k.or_b;
+        a_lo[0] = hsub2_u32(prmt(x0, k.or_a, 0x4240u), sub);
+        a_lo[1] = hsub2_u32(prmt(y0, k.or_a, 0x4240u), sub);
+        a_lo[2] = hsub2_u32(prmt(x0, k.or_a, 0x4341u), sub);
+        a_lo[3] = hsub2_u32(prmt(y0, k.or_a, 0x4341u), sub);
+        a_hi[0] = hsub2_u32(prmt(x1, k.or_a, 0x4240u), sub);
+        a_hi[1] = hsub2_u32(prmt(y1, k.or_a, 0x4240u), sub);
+        a_hi[2] = hsub2_u32(prmt(x1, k.or_a, 0x4341u), sub);
+        a_hi[3] = hsub2_u32(prmt(y1, k.or_a, 0x4341u), sub);
     } else {
         const uint4 r0 = w.q[2 * b];      // row g:   {e0e1, e2e3, e16e17, e18e19} (+4t)
         const uint4 r1 = w.q[2 * b + 1];  // row g+8

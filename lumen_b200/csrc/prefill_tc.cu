@@ -24,8 +24,8 @@
 //               matrices copied by TMA (BF16 layers; LUMEN_MOE_FLAG_PREFILL_F16_WEIGHTS) they
 //               share the gate/up epilogue instead
 //   warp 24     one thread feeds the activation operand (and TMA-fed weights) with
-//               cp.async.bulk.tensor.2d boxes of 64 inputs x 128 rows
-//   warp 25     one elected thread issues tcgen05.mma / tcgen05.commit
+//               cp.async.bulk.tensor.2d boxes of 64 inputs x 32 or 128 rows
+//   warp 25     an elected lane issues tcgen05.mma / tcgen05.commit
 //   warp 26     one thread hands out the tiles: the CTA's first tile is its index, every further
 //               one is claimed from a device-wide counter while the tile before it is being
 //               multiplied, and reaches the roles through a small ring of descriptors
@@ -38,7 +38,7 @@
 // written in the same order so the down product reads it back without any shuffle.
 #include "mma_frag.cuh"
 #include "tc_common.cuh"
-#include <cstdlib>
+#include <type_traits>
 
 namespace lumen {
 
@@ -48,6 +48,8 @@ constexpr int EPI_WARPS = 8, A_WARPS = 16, B_WARPS = 1;  // B: one thread drives
 constexpr int A_WARP0 = EPI_WARPS, B_WARP0 = A_WARP0 + A_WARPS, MMA_WARP = B_WARP0 + B_WARPS;
 constexpr int SCHED_WARP = MMA_WARP + 1;  // one thread hands out the tiles
 constexpr int THREADS = (SCHED_WARP + 1) * 32;
+// rows of an activation box: 32 where tiles are narrow (no more of the operand is copied than the tile has)
+__host__ __device__ constexpr int bbox_rows(int bn) { return bn == 256 ? 128 : 32; }
 constexpr int SCHED_RING = 4;             // tile descriptors in flight between the scheduler and the roles
 
 __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
@@ -68,7 +70,7 @@ __host__ __device__ __forceinline__ int perm_pos(int e) {
 }
 
 struct Args {
-    CUtensorMap tmap;            // activation operand [rows, kdim] f16, box 64 x 128, SWIZZLE_128B (first: 64-byte aligned)
+    CUtensorMap tmap;            // activation operand [rows, kdim] f16, box 64 x 32 or 128, SWIZZLE_128B (first: 64-byte aligned)
     CUtensorMap tmap_a;          // ATMA form: the experts' plain f16 matrices as one 2-D array [E * a_rows_exp, kdim]
     int a_rows_exp;              // rows per expert there: 2 I (gate rows then up rows) or H (down)
     int a_row1;                  // second operand's rows relative to the first: I (up) or 128 (next row tile of down)
@@ -88,63 +90,77 @@ struct Args {
     TcPeerOut peer;              // down mode, expert parallel: output rows go to other ranks' buffers (ret_map null = off)
 };
 
-// Dequantise one lane's share of half a weight tile (16 rows x 64 k: blocks
-// 2*sub and 2*sub+1) into the operand tile: 4 chunks of 16 bytes (rows g, g+8).
-//
-// Lanes with odd g handle the second block of the pair first: the eight lanes of a quarter
+// Lane constants of the dequantiser: where a lane's 16-byte chunks go in the operand tile.
+// Lanes with odd g handle the second block of a pair first: the eight lanes of a quarter
 // warp then hit eight different 16-byte chunk positions (rows are 128 bytes apart, i.e. a
-// whole bank cycle) and the 128-bit stores are conflict-free. The choice is made on the raw
-// words (two selects per block for Q4_0, four for Q8_0), not on the sixteen unpacked ones.
+// whole bank cycle) and the 128-bit stores are conflict-free.
 template <int Q>
-__device__ __forceinline__ void dequant_store(const WTile<Q>& w, int sub, uint32_t a_base, int rtl, int lane) {
+struct DequantLane {
+    uint32_t off[2];   // first / second pass, row g (row g + 8 is 1024 bytes on: the same chunk of the swizzle)
+    uint32_t bsel[2];  // byte selector of the pass's block scale, in both halves
+    bool odd;
+    UnpackConst k = unpack_const_pinned<Q>();
+    __device__ __forceinline__ DequantLane(int rtl, int lane) {
+        const int g = lane >> 2, t = lane & 3;
+        odd = (g & 1) != 0;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int second = p ^ (g & 1);
+            off[p] = (uint32_t)((rtl * 16 + g) * 128 + ((((second << 2) + t) ^ g) << 4));
+            bsel[p] = second ? 0x3232u : 0x1010u;
+        }
+    }
+};
+
+// Dequantise one lane's share of half a weight tile (16 rows x 64 k: blocks 2*sub and 2*sub+1) into the
+// operand tile at a_base: 4 chunks of 16 bytes (rows g, g+8). The kernel issues this for every weight of a call, so its
+// instructions are counted: per 8 weights 1 shift, 4 logic, 4 subtract, 4 multiply, 1 select, 1 scale
+// permute, 1 store with a constant offset.
+template <int Q>
+__device__ __forceinline__ void dequant_store(const WTile<Q>& w, int sub, uint32_t a_base, const DequantLane<Q>& dl) {
     if constexpr (Q == BF16) return;  // BF16 layers feed this path from plain f16 matrices (ATMA): no producers
-    const int g = lane >> 2, t = lane & 3;
-    const bool odd = (g & 1) != 0;
-    const int r0 = rtl * 16 + g, r1 = r0 + 8;
     const uint32_t s_g = (sub == 0) ? w.s.x : w.s.y;   // f16 scales of blocks 2 sub, 2 sub + 1: row g
     const uint32_t s_g8 = (sub == 0) ? w.s.z : w.s.w;  // row g + 8
-#pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-        const bool second = (pass == 1) != odd;  // which block of the pair this lane handles in this pass
-        uint32_t lo[4], hi[4];
-        if (Q == Q4_0) {
-            const uint4 v = w.q[sub];
-            const uint32_t wg = second ? v.z : v.x;   // row g
-            const uint32_t wg8 = second ? v.w : v.y;  // row g+8
-            const uint32_t sub_lo = 0x64086408u;      // 1032 = 1024 + 8
-            const uint32_t sub_hi = 0x54805480u;      // 72   = 64 + 8
-            lo[0] = hsub2_u32(lop_and_or(wg, 0x000F000Fu, 0x64006400u), sub_lo);
-            lo[1] = hsub2_u32(lop_and_or(wg8, 0x000F000Fu, 0x64006400u), sub_lo);
-            lo[2] = hsub2_u32(lop_and_or(wg >> 8, 0x000F000Fu, 0x64006400u), sub_lo);
-            lo[3] = hsub2_u32(lop_and_or(wg8 >> 8, 0x000F000Fu, 0x64006400u), sub_lo);
-            hi[0] = hsub2_u32(lop_and_or(wg, 0x00F000F0u, 0x54005400u), sub_hi);
-            hi[1] = hsub2_u32(lop_and_or(wg8, 0x00F000F0u, 0x54005400u), sub_hi);
-            hi[2] = hsub2_u32(lop_and_or(wg >> 8, 0x00F000F0u, 0x54005400u), sub_hi);
-            hi[3] = hsub2_u32(lop_and_or(wg8 >> 8, 0x00F000F0u, 0x54005400u), sub_hi);
-        } else {
-            const uint4 va = w.q[(2 * sub) % QTraits<Q>::NQ], vb = w.q[(2 * sub + 1) % QTraits<Q>::NQ];
-            // bytes biased by 128 -> unsigned; 0x64xx = 1024 + xx; subtract 1152.
-            const uint32_t sb = 0x64806480u;
-            const uint32_t x0 = (second ? vb.x : va.x) ^ 0x80808080u, x1 = (second ? vb.y : va.y) ^ 0x80808080u;
-            const uint32_t y0 = (second ? vb.z : va.z) ^ 0x80808080u, y1 = (second ? vb.w : va.w) ^ 0x80808080u;
-            lo[0] = hsub2_u32(prmt(x0, 0x64646464u, 0x4240u), sb);
-            lo[1] = hsub2_u32(prmt(y0, 0x64646464u, 0x4240u), sb);
-            lo[2] = hsub2_u32(prmt(x0, 0x64646464u, 0x4341u), sb);
-            lo[3] = hsub2_u32(prmt(y0, 0x64646464u, 0x4341u), sb);
-            hi[0] = hsub2_u32(prmt(x1, 0x64646464u, 0x4240u), sb);
-            hi[1] = hsub2_u32(prmt(y1, 0x64646464u, 0x4240u), sb);
-            hi[2] = hsub2_u32(prmt(x1, 0x64646464u, 0x4341u), sb);
-            hi[3] = hsub2_u32(prmt(y1, 0x64646464u, 0x4341u), sb);
-        }
-        const uint32_t bsel = second ? 0x3232u : 0x1010u;  // the block's scale, in both halves
-        const uint32_t sg2 = prmt(s_g, s_g, bsel);
-        const uint32_t sg82 = prmt(s_g8, s_g8, bsel);
-        const int c = (second ? 4 : 0) + t;
-        sts128(a_base + r0 * 128 + ((c ^ (r0 & 7)) << 4), hmul2_u32(lo[0], sg2), hmul2_u32(hi[0], sg2),
-               hmul2_u32(lo[2], sg2), hmul2_u32(hi[2], sg2));
-        sts128(a_base + r1 * 128 + ((c ^ (r1 & 7)) << 4), hmul2_u32(lo[1], sg82), hmul2_u32(hi[1], sg82),
-               hmul2_u32(lo[3], sg82), hmul2_u32(hi[3], sg82));
+    uint32_t v0[2][2], v1[2][2];  // [pass][row g | g + 8]: the block's words (Q8_0: elements 0..15 | 16..31)
+    if (Q == Q4_0) {
+        const uint4 v = w.q[sub];
+        v0[0][0] = dl.odd ? v.z : v.x;
+        v0[1][0] = dl.odd ? v.x : v.z;
+        v0[0][1] = dl.odd ? v.w : v.y;
+        v0[1][1] = dl.odd ? v.y : v.w;
+    } else {
+        const uint4 va = w.q[(2 * sub) % QTraits<Q>::NQ], vb = w.q[(2 * sub + 1) % QTraits<Q>::NQ];
+        v0[0][0] = dl.odd ? vb.x : va.x;
+        v0[1][0] = dl.odd ? va.x : vb.x;
+        v1[0][0] = dl.odd ? vb.y : va.y;
+        v1[1][0] = dl.odd ? va.y : vb.y;
+        v0[0][1] = dl.odd ? vb.z : va.z;
+        v0[1][1] = dl.odd ? va.z : vb.z;
+        v1[0][1] = dl.odd ? vb.w : va.w;
+        v1[1][1] = dl.odd ? va.w : vb.w;
     }
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint32_t sc = prmt(r ? s_g8 : s_g, 0u, dl.bsel[p]);
+            uint32_t l0, l1, h0, h1;
+            if (Q == Q4_0) {
+                const uint32_t x = v0[p][r], y = x >> 8;
+                l0 = hsub2_u32(lop_and_or(x, 0x000F000Fu, dl.k.or_a), dl.k.sub_a);
+                h0 = hsub2_u32(lop_and_or(x, 0x00F000F0u, dl.k.or_b), dl.k.sub_b);
+                l1 = hsub2_u32(lop_and_or(y, 0x000F000Fu, dl.k.or_a), dl.k.sub_a);
+                h1 = hsub2_u32(lop_and_or(y, 0x00F000F0u, dl.k.or_b), dl.k.sub_b);
+            } else {
+                // bytes biased by 128 -> unsigned; 0x64xx = 1024 + xx; subtract 1152.
+                const uint32_t x = v0[p][r] ^ dl.k.or_b, y = v1[p][r] ^ dl.k.or_b;
+                l0 = hsub2_u32(prmt(x, dl.k.or_a, 0x4240u), dl.k.sub_a);
+                l1 = hsub2_u32(prmt(x, dl.k.or_a, 0x4341u), dl.k.sub_a);
+                h0 = hsub2_u32(prmt(y, dl.k.or_a, 0x4240u), dl.k.sub_a);
+                h1 = hsub2_u32(prmt(y, dl.k.or_a, 0x4341u), dl.k.sub_a);
+            }
+            sts128(a_base + dl.off[p] + r * 1024, hmul2_u32(l0, sc), hmul2_u32(h0, sc), hmul2_u32(l1, sc), hmul2_u32(h1, sc));
+        }
 }
 
 // ATMA: the weight operands are not dequantised here but copied by TMA from plain f16 matrices
@@ -161,7 +177,22 @@ __device__ __forceinline__ void dequant_store(const WTile<Q>& w, int sub, uint32
 // the output rows leave as 256-byte bulk copies (see the epilogue).
 template <int Q, int BN, bool ATMA, bool STG = false>
 struct StagesOf {
-    static constexpr int value = ((BN == 128) ? 4 : 3) - (STG ? 1 : 0);
+    static constexpr bool ring = (BN == 128) && !ATMA && !STG;
+    static constexpr int value = ((BN == 128) ? 4 : 3) - ((STG || ring) ? 1 : 0);
+};
+// Raw weight ring (128-column tiles, dequantised weights). A tile of few columns has little work
+// for the tensor cores, and the register prefetch keeps only one 128-input group (18 KB per SM for
+// Q4_0) on the way. Each producer warp therefore owns a ring of RING of its 16-row tiles in
+// shared memory, filled by bulk copies (quants and scales of a group are contiguous) that run
+// ahead of the dequantisation, across tile boundaries; an operand stage pays for it.
+// The 256-column form keeps the register prefetch: its MMAs take longer than the latency.
+template <int Q, int BN, bool ATMA, bool STG = false>
+struct RingOf {
+    static constexpr int value = !StagesOf<Q, BN, ATMA, STG>::ring ? 0 : (Q == Q4_0) ? 4 : 2;
+};
+template <int Q>
+struct RawTile {  // bytes of one 16-row x 128-input tile: quants, then scales
+    static constexpr int q_bytes = QTraits<Q>::NQ * 512, bytes = q_bytes + 128;
 };
 constexpr int STG_ROW_BYTES = 256 + 16;                 // 128 f16 outputs of one token + padding (bank spread)
 constexpr int STG_BYTES = 2 * 128 * STG_ROW_BYTES;      // two warp groups x 128 tokens
@@ -214,9 +245,12 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
     constexpr int STAGES = StagesOf<Q, BN, ATMA, STG>::value;  // one stage = 64 inputs (one swizzle atom in K)
     constexpr int STAGE_BYTES = NA * SUB_BYTES + BN * 128;  // A operands then B
     constexpr int TMEM_COLS = 512;
+    constexpr int RING = RingOf<Q, BN, ATMA, STG>::value;
+    constexpr int BBOX = bbox_rows(BN);
 
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full_bar[NACC], acc_empty_bar[NACC];
+    __shared__ uint64_t ring_bar[RING ? A_WARPS * RING : 1];
     __shared__ uint32_t tmem_base_s;
     __shared__ uint32_t abort_s;
     // Tiles are handed out dynamically: the CTA's first tile is blockIdx.x, every further one the next
@@ -225,7 +259,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
     // this ring. (With tiles dealt round-robin the slowest CTA of a Zipf-loaded 4096-token call ran
     // 11 % longer than the median one in gate/up and 13 % in down.)
     __shared__ int4 sched_tile_s[SCHED_RING];
-    __shared__ uint64_t sched_full_bar[SCHED_RING], sched_empty_bar[SCHED_RING], sched_go_bar;
+    __shared__ uint64_t sched_full_bar[SCHED_RING], sched_empty_bar[SCHED_RING], sched_go_bar[2];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -234,21 +268,23 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
     if (tid == 0) {
         abort_s = 0u;
         for (int s = 0; s < STAGES; ++s) {
-            mbar_init(smem_u32(&full_bar[s]), ATMA ? 1 : A_WARPS * 32 + 1);  // weight producers + the TMA thread's expect_tx arrive
+            mbar_init(smem_u32(&full_bar[s]), ATMA ? 1 : A_WARPS + 1);  // one arrival per weight-producer warp + the TMA thread's expect_tx
             mbar_init(smem_u32(&empty_bar[s]), 1);
         }
         for (int b = 0; b < NACC; ++b) {
             mbar_init(smem_u32(&acc_full_bar[b]), 1);
-            mbar_init(smem_u32(&acc_empty_bar[b]), (HELP ? EPI_WARPS + A_WARPS : EPI_WARPS) * 32);
+            mbar_init(smem_u32(&acc_empty_bar[b]), HELP ? EPI_WARPS + A_WARPS : EPI_WARPS);
         }
+        for (int i = 0; i < A_WARPS * RING; ++i) mbar_init(smem_u32(&ring_bar[i]), 1);
         // readers of a descriptor: epilogue warps, the producer warps when they dequantise or share the
         // epilogue, the TMA thread and the MMA thread
-        constexpr int SCHED_READERS = EPI_WARPS * 32 + ((!ATMA || HELP) ? A_WARPS * 32 : 0) + 2;
+        constexpr int SCHED_READERS = EPI_WARPS + ((!ATMA || HELP) ? A_WARPS : 0) + 2;
         for (int s = 0; s < SCHED_RING; ++s) {
             mbar_init(smem_u32(&sched_full_bar[s]), 1);
             mbar_init(smem_u32(&sched_empty_bar[s]), SCHED_READERS);
         }
-        mbar_init(smem_u32(&sched_go_bar), 1);
+        mbar_init(smem_u32(&sched_go_bar[0]), 1);
+        mbar_init(smem_u32(&sched_go_bar[1]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == MMA_WARP) {
@@ -270,22 +306,32 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
     const int khs = kgs * 2;       // 64-input pipeline stages per tile
     // every operand is f16 here: BF16 weights are converted exactly (see dequant_store)
     const bool bf16_mode = false;
-    // The n-th tile of this CTA (n counted by the calling thread): false when the list is exhausted
-    // or the kernel gives up. The descriptor is copied and its ring slot released at once.
-    auto next_tile = [&](int& n, int4& tile) -> bool {
+    // The n-th tile of this CTA (n counted by the caller): false when the list is exhausted or the
+    // kernel gives up. The descriptor is copied and its ring slot released at once. WARP: the whole
+    // warp takes it together (one arrival for all lanes), else one thread does.
+    auto take_tile = [&](auto warp_tag, int& n, int4& tile) -> bool {
+        constexpr bool WARP = decltype(warp_tag)::value;
         const int slot = n % SCHED_RING;
-        if (!mbar_wait(smem_u32(&sched_full_bar[slot]), (n / SCHED_RING) & 1, abort_flag)) return false;
+        bool ok = mbar_wait(smem_u32(&sched_full_bar[slot]), (n / SCHED_RING) & 1, abort_flag);
+        if constexpr (WARP) ok = __all_sync(0xffffffffu, ok);
+        if (!ok) return false;
         tile = sched_tile_s[slot];
-        mbar_arrive(smem_u32(&sched_empty_bar[slot]));
+        if constexpr (WARP) __syncwarp();
+        if (!WARP || lane == 0) mbar_arrive(smem_u32(&sched_empty_bar[slot]));
         ++n;
         return tile.z >= 0;
     };
-    // stage of a tile at which the MMA thread lets the scheduler claim the CTA's next tile: late, so
-    // that the last tiles of the list go to the CTAs that are free first, but early enough for the
-    // claim (an atomic and a load, ~2 us) to be back when the producers reach the tile's last group
-    // (the producers take the next descriptor before they fill the last two stages of a tile, so the
-    // signal has to come before the MMA thread needs those: go_kh <= khs - 2)
-    const int go_kh = (khs >= 24) ? khs / 2 - 4 : (khs >= 4 ? 1 : 0);
+    auto next_tile = [&](int& n, int4& tile) -> bool { return take_tile(std::false_type{}, n, tile); };
+    auto next_tile_warp = [&](int& n, int4& tile) -> bool { return take_tile(std::true_type{}, n, tile); };
+    // When the CTA's next tile is claimed: while the MMA warp is in the tile `ahead` before it, at stage go_kh.
+    // Long tiles: late in the tile before, so that the last tiles of the list go to the CTAs that are
+    // free first, but early enough for the claim (an atomic and a load, ~2 us) to be back when the producers reach
+    // the tile's last group. (They take the next descriptor before they fill the last two stages of a
+    // tile, so the signal has to come before the MMA warp needs those: go_kh <= khs - 2.)
+    // Short tiles (the down product, K = I): a tile is over in about the time of a claim, and the producers' ring would
+    // run dry at every tile end; they are claimed two tiles ahead (256 experts, I = 512: 322 -> 250 us per call).
+    const int ahead = (khs >= 24) ? 1 : 2;
+    const int go_kh = (khs >= 24) ? khs / 2 - 4 : 0;
 
     // Epilogue of one tile by one warp: the warp's TMEM lanes are 32 (warp % 4).. (hardware rule);
     // of the tile's 16-column TMEM chunks it takes those with chunk % nparts == part.
@@ -430,7 +476,9 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
             tc_fence_after();
             epilogue_part(tile, per_pass == 2 ? 0 : v % NACC, h, part, EPI_PARTS);
             tc_fence_before();
-            for (int j = 0; j < per_pass; ++j) mbar_arrive(smem_u32(&acc_empty_bar[(v + j) % NACC]));
+            __syncwarp();
+            if (lane == 0)
+                for (int j = 0; j < per_pass; ++j) mbar_arrive(smem_u32(&acc_empty_bar[(v + j) % NACC]));
             v += per_pass;
         }
         return true;
@@ -442,7 +490,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
         bool ok = true;
         int tn = 0;
         int4 tile;
-        while (ok && next_tile(tn, tile)) ok = epilogue_tile(tile, v, warp >> 2);
+        while (ok && next_tile_warp(tn, tile)) ok = epilogue_tile(tile, v, warp >> 2);
         if constexpr (STG) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // every row has been written
     } else if (warp < B_WARP0) {
         // --------------------------- weight producers --------------------------
@@ -468,49 +516,117 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                 sb = a.L.down_s(e);
                 tidx = (tile.w * 16 + pw) * kgs + kg;
             }
-            qp = qb + ((size_t)tidx * QTraits<Q>::NQ) * 32 + lane;
+            qp = qb + ((size_t)tidx * QTraits<Q>::NQ) * 32;
             sp = sb + (size_t)tidx * 8;
         };
         auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool { return mbar_wait(bar, parity, abort_flag); };
         auto warp_arrive = [&](uint32_t bar) {
-            fence_proxy_async();
-            mbar_arrive(bar);
+            fence_proxy_async();  // every lane's own stores, before the warp's one arrival
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar);
         };
-        if constexpr (!ATMA) {
+        const DequantLane<Q> dl(rtl, lane);
+        int s = 0, ph = 0;  // operand stage and its parity
+        // one half tile into the next stage
+        auto produce = [&](const WTile<Q>& w, int sub) -> bool {
+            const bool r = __all_sync(0xffffffffu, warp_wait(smem_u32(&empty_bar[s]), ph ^ 1));
+            if (r) {
+                dequant_store<Q>(w, sub, stage0 + s * STAGE_BYTES + op * SUB_BYTES, dl);
+                warp_arrive(smem_u32(&full_bar[s]));
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+            return r;
+        };
+        if constexpr (RING > 0) {
+            // Groups flow through this warp's ring in the order of the tile list: `issued` counts the
+            // groups requested, `taken` those copied to registers; a slot is refilled as soon as its
+            // words are in registers. The descriptor of the CTA's next tile is taken only when it is
+            // there already (or when nothing is left to do): waiting for it with groups of the current
+            // tile undone would wait for the MMA warp, which waits for those groups.
+            constexpr uint32_t RAW = RawTile<Q>::bytes, RAW_Q = RawTile<Q>::q_bytes;
+            const uint32_t ring0 = stage0 + STAGES * STAGE_BYTES + (uint32_t)pw * RING * RAW;
+            const uint32_t bar0 = smem_u32(&ring_bar[pw * RING]);
+            int4 tile = make_int4(0, 0, -1, 0);
+            int issued = 0, taken = 0, pkg = kgs;
+            bool more = true;  // the list may hold further tiles
+            const uint4 *qp = nullptr, *sp = nullptr;
+            auto top_up = [&]() {
+                while (issued - taken < RING) {
+                    if (pkg == kgs) {
+                        if (!more) return;
+                        if (issued != taken) {
+                            const int slot = tn % SCHED_RING;
+                            const bool there = mbar_try(smem_u32(&sched_full_bar[slot]), (tn / SCHED_RING) & 1);
+                            if (!__all_sync(0xffffffffu, there)) return;
+                        }
+                        more = next_tile_warp(tn, tile);
+                        if (!more) return;
+                        pkg = 0;
+                        tile_ptrs(tile, 0, qp, sp);
+                    }
+                    if (elect_one()) {
+                        const int slot = issued % RING;
+                        const uint32_t bar = bar0 + slot * 8, dst = ring0 + slot * RAW;
+                        mbar_expect_tx(bar, RAW);
+                        bulk_load(dst, qp, RAW_Q, bar);
+                        bulk_load(dst + RAW_Q, sp, RAW - RAW_Q, bar);
+                    }
+                    __syncwarp();
+                    qp += RAW_Q / 16;
+                    sp += 8;
+                    ++issued;
+                    ++pkg;
+                }
+            };
+            top_up();
+            while (ok && issued != taken) {
+                const int slot = taken % RING;
+                ok = __all_sync(0xffffffffu, warp_wait(bar0 + slot * 8, (taken / RING) & 1));
+                if (!ok) break;
+                WTile<Q> cur;
+                const uint32_t src = ring0 + slot * RAW;
+#pragma unroll
+                for (int j = 0; j < QTraits<Q>::NQ; ++j) cur.q[j] = lds128(src + j * 512 + lane * 16);
+                cur.s = lds128(src + RAW_Q + (lane >> 2) * 16);
+                ++taken;
+                // (the slot is refilled behind the first half's proxy fence and warp barrier: every lane's reads of
+                // it are then ordered before the bulk copy's writes)
+                ok = produce(cur, 0);
+                if (!ok) break;
+                top_up();
+                ok = produce(cur, 1);
+            }
+            // give-up: the copies still in flight land before the shared memory goes away
+            for (; taken != issued; ++taken)
+                for (int i = 0; i < (1 << 16) && !mbar_try(bar0 + (taken % RING) * 8, (taken / RING) & 1); ++i) {}
+        } else if constexpr (!ATMA) {
             WTile<Q> cur, nxt;
             auto issue = [&](const int4& tile, int kg, WTile<Q>& dst) {
                 const uint4 *qp, *sp;
                 tile_ptrs(tile, kg, qp, sp);
     #pragma unroll
-                for (int j = 0; j < QTraits<Q>::NQ; ++j) dst.q[j] = ldg_stream(qp + j * 32);
+                for (int j = 0; j < QTraits<Q>::NQ; ++j) dst.q[j] = ldg_stream(qp + j * 32 + lane);
                 if (Q != BF16) dst.s = ldg_stream(sp + (lane >> 2));
             };
             // The next tile's descriptor is taken before the last group of the current tile, so that
             // the first group of the next tile is in flight while the last one is dequantised.
             int4 tile_c, tile_n = make_int4(0, 0, -1, 0);
-            bool have_c = next_tile(tn, tile_c), have_n = false;
+            bool have_c = next_tile_warp(tn, tile_c), have_n = false;
             if (have_c) issue(tile_c, 0, cur);
-            int it = 0, kg = 0;
-            long long tr_w = 0;
-            const long long tr_t0 = clock64();
+            int kg = 0;
             while (ok && have_c) {
                 bool more = true;  // a group follows this one
                 if (kg + 1 < kgs) {
                     issue(tile_c, kg + 1, nxt);
                 } else {
-                    have_n = next_tile(tn, tile_n);
+                    have_n = next_tile_warp(tn, tile_n);
                     if (have_n) issue(tile_n, 0, nxt);
                     more = have_n;
                 }
-    #pragma unroll
-                for (int sub = 0; sub < 2; ++sub, ++it) {
-                    const int s = it % STAGES, ph = (it / STAGES) & 1;
-                    ok = ok && TRACE_WAIT(tr_w, warp_wait(smem_u32(&empty_bar[s]), ph ^ 1));
-                    if (ok) {
-                        dequant_store<Q>(cur, sub, stage0 + s * STAGE_BYTES + op * SUB_BYTES, rtl, lane);
-                        warp_arrive(smem_u32(&full_bar[s]));
-                    }
-                }
+                ok = produce(cur, 0) && produce(cur, 1);
                 if (more) cur = nxt;
                 if (++kg == kgs) {
                     kg = 0;
@@ -519,23 +635,18 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                     have_n = false;
                 }
             }
-            if (pw == 0 && lane == 0) {
-                TRACE_PUT(0, tr_w);
-                TRACE_PUT(1, clock64() - tr_t0);
-            }
-            (void)tr_w;
-            (void)tr_t0;
         }
         if constexpr (HELP) {
             // TMA-fed weights, one accumulator set: nothing to dequantise, the warp takes a share of
             // every tile's epilogue instead
             int4 tile;
             int v = 0;
-            while (ok && next_tile(tn, tile)) ok = epilogue_tile(tile, v, EPI_WARPS / 4 + (pw >> 2));
+            while (ok && next_tile_warp(tn, tile)) ok = epilogue_tile(tile, v, EPI_WARPS / 4 + (pw >> 2));
         }
         (void)warp_wait;
         (void)warp_arrive;
         (void)tile_ptrs;
+        (void)produce;
     } else if (warp < MMA_WARP) {
         // ------------------------- activation producers ------------------------
         // One thread feeds the activation operand with TMA: per 64-input stage one or two
@@ -554,7 +665,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                     int4 tile;
                     if (!next_tile(tn, tile)) break;
                     row0 = tile.y;
-                    nbox = (BN > 128 && tile.z > 128) ? 2 : 1;
+                    nbox = (tile.z + BBOX - 1) / BBOX;
                     arow0 = tile.x * a.a_rows_exp + tile.w * (MODE == 0 ? 128 : 256);
                 }
                 const int s = n % STAGES, ph = (n / STAGES) & 1;
@@ -564,7 +675,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                 const uint32_t bbase = stage0 + s * STAGE_BYTES + NA * SUB_BYTES;
                 // (test hook: with debug_extra_tx the very first stage can never complete)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                             "r"((nbox + (ATMA ? NA : 0)) * SUB_BYTES + (n == 0 ? a.debug_extra_tx : 0))
+                             "r"(nbox * BBOX * 128 + (ATMA ? NA : 0) * SUB_BYTES + (n == 0 ? a.debug_extra_tx : 0))
                              : "memory");
                 if (ATMA) {
 #pragma unroll
@@ -578,23 +689,23 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                 for (int q = 0; q < nbox; ++q)
                     asm volatile(
                         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                        "[%0], [%1, {%2, %3}], [%4];" ::"r"(bbase + q * SUB_BYTES),
-                        "l"(tmap_addr), "r"(kh * 64), "r"(row0 + q * 128), "r"(bar)
+                        "[%0], [%1, {%2, %3}], [%4];" ::"r"(bbase + q * BBOX * 128),
+                        "l"(tmap_addr), "r"(kh * 64), "r"(row0 + q * BBOX), "r"(bar)
                         : "memory");
             }
         }
         __syncwarp();
     } else if (warp == MMA_WARP) {
         // -------------------------------- MMA ---------------------------------
-        if (lane == 0) {
-            int it = 0, tl = 0;
+        {
+            int tl = 0, s = 0, ph = 0;  // operand stage and its parity
             bool ok = true;
             long long tr_wf = 0, tr_wa = 0;
             const long long tr_t0 = clock64();
             int v = 0;  // accumulator sets taken so far (see the epilogue)
             int tn = 0;
             int4 tile;
-            for (; ok && next_tile(tn, tile); ++tl) {
+            for (; ok && next_tile_warp(tn, tile); ++tl) {
                 const int n16 = (tile.z + 15) & ~15;
                 // down: D[128 tokens, 256 output rows] = X[128, k] W[256, k]^T, the two adjacent 128-row
                 // weight operands of a stage forming one 256-row N operand; a tile of more than 128
@@ -605,43 +716,49 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                     const int ab = (v + h) % NACC, use = (v + h) / NACC;
                     ok = TRACE_WAIT(tr_wa, mbar_wait(smem_u32(&acc_empty_bar[ab]), (use & 1) ^ 1, abort_flag));
                 }
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acc0 = tmem_base + (v % NACC) * ACC_COLS, acc1 = tmem_base + ((v + 1) % NACC) * ACC_COLS;
-                for (int kh = 0; kh < khs; ++kh, ++it) {
-                    const int s = it % STAGES, ph = (it / STAGES) & 1;
-                    if (kh == go_kh) mbar_arrive(smem_u32(&sched_go_bar));  // the CTA's next tile may be claimed now
-                    ok = TRACE_WAIT(tr_wf, mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag));
+                for (int kh = 0; kh < khs; ++kh) {
+                    if (kh == go_kh && lane == 0) mbar_arrive(smem_u32(&sched_go_bar[tl % ahead]));  // the CTA's next tile may be claimed now
+                    ok = __all_sync(0xffffffffu, TRACE_WAIT(tr_wf, mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag)));
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t sbase = stage0 + s * STAGE_BYTES;
-                    const uint32_t bbase = sbase + NA * SUB_BYTES;
+                    if (elect_one()) {
+                        const uint64_t w0 = make_desc(stage0 + s * STAGE_BYTES), b0 = w0 + (NA * SUB_BYTES >> 4);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint64_t bdesc = make_desc(bbase + j * 32);
-                        const uint32_t acc = (kh > 0 || j > 0) ? 1u : 0u;
-                        if (MODE == 1) {
-                            const uint64_t wdesc = make_desc(sbase + j * 32);
-                            umma(acc0, bdesc, wdesc, idesc, acc);
-                            if (nh == 2) umma(acc1, make_desc(bbase + SUB_BYTES + j * 32), wdesc, idesc, acc);
-                        } else {
+                        for (int j = 0; j < 4; ++j) {
+                            const uint32_t acc = (kh > 0 || j > 0) ? 1u : 0u;
+                            if (MODE == 1) {
+                                umma(acc0, b0 + j * 2, w0 + j * 2, idesc, acc);
+                                if (nh == 2) umma(acc1, b0 + (SUB_BYTES >> 4) + j * 2, w0 + j * 2, idesc, acc);
+                            } else {
 #pragma unroll
-                            for (int op = 0; op < NA; ++op) {
-                                const uint64_t adesc = make_desc(sbase + op * SUB_BYTES + j * 32);
-                                umma((nh == 2 ? tmem_base : acc0) + op * BN, adesc, bdesc, idesc, acc);
+                                for (int op = 0; op < NA; ++op)
+                                    umma((nh == 2 ? tmem_base : acc0) + op * BN, w0 + op * (SUB_BYTES >> 4) + j * 2, b0 + j * 2,
+                                         idesc, acc);
                             }
                         }
+                        umma_commit(smem_u32(&empty_bar[s]));
+                        if (kh == khs - 1)
+                            for (int h = 0; h < nh; ++h) umma_commit(smem_u32(&acc_full_bar[(v + h) % NACC]));
                     }
-                    umma_commit(smem_u32(&empty_bar[s]));
+                    __syncwarp();
+                    if (++s == STAGES) {
+                        s = 0;
+                        ph ^= 1;
+                    }
                 }
                 if (!ok) break;
-                for (int h = 0; h < nh; ++h) umma_commit(smem_u32(&acc_full_bar[(v + h) % NACC]));
                 v += nh;
             }
-            TRACE_PUT(2, tr_wf);
-            TRACE_PUT(3, tr_wa);
-            TRACE_PUT(4, clock64() - tr_t0);
-            TRACE_PUT(5, tl);
+            if (lane == 0) {
+                TRACE_PUT(2, tr_wf);
+                TRACE_PUT(3, tr_wa);
+                TRACE_PUT(4, clock64() - tr_t0);
+                TRACE_PUT(5, tl);
+            }
             (void)tr_wf;
             (void)tr_wa;
             (void)tr_t0;
@@ -652,11 +769,14 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
         if (lane == 0) {
             for (int n = 0;; ++n) {
                 const int slot = n % SCHED_RING;
-                // tile n >= 1 is claimed once the MMA thread is far enough into tile n - 1 (the thread
-                // cannot get two tiles ahead of this wait: tile n is not handed out before it)
-                if (n > 0 && !mbar_wait(smem_u32(&sched_go_bar), (n - 1) & 1, abort_flag)) break;
+                // tile n is claimed once the MMA warp is far enough into tile n - ahead (one barrier per parity
+                // of that tile when ahead = 2: the warp cannot come round to the same barrier before this wait is over,
+                // because tile n is not handed out before it)
+                const int m = n - ahead;
+                if (m >= 0 && !mbar_wait(smem_u32(&sched_go_bar[m % ahead]), (m / ahead) & 1, abort_flag)) break;
                 if (!mbar_wait(smem_u32(&sched_empty_bar[slot]), ((n / SCHED_RING) & 1) ^ 1, abort_flag)) break;
-                const int t = (n == 0) ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(a.n_tiles + 2 + MODE, 1);
+                // the first `ahead` tiles are the CTA's by its index
+                const int t = (n < ahead) ? (int)blockIdx.x + n * (int)gridDim.x : ahead * (int)gridDim.x + atomicAdd(a.n_tiles + 2 + MODE, 1);
                 sched_tile_s[slot] = (t < ntiles) ? a.tiles[t] : make_int4(0, 0, -1, 0);  // columns < 0: no more tiles
                 mbar_arrive(smem_u32(&sched_full_bar[slot]));
                 if (t >= ntiles) break;
@@ -779,7 +899,8 @@ template <int Q, int MODE, int BN, bool ATMA = false, bool STG = false>
 static cudaError_t launch_tc_one(const tc::Args& a, int grid, cudaStream_t st) {
     constexpr int NA = 2;
     constexpr int STAGES = tc::StagesOf<Q, BN, ATMA, STG>::value;
-    const int smem = STAGES * (NA * tc::SUB_BYTES + BN * 128) + 1024 + (STG ? tc::STG_BYTES : 0);
+    const int smem = STAGES * (NA * tc::SUB_BYTES + BN * 128) + 1024 + (STG ? tc::STG_BYTES : 0) +
+                     tc::A_WARPS * tc::RingOf<Q, BN, ATMA, STG>::value * tc::RawTile<Q>::bytes;
     static SmemOptIn optin;
     {
         cudaError_t e = ensure_dyn_smem(tc::grouped_gemm_tc_kernel<Q, MODE, BN, ATMA, STG>, (size_t)smem, optin);
@@ -804,7 +925,7 @@ cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, c
     const bool stg = (peer != nullptr) && !dn256;
     const int mt_gu = p.L.I / 128;
     tc::Args gu{};
-    cudaError_t te = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, 128, &gu.tmap);
+    cudaError_t te = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, tc::bbox_rows(gu_cols), &gu.tmap);
     if (te != cudaSuccess) return te;
     gu.L = p.L;
     gu.col_src_tok = p.R.col_src_tok;
@@ -819,7 +940,7 @@ cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, c
     gu.kdim = p.L.H;
     gu.out_ld = p.L.I;
     tc::Args dn = gu;
-    te = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, 128, &dn.tmap);
+    te = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, tc::bbox_rows(dn256 ? 256 : 128), &dn.tmap);
     if (te != cudaSuccess) return te;
     dn.col_src_tok = nullptr;
     dn.debug_extra_tx = 0;  // the hook applies to the first kernel of the pair
