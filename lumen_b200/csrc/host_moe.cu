@@ -466,6 +466,13 @@ Status encode_route_only(CudaMoeScratch* s, const MoeLayer* layer, const float* 
     return Status::Ok();
 }
 
+// Which prompts take the streaming kernels: those whose experts have so few columns on average that
+// the call is bound by reading the weights, not by multiplying. (BF16 layers have their f16 matrices copied by
+// TMA on the tcgen05 path, which then is bound by HBM as well: 240 against 224 us at 64 tokens.)
+static bool prefill_streams(int columns, int E, int H, int I, int quant, const void* normed) {
+    return quant != BF16 && H % 128 == 0 && I % 128 == 0 && H >= 256 && columns <= STREAM_MAX_COLS * E && reinterpret_cast<uintptr_t>(normed) % 16 == 0;
+}
+
 // cuda/moe.rs:1900-2760
 Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, const void* normed, int act_dtype,
                                       const float* residual, float* output, int batch, cudaStream_t st,
@@ -515,9 +522,23 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
     const bool tc_ok = (s->H % 256 == 0) && (s->I % 128 == 0) && (reinterpret_cast<uintptr_t>(normed) % 16 == 0) &&
                        (reinterpret_cast<uintptr_t>(out16_rows) % 32 == 0);
     p.impl = (s->prefill_impl == 1 || !tc_ok) ? 1 : 0;
+    if (s->prefill_impl == 0 && prefill_streams(batch * s->K, s->E, s->H, s->I, layer.dev.quant, normed)) {
+        p.impl = 2;
+        p.stream_starts = reinterpret_cast<int32_t*>(s->R.work);  // (decode's work records: 8 KB, unused by a prefill)
+    }
+    const bool own_router = ids_in == nullptr && s->logits_override == nullptr;
     CUDA_TRY(launch_route_large(p, st));
     const bool bf16_mode = (layer.dev.quant == BF16);
-    if (p.impl == 0) {
+    if (p.impl == 2) {
+        // the router has left the activations' f16 planes; with routing from elsewhere they are made here
+        if (!own_router) CUDA_TRY(launch_split_x16(normed, act_dtype, batch, s->H, s->xr16, nullptr, st));
+        if (s->expire_next[1]) {
+            p.debug_extra_tx = 1;
+            s->expire_next[1] = 0;
+        }
+        CUDA_TRY(launch_stream_prefill(p, s->xr16, out16_rows, st));
+        if (out16_rows) return Status::Ok();
+    } else if (p.impl == 0) {
         CUDA_TRY(launch_gather_permute_x16(normed, act_dtype, s->R.col_src_tok, batch * s->K, s->H, s->x16, st,
                                            layer.dev.gu16 != nullptr));
         // persistent grid, one CTA per SM; LUMEN_MOE_FLAG_TC_CTAS leaves some SMs to kernels that run beside it

@@ -179,6 +179,7 @@ struct PrefillArgs {
     __half* w16;            // [2, E, H] router weight split into f16 high and low planes (per call, when the layer has none)
     __half* xr16;           // [2, T, H] activations split into f16 high and low planes (tcgen05 router)
     float* rpart;           // [ksplit, T, E] partial logits of the tcgen05 router
+    int32_t* stream_starts; // [2][sms + 1] first item of every CTA of the streaming gate/up and down kernels
     int32_t* any_lo;        // [1] some low part of the activations is non-zero
     int sms;                // multiprocessors of the device
     __half* s16;            // [C, I] f16 SwiGLU output, row-major by compact column
@@ -191,13 +192,15 @@ struct PrefillArgs {
     unsigned wait_limit_us; // limit of the device-side waits (0 = two seconds)
     int debug_extra_tx;     // test hook: the first stage barrier expects this many bytes more than arrive
     int tc_ctas;            // cap of the persistent tcgen05 grid (0 = every SM)
-    int impl;               // 0 = tcgen05 path, 1 = mma.sync grouped fallback
+    int impl;               // 0 = tcgen05 path, 1 = mma.sync grouped fallback, 2 = streaming kernels (few columns per expert)
     const uint32_t* ids_in;  // caller-supplied routing [T,K] (null = route here)
     const float* weights_in; // [T,K] or null (= 1)
 };
 cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st);
 // tcgen05 router (route_tc.cu)
 cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, cudaStream_t st);
+// f16 planes of the activations in the weight planes' element order (see route_tc.cu); any_lo null = high plane only
+cudaError_t launch_split_x16(const void* x, int act_dtype, int T, int H, __half* x16, int32_t* any_lo, cudaStream_t st);
 int router_tc_ksplit(int T, int E, int H, int sms);
 bool router_tc_applicable(int T, int E, int H, const void* x);
 cudaError_t launch_router_logits_tc(const void* x, int act_dtype, const __half* w16, int T, int E, int H, int ksplit,
@@ -220,10 +223,17 @@ struct TcPlan {
     int gu_cols;   // columns per gate/up tile the tile lists were built with (128 or 256)
 };
 // tile lists {expert, col_start, ncols, m_tile} of both grouped GEMMs from per-expert column counts
-// left in R.expert_bounds[0..E) (turned into bounds in place), plus R.uexp / R.n_uexp
+// left in R.expert_bounds[0..E) (turned into bounds in place), plus R.uexp / R.n_uexp. stream_mode (null = off): device
+// word that says whether the call's work goes to the streaming kernels (chunks, starts) instead
 cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_cap, int gu_cols, int4* tiles,
-                             int32_t* n_tiles, cudaStream_t st);
-cudaError_t launch_prefill(const PrefillArgs& a, cudaStream_t st);
+                             int32_t* n_tiles, cudaStream_t st, const int32_t* stream_mode, int4* chunks, int32_t* starts,
+                             int sms);
+// expert products of short prompts (stream.cu)
+cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __half* out16_rows, cudaStream_t st,
+                                  const TcPeerOut* peer = nullptr);
+constexpr int STREAM_MAX_COLS = 12;
+constexpr int STREAM_SHIFT = 5;
+constexpr int STREAM_CHUNK = 1 << STREAM_SHIFT;  // columns of an expert that one item of the streaming kernels multiplies
 
 void count_launch(int n = 1);
 

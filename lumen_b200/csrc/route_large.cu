@@ -256,33 +256,54 @@ router_logits_mma_kernel(const XT* __restrict__ x, const __half* __restrict__ w1
     }
 }
 
-// nparts > 0: the logits arrive as `nparts` partial sums [nparts][T][E] (k ranges of the tcgen05
-// router); they are added in a fixed order and the sum is left in logits_out.
-constexpr int TK_WARPS = 8;
+// Gating + top-k of a batch, one warp per token. NP > 0: the logits arrive as NP partial sums
+// [NP][T][E] (k ranges of the tcgen05 router); they are added in a fixed order and the sum is left in
+// logits_out. NP = 0: plain logits. NS * 32 >= E.
+// A warp's chain of dependent steps is what this kernel costs (4096 tokens are 28 warps per SM), so
+// all NS * NP logits of a lane are requested at once (one after the other they were 16 L2 round trips, two
+// thirds of 22 us), and the exps of a lane are inline and independent of one another, their table
+// in shared memory.
 // blk_hist (null = none): the per-expert pair counts of this block's TK_WARPS tokens, the first
 // step of the counting sort (one histogram per chunk of SORT_TOK = TK_WARPS tokens), written here
 // instead of by a launch of its own.
+constexpr int TK_WARPS = 8;
+template <int NS, int NP>
 __global__ void __launch_bounds__(TK_WARPS * 32)
-topk_large_kernel(const float* __restrict__ logits, int nparts, float* __restrict__ logits_out, int T, int E, int K,
+topk_large_kernel(const float* __restrict__ logits, float* __restrict__ logits_out, int T, int E, int K,
                   int gating, uint32_t* __restrict__ ids, float* __restrict__ weights, int32_t* __restrict__ blk_hist) {
-    grid_dep_sync();
-    __shared__ __align__(16) float p_s[TK_WARPS][MAX_EXPERTS];
-    __shared__ __align__(16) float lg_s[TK_WARPS][MAX_EXPERTS];
-    __shared__ int h[MAX_EXPERTS];
+    __shared__ __align__(16) float p_s[TK_WARPS][NS * 32];
+    __shared__ unsigned long long tab_s[32];
+    __shared__ int h[NS * 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * TK_WARPS + warp;
-    for (int e = threadIdx.x; e < E; e += TK_WARPS * 32) h[e] = 0;
+    if (threadIdx.x < 32) tab_s[threadIdx.x] = lumen_exact::exp2_tab_entry(threadIdx.x);
+    if (threadIdx.x < NS * 32) h[threadIdx.x] = 0;
+    grid_dep_sync();
     __syncthreads();
     if (t < T) {
-        for (int i = lane; i < E; i += 32) {
-            float v = logits[(size_t)t * E + i];
-            for (int q = 1; q < nparts; ++q) v += logits[((size_t)q * T + t) * E + i];
-            if (nparts > 0) logits_out[(size_t)t * E + i] = v;
-            lg_s[warp][i] = v;
+        constexpr int NL = NP > 0 ? NP : 1;
+        float v[NL][NS];
+#pragma unroll
+        for (int q = 0; q < NL; ++q)
+#pragma unroll
+            for (int i = 0; i < NS; ++i) {
+                const int e = lane + 32 * i;
+                v[q][i] = (e < E) ? __ldg(&logits[((size_t)q * T + t) * E + e]) : -INFINITY;
+            }
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            const int e = lane + 32 * i;
+#pragma unroll
+            for (int q = 1; q < NL; ++q) v[0][i] += v[q][i];
+            if (NP > 0 && e < E) logits_out[(size_t)t * E + e] = v[0][i];
         }
-        __syncwarp();
-        warp_topk(lg_s[warp], E, K, gating, p_s[warp], nullptr, ids + (size_t)t * K, weights + (size_t)t * K);
-        if (blk_hist != nullptr && lane < K) atomicAdd(&h[ids[(size_t)t * K + lane]], 1);  // (the lane's own store)
+        int id;
+        const float w = warp_route<NS>(v[0], E, K, gating, p_s[warp], reinterpret_cast<const uint64_t*>(tab_s), id);
+        if (lane < K) {
+            ids[(size_t)t * K + lane] = (uint32_t)id;
+            weights[(size_t)t * K + lane] = w;
+            if (blk_hist != nullptr) atomicAdd(&h[id], 1);
+        }
     }
     if (blk_hist == nullptr) return;
     __syncthreads();
@@ -342,100 +363,193 @@ sort_rowscan_kernel(int32_t* __restrict__ blk_hist, int nchunks, RouteDev R) {
     if (lane == 0) R.expert_bounds[e] = run;
 }
 
-// One CTA of 256 threads (E <= 256): expert segment bounds from the row totals and the
-// tile lists. tile entry: {expert, col_start, ncols, m_tile}.
-__global__ void __launch_bounds__(256)
-sort_scan_kernel(int nchunks, int E, RouteDev R, int tile_cols, int tile_cols_dn,
-                 int mt_gu, int mt_dn, int4* __restrict__ tiles_gu, int4* __restrict__ tiles_dn,
-                 int32_t* __restrict__ n_tiles, int max_tiles_gu, int max_tiles_dn) {
-    grid_dep_sync();
-    __shared__ int cnt_s[MAX_EXPERTS];
-    __shared__ int bounds_s[MAX_EXPERTS + 1];
-    __shared__ int tile_off_s[MAX_EXPERTS + 1];
-    __shared__ int tile_off_dn_s[MAX_EXPERTS + 1];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid < E) cnt_s[tid] = R.expert_bounds[tid];
+// What the plan of a call consists of besides the sorted pairs: expert segment bounds and the tile
+// lists of the expert products. tile entry: {expert, col_start, ncols, m_tile}.
+struct PlanArgs {
+    int E, tile_shift, tile_shift_dn, mt_gu, mt_dn;  // log2 of the columns per tile
+    int4 *tiles_gu, *tiles_dn;
+    int32_t* n_tiles;
+    int max_tiles_gu, max_tiles_dn;
+    int32_t* any_lo;    // the router's "some low part is non-zero" word: zeroed for the next call
+    int32_t* starts;    // item shares of the streaming kernels (null = none)
+    int ctas, rt_gu, rt_dn;
+    // expert parallel: whether this call's work goes to the streaming kernels is known on the device only (null =
+    // the lists above are what the host decided on); then their chunk list, and no tiles
+    const int32_t* stream_mode;
+    int4* chunks;
+};
+
+// By one CTA of PLAN_THREADS threads: plan from the experts' column counts in shared memory (E <= 256
+// entries); bounds_s[0..E) receives the segment bounds.
+// This runs once per call, alone, and every dependent instruction of its longest chain costs a few ns: the four
+// scans run side by side on eight warps each (thread = expert), and so do the lists that follow. (One
+// warp doing all scans with eight experts per lane took the one-CTA sort 9-12 us.)
+constexpr int PLAN_THREADS = 1024;
+__device__ __forceinline__ void emit_plan(const PlanArgs& a, const RouteDev& R, const int* cnt_s, int* bounds_s) {
+    enum { COLS, TILES, TILES_DN, COST };  // TILES: chunks of the first list in the low, experts with work in the high half
+    __shared__ int off_s[4][MAX_EXPERTS];  // exclusive sums over the experts
+    __shared__ int tot_s[4];
+    __shared__ __align__(16) int wsum_s[4][8];
+    const int tid = threadIdx.x, lane = tid & 31, E = a.E;
+    const int v = tid >> 8, e = tid & 255, wv = e >> 5;
+    // the router's "some low part is non-zero" word, read by now, is zero again for the next call
+    if (a.any_lo != nullptr && tid == 0) *a.any_lo = 0;
+    if (tid >= 1022) a.n_tiles[2 + (tid & 1)] = 0;  // tile counters of the grouped products (tiles are claimed dynamically)
+    const bool to_stream = a.stream_mode != nullptr && *a.stream_mode != 0;
+    const bool to_tc = a.stream_mode != nullptr && !to_stream;
+    const int tsh = to_stream ? STREAM_SHIFT : a.tile_shift, tc = 1 << tsh;
+    // An item of the streaming kernels costs ~1 + n for a chunk of up to 8 n columns: unpacking the
+    // weights, then every group of eight columns.
+    const int full_cost = 1 + (tc >> 3);
+    const int c = (e < E) ? cnt_s[e] : 0;
+    int x = c;
+    if (v == TILES) x = ((c + tc - 1) >> tsh) | (c > 0 ? 1 << 20 : 0);
+    if (v == TILES_DN) x = (c + (1 << a.tile_shift_dn) - 1) >> a.tile_shift_dn;
+    if (v == COST) {
+        const int rest = c & (tc - 1);
+        x = (c >> tsh) * full_cost + (rest ? 1 + ((rest + 7) >> 3) : 0);
+    }
+    int inc = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int w = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += w;
+    }
+    if (lane == 31) wsum_s[v][wv] = inc;
     __syncthreads();
-    if (warp == 0) {
-        int local[8], ltiles[8], ltiles_dn[8], lsum = 0, lnz = 0, ltl = 0, ltd = 0;
+    {
+        const int4 s0 = *reinterpret_cast<const int4*>(&wsum_s[v][0]), s1 = *reinterpret_cast<const int4*>(&wsum_s[v][4]);
+        const int ws[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        int base = 0, total = 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int ee = lane * 8 + j;
-            local[j] = (ee < E) ? cnt_s[ee] : 0;
-            ltiles[j] = (local[j] + tile_cols - 1) / tile_cols;
-            ltiles_dn[j] = (local[j] + tile_cols_dn - 1) / tile_cols_dn;
-            lsum += local[j];
-            lnz += (local[j] > 0);
-            ltl += ltiles[j];
-            ltd += ltiles_dn[j];
+        for (int w = 0; w < 8; ++w) {
+            base += (w < wv) ? ws[w] : 0;
+            total += ws[w];
         }
-        int isum = lsum, inz = lnz, itl = ltl, itd = ltd;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v1 = __shfl_up_sync(0xffffffffu, isum, o);
-            const int v2 = __shfl_up_sync(0xffffffffu, inz, o);
-            const int v3 = __shfl_up_sync(0xffffffffu, itl, o);
-            const int v4 = __shfl_up_sync(0xffffffffu, itd, o);
-            if (lane >= o) {
-                isum += v1;
-                inz += v2;
-                itl += v3;
-                itd += v4;
-            }
+        const int o = inc - x + base;
+        off_s[v][e] = (v == TILES) ? o & 0xfffff : o;
+        if (v == COLS && e < E) {
+            R.expert_bounds[e] = o;
+            bounds_s[e] = o;
         }
-        int run = isum - lsum, unz = inz - lnz, trun = itl - ltl, drun = itd - ltd;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int ee = lane * 8 + j;
-            if (ee < E) {
-                bounds_s[ee] = run;
-                tile_off_s[ee] = trun;
-                tile_off_dn_s[ee] = drun;
-                R.expert_bounds[ee] = run;
-                if (local[j] > 0) R.uexp[unz++] = ee;
-                run += local[j];
-                trun += ltiles[j];
-                drun += ltiles_dn[j];
-            }
-        }
-        if (lane == 31) {
-            bounds_s[E] = isum;
-            tile_off_s[E] = itl;
-            tile_off_dn_s[E] = itd;
-            R.expert_bounds[E] = isum;
-            *R.n_uexp = inz;
-            n_tiles[0] = min(itl * mt_gu, max_tiles_gu);
-            n_tiles[1] = min(itd * mt_dn, max_tiles_dn);
-            n_tiles[2] = 0;  // tile counters of the two grouped products (tiles are claimed dynamically)
-            n_tiles[3] = 0;
+        if (v == TILES && c > 0) R.uexp[o >> 20] = e;
+        if (e == 0) {
+            tot_s[v] = (v == TILES) ? total & 0xfffff : total;
+            if (v == COLS) R.expert_bounds[E] = total;
+            if (v == TILES) *R.n_uexp = total >> 20;
+            if (v == TILES) a.n_tiles[0] = to_stream ? 0 : min((total & 0xfffff) * a.mt_gu, a.max_tiles_gu);
+            if (v == TILES_DN) a.n_tiles[1] = to_stream ? 0 : min(total * a.mt_dn, a.max_tiles_dn);
         }
     }
     __syncthreads();
-    // Column tiles in expert order, all threads emitting: thread takes column chunk c, finds its
-    // expert by bisection of the chunk offsets, writes the chunk's m-tiles. The m-tile is the fastest
-    // index so that CTAs running side by side share the same activation tile. (One thread per
-    // expert used to emit all of a loaded expert's tiles alone: 8.7 us of a 4096-token call.)
-    auto emit = [&](const int* off_s, int tcols, int mt_n, int4* __restrict__ tiles, int max_tiles) {
-        if (tiles == nullptr) return;
-        const int total = off_s[E];
-        for (int c = tid; c < total; c += 256) {
-            int lo = 0, hi = E;  // largest e with off_s[e] <= c
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (off_s[mid] <= c) lo = mid;
-                else hi = mid;
-            }
-            const int e = lo, ct = c - off_s[e];
-            const int cs = bounds_s[e] + ct * tcols;
-            const int nc = min(tcols, cnt_s[e] - ct * tcols);
-            for (int mt = 0; mt < mt_n; ++mt) {
-                const int idx = c * mt_n + mt;
-                if (idx < max_tiles) tiles[idx] = make_int4(e, cs, nc, mt);
-            }
+    // largest expert with off[e] <= y (y below the total)
+    auto expert_of = [&](const int* off, int y) {
+        int lo = 0, hi = E;
+#pragma unroll 1
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (off[mid] <= y) lo = mid;
+            else hi = mid;
         }
+        return lo;
     };
-    emit(tile_off_s, tile_cols, mt_gu, tiles_gu, max_tiles_gu);
-    emit(tile_off_dn_s, tile_cols_dn, mt_dn, tiles_dn, max_tiles_dn);
+    if (v < 3) {
+        // Column tiles in expert order: a thread takes column chunk q, finds its expert by bisection of the
+        // chunk offsets, writes the chunk's m-tiles. The m-tile is the fastest index so that CTAs
+        // running side by side share the same activation tile.
+        const bool dn = (v == 2);
+        int4* tiles = dn ? (to_stream ? nullptr : a.tiles_dn) : to_stream ? a.chunks : a.tiles_gu;
+        const int* off = off_s[dn ? TILES_DN : TILES];
+        const int total = tiles ? tot_s[dn ? TILES_DN : TILES] : 0;
+        const int sh = dn ? a.tile_shift_dn : tsh, mt_n = dn ? a.mt_dn : to_stream ? 1 : a.mt_gu, max_tiles = dn ? a.max_tiles_dn : a.max_tiles_gu;
+#pragma unroll 1
+        for (int q = dn ? e : tid; q < total; q += dn ? 256 : 512) {
+            const int ee = expert_of(off, q), ct = q - off[ee];
+            const int cs = bounds_s[ee] + (ct << sh), nc = min(1 << sh, cnt_s[ee] - (ct << sh));
+#pragma unroll 1
+            for (int mt = 0, idx = q * mt_n; mt < mt_n && idx < max_tiles; ++mt, ++idx) tiles[idx] = make_int4(ee, cs, nc, mt);
+        }
+    } else if (a.starts != nullptr) {
+        // shares of the streaming kernels' CTAs: contiguous item ranges of equal cost
+        const float per_cta = (float)tot_s[COST] / (float)a.ctas;
+#pragma unroll 1
+        for (int i = e; i <= a.ctas; i += 256) {
+            int chunk = to_tc ? 0 : tot_s[TILES];
+            float frac = 0.0f;
+            if (i < a.ctas && !to_tc) {
+                const float want = per_cta * (float)i;
+                const int ee = expert_of(off_s[COST], min((int)want, tot_s[COST] - 1));
+                const float rest = want - (float)off_s[COST][ee];
+                const int ct = (int)rest / full_cost;
+                chunk = off_s[TILES][ee] + ct;
+                frac = __fdividef(rest - (float)(ct * full_cost), (float)(1 + ((min(tc, cnt_s[ee] - (ct << tsh)) + 7) >> 3)));
+            }
+            a.starts[i] = chunk * a.rt_gu + min((int)(frac * (float)a.rt_gu), a.rt_gu);
+            a.starts[a.ctas + 1 + i] = chunk * a.rt_dn + min((int)(frac * (float)a.rt_dn), a.rt_dn);
+        }
+    }
+}
+
+// One CTA: the plan from the row totals that sort_rowscan_kernel (or an expert-parallel plan) left in expert_bounds.
+__global__ void __launch_bounds__(PLAN_THREADS)
+sort_scan_kernel(const __grid_constant__ PlanArgs a, RouteDev R) {
+    grid_dep_sync();
+    __shared__ int cnt_s[MAX_EXPERTS];
+    __shared__ int bounds_s[MAX_EXPERTS];
+    if (threadIdx.x < a.E) cnt_s[threadIdx.x] = R.expert_bounds[threadIdx.x];
+    __syncthreads();
+    emit_plan(a, R, cnt_s, bounds_s);
+}
+
+// The whole sort of a short batch (up to SORT1_MAX pairs) in one CTA: a warp owns a contiguous
+// run of pairs, counts them per expert (lanes with the same expert find each other by a match, so no
+// atomics), the counts are scanned over warps and experts, and the warp places its pairs. One
+// launch for the three below: at 77 tokens they took 11 us of a 217 us call, this one 5.
+constexpr int SORT1_MAX = 2048, SORT1_WARPS = PLAN_THREADS / 32;
+__global__ void __launch_bounds__(SORT1_WARPS * 32)
+sort_one_kernel(const uint32_t* __restrict__ ids, int C, int K, RouteDev R, const __grid_constant__ PlanArgs a) {
+    __shared__ int wcnt[SORT1_WARPS * MAX_EXPERTS];  // [warp][E]
+    __shared__ int cnt_s[MAX_EXPERTS];
+    __shared__ int bounds_s[MAX_EXPERTS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, E = a.E;
+    for (int i = tid; i < SORT1_WARPS * E; i += SORT1_WARPS * 32) wcnt[i] = 0;
+    grid_dep_sync();
+    __syncthreads();
+    int* my = wcnt + warp * E;
+    const int per = (C + SORT1_WARPS * 32 - 1) / (SORT1_WARPS * 32);  // 32-pair steps of a warp
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll 1
+        for (int i = 0; i < per; ++i) {
+            const int p = (warp * per + i) * 32 + lane;
+            const int e = (p < C) ? (int)ids[p] : -1 - lane;  // padding lanes match nobody
+            const unsigned same = __match_any_sync(0xffffffffu, e), below = same & ((1u << lane) - 1u);
+            if (pass == 1 && e >= 0) {
+                const int col = bounds_s[e] + my[e] + __popc(below);
+                R.col_expert[col] = e;
+                R.col_src_tok[col] = p / K;
+                R.dst_to_col[p] = col;
+            }
+            __syncwarp();
+            if (e >= 0 && below == 0u) my[e] += __popc(same);  // one leader per expert
+            __syncwarp();
+        }
+        if (pass == 1) break;
+        __syncthreads();
+        if (tid < E) {
+            int run = 0;
+#pragma unroll 4
+            for (int w = 0; w < SORT1_WARPS; ++w) {
+                const int c = wcnt[w * E + tid];
+                wcnt[w * E + tid] = run;
+                run += c;
+            }
+            cnt_s[tid] = run;
+        }
+        __syncthreads();
+        emit_plan(a, R, cnt_s, bounds_s);
+        __syncthreads();
+    }
 }
 
 // One warp per chunk of SORT_TOK tokens: the chunk's (token, slot) pairs are taken 32 at
@@ -501,8 +615,11 @@ build_xf_kernel(const XT* __restrict__ x, int T, int H, int nblk_pad, bool bf16_
 // ---------------------------------------------------------------------------
 // scatter-accumulate
 // ---------------------------------------------------------------------------
-// One thread per 8 consecutive outputs (16-byte loads of the f16 rows); the slots are taken four
-// at a time so that their rows are in flight together, and added in slot order.
+// One thread per 8 consecutive outputs (16-byte loads of the f16 rows); the slots are taken S
+// at a time so that their rows are in flight together, and added in slot order: eight for a short batch, where the
+// chain of round trips is the time (77 tokens: 6 -> 4 us), four when the rows come from HBM (4096 tokens: 33 us, 51
+// with eight: fewer warps resident).
+template <int S>  // slots in flight
 __global__ void __launch_bounds__(256)
 scatter_accum_kernel(const __half* __restrict__ d16, const float* residual,
                      const float* __restrict__ weights, const int32_t* __restrict__ dst_to_col,
@@ -519,18 +636,21 @@ scatter_accum_kernel(const __half* __restrict__ d16, const float* residual,
         acc[0] = r0.x; acc[1] = r0.y; acc[2] = r0.z; acc[3] = r0.w;
         acc[4] = r1.x; acc[5] = r1.y; acc[6] = r1.z; acc[7] = r1.w;
     }
-    for (int s0 = 0; s0 < K; s0 += 4) {
-        uint4 d[4];
-        float w[4];
+    for (int s0 = 0; s0 < K; s0 += S) {
+        int col[S];
+        uint4 d[S];
+        float w[S];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int slot = min(s0 + j, K - 1);
-            const int col = dst_to_col[(size_t)t * K + slot];
-            w[j] = weights[(size_t)t * K + slot];
-            d[j] = *reinterpret_cast<const uint4*>(d16 + (size_t)col * H + h8 * 8);
+        for (int j = 0; j < S; ++j) {
+            const size_t p = (size_t)t * K + min(s0 + j, K - 1);
+            col[j] = dst_to_col[p];
+            w[j] = weights[p];
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < S; ++j)
+            if (s0 + j < K) d[j] = *reinterpret_cast<const uint4*>(d16 + (size_t)col[j] * H + h8 * 8);
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
             if (s0 + j < K) {
                 const __half2* hp = reinterpret_cast<const __half2*>(&d[j]);
 #pragma unroll
@@ -549,7 +669,7 @@ scatter_accum_kernel(const __half* __restrict__ d16, const float* residual,
 cudaError_t launch_scatter_accum(const __half* d16, const float* residual, const RouteDev& R, float* out,
                                  int T, int H, int K, cudaStream_t st) {
     count_launch();
-    return launch_dep(scatter_accum_kernel, dim3(T, (H / 8 + 255) / 256), dim3(256), 0, st, d16, residual, R.weights,
+    return launch_dep(T <= 512 ? scatter_accum_kernel<8> : scatter_accum_kernel<4>, dim3(T, (H / 8 + 255) / 256), dim3(256), 0, st, d16, residual, R.weights,
                       R.dst_to_col, out, T, H, K);
 }
 
@@ -608,6 +728,26 @@ __global__ void set_routing_kernel(const uint32_t* __restrict__ ids_in, const fl
     }
 }
 
+static int log2i(int v) { return v <= 1 ? 0 : 1 + log2i(v / 2); }
+
+template <int NS>
+static cudaError_t launch_topk_n(const PrefillArgs& a, const float* lg, int nparts, int32_t* hist, cudaStream_t st) {
+    const dim3 grid((a.T + TK_WARPS - 1) / TK_WARPS), block(TK_WARPS * 32);
+    auto go = [&](auto kern) {
+        return launch_dep(kern, grid, block, 0, st, lg, a.R.logits, a.T, a.L.E, a.K, a.gating, a.R.ids, a.R.weights, hist);
+    };
+    switch (nparts) {
+        case 0: return go(topk_large_kernel<NS, 0>);
+        case 1: return go(topk_large_kernel<NS, 1>);
+        case 2: return go(topk_large_kernel<NS, 2>);
+        default: return go(topk_large_kernel<NS, 4>);
+    }
+}
+static cudaError_t launch_topk(const PrefillArgs& a, const float* lg, int nparts, int32_t* hist, cudaStream_t st) {
+    if (a.L.E <= 32) return launch_topk_n<1>(a, lg, nparts, hist, st);
+    return (a.L.E <= 128) ? launch_topk_n<4>(a, lg, nparts, hist, st) : launch_topk_n<8>(a, lg, nparts, hist, st);
+}
+
 // Router + tables for any T. tile lists are optional (tiles == nullptr skips them).
 cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st) {
     const int T = a.T, E = a.L.E, H = a.L.H, K = a.K;
@@ -656,36 +796,43 @@ cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st) {
         }
         lg = a.R.logits;
     }
-    count_launch(4);
     const int nchunks = (T + SORT_TOK - 1) / SORT_TOK;
+    const bool one_cta = T * K <= SORT1_MAX;
+    count_launch(one_cta ? 2 : 4);
     if (a.ids_in == nullptr)
-        CUDA_RET(launch_dep(topk_large_kernel, dim3(nchunks), dim3(TK_WARPS * 32), 0, st, lg, nparts, a.R.logits, T, E, K,
-                            a.gating, a.R.ids, a.R.weights, a.blk_hist));
-    else
+        CUDA_RET(launch_topk(a, lg, nparts, one_cta ? nullptr : a.blk_hist, st));
+    else if (!one_cta)
         CUDA_RET(launch_dep(sort_hist_kernel, dim3(nchunks), dim3(256), 0, st, a.R.ids, T, K, E, a.blk_hist));
     const int C = T * K;
     // columns per grouped-GEMM tile: 128 or 256, the same for gate/up and down
-    const int tile_cols = tc_gu_tile_cols(C, E), tile_cols_dn = tile_cols;
+    // (the streaming kernels share one list of column chunks and cut the rows themselves)
+    const bool stream = (a.impl == 2);
+    const int tile_cols = stream ? STREAM_CHUNK : tc_gu_tile_cols(C, E), tile_cols_dn = tile_cols;
     const int max_ct = C / tile_cols + E, max_ct_dn = C / tile_cols_dn + E;
-    const int mt_gu = a.L.I / 128, mt_dn = a.L.H / 256;  // m-tiles: 128 gate + 128 up rows | 256 down rows
+    const int mt_gu = stream ? 1 : a.L.I / 128, mt_dn = a.L.H / 256;  // m-tiles: 128 gate + 128 up rows | 256 down rows
     int4* tiles_gu = a.tiles;
-    int4* tiles_dn = a.tiles ? a.tiles + (size_t)max_ct * (mt_gu > 0 ? mt_gu : 1) : nullptr;
+    int4* tiles_dn = (a.tiles && !stream) ? a.tiles + (size_t)max_ct * (mt_gu > 0 ? mt_gu : 1) : nullptr;
+    const PlanArgs plan{E, log2i(tile_cols), log2i(tile_cols_dn), mt_gu, mt_dn, tiles_gu, tiles_dn, a.n_tiles, max_ct * mt_gu, max_ct_dn * mt_dn,
+                        a.any_lo, stream ? a.stream_starts : nullptr, a.sms, a.L.I / 16, a.L.H / 16};
+    if (one_cta) return launch_dep(sort_one_kernel, dim3(1), dim3(SORT1_WARPS * 32), 0, st, a.R.ids, C, K, a.R, plan);
     CUDA_RET(launch_dep(sort_rowscan_kernel, dim3(E), dim3(32), 0, st, a.blk_hist, nchunks, a.R));
-    CUDA_RET(launch_dep(sort_scan_kernel, dim3(1), dim3(256), 0, st, nchunks, E, a.R, tile_cols, tile_cols_dn, mt_gu, mt_dn,
-                        tiles_gu, tiles_dn, a.n_tiles, max_ct * mt_gu, max_ct_dn * mt_dn));
+    CUDA_RET(launch_dep(sort_scan_kernel, dim3(1), dim3(PLAN_THREADS), 0, st, plan, a.R));
     return launch_dep(sort_place_kernel, dim3((nchunks + 7) / 8), dim3(256), 0, st, a.R.ids, T, K, E, a.blk_hist, nchunks,
                       a.R);
 }
 
 cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_cap, int gu_cols, int4* tiles,
-                             int32_t* n_tiles, cudaStream_t st) {
+                             int32_t* n_tiles, cudaStream_t st, const int32_t* stream_mode, int4* chunks, int32_t* starts,
+                             int sms) {
     const int max_ct = rows_cap / gu_cols + E, max_ct_dn = rows_cap / 128 + E;
     const int mt_gu = I / 128, mt_dn = H / 256;
     count_launch();
     // (down tiles of 128 tokens here: an expert-parallel down product stores its rows into other GPUs'
     // memory, which only the always-overlapped epilogue of the 128-token form hides)
-    return launch_dep(sort_scan_kernel, dim3(1), dim3(256), 0, st, 0, E, R, gu_cols, 128, mt_gu, mt_dn, tiles,
-                      tiles + (size_t)max_ct * (mt_gu > 0 ? mt_gu : 1), n_tiles, max_ct * mt_gu, max_ct_dn * mt_dn);
+    const PlanArgs plan{E, log2i(gu_cols), 7, mt_gu, mt_dn, tiles, tiles + (size_t)max_ct * (mt_gu > 0 ? mt_gu : 1), n_tiles,
+                        max_ct * mt_gu, max_ct_dn * mt_dn, nullptr, stream_mode ? starts : nullptr, sms, I / 16, H / 16,
+                        stream_mode, chunks};
+    return launch_dep(sort_scan_kernel, dim3(1), dim3(PLAN_THREADS), 0, st, plan, R);
 }
 
 // ---------------------------------------------------------------------------

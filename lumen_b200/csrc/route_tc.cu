@@ -20,6 +20,7 @@
 // All mbarrier waits are bounded; on expiry the kernel raises the context's status word,
 // frees its TMEM and returns.
 #include "tc_common.cuh"
+#include <type_traits>
 
 namespace lumen {
 
@@ -27,10 +28,16 @@ namespace rtc {
 
 using namespace tc;
 
-constexpr int STAGES = 3;
-constexpr int STAGE_BYTES = 4 * SUB_BYTES;  // W_hi | W_lo | x_hi | x_lo, each [128 rows x 64 k] f16
+// Tokens per tile: 128, or 32 for batches whose 128-token tiles would leave most of the chip idle. A logit is
+// the same in both: the tile width only says how many columns one MMA covers. (77 tokens: 11 -> 6 us,
+// with the set-up and the first weight boxes moved ahead of the wait for the kernel before.)
+template <int BN>
+struct Cfg {
+    static constexpr int STAGES = (BN == 128) ? 3 : 5;
+    static constexpr int X_BYTES = BN * 128;                           // [BN rows x 64 k] f16
+    static constexpr int STAGE_BYTES = 2 * SUB_BYTES + 2 * X_BYTES;    // W_hi | W_lo ([128 rows x 64 k] each) | x_hi | x_lo
+};
 constexpr int THREADS = 6 * 32;
-constexpr int BN = 128;  // tokens per tile
 
 struct Args {
     CUtensorMap tmap_w;   // [2 E, H] f16: rows [0, E) high parts, [E, 2 E) low parts
@@ -43,8 +50,10 @@ struct Args {
     int T, E, H, ksplit, m_tiles;
 };
 
+template <int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 router_logits_tc_kernel(const __grid_constant__ Args a) {
+    constexpr int STAGES = Cfg<BN>::STAGES, STAGE_BYTES = Cfg<BN>::STAGE_BYTES, X_BYTES = Cfg<BN>::X_BYTES;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_bar;
     __shared__ uint32_t tmem_base_s;
@@ -62,13 +71,10 @@ router_logits_tc_kernel(const __grid_constant__ Args a) {
     const int t0 = tt * BN, e0 = mt * 128;
     const int kh_per = (a.H / 64) / a.ksplit;  // 64-input stages of this CTA's k range
     const int kh0 = ks * kh_per;
-    grid_dep_sync();  // (the planes of x and the flag come from the split kernel before this one)
-    const bool use_lo = (*a.any_lo != 0);
-
     if (tid == 0) {
         abort_s = 0u;
         for (int s = 0; s < STAGES; ++s) {
-            mbar_init(smem_u32(&full_bar[s]), 1);
+            mbar_init(smem_u32(&full_bar[s]), 2);  // the weight boxes' and the activation boxes' expect_tx
             mbar_init(smem_u32(&empty_bar[s]), 1);
         }
         mbar_init(smem_u32(&acc_bar), 1);
@@ -76,7 +82,7 @@ router_logits_tc_kernel(const __grid_constant__ Args a) {
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
-                     "r"((uint32_t)BN)
+                     "r"((uint32_t)BN)  // (a power of two, 32 at least)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -85,48 +91,62 @@ router_logits_tc_kernel(const __grid_constant__ Args a) {
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
 
+    // The weight planes are static: their boxes of the first stages are requested before the wait for the split
+    // kernel, whose output (the planes of x and the flag) everything else here depends on.
+    auto load_w = [&](int n) {
+        const int s = n % STAGES, k = (kh0 + n) * 64;
+        const uint32_t bar = smem_u32(&full_bar[s]), base = stage0 + s * STAGE_BYTES;
+        mbar_expect_tx(bar, 2 * SUB_BYTES);
+        tma_load_2d(base, &a.tmap_w, k, e0, bar);
+        tma_load_2d(base + SUB_BYTES, &a.tmap_w, k, a.E + e0, bar);
+    };
+    if (tid == 0)
+        for (int n = 0; n < STAGES && n < kh_per; ++n) load_w(n);
+    grid_dep_sync();
+    const bool use_lo = (*a.any_lo != 0);
+
     if (warp == 0) {
         if (lane == 0) {
             bool ok = true;
             for (int n = 0; ok && n < kh_per; ++n) {
                 const int s = n % STAGES, ph = (n / STAGES) & 1;
-                ok = mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag);
-                if (!ok) break;
-                const uint32_t bar = smem_u32(&full_bar[s]);
-                const uint32_t base = stage0 + s * STAGE_BYTES;
+                if (n >= STAGES) {
+                    ok = mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag);
+                    if (!ok) break;
+                    load_w(n);
+                }
+                const uint32_t bar = smem_u32(&full_bar[s]), base = stage0 + s * STAGE_BYTES + 2 * SUB_BYTES;
                 const int k = (kh0 + n) * 64;
-                mbar_expect_tx(bar, (use_lo ? 4 : 3) * SUB_BYTES);
-                tma_load_2d(base + 0 * SUB_BYTES, &a.tmap_w, k, e0, bar);
-                tma_load_2d(base + 1 * SUB_BYTES, &a.tmap_w, k, a.E + e0, bar);
-                tma_load_2d(base + 2 * SUB_BYTES, &a.tmap_x, k, t0, bar);
-                if (use_lo) tma_load_2d(base + 3 * SUB_BYTES, &a.tmap_x, k, a.T + t0, bar);
+                mbar_expect_tx(bar, (use_lo ? 2 : 1) * X_BYTES);
+                tma_load_2d(base, &a.tmap_x, k, t0, bar);
+                if (use_lo) tma_load_2d(base + X_BYTES, &a.tmap_x, k, a.T + t0, bar);
             }
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc(BN, false);
-            bool ok = true;
-            for (int n = 0; ok && n < kh_per; ++n) {
-                const int s = n % STAGES, ph = (n / STAGES) & 1;
-                ok = mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t base = stage0 + s * STAGE_BYTES;
+        const uint32_t idesc = make_idesc(BN, false);
+        bool ok = true;
+        for (int n = 0, s = 0, ph = 0; n < kh_per; ++n) {
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+                const uint64_t w0 = make_desc(stage0 + s * STAGE_BYTES), x0 = w0 + (2 * SUB_BYTES >> 4);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const uint64_t whi = make_desc(base + 0 * SUB_BYTES + j * 32);
-                    const uint64_t wlo = make_desc(base + 1 * SUB_BYTES + j * 32);
-                    const uint64_t xhi = make_desc(base + 2 * SUB_BYTES + j * 32);
-                    umma(tmem_base, whi, xhi, idesc, (n > 0 || j > 0) ? 1u : 0u);
-                    umma(tmem_base, wlo, xhi, idesc, 1u);
-                    if (use_lo) umma(tmem_base, whi, make_desc(base + 3 * SUB_BYTES + j * 32), idesc, 1u);
+                    umma(tmem_base, w0 + j * 2, x0 + j * 2, idesc, (n > 0 || j > 0) ? 1u : 0u);
+                    umma(tmem_base, w0 + (SUB_BYTES >> 4) + j * 2, x0 + j * 2, idesc, 1u);
+                    if (use_lo) umma(tmem_base, w0 + j * 2, x0 + (X_BYTES >> 4) + j * 2, idesc, 1u);
                 }
                 umma_commit(smem_u32(&empty_bar[s]));
+                if (n == kh_per - 1) umma_commit(smem_u32(&acc_bar));
             }
-            if (ok) umma_commit(smem_u32(&acc_bar));
+            __syncwarp();
+            if (++s == STAGES) {
+                s = 0;
+                ph ^= 1;
+            }
         }
-        __syncwarp();
     } else {
         // epilogue: warp w reads TMEM lanes 32 * (w % 4) ..; lane = expert row of the tile
         const int q = warp & 3;
@@ -156,7 +176,11 @@ router_logits_tc_kernel(const __grid_constant__ Args a) {
     if (tid == 0 && abort_s) raise_status(a.status, a.status_host, 4);  // LUMEN_MOE_TIMEOUT
 }
 
-// x [T, H] (f32 or bf16) -> f16 planes [2][T][H]: high part, low part; *any_lo |= (some low part != 0)
+// x [T, H] (f32, bf16 or f16) -> f16 planes [2][T][H] in the weight planes' element order: high part, low
+// part; *any_lo |= (some low part != 0). The high plane is also the activation operand of the expert
+// products of short prompts. any_lo null: no low plane wanted (routing supplied by the caller).
+// One thread per 16-byte output chunk: chunk t of a 32-block holds inputs
+// (4t, 4t+2, 16+4t, 16+4t+2, 4t+1, 4t+3, 16+4t+1, 16+4t+3).
 template <typename XT>
 __global__ void __launch_bounds__(256)
 split_x16_kernel(const XT* __restrict__ x, size_t n8, size_t plane, __half* __restrict__ out, int32_t* any_lo) {
@@ -164,20 +188,26 @@ split_x16_kernel(const XT* __restrict__ x, size_t n8, size_t plane, __half* __re
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
     unsigned nz = 0u;
     if (i < n8) {
-        float f[8];
+        const size_t oa = (i >> 2) * 32 + (i & 3) * 4;
+        float4 p, q;  // inputs 4t.. and 16+4t..
         if (sizeof(XT) == 4) {
-            const float4 p = reinterpret_cast<const float4*>(x)[2 * i], q = reinterpret_cast<const float4*>(x)[2 * i + 1];
-            f[0] = p.x; f[1] = p.y; f[2] = p.z; f[3] = p.w;
-            f[4] = q.x; f[5] = q.y; f[6] = q.z; f[7] = q.w;
+            p = *reinterpret_cast<const float4*>(x + oa);
+            q = *reinterpret_cast<const float4*>(x + oa + 16);
         } else {
-            const uint4 v = reinterpret_cast<const uint4*>(x)[i];
-            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                f[2 * j] = __uint_as_float(u[j] << 16);
-                f[2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
+            const uint2 u = *reinterpret_cast<const uint2*>(x + oa), v = *reinterpret_cast<const uint2*>(x + oa + 16);
+            if (std::is_same<XT, __half>::value) {
+                const float2 u0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), u1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+                const float2 v0 = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), v1 = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+                p = make_float4(u0.x, u0.y, u1.x, u1.y);
+                q = make_float4(v0.x, v0.y, v1.x, v1.y);
+            } else {
+                p = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                                __uint_as_float(u.y & 0xffff0000u));
+                q = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                                __uint_as_float(v.y & 0xffff0000u));
             }
         }
+        const float f[8] = {p.x, p.z, q.x, q.z, p.y, p.w, q.y, q.w};
         __align__(16) __half hi[8], lo[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -186,21 +216,24 @@ split_x16_kernel(const XT* __restrict__ x, size_t n8, size_t plane, __half* __re
             nz |= (unsigned)(__half_as_ushort(lo[j]) & 0x7fffu);
         }
         reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(hi);
-        reinterpret_cast<uint4*>(out + plane)[i] = *reinterpret_cast<const uint4*>(lo);
+        if (any_lo != nullptr) reinterpret_cast<uint4*>(out + plane)[i] = *reinterpret_cast<const uint4*>(lo);
     }
-    if (__any_sync(0xffffffffu, nz != 0u) && (threadIdx.x & 31) == 0) atomicOr(any_lo, 1);
+    if (any_lo != nullptr && __any_sync(0xffffffffu, nz != 0u) && (threadIdx.x & 31) == 0 && *reinterpret_cast<volatile int32_t*>(any_lo) == 0)
+        atomicOr(any_lo, 1);  // (one warp's finding is enough: the word is read first, so that thousands of atomics do not queue on it)
 }
 
 }  // namespace rtc
 
-// W_r [E, H] f32 -> f16 planes [2][E][H] (high, low): once per layer
+// W_r [E, H] f32 -> f16 planes [2][E][H] (high, low) in the same element order as x: once per layer
 __global__ void split_router_w16_kernel(const float* __restrict__ w, __half* __restrict__ w16, size_t n) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float v = w[i];
     const __half hi = __float2half_rn(v);
-    w16[i] = hi;
-    w16[n + i] = __float2half_rn(v - __half2float(hi));
+    const int el = (int)(i & 31), t = (el & 15) >> 2, m = el & 3;
+    const size_t o = (i & ~(size_t)31) + t * 8 + ((m & 1) ? 4 : 0) + ((el >> 4) ? 2 : 0) + (m >> 1);
+    w16[o] = hi;
+    w16[n + o] = __float2half_rn(v - __half2float(hi));
 }
 
 cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, cudaStream_t st) {
@@ -227,24 +260,39 @@ bool router_tc_applicable(int T, int E, int H, const void* x) {
     return H % 64 == 0 && E >= 1 && E <= 256 && T >= 1 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
 }
 
+cudaError_t launch_split_x16(const void* x, int act_dtype, int T, int H, __half* x16, int32_t* any_lo, cudaStream_t st) {
+    const size_t n8 = (size_t)T * H / 8, plane = (size_t)T * H;
+    const dim3 grid((unsigned)((n8 + 255) / 256));
+    count_launch();
+    if (act_dtype == 0) return launch_dep(rtc::split_x16_kernel<float>, grid, dim3(256), 0, st, (const float*)x, n8, plane, x16, any_lo);
+    if (act_dtype == 2) return launch_dep(rtc::split_x16_kernel<__half>, grid, dim3(256), 0, st, (const __half*)x, n8, plane, x16, any_lo);
+    return launch_dep(rtc::split_x16_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, (const __nv_bfloat16*)x, n8, plane, x16, any_lo);
+}
+
+template <int BN>
+static cudaError_t launch_rtc(const rtc::Args& a, cudaStream_t st) {
+    const int smem = rtc::Cfg<BN>::STAGES * rtc::Cfg<BN>::STAGE_BYTES + 1024;
+    static SmemOptIn optin;
+    const cudaError_t e = ensure_dyn_smem(rtc::router_logits_tc_kernel<BN>, (size_t)smem, optin);
+    if (e != cudaSuccess) return e;
+    const int grid = ((a.T + BN - 1) / BN) * a.m_tiles * a.ksplit;
+    return launch_dep(rtc::router_logits_tc_kernel<BN>, dim3(grid), dim3(rtc::THREADS), (size_t)smem, st, a);
+}
+
 // logits partials of the whole batch; x16 / any_lo / part are scratch of the context
 cudaError_t launch_router_logits_tc(const void* x, int act_dtype, const __half* w16, int T, int E, int H, int ksplit,
                                     __half* x16, int32_t* any_lo, float* part, int32_t* status, int32_t* status_host,
                                     unsigned wait_limit_us, cudaStream_t st) {
-    const size_t n8 = (size_t)T * H / 8, plane = (size_t)T * H;
-    cudaError_t e = cudaMemsetAsync(any_lo, 0, sizeof(int32_t), st);
+    cudaError_t e = launch_split_x16(x, act_dtype, T, H, x16, any_lo, st);
     if (e != cudaSuccess) return e;
-    count_launch(2);
-    const dim3 sgrid((unsigned)((n8 + 255) / 256));
-    e = (act_dtype == 0)
-            ? launch_dep(rtc::split_x16_kernel<float>, sgrid, dim3(256), 0, st, (const float*)x, n8, plane, x16, any_lo)
-            : launch_dep(rtc::split_x16_kernel<__nv_bfloat16>, sgrid, dim3(256), 0, st, (const __nv_bfloat16*)x, n8, plane, x16,
-                         any_lo);
-    if (e != cudaSuccess) return e;
+    count_launch();
     rtc::Args a{};
+    a.m_tiles = (E + 127) / 128;
     e = make_tmap_f16(w16, (uint64_t)2 * E, (uint64_t)H, 128, &a.tmap_w);
     if (e != cudaSuccess) return e;
-    e = make_tmap_f16(x16, (uint64_t)2 * T, (uint64_t)H, 128, &a.tmap_x);
+    const bool narrow = (T + 127) / 128 * a.m_tiles * ksplit < 148 / 2;
+    const int bn = narrow ? 32 : 128;
+    e = make_tmap_f16(x16, (uint64_t)2 * T, (uint64_t)H, bn, &a.tmap_x);
     if (e != cudaSuccess) return e;
     a.part = part;
     a.any_lo = any_lo;
@@ -255,13 +303,7 @@ cudaError_t launch_router_logits_tc(const void* x, int act_dtype, const __half* 
     a.E = E;
     a.H = H;
     a.ksplit = ksplit;
-    a.m_tiles = (E + 127) / 128;
-    const int smem = rtc::STAGES * rtc::STAGE_BYTES + 1024;
-    static SmemOptIn optin;
-    e = ensure_dyn_smem(rtc::router_logits_tc_kernel, (size_t)smem, optin);
-    if (e != cudaSuccess) return e;
-    const int grid = ((T + rtc::BN - 1) / rtc::BN) * a.m_tiles * ksplit;
-    return launch_dep(rtc::router_logits_tc_kernel, dim3(grid), dim3(rtc::THREADS), (size_t)smem, st, a);
+    return narrow ? launch_rtc<32>(a, st) : launch_rtc<128>(a, st);
 }
 
 }  // namespace lumen

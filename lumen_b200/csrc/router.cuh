@@ -37,7 +37,8 @@ namespace lumen {
 // Double-precision instructions issue slowly on this part, and the exp is the only
 // place that needs them, so the exps of one token can be shared by `nsub` warps
 // (warp_gate_probs with sub = 0..nsub-1, the caller synchronises them) before one
-// warp finishes the token (warp_select). warp_topk is the one-warp form.
+// warp finishes the token (warp_select). warp_topk is the one-warp form; warp_route the one-warp form with
+// the logits in registers.
 
 // One body for all call sites: the exp is ~60 double-precision instructions and the code of
 // these routines runs once per launch, so its size is paid in instruction fetches.
@@ -214,6 +215,101 @@ __device__ __forceinline__ void warp_topk(const float* __restrict__ logits, int 
     warp_gate_probs(logits, E, gating, smem_p, tab, 0, 1);
     __syncwarp();
     warp_select(smem_p, E, K, gating, out_ids, out_w);
+}
+
+// The whole routing of one token by one warp with its logits in registers: expert lane + 32 i in
+// lg[i] (-inf past E). Lane k < K returns the weight of the k-th selected expert, its id in id_out. Same operations in the
+// same order as warp_gate_probs + warp_select; what differs is the latency: the NS exps of a lane are independent and
+// inline, a lane keeps its probabilities sorted (largest first, lower index first among equals) so that a
+// selection round is one reduction and one vote, and the winners' ids go through shared memory
+// instead of a second reduction. smem_p: NS * 32 floats, 16-byte aligned, private to the warp.
+template <int NS>
+__device__ __forceinline__ float warp_route(const float (&lg)[NS], int E, int K, int gating, float* smem_p,
+                                            const uint64_t* tab, int& id_out) {
+    const int lane = threadIdx.x & 31;
+    float m = 0.0f;
+    if (gating == 0) {
+        m = lg[0];
+#pragma unroll
+        for (int i = 1; i < NS; ++i) m = fmaxf(m, lg[i]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    }
+    float p[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+        const float ex = lumen_exact::expf_libm_tab((gating == 0) ? lg[i] - m : -lg[i], lumen_exact::Exp2TabPtr{tab});
+        p[i] = (gating == 0) ? ex : __fdiv_rn(1.0f, __fadd_rn(1.0f, ex));
+    }
+    if (gating == 0) {
+#pragma unroll
+        for (int i = 0; i < NS; ++i) smem_p[lane + 32 * i] = p[i];
+        __syncwarp();
+        // sequential f32 sum over e ascending, on every lane; entries past E are exp(-inf) = +0, which change nothing
+        float sum = 0.0f;
+        const float4* p4 = reinterpret_cast<const float4*>(smem_p);
+#pragma unroll
+        for (int e = 0; e < NS * 8; ++e) {
+            const float4 c = p4[e];
+            sum = __fadd_rn(sum, c.x);
+            sum = __fadd_rn(sum, c.y);
+            sum = __fadd_rn(sum, c.z);
+            sum = __fadd_rn(sum, c.w);
+        }
+#pragma unroll
+        for (int i = 0; i < NS; ++i) p[i] = __fdiv_rn(p[i], sum);
+        __syncwarp();
+    }
+    unsigned key[NS];  // bit pattern + 1 (probabilities are >= 0: unsigned order is value order); 0 = none
+    int slot[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+        key[i] = (lane + 32 * i < E) ? __float_as_uint(p[i]) + 1u : 0u;
+        slot[i] = i;
+    }
+#pragma unroll
+    for (int a = 0; a < NS - 1; ++a)  // (a strict comparison keeps the lower index first among equals)
+#pragma unroll
+        for (int b = 0; b < NS - 1 - a; ++b) {
+            const bool sw = key[b + 1] > key[b];
+            const unsigned k0 = sw ? key[b + 1] : key[b], k1 = sw ? key[b] : key[b + 1];
+            const int s0 = sw ? slot[b + 1] : slot[b], s1 = sw ? slot[b] : slot[b + 1];
+            key[b] = k0;
+            key[b + 1] = k1;
+            slot[b] = s0;
+            slot[b + 1] = s1;
+        }
+    int* win_s = reinterpret_cast<int*>(smem_p);
+    float my_sel = 0.0f, renorm = 0.0f;
+#pragma unroll 1
+    for (int k = 0; k < K; ++k) {
+        const unsigned mk = __reduce_max_sync(0xffffffffu, key[0]);
+        const bool top = key[0] == mk;
+        const unsigned who = __ballot_sync(0xffffffffu, top);
+        const int idx = lane + 32 * slot[0];
+        bool win = top;
+        if (who & (who - 1u)) {  // (uniform: every lane takes part in the reduction)
+            const int lowest = __reduce_min_sync(0xffffffffu, top ? idx : 0x7fffffff);
+            win = top && idx == lowest;
+        }
+        float sel = __uint_as_float(mk - 1u);
+        if (mk == 0u) sel = -1.0f;  // nothing left: the reference's fold starts at (index 0, -1.0)
+        renorm = __fadd_rn(renorm, sel);  // sel[0] + sel[1] + ... in order, on every lane
+        if (lane == k) my_sel = sel;
+        if (win) {
+            win_s[k] = (mk == 0u) ? 0 : idx;
+#pragma unroll
+            for (int i = 0; i < NS - 1; ++i) {
+                key[i] = key[i + 1];
+                slot[i] = slot[i + 1];
+            }
+            key[NS - 1] = 0u;
+        }
+    }
+    __syncwarp();
+    id_out = (lane < K) ? win_s[lane] : 0;
+    // gating 2: the sigmoid value itself (shared-expert gate); 3: unit weight
+    return (gating == 3) ? 1.0f : (gating != 2 && renorm > 0.0f) ? __fdiv_rn(my_sel, renorm) : my_sel;
 }
 
 }  // namespace lumen
