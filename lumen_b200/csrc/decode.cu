@@ -11,8 +11,8 @@
 //   gate_up_kernel        per (distinct expert, 16 rows of I): gate and up rows
 //                         times the tokens routed to the expert, SwiGLU
 //                         (cuda/shaders/moe_expert_q4_0.cu:58-108, moe_expert.cu:62-97).
-//                         The general form; Q4_0 layers take gate_up_stream_kernel and the
-//                         other small-batch forms of decode_small.cu.
+//                         The form of the mma.sync prefill path; decode batches take
+//                         gate_up_stream_kernel (decode_small.cu) or the kernel of stream.cu.
 //   down_combine_kernel   per 16 rows of H: down rows of every selected expert
 //                         (moe_expert_q4_0.cu:118-151; integer tensor cores on int8 SwiGLU
 //                         values after gate_up_stream_kernel) and the weighted combine
@@ -33,134 +33,235 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 
 constexpr int RS_THREADS = 512;  // 16 warps: the last CTA gates one token per warp at batches up to 16
 constexpr int RS_WARPS = RS_THREADS / 32;
+constexpr int RS_BLOCKS = RS_THREADS / 8;  // 32-input blocks of the activation operand an operand CTA builds
 
+// Sums v[0..15] over the warp's lanes in 16 shuffles instead of 80: every step halves the values a lane
+// is responsible for. Returns the total of value lane >> 1.
+__device__ __forceinline__ float warp_sum16(float (&v)[16]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16, n = 8; n >= 1; o >>= 1, n >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float keep = up ? v[i + n] : v[i], give = up ? v[i] : v[i + n];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// The tables of the C = T*K <= 256 routed pairs (expert ids in ids_s), by one CTA: stable sort by expert, list of the
+// experts with work and their work records. A pair's column is the number of pairs in front of it, which its
+// threads count directly (a scan over 256 experts was most of the time of this step).
+__device__ __forceinline__ void decode_tables(const RouteDev& R, const int* ids_s, int C, int E, int K, unsigned* mask_s, int* c0_s) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid < MAX_EXPERTS / 32) mask_s[tid] = 0u;
+    __syncthreads();
+    // four threads per pair at up to 128 pairs, two above; each takes every 4th (2nd) quadruple of pairs
+    const int sh = (C <= RS_THREADS / 4) ? 2 : 1, per = 1 << sh, part = tid & (per - 1), p = tid >> sh;
+    const int e = (p < C) ? ids_s[p] : 0;
+    if (p < C && part == 0) atomicOr(&mask_s[e >> 5], 1u << (e & 31));
+    int less = 0, before = 0, same = 0;  // smaller experts; same expert, lower pair; same expert
+    if (p < C) {
+#pragma unroll 2
+        for (int q = part * 4; q < C; q += per * 4) {
+            const int4 v = *reinterpret_cast<const int4*>(&ids_s[q]);  // (padded with ids no expert has)
+            const int x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                less += x[i] < e;
+                same += x[i] == e;
+                before += (x[i] == e) && (q + i < p);
+            }
+        }
+    }
+    for (int o = 1; o < per; o <<= 1) {
+        less += __shfl_xor_sync(0xffffffffu, less, o);
+        same += __shfl_xor_sync(0xffffffffu, same, o);
+        before += __shfl_xor_sync(0xffffffffu, before, o);
+    }
+    __syncthreads();
+    auto rank_of = [&](int ex) {  // experts with work below ex
+        int u = 0;
+#pragma unroll
+        for (int w = 0; w < MAX_EXPERTS / 32; ++w) {
+            const unsigned m = mask_s[w];
+            u += (w < (ex >> 5)) ? __popc(m) : (w == (ex >> 5)) ? __popc(m & ((1u << (ex & 31)) - 1u)) : 0;
+        }
+        return u;
+    };
+    const int U = rank_of(MAX_EXPERTS - 1) + (int)(mask_s[MAX_EXPERTS / 32 - 1] >> 31);
+    if (p < C && part == 0) {
+        const int col = less + before, u = rank_of(e), tok = p / K;
+        R.col_expert[col] = e;
+        R.col_src_tok[col] = tok;
+        R.dst_to_col[p] = col;
+        // source tokens of the expert's first four columns ride in its work record, which a consumer
+        // CTA reads in a single round trip {expert, first column, columns}
+        if (before < 4) reinterpret_cast<int*>(R.work)[8 * u + 4 + before] = tok;
+        if (before == 0) {
+            R.work[2 * u] = make_int4(e, less, same, 0);
+            R.uexp[u] = e;
+            c0_s[u] = less;
+        }
+    }
+    if (tid == 0) *R.n_uexp = U;
+    const int nu_max = (C < E) ? C : E;
+    if (tid >= U && tid < nu_max) R.work[2 * tid] = make_int4(-1, 0, 0, 0);
+    __syncthreads();
+    if (tid <= E) {
+        // bound of expert tid: first column of the next expert with work
+        const int u = (tid < MAX_EXPERTS) ? rank_of(tid) : U;
+        R.expert_bounds[tid] = (u < U) ? c0_s[u] : C;
+    }
+    (void)lane;
+}
+
+// Router of a decode batch. The first CTAs: the logits of an expert row (or two) for all tokens; the CTAs after them: the
+// activation operand (and the normed activations), one token and RS_BLOCKS blocks each; the last
+// CTA to finish (fence + ticket, no spin) routes: one warp per token, then the tables.
+// Bound by the chain of dependent steps, so each of them is as short as it goes: all tokens' inputs of a thread are
+// requested together, the fused RMSNorm needs no pass of its own (a logit is scaled by its token's
+// 1 / rms after the sum, whose squares ride along), sixteen sums cross the warp in 16 shuffles. (One token after
+// the other, with a shared two-term reduction each, this kernel took 25 us at 16 tokens; now ~10.)
+// ROWS: expert rows of a logit CTA: two for 256 experts, so that the CTAs (one per SM: 128 registers a thread) are one wave.
+template <int NS, int ROWS>  // NS * 32 >= E
 __global__ void __launch_bounds__(RS_THREADS)
-router_small_kernel(const __grid_constant__ DecodeArgs a) {
-    __shared__ float red_s[RS_WARPS][DECODE_MAX_TOKENS];
-    __shared__ float scale_s[DECODE_MAX_TOKENS];
-    __shared__ __align__(16) float p_s[RS_WARPS][MAX_EXPERTS];
-    __shared__ __align__(16) float lg_s[RS_WARPS][MAX_EXPERTS];
-    __shared__ int ids_s[DECODE_MAX_TOKENS * MAX_TOP_K];
-    __shared__ int cnt_s[MAX_EXPERTS];
-    __shared__ int cntw_s[DECODE_MAX_TOKENS * MAX_TOP_K / 32][MAX_EXPERTS];
-    __shared__ int bounds_s[MAX_EXPERTS + 1];
-    __shared__ int uidx_s[MAX_EXPERTS];
+router_small_kernel(const __grid_constant__ DecodeArgs a, const int logit_ctas, const int parts) {
+    __shared__ float red_s[ROWS][RS_WARPS][DECODE_MAX_TOKENS], ssq_s[RS_WARPS][DECODE_MAX_TOKENS];
+    __shared__ __align__(16) float p_s[RS_WARPS][NS * 32];
+    __shared__ __align__(16) int ids_s[DECODE_MAX_TOKENS * MAX_TOP_K];
+    __shared__ int c0_s[MAX_EXPERTS];
+    __shared__ unsigned mask_s[MAX_EXPERTS / 32];
     __shared__ int is_last_s;
     __shared__ unsigned long long tab_s[32];
 
     pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int e = blockIdx.x;
     const int H = a.L.H, E = a.L.E, T = a.T, K = a.K;
     const int H4 = H >> 2;
-    const bool want_logits = (a.logits_override == nullptr);
+    const bool is_logit = (int)blockIdx.x < logit_ctas;
+    if (tid < 32) tab_s[tid] = lumen_exact::exp2_tab_entry(tid);
 
-    // Router row in registers before waiting on the previous kernel (weights are static).
-    constexpr int MAXV = 4;  // covers H <= 4096 without re-reading
-    float4 wv[MAXV];
-    const float4* wrow = reinterpret_cast<const float4*>(a.L.router_w + (size_t)e * H);
+    if (is_logit) {
+        const int e0 = blockIdx.x * ROWS;
+        const float4* wrow[ROWS];
+        float4 w4[ROWS];
+        // first part of the router rows in registers before waiting on the previous kernel (weights are static)
 #pragma unroll
-    for (int j = 0; j < MAXV; ++j) {
-        const int i4 = tid + j * RS_THREADS;
-        wv[j] = (want_logits && i4 < H4) ? __ldg(wrow + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    pdl_wait();
-
-    // fused FFN RMSNorm scale per token
-    if (a.gamma != nullptr) {
-        for (int t = 0; t < T; ++t) {
-            const float4* xr = reinterpret_cast<const float4*>(a.x + (size_t)t * H);
+        for (int r = 0; r < ROWS; ++r) {
+            wrow[r] = reinterpret_cast<const float4*>(a.L.router_w + (size_t)min(e0 + r, E - 1) * H);
+            w4[r] = (tid < H4) ? __ldg(wrow[r] + tid) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        pdl_wait();
+        float acc[ROWS][DECODE_MAX_TOKENS], sq[DECODE_MAX_TOKENS];
+#pragma unroll
+        for (int t = 0; t < DECODE_MAX_TOKENS; ++t) {
+            sq[t] = 0.0f;
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) acc[r][t] = 0.0f;
+        }
+#pragma unroll 1
+        for (int i4 = tid; i4 < H4; i4 += RS_THREADS) {
+            if (i4 != tid) {
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) w4[r] = __ldg(wrow[r] + i4);
+            }
+            if (a.gamma != nullptr) {
+                const float4 g = __ldg(reinterpret_cast<const float4*>(a.gamma) + i4);
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) w4[r] = make_float4(w4[r].x * g.x, w4[r].y * g.y, w4[r].z * g.z, w4[r].w * g.w);
+            }
+            constexpr int TB = DECODE_MAX_TOKENS / ROWS;  // tokens whose inputs are in flight together
+#pragma unroll
+            for (int t0 = 0; t0 < DECODE_MAX_TOKENS; t0 += TB) {
+                float4 xv[TB];
+#pragma unroll
+                for (int t = 0; t < TB; ++t)
+                    if (t0 + t < T) xv[t] = reinterpret_cast<const float4*>(a.x + (size_t)(t0 + t) * H)[i4];
+#pragma unroll
+                for (int t = 0; t < TB; ++t)
+                    if (t0 + t < T) {
+#pragma unroll
+                        for (int r = 0; r < ROWS; ++r)
+                            acc[r][t0 + t] += w4[r].x * xv[t].x + w4[r].y * xv[t].y + w4[r].z * xv[t].z + w4[r].w * xv[t].w;
+                        if (a.gamma != nullptr)
+                            sq[t0 + t] += xv[t].x * xv[t].x + xv[t].y * xv[t].y + xv[t].z * xv[t].z + xv[t].w * xv[t].w;
+                    }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const float v = warp_sum16(acc[r]);
+            if ((lane & 1) == 0) red_s[r][warp][lane >> 1] = v;
+        }
+        if (a.gamma != nullptr) {
+            const float q = warp_sum16(sq);
+            if ((lane & 1) == 0) ssq_s[warp][lane >> 1] = q;
+        }
+        __syncthreads();
+        const int tt = tid & (DECODE_MAX_TOKENS - 1), rr = tid / DECODE_MAX_TOKENS;
+        if (rr < ROWS && tt < T && e0 + rr < E) {
+            float sum = 0.0f, ss = 0.0f;
+#pragma unroll
+            for (int w = 0; w < RS_WARPS; ++w) sum += red_s[rr][w][tt];
+            if (a.gamma != nullptr) {
+#pragma unroll
+                for (int w = 0; w < RS_WARPS; ++w) ss += ssq_s[w][tt];
+                sum *= 1.0f / sqrtf(ss / (float)H + a.eps);
+            }
+            a.R.logits[(size_t)tt * E + e0 + rr] = sum;
+        }
+    } else if (parts > 0) {
+        // activation operand of the gate/up kernel (and the normed output of the fused-norm entry
+        // point): two-term int8 blocks for Q4_0 weights, 16-bit hi + lo fragments otherwise
+        const int o = blockIdx.x - logit_ctas, t = o / parts, b = (o - t * parts) * RS_BLOCKS + (tid >> 3);
+        const int nblk = H >> 5, nblk_pad = a.L.kg_h * 4, sub = tid & 7;
+        const float4* xr = reinterpret_cast<const float4*>(a.x + (size_t)t * H);
+        pdl_wait();
+        float scale = 1.0f;
+        if (a.gamma != nullptr) {
             float ss = 0.0f;
             for (int i4 = tid; i4 < H4; i4 += RS_THREADS) {
                 const float4 v = xr[i4];
                 ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
             }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            if (lane == 0) red_s[warp][t] = ss;
-        }
-        __syncthreads();
-        if (tid < T) {
-            float ss = 0.0f;
-            for (int w = 0; w < RS_WARPS; ++w) ss += red_s[w][tid];
-            scale_s[tid] = 1.0f / sqrtf(ss / (float)H + a.eps);
-        }
-        __syncthreads();
-    }
-    auto load_x4 = [&](int t, int i4) -> float4 {
-        float4 v = reinterpret_cast<const float4*>(a.x + (size_t)t * H)[i4];
-        if (a.gamma != nullptr) {
-            const float4 g = __ldg(reinterpret_cast<const float4*>(a.gamma) + i4);
-            const float sc = scale_s[t];
-            v.x = v.x * sc * g.x;
-            v.y = v.y * sc * g.y;
-            v.z = v.z * sc * g.z;
-            v.w = v.w * sc * g.w;
-        }
-        return v;
-    };
-
-    // logits for this expert row, all tokens (token loop rolled: the code of this kernel runs
-    // once per launch, so its size is paid in instruction fetches)
-    if (want_logits) {
-#pragma unroll 4
-        for (int t = 0; t < T; ++t) {
-            float acc = 0.0f;
+            for (int k = 16; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
+            if (lane == 0) ssq_s[warp][0] = ss;
+            __syncthreads();
+            ss = 0.0f;
 #pragma unroll
-            for (int j = 0; j < MAXV; ++j) {
-                const int i4 = tid + j * RS_THREADS;
-                if (i4 < H4) {
-                    const float4 xv = load_x4(t, i4);
-                    acc += wv[j].x * xv.x + wv[j].y * xv.y + wv[j].z * xv.z + wv[j].w * xv.w;
-                }
+            for (int w = 0; w < RS_WARPS; ++w) ss += ssq_s[w][0];
+            scale = 1.0f / sqrtf(ss / (float)H + a.eps);
+        }
+        auto load_x4 = [&](int i4) -> float4 {
+            float4 v = xr[i4];
+            if (a.gamma != nullptr) {
+                const float4 g = __ldg(reinterpret_cast<const float4*>(a.gamma) + i4);
+                v.x = v.x * scale * g.x;
+                v.y = v.y * scale * g.y;
+                v.z = v.z * scale * g.z;
+                v.w = v.w * scale * g.w;
             }
-#pragma unroll 1
-            for (int i4 = tid + MAXV * RS_THREADS; i4 < H4; i4 += RS_THREADS) {  // H > 4096
-                const float4 w4 = __ldg(wrow + i4);
-                const float4 xv = load_x4(t, i4);
-                acc += w4.x * xv.x + w4.y * xv.y + w4.z * xv.z + w4.w * xv.w;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) red_s[warp][t] = acc;
-        }
-        __syncthreads();
-        if (tid < T) {
-            float v = 0.0f;
-            for (int w = 0; w < RS_WARPS; ++w) v += red_s[w][tid];
-            a.R.logits[(size_t)tid * E + e] = v;
-        }
-    }
-
-    // activation operand of the gate/up kernel (and the normed output of the fused-norm entry
-    // point): two-term int8 blocks for Q4_0 weights, f16 hi+lo fragments otherwise
-    if (a.xq != nullptr) {
-        const int nblk = H >> 5, nblk_pad = a.L.kg_h * 4;
-        const int sub = tid & 7;
-        const int xq_tok = dcommon::xq_tok_words(nblk_pad);
-        for (int item = blockIdx.x * (RS_THREADS / 8) + (tid >> 3); item < T * nblk;
-             item += gridDim.x * (RS_THREADS / 8)) {
-            const int t = item / nblk, b = item - t * nblk;
-            const float4 v = load_x4(t, b * 8 + sub);
-            dcommon::build_xq_block(v, sub, lane, a.xq + (size_t)t * xq_tok, nblk_pad, b);
-            if (a.gamma != nullptr && a.normed_out != nullptr)
-                reinterpret_cast<float4*>(a.normed_out + (size_t)t * H)[b * 8 + sub] = v;
-        }
-    } else if (a.xf != nullptr) {
-        const int nblk = H >> 5, nblk_pad = a.L.kg_h * 4;
-        const bool bf16_mode = (a.L.quant == BF16);
-        const int sub = tid & 7, hl = sub >> 2, t4 = sub & 3;
-        for (int item = blockIdx.x * (RS_THREADS / 8) + (tid >> 3); item < T * nblk;
-             item += gridDim.x * (RS_THREADS / 8)) {
-            const int t = item / nblk, b = item - t * nblk;
-            const float4 lo4 = load_x4(t, b * 8 + t4);
-            const float4 hi4 = load_x4(t, b * 8 + 4 + t4);
-            a.xf[((size_t)(t * 2 + hl) * nblk_pad + b) * 4 + t4] = make_act_frag(lo4, hi4, hl, bf16_mode);
-            if (a.gamma != nullptr && a.normed_out != nullptr) {
-                float4* o = reinterpret_cast<float4*>(a.normed_out + (size_t)t * H);
-                o[b * 8 + (hl ? 4 : 0) + t4] = hl ? hi4 : lo4;
+            return v;
+        };
+        if (b < nblk) {  // (the eight lanes of a block agree)
+            float4* normed = (a.gamma != nullptr && a.normed_out != nullptr) ? reinterpret_cast<float4*>(a.normed_out + (size_t)t * H) : nullptr;
+            if (a.xq != nullptr) {
+                const float4 v = load_x4(b * 8 + sub);
+                dcommon::build_xq_block(v, sub, lane, a.xq + (size_t)t * dcommon::xq_tok_words(nblk_pad), nblk_pad, b);
+                if (normed) normed[b * 8 + sub] = v;
+            } else {
+                const int hl = sub >> 2, t4 = sub & 3;
+                const float4 lo4 = load_x4(b * 8 + t4), hi4 = load_x4(b * 8 + 4 + t4);
+                a.xf[((size_t)(t * 2 + hl) * nblk_pad + b) * 4 + t4] = make_act_frag(lo4, hi4, hl, a.L.quant == BF16);
+                if (normed) normed[b * 8 + (hl ? 4 : 0) + t4] = hl ? hi4 : lo4;
             }
         }
+    } else {
+        pdl_wait();  // (logits supplied, no operand wanted: this CTA only routes)
     }
 
     // last-CTA election: the CTA barrier orders every thread's stores before
@@ -175,112 +276,23 @@ router_small_kernel(const __grid_constant__ DecodeArgs a) {
     __syncthreads();
     if (!is_last_s) return;
 
-    const float* lg = want_logits ? a.R.logits : a.logits_override;
-    if (tid < 32) tab_s[tid] = lumen_exact::exp2_tab_entry(tid);
+    const float* lg = (a.logits_override == nullptr) ? a.R.logits : a.logits_override;
+    if (tid < DECODE_MAX_TOKENS * MAX_TOP_K) ids_s[tid] = 0x7fffffff;  // padding: an id no expert has
     __syncthreads();
-    // The exact exps are the long part: the 16 warps share a token's exps 4-, 2- or 1-way
-    // (consecutive warps form a token's group), then the group's first warp selects.
-    {
-        const int nsub = (T <= 4) ? 4 : (T <= 8) ? 2 : 1;
-        const int t = warp / nsub, sub = warp - t * nsub;
-        if (t < T) {
-            for (int i = lane; i < E; i += 32) lg_s[warp][i] = __ldcg(lg + (size_t)t * E + i);
-            __syncwarp();
-            float* p = p_s[warp - sub];
-            warp_gate_probs(lg_s[warp], E, a.gating, p, tab_s, sub, nsub);
-            if (nsub > 1) asm volatile("bar.sync %0, %1;" ::"r"(1 + t), "r"(nsub * 32) : "memory");
-            else __syncwarp();
-            if (sub == 0) {
-                warp_select(p, E, K, a.gating, a.R.ids + (size_t)t * K, a.R.weights + (size_t)t * K);
-                if (lane < K) ids_s[t * K + lane] = (int)a.R.ids[(size_t)t * K + lane];
-            }
-        }
-    }
-    __syncthreads();
-    // Stable counting sort of the C = T*K <= 128 pairs by expert, one pair per thread: pairs
-    // of one warp that share an expert rank themselves with a match, and a small table of
-    // per-warp counts orders the warps; no loop over the pairs anywhere.
-    const int C = T * K;
-    const int npw = (C + 31) >> 5;
-    for (int i = tid; i < npw * E; i += RS_THREADS) cntw_s[i / E][i % E] = 0;
-    __syncthreads();
-    int my_e = -1, my_rank = 0;
-    if (warp < npw) {
-        const int p = warp * 32 + lane;
-        my_e = (p < C) ? ids_s[p] : -1 - lane;  // padding lanes match nobody
-        const unsigned same = __match_any_sync(0xffffffffu, my_e);
-        my_rank = __popc(same & ((1u << lane) - 1u));
-        if (p < C && my_rank == 0) cntw_s[warp][my_e] = __popc(same);
-    }
-    __syncthreads();
-    if (tid < E) {
-        int c = 0;
-        for (int w = 0; w < npw; ++w) c += cntw_s[w][tid];
-        cnt_s[tid] = c;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        // exclusive scan over experts, 8 per lane (E <= 256), and the ascending
-        // list of experts that received at least one token
-        int local[8], lsum = 0, lnz = 0;
+    if (warp < T) {
+        float v[NS];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int ee = lane * 8 + j;
-            local[j] = (ee < E) ? cnt_s[ee] : 0;
-            lsum += local[j];
-            lnz += (local[j] > 0);
-        }
-        int isum = lsum, inz = lnz;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v1 = __shfl_up_sync(0xffffffffu, isum, o);
-            const int v2 = __shfl_up_sync(0xffffffffu, inz, o);
-            if (lane >= o) {
-                isum += v1;
-                inz += v2;
-            }
-        }
-        int run = isum - lsum, unz = inz - lnz;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int ee = lane * 8 + j;
-            if (ee < E) {
-                bounds_s[ee] = run;
-                a.R.expert_bounds[ee] = run;
-                uidx_s[ee] = -1;
-                if (local[j] > 0) {
-                    // work descriptor of the unz-th expert with work: one 32-byte record that a
-                    // consumer CTA reads in a single round trip {expert, first column, columns}
-                    a.R.work[2 * unz] = make_int4(ee, run, local[j], 0);
-                    uidx_s[ee] = unz;
-                    a.R.uexp[unz++] = ee;
-                }
-                run += local[j];
-            }
-        }
-        const int total_u = __shfl_sync(0xffffffffu, inz, 31);
-        const int nu_max = (C < E) ? C : E;
-        for (int uu = total_u + lane; uu < nu_max; uu += 32) a.R.work[2 * uu] = make_int4(-1, 0, 0, 0);
-        if (lane == 31) {
-            bounds_s[E] = isum;
-            a.R.expert_bounds[E] = isum;
-            *a.R.n_uexp = inz;
+        for (int i = 0; i < NS; ++i) v[i] = (lane + 32 * i < E) ? __ldcg(lg + (size_t)warp * E + lane + 32 * i) : -INFINITY;
+        int id;
+        const float w = warp_route<NS>(v, E, K, a.gating, p_s[warp], reinterpret_cast<const uint64_t*>(tab_s), id);
+        if (lane < K) {
+            a.R.ids[(size_t)warp * K + lane] = (uint32_t)id;
+            a.R.weights[(size_t)warp * K + lane] = w;
+            ids_s[warp * K + lane] = id;
         }
     }
     __syncthreads();
-    if (warp < npw) {
-        const int p = warp * 32 + lane;
-        if (p < C) {
-            int before = my_rank;  // same expert, lower pair index
-            for (int w = 0; w < warp; ++w) before += cntw_s[w][my_e];
-            const int col = bounds_s[my_e] + before;
-            a.R.col_expert[col] = my_e;
-            a.R.col_src_tok[col] = p / K;
-            a.R.dst_to_col[p] = col;
-            // source tokens of the expert's first four columns ride in its work record
-            if (before < 4) reinterpret_cast<int*>(a.R.work)[8 * uidx_s[my_e] + 4 + before] = p / K;
-        }
-    }
+    decode_tables(a.R, ids_s, T * K, E, K, mask_s, c0_s);
     if (tid == 0) *a.R.ticket = 0u;
 }
 
@@ -450,265 +462,6 @@ gate_up_kernel(const __grid_constant__ DecodeArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// down + weighted combine (decode: every expert has at most 16 columns)
-// ---------------------------------------------------------------------------
-constexpr int DC_THREADS = 512;
-constexpr int DC_WARPS = DC_THREADS / 32;
-constexpr int DC_MAX_COLS = DECODE_MAX_TOKENS * MAX_TOP_K;
-
-template <int Q>
-struct DcRing {  // weight tiles in flight per warp
-    static constexpr int value = (Q == Q4_0) ? 6 : (Q == Q8_0) ? 4 : 3;
-};
-
-__device__ __forceinline__ void cp_async16_dc(void* smem_dst, const void* gsrc) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
-}
-
-// I8 (Q4_0 only): the SwiGLU outputs arrive as two-term int8 blocks (a.sq, written by
-// gate_up_stream_kernel) and the products run on the integer tensor cores, raw nibbles against
-// int8, as in the gate/up kernels: ~20 instead of ~33 instructions per 32-input block.
-template <int Q, bool I8 = false>
-__global__ void __launch_bounds__(DC_THREADS)
-down_combine_kernel(const __grid_constant__ DecodeArgs a) {
-    __shared__ float dsm[DC_MAX_COLS][16];
-    __shared__ int exp_s[MAX_EXPERTS], c0_s[MAX_EXPERTS], nc_s[MAX_EXPERTS];
-    // The routing tables come from the router kernel, which had completed before the gate/up kernel
-    // (the immediate predecessor) released this launch: they are read, and the first weight tiles
-    // they determine requested, before waiting for gate/up.
-    pdl_trigger();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int gq = lane >> 2, t4 = lane & 3;
-    const int rt = blockIdx.x;
-    const int U = *a.R.n_uexp;
-    const int kg_i = a.L.kg_i, H = a.L.H, K = a.K, T = a.T;
-    const int nblk_i_pad = kg_i * 4;
-    // expert id, first column and column count of every expert with work, once per CTA: the
-    // per-item lookups below then stay out of the chain of dependent global loads
-    for (int u = tid; u < U; u += DC_THREADS) {
-        const int ee = a.R.uexp[u];
-        const int b0 = a.R.expert_bounds[ee];
-        exp_s[u] = ee;
-        c0_s[u] = b0;
-        nc_s[u] = min(16, a.R.expert_bounds[ee + 1] - b0);
-    }
-    __syncthreads();
-
-    // flattened (expert, k-group) items of this warp; a ring of DC_RING tiles per warp is kept
-    // in flight with cp.async (one commit group per item, empty past the end), so that the
-    // bytes in flight per SM cover the HBM latency
-    extern __shared__ uint4 dc_ring[];  // [DC_WARPS][DC_RING][NQ * 32 + 8]
-    constexpr int NQ32 = QTraits<Q>::NQ * 32, TU4 = NQ32 + 8;
-    uint4* my_ring = dc_ring + (size_t)warp * DcRing<Q>::value * TU4;
-    const int n_exp_w = (U > warp) ? (U - warp + DC_WARPS - 1) / DC_WARPS : 0;
-    const int nitems = n_exp_w * kg_i;
-    // (expert slot, k-group) of the next item to request / to prefetch activations for / to multiply:
-    // three cursors stepped by one item, no division in the loop
-    int is_u = warp, is_kg = 0, is_slot = 0;
-    const uint4 *is_q = nullptr, *is_s = nullptr;  // this lane's source words of the next item
-    auto issue = [&]() {
-        if (is_u < U) {
-            if (is_kg == 0) {
-                const int ee = exp_s[is_u];
-                is_q = a.L.down_q(ee) + (size_t)rt * kg_i * NQ32 + lane;
-                is_s = a.L.down_s(ee) + (size_t)rt * kg_i * 8 + lane;
-            }
-            uint4* slot = my_ring + (size_t)is_slot * TU4;
-#pragma unroll
-            for (int j = 0; j < QTraits<Q>::NQ; ++j) cp_async16_dc(slot + j * 32 + lane, is_q + j * 32);
-            if (Q != BF16 && lane < 8) cp_async16_dc(slot + NQ32 + lane, is_s);
-            is_q += NQ32;
-            is_s += 8;
-            if (++is_kg == kg_i) {
-                is_kg = 0;
-                is_u += DC_WARPS;
-            }
-        }
-        if (++is_slot == DcRing<Q>::value) is_slot = 0;
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-#pragma unroll 1
-    for (int i = 0; i < DcRing<Q>::value; ++i) issue();
-    pdl_wait();  // the SwiGLU outputs are final from here on
-    float acc[4][4];
-    int c0 = 0, ncol = 0, ng = 0;
-    // activation fragments of the first column group (an expert rarely has more than four columns
-    // here) are fetched one item ahead, so that their L2 latency is not paid tile by tile
-    const int sq_term = dcommon::xq_term_words(nblk_i_pad), sq_tok = dcommon::xq_tok_words(nblk_i_pad);
-    // B operand of block b of item (expert slot u_slot, k-group kgx), column group g. f16 form: the
-    // lane's fragment of the hi / lo plane of its column. Int8 form: {word pair of the lane's
-    // column and term, {sx, 8 sx sum q} of the column of the lane's accumulators}.
-    auto load_b = [&](int u_slot, int kgx, int g, int b) -> uint4 {
-        const int ncu = nc_s[u_slot], c0u = c0_s[u_slot];
-        const int colr = 4 * g + (gq >> 1);
-        if (I8) {
-            const int cols = 4 * g + t4;
-            uint2 w = make_uint2(0u, 0u);
-            if (colr < ncu)
-                w = __ldg(reinterpret_cast<const uint2*>(a.sq + (size_t)(c0u + colr) * sq_tok + (gq & 1) * sq_term +
-                                                         (size_t)(kgx * 4 + b) * 8 + t4 * 2));
-            const float2 sc = __ldg(reinterpret_cast<const float2*>(a.sq + (size_t)(c0u + (cols < ncu ? cols : 0)) * sq_tok +
-                                                                    2 * sq_term) + kgx * 4 + b);
-            return make_uint4(w.x, w.y, __float_as_uint(sc.x), __float_as_uint(sc.y));
-        }
-        if (colr >= ncu) return make_uint4(0u, 0u, 0u, 0u);
-        return ldg_cached(a.sf + ((size_t)((c0u + colr) * 2 + (gq & 1)) * nblk_i_pad) * 4 + t4 + (size_t)kgx * 16 + b * 4);
-    };
-    // group 0 of the next item: running pointers, recomputed when the expert changes (null = no column)
-    int pb_u = warp, pb_kg = 0;
-    const unsigned* pb_w = nullptr;  // int8 form: word pairs of the lane's column and term | f16 form: fragments
-    const float2* pb_s = nullptr;    // int8 form: scales of the column of the lane's accumulators
-    uint4 bnx[4];
-    auto b0_next = [&]() {
-        if (pb_u < U) {
-            if (pb_kg == 0) {
-                const int ncu = nc_s[pb_u], c0u = c0_s[pb_u];
-                const int colr = gq >> 1;
-                if (I8) {
-                    pb_w = (colr < ncu) ? a.sq + (size_t)(c0u + colr) * sq_tok + (gq & 1) * sq_term + t4 * 2 : nullptr;
-                    pb_s = reinterpret_cast<const float2*>(a.sq + (size_t)(c0u + (t4 < ncu ? t4 : 0)) * sq_tok + 2 * sq_term);
-                } else {
-                    pb_w = (colr < ncu) ? reinterpret_cast<const unsigned*>(
-                                              a.sf + ((size_t)((c0u + colr) * 2 + (gq & 1)) * nblk_i_pad) * 4 + t4)
-                                        : nullptr;
-                }
-            }
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                if (I8) {
-                    const uint2 w = pb_w ? __ldg(reinterpret_cast<const uint2*>(pb_w) + b * 4) : make_uint2(0u, 0u);
-                    const float2 sc = __ldg(pb_s + b);
-                    bnx[b] = make_uint4(w.x, w.y, __float_as_uint(sc.x), __float_as_uint(sc.y));
-                } else {
-                    bnx[b] = pb_w ? ldg_cached(reinterpret_cast<const uint4*>(pb_w) + b * 4) : make_uint4(0u, 0u, 0u, 0u);
-                }
-            }
-            if (pb_w) pb_w += I8 ? 32 : 64;  // one k-group on: 4 blocks x 8 words | 16 uint4
-            pb_s += 4;
-            if (++pb_kg == kg_i) {
-                pb_kg = 0;
-                pb_u += DC_WARPS;
-            }
-        } else {
-#pragma unroll
-            for (int b = 0; b < 4; ++b) bnx[b] = make_uint4(0u, 0u, 0u, 0u);
-        }
-    };
-    b0_next();
-    int uu = warp - DC_WARPS, kg = kg_i - 1, rslot = 0;
-#pragma unroll 1
-    for (int n = 0; n < nitems; ++n) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(DcRing<Q>::value - 1) : "memory");
-        __syncwarp();
-        WTile<Q> cur;
-        {
-            const uint4* slot = my_ring + (size_t)rslot * TU4;
-#pragma unroll
-            for (int j = 0; j < QTraits<Q>::NQ; ++j) cur.q[j] = slot[j * 32 + lane];
-            if (Q != BF16) cur.s = slot[NQ32 + (lane >> 2)];
-            if (++rslot == DcRing<Q>::value) rslot = 0;
-        }
-        __syncwarp();
-        issue();  // refill the slot just read
-        uint4 bcur[4];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) bcur[b] = bnx[b];
-        b0_next();
-        if (++kg == kg_i) {
-            kg = 0;
-            uu += DC_WARPS;
-        }
-        if (kg == 0) {
-            c0 = c0_s[uu];
-            ncol = nc_s[uu];
-            ng = (ncol + 3) >> 2;
-#pragma unroll
-            for (int g = 0; g < 4; ++g)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[g][i] = 0.0f;
-        }
-        // Group 0 from the prefetched registers, further groups fetched in place. An expert with more
-        // than four columns is rare in a decode batch, so the one-group case gets code of its own:
-        // in the four-group form the compiler predicates the other groups' bodies instead of
-        // branching around them, and a tile then costs ~400 issued instructions instead of ~150.
-        auto tile_blocks = [&](auto ng_tag) {
-            constexpr int NG = decltype(ng_tag)::value;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const float2 sc = block_scales<Q>(cur, b);
-                if (I8) {
-                    const uint4 qv = cur.q[(b >> 1) % QTraits<Q>::NQ];
-                    const unsigned w0 = (b & 1) ? qv.z : qv.x, w8 = (b & 1) ? qv.w : qv.y;
-                    const unsigned a0 = w0 & 0x0F0F0F0Fu, a1 = w8 & 0x0F0F0F0Fu;
-                    const unsigned a2 = (w0 >> 4) & 0x0F0F0F0Fu, a3 = (w8 >> 4) & 0x0F0F0F0Fu;
-#pragma unroll
-                    for (int g = 0; g < NG; ++g) {
-                        if (g == 0 || g < ng) {
-                            const uint4 bf = (g == 0) ? bcur[b] : load_b(uu, kg, g, b);
-                            int c[4] = {0, 0, 0, 0};
-                            dcommon::mma_u8s8(c, a0, a1, a2, a3, bf.x, bf.y);
-                            const float sx = __uint_as_float(bf.z), off = __uint_as_float(bf.w);
-                            const float k1 = 1.0f / 254.0f;
-                            acc[g][0] = fmaf(sc.x, fmaf(sx, fmaf((float)c[1], k1, (float)c[0]), -off), acc[g][0]);
-                            acc[g][2] = fmaf(sc.y, fmaf(sx, fmaf((float)c[3], k1, (float)c[2]), -off), acc[g][2]);
-                        }
-                    }
-                } else {
-                    uint32_t a_lo[4], a_hi[4];
-                    unpack_block<Q>(cur, b, a_lo, a_hi);
-#pragma unroll
-                    for (int g = 0; g < NG; ++g) {
-                        if (g == 0 || g < ng) {
-                            const uint4 bf = (g == 0) ? bcur[b] : load_b(uu, kg, g, b);
-                            float c[4] = {0.f, 0.f, 0.f, 0.f};
-                            if (Q == BF16) {
-                                mma_bf16(c, a_lo, bf.x, bf.y);
-                                mma_bf16(c, a_hi, bf.z, bf.w);
-                            } else {
-                                mma_f16(c, a_lo, bf.x, bf.y);
-                                mma_f16(c, a_hi, bf.z, bf.w);
-                            }
-                            acc[g][0] = fmaf(sc.x, c[0], acc[g][0]);
-                            acc[g][1] = fmaf(sc.x, c[1], acc[g][1]);
-                            acc[g][2] = fmaf(sc.y, c[2], acc[g][2]);
-                            acc[g][3] = fmaf(sc.y, c[3], acc[g][3]);
-                        }
-                    }
-                }
-            }
-        };
-        if (ng <= 1) tile_blocks(std::integral_constant<int, 1>{});
-        else tile_blocks(std::integral_constant<int, 4>{});
-        if (kg == kg_i - 1) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                const int tokc = 4 * g + t4;
-                if (tokc < ncol) {
-                    dsm[c0 + tokc][gq] = acc[g][0] + acc[g][1];
-                    dsm[c0 + tokc][gq + 8] = acc[g][2] + acc[g][3];
-                }
-            }
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    {
-        const int row = tid & 15, t = tid >> 4;
-        if (t < T) {
-            const size_t o = (size_t)t * H + rt * 16 + row;
-            float accv = a.residual[o];
-            for (int slot = 0; slot < K; ++slot) {
-                const int col = a.R.dst_to_col[t * K + slot];
-                const float w = a.R.weights[t * K + slot];
-                accv = __fadd_rn(accv, __fmul_rn(w, dsm[col][row]));
-            }
-            a.out[o] = accv;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // down projection for any number of columns per expert (mma.sync grouped path of
 // the prefill entry point): one CTA per (16 rows of H, expert), k-groups split
 // across warps, output f16 by compact column for the scatter-accumulate.
@@ -792,77 +545,30 @@ cudaError_t launch_grouped_mma(const DecodeArgs& a, __half* d16, cudaStream_t st
 // ---------------------------------------------------------------------------
 // launch
 // ---------------------------------------------------------------------------
-template <typename Kern>
-static cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, cudaStream_t st, const DecodeArgs& a) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    count_launch();
-    return cudaLaunchKernelEx(&cfg, kern, a);
-}
-
-template <int Q, bool I8 = false>
-static cudaError_t launch_down_combine(const DecodeArgs& a, dim3 grid, cudaStream_t st) {
-    const size_t smem = (size_t)DC_WARPS * DcRing<Q>::value * (QTraits<Q>::NQ * 32 + 8) * 16;
-    static SmemOptIn optin;
-    {
-        cudaError_t e = ensure_dyn_smem(down_combine_kernel<Q, I8>, smem, optin);
-        if (e != cudaSuccess) return e;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(DC_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    count_launch();
-    return cudaLaunchKernelEx(&cfg, down_combine_kernel<Q, I8>, a);
-}
-
 cudaError_t launch_route_small(const DecodeArgs& a, cudaStream_t st) {
-    return launch_pdl(router_small_kernel, dim3(a.L.E), dim3(RS_THREADS), st, a);
+    const int rows = (a.L.E > 128) ? 2 : 1;
+    const int logit_ctas = (a.logits_override == nullptr) ? (a.L.E + rows - 1) / rows : 0;
+    const int parts = (a.xq != nullptr || a.xf != nullptr) ? (a.L.H / 32 + RS_BLOCKS - 1) / RS_BLOCKS : 0;
+    const int grid = logit_ctas + a.T * parts;
+    count_launch();
+    auto go = [&](auto kern) {
+        return launch_dep(kern, dim3(grid > 0 ? grid : 1), dim3(RS_THREADS), 0, st, a, logit_ctas, parts);
+    };
+    return (a.L.E <= 32) ? go(router_small_kernel<1, 1>) : (a.L.E <= 128) ? go(router_small_kernel<4, 1>) : go(router_small_kernel<8, 2>);
 }
 
-bool decode_small_applicable(const DecodeArgs& a, int phase);
 bool decode_stream_applicable(const DecodeArgs& a);
-cudaError_t launch_decode_small_phase(const DecodeArgs& a, int phase, cudaStream_t st);
+cudaError_t launch_gate_up_stream(const DecodeArgs& a, cudaStream_t st);
 
 cudaError_t launch_decode_phase(const DecodeArgs& a_in, int phase, cudaStream_t st) {
-    // the int8 activation form belongs to the Q4_0 gate/up kernel that walks columns four at a time
     DecodeArgs a = a_in;
-    if (!(a.xq != nullptr && a.xf != nullptr && a.L.quant == Q4_0 && decode_small_applicable(a, 1))) a.xq = nullptr;
-    // 5..16 tokens, Q4_0: streaming gate/up that hands the down product int8 activations
-    const bool stream = decode_stream_applicable(a);
-    if (!stream) a.sq = nullptr;
+    // Q4_0 layers that gate_up_stream_kernel takes: int8 activations for both products; every other format and shape:
+    // hi + lo fragments and the general streaming kernel
+    const bool int8 = decode_stream_applicable(a);
+    if (!int8) a.xq = a.sq = nullptr;
     if (phase == 0) return launch_route_small(a, st);
-    if (stream && phase == 2) return launch_down_combine<Q4_0, true>(a, dim3(a.L.rt_h), st);  // consumes the int8 SwiGLU values
-    if (decode_small_applicable(a, phase)) return launch_decode_small_phase(a, phase, st);
-    const int C = a.T * a.K;
-    const int nu = C < a.L.E ? C : a.L.E;
-    const dim3 g_gu(a.L.rt_i, nu), g_dc(a.L.rt_h);
-    if (phase == 1) {
-        switch (a.L.quant) {
-            case Q4_0: return launch_pdl(gate_up_kernel<Q4_0>, g_gu, dim3(GU_THREADS), st, a);
-            case Q8_0: return launch_pdl(gate_up_kernel<Q8_0>, g_gu, dim3(GU_THREADS), st, a);
-            default: return launch_pdl(gate_up_kernel<BF16>, g_gu, dim3(GU_THREADS), st, a);
-        }
-    }
-    switch (a.L.quant) {
-        case Q4_0: return launch_down_combine<Q4_0>(a, g_dc, st);
-        case Q8_0: return launch_down_combine<Q8_0>(a, g_dc, st);
-        default: return launch_down_combine<BF16>(a, g_dc, st);
-    }
+    if (phase == 1) return int8 ? launch_gate_up_stream(a, st) : launch_stream_gate_up(a, st);
+    return launch_stream_down(a, int8, st);
 }
 
 bool decode_fused_applicable(const DecodeArgs& a);

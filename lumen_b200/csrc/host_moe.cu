@@ -147,12 +147,12 @@ Status build_repacked(const CudaMoeScratch& sc, const void* layer_buf, size_t bl
 }
 
 static size_t tok_arena_bytes(const CudaMoeScratch& s, int cap, size_t* offs) {
-    // order: logits, ids, weights, col_expert, col_src_tok, dst_to_col, blk_hist, tiles, s16, d16, x16, xf, sf, w16, xq, xr16, rpart, sq
+    // order: logits, ids, weights, col_expert, col_src_tok, dst_to_col, blk_hist, tiles, s16, d16, x16, xf, sf, w16, xq, xr16, rpart, sq, d32
     const size_t C = (size_t)cap * s.K;
     const size_t nblk_h_pad = (size_t)((s.H / 32 + 3) / 4) * 4, nblk_i_pad = (size_t)((s.I / 32 + 3) / 4) * 4;
     const size_t max_ct = C / 128 + s.E, max_ct_dn = C / 128 + s.E;  // gate/up tiles of 128 or 256 columns (sized for 128), down tiles of 128
     const size_t n_tile_entries = max_ct * ((size_t)s.I / 128 + 1) + max_ct_dn * ((size_t)s.H / 256 + 1);
-    size_t sizes[18] = {
+    size_t sizes[19] = {
         (size_t)cap * s.E * 4, C * 4, C * 4, C * 4, C * 4, C * 4,
         (size_t)((cap + 7) / 8) * s.E * 4,  // one histogram per chunk of 8 tokens (SORT_TOK in route_large.cu)
         n_tile_entries * sizeof(int4),
@@ -162,9 +162,10 @@ static size_t tok_arena_bytes(const CudaMoeScratch& s, int cap, size_t* offs) {
         (size_t)DECODE_MAX_TOKENS * (18 * nblk_h_pad + 16) * 4,  // xq_tok_words(nblk_h_pad) words per token
         (size_t)cap * s.H * 2 * 2,
         (size_t)ROUTER_TC_MAX_KSPLIT * cap * s.E * 4,
-        (size_t)DECODE_MAX_TOKENS * s.K * (18 * nblk_i_pad + 16) * 4};  // xq_tok_words(nblk_i_pad) words per decode column
+        (size_t)DECODE_MAX_TOKENS * s.K * (18 * nblk_i_pad + 16) * 4,  // xq_tok_words(nblk_i_pad) words per decode column
+        (size_t)DECODE_MAX_TOKENS * s.K * s.H * 4};
     size_t off = 0;
-    for (int i = 0; i < 18; ++i) {
+    for (int i = 0; i < 19; ++i) {
         offs[i] = off;
         off += align_up(sizes[i], 256);
     }
@@ -172,7 +173,7 @@ static size_t tok_arena_bytes(const CudaMoeScratch& s, int cap, size_t* offs) {
 }
 
 static Status alloc_tok_arena(CudaMoeScratch* s, int cap) {
-    size_t offs[18];
+    size_t offs[19];
     const size_t bytes = tok_arena_bytes(*s, cap, offs);
     void* p = nullptr;
     CUDA_TRY(cudaMalloc(&p, bytes));
@@ -201,6 +202,7 @@ static Status alloc_tok_arena(CudaMoeScratch* s, int cap) {
     s->xr16 = reinterpret_cast<__half*>(b + offs[15]);
     s->rpart = reinterpret_cast<float*>(b + offs[16]);
     s->sq = reinterpret_cast<unsigned*>(b + offs[17]);
+    s->d32 = reinterpret_cast<float*>(b + offs[18]);
     return Status::Ok();
 }
 
@@ -355,6 +357,8 @@ static DecodeArgs make_decode_args(CudaMoeScratch* s, const MoeLayer& layer, int
     a.s_f32 = nullptr;
     a.T = tokens;
     a.K = s->K;
+    a.sms = s->sms;
+    a.d32 = s->d32;
     a.gating = s->gating;
     a.logits_override = s->logits_override;
     a.bar = (s->decode_impl == 0) ? s->bar : nullptr;
@@ -522,7 +526,8 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
     const bool tc_ok = (s->H % 256 == 0) && (s->I % 128 == 0) && (reinterpret_cast<uintptr_t>(normed) % 16 == 0) &&
                        (reinterpret_cast<uintptr_t>(out16_rows) % 32 == 0);
     p.impl = (s->prefill_impl == 1 || !tc_ok) ? 1 : 0;
-    if (s->prefill_impl == 0 && prefill_streams(batch * s->K, s->E, s->H, s->I, layer.dev.quant, normed)) {
+    // (the streaming kernels wait for nothing that could fail to come: the test hook takes the tcgen05 path)
+    if (s->prefill_impl == 0 && !s->expire_next[1] && prefill_streams(batch * s->K, s->E, s->H, s->I, layer.dev.quant, normed)) {
         p.impl = 2;
         p.stream_starts = reinterpret_cast<int32_t*>(s->R.work);  // (decode's work records: 8 KB, unused by a prefill)
     }
@@ -532,10 +537,6 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
     if (p.impl == 2) {
         // the router has left the activations' f16 planes; with routing from elsewhere they are made here
         if (!own_router) CUDA_TRY(launch_split_x16(normed, act_dtype, batch, s->H, s->xr16, nullptr, st));
-        if (s->expire_next[1]) {
-            p.debug_extra_tx = 1;
-            s->expire_next[1] = 0;
-        }
         CUDA_TRY(launch_stream_prefill(p, s->xr16, out16_rows, st));
         if (out16_rows) return Status::Ok();
     } else if (p.impl == 0) {

@@ -100,6 +100,7 @@ struct CudaMoeScratch {
     unsigned* xq = nullptr; // decode activations as two-term int8 blocks (Q4_0 gate/up of the three-kernel chain)
     unsigned* sq = nullptr; // SwiGLU outputs of a 5..16-token Q4_0 decode in the same form, per compact column
     uint4* sf = nullptr;    // decode SwiGLU fragments
+    float* d32 = nullptr;   // decode down outputs by compact column
     float* s_f32 = nullptr; // optional debug copy
     // prefill (grow-only)
     int32_t* blk_hist = nullptr;

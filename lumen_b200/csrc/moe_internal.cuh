@@ -99,6 +99,8 @@ struct DecodeArgs {
     uint4* sf;              // SwiGLU fragments     [C][2][kg_i*4][4]
     float* s_f32;           // optional [C,I] f32 copy of the SwiGLU output (null = skip)
     int T, K, gating;
+    int sms;                // multiprocessors of the device
+    float* d32;             // [C,H] unweighted down outputs by compact column (three-kernel chain)
     unsigned int* bar;      // grid barrier of the fused kernel: arrival counter + per-CTA barrier counts (1024 words); null = three-kernel chain
     int32_t* status;        // context status word (non-zero after a bounded wait expired)
     int32_t* status_host;   // the same code for the host: a word of mapped pinned host memory (null = none)
@@ -228,7 +230,9 @@ struct TcPlan {
 cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_cap, int gu_cols, int4* tiles,
                              int32_t* n_tiles, cudaStream_t st, const int32_t* stream_mode, int4* chunks, int32_t* starts,
                              int sms);
-// expert products of short prompts (stream.cu)
+// gate/up of a decode batch, expert products of short prompts (stream.cu)
+cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st);
+cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, cudaStream_t st);
 cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __half* out16_rows, cudaStream_t st,
                                   const TcPeerOut* peer = nullptr);
 constexpr int STREAM_MAX_COLS = 12;

@@ -3,25 +3,27 @@
 //
 // With a handful of columns per expert a layer call reads every selected expert's weights (340 MB
 // at H=2048, I=768, E=128, Q4_0) for little arithmetic. The tcgen05 kernel (prefill_tc.cu) has
-// to write each dequantised weight to shared memory as a rounded f16 operand: ~350 instructions per
-// 16 x 128 tile, which is what bounds it there (60 % issue slots, 1.9 TB/s at 77 tokens). Here a
+// to write each dequantised weight to shared memory as a rounded f16 operand: ~340 instructions per
+// 16 x 128 tile, which is what bounds it there (1.9 TB/s at 77 tokens). Here a
 // weight goes from the quant planes to an mma.sync fragment as an exact small integer, the f32 scale is
-// applied to the block's sums, and nothing is written back: ~110 instructions per tile at up to
-// eight columns, ~30 more per further eight.
+// applied to the block's sums, and nothing is written back.
 //
 // A WARP owns an item (16 output rows of one expert times one chunk of its columns, all inputs). Items are
-// dealt to the CTAs (one per SM) as equal contiguous ranges, so that the warps of an SM work on neighbouring
-// rows of one expert and share its activations in L1; inside the range the warps take every
-// WARPS-th item. Each warp keeps a ring of 128-input groups in flight with bulk copies on its own
-// mbarriers, across item boundaries: no CTA-wide synchronisation anywhere in the loop.
+// dealt to the CTAs (one per SM) as contiguous ranges of equal cost, experts outermost, so that the warps of an SM work
+// on neighbouring rows of one or two experts and find their activations in L1; inside the range the warps take
+// every WARPS-th item; no CTA-wide synchronisation anywhere. (A down kernel with the rows outermost, whose CTAs could combine their rows
+// themselves, had every warp on another expert and waited for L2 at each 32-input block: 25 instead of 20 us at
+// 16 tokens.) Each warp keeps a ring of its own in flight in shared memory, filled by bulk copies on its own
+// mbarriers across item boundaries. (cp.async by all lanes instead: 124 -> 138 us at 77 tokens, 193 -> 201 us for a 13-token
+// Q8_0 decode at H = 4096.)
 //
-//   gate_up   16 rows of I: gate and up tiles together, SwiGLU at the end
-//             (cuda/shaders/moe_expert_q4_0.cu:58-108, moe_expert.cu:47-97)
-//   down      16 rows of H (moe_grouped.cu:1202-1510); the weighted sum follows in scatter_accum_kernel
-//
-// TERMS = 1 (prompts): activations are single f16 rows in the planes' element order (x16, s16), the
-// precision of the tcgen05 path. TERMS = 2 (decode): hi + lo fragments, two MMA columns per token.
-// Every wait is bounded; a warp whose wait runs out raises the context's status word.
+//   GATE_UP_1 / DOWN_1    prompts: single f16 activation rows in the planes' element order (x16, s16), the precision
+//                         of the tcgen05 path; f16 rows out (moe_grouped.cu:1202-1510); the weighted sum
+//                         follows in scatter_accum_kernel
+//   GATE_UP_2 / DOWN_2    decode batches: hi + lo fragments, two MMA columns per token; f32 sums out
+//   DOWN_2I               the same on the integer tensor cores: Q4_0 nibbles against the two-term int8 SwiGLU blocks of
+//                         gate_up_stream_kernel
+//   (gate/up: cuda/shaders/moe_expert_q4_0.cu:58-108, moe_expert.cu:47-97; down: moe_expert_q4_0.cu:118-151)
 #include "decode_common.cuh"
 #include "tc_common.cuh"
 #include <type_traits>
@@ -32,43 +34,52 @@ namespace stream {
 
 using namespace dcommon;
 
+enum Mode { GATE_UP_1, DOWN_1, GATE_UP_2, DOWN_2, DOWN_2I };
+
+// warps per SM and groups in flight per warp: 131..147 KB on the way per SM (the copy peak times the latency is
+// ~55 KB), the rest of the 256 KB is L1 for the activations
 template <int Q>
-struct Cfg;  // a ring slot holds up to GRP 128-input groups (of each matrix); RING_GU / RING_DN slots per warp
-// (the copy peak times the latency is ~55 KB per SM in flight; the rings hold 139..184 KB)
+struct Cfg;
 template <>
 struct Cfg<Q4_0> {
-    static constexpr int WARPS = 16, GRP = 2, RING_GU = 2, RING_DN = 4;
+    static constexpr int WARPS = 16, RING_GU = 4, RING_DN = 8;
 };
 template <>
 struct Cfg<Q8_0> {
-    static constexpr int WARPS = 16, GRP = 1, RING_GU = 2, RING_DN = 4;
+    static constexpr int WARPS = 16, RING_GU = 2, RING_DN = 4;
 };
 template <>
 struct Cfg<BF16> {
-    static constexpr int WARPS = 8, GRP = 1, RING_GU = 2, RING_DN = 4;
+    static constexpr int WARPS = 8, RING_GU = 2, RING_DN = 4;
 };
 
-template <int Q>
-struct Raw {  // one 16-row x 128-input tile: quants then scales
-    static constexpr int q_bytes = QTraits<Q>::NQ * 512, s_bytes = (Q == BF16) ? 0 : 128, bytes = q_bytes + s_bytes;
+template <int Q, int MODE>
+struct Shape {
+    static constexpr bool down = (MODE == DOWN_1 || MODE == DOWN_2 || MODE == DOWN_2I), int8 = (MODE == DOWN_2I);
+    static constexpr int terms = (MODE == GATE_UP_1 || MODE == DOWN_1) ? 1 : 2;
+    static constexpr int nm = down ? 1 : 2;  // matrices of an item: down | gate and up
+    static constexpr int grp = (Q == Q4_0) ? 2 : 1;  // 128-input groups of a ring slot
+    static constexpr int warps = Cfg<Q>::WARPS, ring = (down ? Cfg<Q>::RING_DN : Cfg<Q>::RING_GU) / grp;
+    static constexpr uint32_t q_bytes = QTraits<Q>::NQ * 512, s_bytes = (Q == BF16 ? 0 : 128);  // of a tile: quants, scales
+    static constexpr uint32_t tile = grp * (q_bytes + s_bytes);
+    static constexpr uint32_t slot = nm * tile;
+    static constexpr size_t smem = (size_t)warps * ring * slot;
 };
 
 struct Args {
     LayerDev L;
-    const int4* chunks;         // {expert, first column, columns, -}
+    const int4* chunks;         // {expert, first column, columns, -}, `chunk_stride` entries apart
+    int chunk_stride;
     const int32_t* starts;      // [CTAs + 1] first item of every CTA (null: equal shares of n_chunks)
     const int32_t* n_chunks;
-    const int32_t* col_src_tok;
-    const uint4* b;             // activation rows: TERMS 1: f16 [row][kdim]; TERMS 2: fragments [row][2][nblk_pad][4]
+    const int32_t* col_src_tok; // gate/up: activation row of a compact column (null = the column itself)
+    const uint4* b;             // activation rows: f16 [row][kdim] | fragments [row][2][nblk_pad][4] | int8 blocks [row][sq]
     size_t b_row;               // uint4 per row (TERMS 2: per row and term)
-    __half* out16;              // TERMS 1: s16 [C, I] (permuted order) | d16 [C, H]
-    uint4* sf;                  // TERMS 2 gate/up: SwiGLU fragments
-    int32_t* status;
-    int32_t* status_host;
-    uint64_t wait_limit_ns;
-    int debug_extra_tx;             // test hook: every warp's first group expects this many bytes too many
-    const int32_t* out_row_map;     // down: output row of compact column c (null = c itself)
-    TcPeerOut peer;                 // down, expert parallel: output rows go to other ranks' buffers (ret_map null = off)
+    __half* out16;              // GATE_UP_1: s16 [C, I] (permuted order); DOWN_1: d16 [C, H]
+    uint4* sf;                  // GATE_UP_2: SwiGLU fragments
+    float* d32;                 // DOWN_2(I): [C, H]
+    const int32_t* out_row_map; // DOWN_1: output row of compact column c (null = c itself)
+    TcPeerOut peer;             // DOWN_1, expert parallel: output rows go to other ranks' buffers (ret_map null = off)
 };
 
 // b fragments of the block's two MMAs out of one 16-byte chunk (the two layouts order them differently)
@@ -139,19 +150,18 @@ __device__ __forceinline__ int perm32(int e) {
     return t * 8 + ((m & 1) ? 4 : 0) + (hi ? 2 : 0) + ((m >> 1) & 1);
 }
 
-template <int Q, int TERMS, bool DOWN>
+template <int Q, int MODE>
 __global__ void __launch_bounds__(Cfg<Q>::WARPS * 32, 1)
 stream_kernel(const __grid_constant__ Args a) {
-    static_assert(!DOWN || TERMS == 1, "the decode chain has its own down kernel");
-    constexpr int WARPS = Cfg<Q>::WARPS, RING = DOWN ? Cfg<Q>::RING_DN : Cfg<Q>::RING_GU;
-    constexpr int NM = DOWN ? 1 : 2;  // matrices of an item: down | gate and up
-    constexpr int GRP = Cfg<Q>::GRP;
-    constexpr uint32_t RAW_Q = Raw<Q>::q_bytes, RAW_S = Raw<Q>::s_bytes, RAW = GRP * (RAW_Q + RAW_S), SLOT = NM * RAW;
-    extern __shared__ __align__(128) uint8_t ring_smem[];  // [WARPS][RING][NM][quants of GRP groups | scales of GRP groups]
+    using S = Shape<Q, MODE>;
+    constexpr bool DOWN = S::down, I8 = S::int8;
+    constexpr int WARPS = S::warps, RING = S::ring, NM = S::nm, TERMS = S::terms, NQ = QTraits<Q>::NQ, GRP = S::grp;
+    static_assert(!I8 || Q == Q4_0, "the integer form is for Q4_0 nibbles");
+    extern __shared__ __align__(128) uint8_t ring_smem[];  // [WARPS][RING][NM][quants of GRP groups | their scales]
     __shared__ uint64_t bar_s[WARPS * RING];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gq = lane >> 2, t4 = lane & 3;
-    const uint32_t ring0 = tc::smem_u32(ring_smem) + (uint32_t)warp * RING * SLOT;
+    const uint32_t ring = tc::smem_u32(ring_smem) + (uint32_t)warp * RING * S::slot;
     const uint32_t bar0 = tc::smem_u32(&bar_s[warp * RING]);
     if (lane < RING) tc::mbar_init(bar0 + lane * 8, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -163,6 +173,7 @@ stream_kernel(const __grid_constant__ Args a) {
         pdl_trigger();
     }
     const int rt_n = DOWN ? a.L.rt_h : a.L.rt_i, kg_n = DOWN ? a.L.kg_i : a.L.kg_h;
+    const int nblk_pad = kg_n * 4;
     int i0, i1;
     if (a.starts != nullptr) {
         i0 = a.starts[blockIdx.x];
@@ -173,76 +184,84 @@ stream_kernel(const __grid_constant__ Args a) {
         i1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
     }
 
-    // request cursor: next group (item pi, group pkg) to copy
-    int pi = i0 + warp, pkg = 0, issued = 0, taken = 0;
+    // request cursor: the next groups (of item pi, from group pkg on) to copy, into ring slot wslot
+    int pi = i0 + warp, pkg = 0, wslot = 0, rslot = 0;
+    uint32_t rphase = 0;
     const uint4 *pq[NM], *ps[NM];
-    auto top_up = [&]() {
-        while (issued - taken < RING && pi < i1) {
-            if (pkg == 0) {
-                const int c = pi / rt_n;
-                const size_t t0 = (size_t)(pi - c * rt_n) * kg_n;
-                const int e = __ldg(&a.chunks[c]).x;
-                pq[0] = (DOWN ? a.L.down_q(e) : a.L.gate_q(e)) + t0 * (RAW_Q / 16);
-                ps[0] = (DOWN ? a.L.down_s(e) : a.L.gate_s(e)) + t0 * 8;
-                if constexpr (!DOWN) {
-                    pq[1] = a.L.up_q(e) + t0 * (RAW_Q / 16);
-                    ps[1] = a.L.up_s(e) + t0 * 8;
-                }
-            }
-            const int slot = issued % RING;
-            const uint32_t n = (GRP > 1) ? (uint32_t)min(GRP, kg_n - pkg) : 1u;
-            if (lane == 0) {
-                const uint32_t bar = bar0 + slot * 8, dst = ring0 + slot * SLOT;
-                tc::mbar_expect_tx(bar, NM * n * (RAW_Q + RAW_S) + (issued == 0 ? (uint32_t)a.debug_extra_tx : 0u));
-#pragma unroll
-                for (int m = 0; m < NM; ++m) {
-                    tc::bulk_load(dst + m * RAW, pq[m], n * RAW_Q, bar);
-                    if (RAW_S) tc::bulk_load(dst + m * RAW + GRP * RAW_Q, ps[m], n * RAW_S, bar);
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < NM; ++m) {
-                pq[m] += GRP * RAW_Q / 16;
-                ps[m] += GRP * 8;
-            }
-            ++issued;
-            if ((pkg += GRP) >= kg_n) {
-                pkg = 0;
-                pi += WARPS;
+    auto request = [&]() {
+        if (pi >= i1) return;
+        if (pkg == 0) {
+            const int c = pi / rt_n;
+            const size_t t0 = (size_t)(pi - c * rt_n) * kg_n;
+            const int e = __ldg(&a.chunks[c * a.chunk_stride]).x;
+            pq[0] = (DOWN ? a.L.down_q(e) : a.L.gate_q(e)) + t0 * (NQ * 32);
+            ps[0] = (DOWN ? a.L.down_s(e) : a.L.gate_s(e)) + t0 * 8;
+            if constexpr (!DOWN) {
+                pq[1] = a.L.up_q(e) + t0 * (NQ * 32);
+                ps[1] = a.L.up_s(e) + t0 * 8;
             }
         }
+        const uint32_t n = (GRP > 1) ? (uint32_t)min(GRP, kg_n - pkg) : 1u;
+        if (tc::elect_one()) {
+            const uint32_t bar = bar0 + wslot * 8, dst = ring + wslot * S::slot;
+            tc::mbar_expect_tx(bar, NM * n * (S::q_bytes + S::s_bytes));
+#pragma unroll
+            for (int m = 0; m < NM; ++m) {
+                tc::bulk_load(dst + m * S::tile, pq[m], n * S::q_bytes, bar);
+                if (S::s_bytes) tc::bulk_load(dst + m * S::tile + GRP * S::q_bytes, ps[m], n * S::s_bytes, bar);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < NM; ++m) {
+            pq[m] += GRP * NQ * 32;
+            ps[m] += GRP * 8;
+        }
+        if (++wslot == RING) wslot = 0;
+        if ((pkg += GRP) >= kg_n) {
+            pkg = 0;
+            pi += WARPS;
+        }
     };
-    top_up();
+#pragma unroll 1
+    for (int i = 0; i < RING; ++i) request();
     if (DOWN) {
         pdl_wait();
         pdl_trigger();
     }
-    bool ok = true;
-    auto wait_slot = [&]() -> bool {
-        const uint32_t bar = bar0 + (taken % RING) * 8, ph = (taken / RING) & 1;
-        bool r = tc::mbar_try(bar, ph);
-        if (!r) {
-            const uint64_t t0 = tc::globaltimer_ns();
-            do {
-                r = tc::mbar_try(bar, ph);
-            } while (!r && tc::globaltimer_ns() - t0 < a.wait_limit_ns);
-        }
-        return __all_sync(0xffffffffu, r);
-    };
-
     const UnpackConst kc = unpack_const_pinned<Q>();
+    const int sq_term = xq_term_words(nblk_pad), sq_tok = xq_tok_words(nblk_pad);
+
     auto item = [&](auto ng_tag, const int4& ch, int rt) {
         constexpr int NG = decltype(ng_tag)::value;
         constexpr int CPG = (TERMS == 1) ? 8 : 4;  // columns of an MMA group
+        // This lane's B column of every group (a column past the end repeats the chunk's last one: its sums are not
+        // stored). I8: bp = word pairs of the column and term (8 bytes per block), sp = {sx, 8 sx sum q} of the column of
+        // the lane's accumulators.
         const uint4* bp[NG];
+        const float2* sp[NG];
 #pragma unroll
         for (int g = 0; g < NG; ++g) {
-            // this lane's B column; a column past the end repeats the chunk's last one (its sums are not stored)
             const int n = (TERMS == 1) ? g * CPG + gq : g * CPG + (gq >> 1);
             const int col = ch.y + min(n, ch.z - 1);
-            const int row = (DOWN || a.col_src_tok == nullptr) ? col : a.col_src_tok[col];
-            bp[g] = a.b + ((TERMS == 1) ? (size_t)row : (size_t)row * 2 + (gq & 1)) * a.b_row + t4;
+            if constexpr (I8) {
+                const unsigned* sq = reinterpret_cast<const unsigned*>(a.b);
+                bp[g] = reinterpret_cast<const uint4*>(sq + (size_t)col * sq_tok + (gq & 1) * sq_term + t4 * 2);
+                sp[g] = reinterpret_cast<const float2*>(sq + (size_t)(ch.y + min(g * CPG + t4, ch.z - 1)) * sq_tok + 2 * sq_term);
+            } else {
+                const int row = (DOWN || a.col_src_tok == nullptr) ? col : a.col_src_tok[col];
+                bp[g] = a.b + ((TERMS == 1) ? (size_t)row : (size_t)row * 2 + (gq & 1)) * a.b_row + t4;
+            }
         }
+        auto load_b = [&](int g, int b) -> uint4 {  // operand of block b of the group at hand
+            if constexpr (I8) {
+                const uint2 w = __ldg(reinterpret_cast<const uint2*>(bp[g]) + b * 4);
+                const float2 sc = __ldg(sp[g] + b);
+                return make_uint4(w.x, w.y, __float_as_uint(sc.x), __float_as_uint(sc.y));
+            } else {
+                return __ldg(bp[g] + b * 4);
+            }
+        };
         float acc[NM][NG][4];
 #pragma unroll
         for (int m = 0; m < NM; ++m)
@@ -251,64 +270,89 @@ stream_kernel(const __grid_constant__ Args a) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[m][g][i] = 0.0f;
         // The next block's activations are loaded one block ahead (at the end of a row that is the first
-        // chunk of whatever follows it in the context's memory: loaded, never used).
-        uint4 bn[NG];
+        // chunk of whatever follows it in the context's memory: loaded, never used), registers permitting.
+        constexpr bool AHEAD = NG * NM <= 4;
+        uint4 bn[AHEAD ? NG : 1];
+        if constexpr (AHEAD) {
 #pragma unroll
-        for (int g = 0; g < NG; ++g) bn[g] = __ldg(bp[g]);
-        int sub = GRP;  // next group within the slot
-        uint32_t src = 0;
+            for (int g = 0; g < NG; ++g) bn[g] = load_b(g, 0);
+        }
+        int sub = 0;
 #pragma unroll 1
         for (int kg = 0; kg < kg_n; ++kg) {
-            if (GRP == 1 || sub == GRP) {
-                ok = wait_slot();
-                if (!ok) return;
-                src = ring0 + (taken % RING) * SLOT;
-                sub = 0;
+            if (sub == 0) {
+                // (the warp's own copies: they arrive; the limit only keeps a broken launch from spinning for good)
+                for (int k = 0; k < (1 << 22) && !tc::mbar_try(bar0 + rslot * 8, rphase); ++k) {}
             }
             WTile<Q> w[NM];
+            const uint32_t src = ring + rslot * S::slot;
 #pragma unroll
             for (int m = 0; m < NM; ++m) {
 #pragma unroll
-                for (int j = 0; j < QTraits<Q>::NQ; ++j) w[m].q[j] = tc::lds128(src + m * RAW + sub * RAW_Q + j * 512 + lane * 16);
-                if (Q != BF16) w[m].s = tc::lds128(src + m * RAW + GRP * RAW_Q + sub * RAW_S + gq * 16);
+                for (int j = 0; j < NQ; ++j) w[m].q[j] = tc::lds128(src + m * S::tile + sub * S::q_bytes + j * 512 + lane * 16);
+                if (Q != BF16) w[m].s = tc::lds128(src + m * S::tile + GRP * S::q_bytes + sub * S::s_bytes + gq * 16);
             }
             if (GRP == 1 || ++sub == GRP || kg + 1 == kg_n) {
+                sub = 0;
+                if (++rslot == RING) {
+                    rslot = 0;
+                    rphase ^= 1u;
+                }
                 // every lane's reads of the slot are ordered before the bulk copy that fills it again
                 tc::fence_proxy_async();
                 __syncwarp();
-                ++taken;
-                top_up();
+                request();
             }
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 uint4 bc[NG];
 #pragma unroll
                 for (int g = 0; g < NG; ++g) {
-                    bc[g] = bn[g];
-                    bn[g] = __ldg(bp[g] + (b + 1) * 4);
+                    if constexpr (AHEAD) {
+                        bc[g] = bn[g];
+                        bn[g] = load_b(g, b + 1);
+                    } else {
+                        bc[g] = load_b(g, b);
+                    }
                 }
 #pragma unroll
                 for (int m = 0; m < NM; ++m) {
-                    uint32_t lo[4], hi[4];
-                    unpack<Q, TERMS>(w[m], b, lo, hi, kc);
                     const float2 sc = block_scales<Q>(w[m], b);
+                    if constexpr (I8) {
+                        const uint4 qv = w[m].q[(b >> 1) % NQ];
+                        const unsigned w0 = (b & 1) ? qv.z : qv.x, w8 = (b & 1) ? qv.w : qv.y;
 #pragma unroll
-                    for (int g = 0; g < NG; ++g) block_mma<Q, TERMS>(lo, hi, sc, bc[g], acc[m][g]);
+                        for (int g = 0; g < NG; ++g) {
+                            int c[4] = {0, 0, 0, 0};
+                            mma_u8s8(c, w0 & 0x0F0F0F0Fu, w8 & 0x0F0F0F0Fu, (w0 >> 4) & 0x0F0F0F0Fu, (w8 >> 4) & 0x0F0F0F0Fu,
+                                     bc[g].x, bc[g].y);
+                            const float sx = __uint_as_float(bc[g].z), off = __uint_as_float(bc[g].w), k1 = 1.0f / 254.0f;
+                            acc[m][g][0] = fmaf(sc.x, fmaf(sx, fmaf((float)c[1], k1, (float)c[0]), -off), acc[m][g][0]);
+                            acc[m][g][2] = fmaf(sc.y, fmaf(sx, fmaf((float)c[3], k1, (float)c[2]), -off), acc[m][g][2]);
+                        }
+                    } else {
+                        uint32_t lo[4], hi[4];
+                        unpack<Q, TERMS>(w[m], b, lo, hi, kc);
+#pragma unroll
+                        for (int g = 0; g < NG; ++g) block_mma<Q, TERMS>(lo, hi, sc, bc[g], acc[m][g]);
+                    }
                 }
             }
 #pragma unroll
-            for (int g = 0; g < NG; ++g) bp[g] += 16;
+            for (int g = 0; g < NG; ++g) {
+                bp[g] += I8 ? 8 : 16;  // one group on: 4 blocks x 32 | 64 bytes
+                if (I8) sp[g] += 4;
+            }
         }
         // lane: rows gq and gq + 8 of the tile, MMA columns 2 t4, 2 t4 + 1 of each group
         const int r0 = rt * 16 + gq;
 #pragma unroll
         for (int g = 0; g < NG; ++g) {
-            if constexpr (DOWN) {
+            if constexpr (MODE == DOWN_1) {
                 // transposed through the tensor path's 8 x 8 move, so that a lane holds two neighbouring rows of one
                 // column: four lanes then write 16 bytes of an output row
-                uint32_t p0 = h2_bits(acc[0][g][0], acc[0][g][1]), p1 = h2_bits(acc[0][g][2], acc[0][g][3]);
-                p0 = movmatrix_trans(p0);
-                p1 = movmatrix_trans(p1);
+                const uint32_t p0 = movmatrix_trans(h2_bits(acc[0][g][0], acc[0][g][1]));
+                const uint32_t p1 = movmatrix_trans(h2_bits(acc[0][g][2], acc[0][g][3]));
                 const int n = g * 8 + gq;
                 if (n < ch.z) {
                     int orow = ch.y + n;
@@ -329,17 +373,15 @@ stream_kernel(const __grid_constant__ Args a) {
                         d[4] = p1;
                     }
                 }
-            } else if constexpr (TERMS == 1) {
+            } else if constexpr (MODE == GATE_UP_1) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int n = g * 8 + 2 * t4 + (i & 1), row = r0 + (i >> 1) * 8;
                     if (n < ch.z) {
-                        {
-                            // fast exp and divide: their error (~2^-21) is far below the f16 rounding that follows
-                            const float gt = acc[0][g][i];
-                            a.out16[(size_t)(ch.y + n) * a.L.I + (row & ~31) + perm32(row & 31)] =
-                                __float2half_rn(__fdividef(gt, 1.0f + __expf(-gt)) * acc[NM - 1][g][i]);
-                        }
+                        // fast exp and divide: their error (~2^-21) is far below the f16 rounding that follows
+                        const float gt = acc[0][g][i];
+                        a.out16[(size_t)(ch.y + n) * a.L.I + (row & ~31) + perm32(row & 31)] =
+                            __float2half_rn(__fdividef(gt, 1.0f + __expf(-gt)) * acc[NM - 1][g][i]);
                     }
                 }
             } else {
@@ -347,80 +389,135 @@ stream_kernel(const __grid_constant__ Args a) {
                 if (n < ch.z) {
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
-                        const float gt = acc[0][g][2 * i] + acc[0][g][2 * i + 1];
-                        const float up = acc[NM - 1][g][2 * i] + acc[NM - 1][g][2 * i + 1];
-                        store_swiglu_frag<Q>(a.sf, ch.y + n, r0 + i * 8, a.L.kg_i * 4, (gt / (1.0f + expf(-gt))) * up);
+                        const float v = acc[0][g][2 * i] + acc[0][g][2 * i + 1];
+                        if constexpr (DOWN) {
+                            __stcg(a.d32 + (size_t)(ch.y + n) * a.L.H + r0 + i * 8, v);
+                        } else {
+                            const float up = acc[NM - 1][g][2 * i] + acc[NM - 1][g][2 * i + 1];
+                            store_swiglu_frag<Q>(a.sf, ch.y + n, r0 + i * 8, a.L.kg_i * 4, (v / (1.0f + expf(-v))) * up);
+                        }
                     }
                 }
             }
         }
     };
-    for (int i = i0 + warp; i < i1 && ok; i += WARPS) {
+    for (int i = i0 + warp; i < i1; i += WARPS) {
         const int c = i / rt_n;
-        const int4 ch = __ldg(&a.chunks[c]);
+        const int4 ch = __ldg(&a.chunks[c * a.chunk_stride]);
         const int rt = i - c * rt_n;
         const int ng = (TERMS == 1) ? (ch.z + 7) >> 3 : (ch.z + 3) >> 2;
         if (ng == 1) item(std::integral_constant<int, 1>{}, ch, rt);
         else if (ng == 2) item(std::integral_constant<int, 2>{}, ch, rt);
-        else if (ng == 3) item(std::integral_constant<int, 3>{}, ch, rt);
         else item(std::integral_constant<int, 4>{}, ch, rt);
     }
-    if (!ok) {
-        // give-up: let the copies in flight land before the shared memory goes away
-        for (; taken != issued; ++taken)
-            for (int k = 0; k < (1 << 16) && !tc::mbar_try(bar0 + (taken % RING) * 8, (taken / RING) & 1); ++k) {}
-        if (lane == 0) raise_status(a.status, a.status_host, 4);  // LUMEN_MOE_TIMEOUT
-    }
 }
 
-template <int Q, int TERMS, bool DOWN>
+// out[t] = residual[t] + sum_slot w * d32[column of the slot], in slot order (cuda/shaders/moe_accum.cu:22-46)
+__global__ void __launch_bounds__(128)
+combine_f32_kernel(const float* __restrict__ d32, RouteDev R, const float* residual, float* out, int H, int K) {
+    const int t = blockIdx.x, h = (blockIdx.y * 128 + threadIdx.x) * 2;
+    // (the tables are the router's, complete before the down kernel started)
+    int col[MAX_TOP_K];
+    float w[MAX_TOP_K];
+#pragma unroll
+    for (int s = 0; s < MAX_TOP_K; ++s)
+        if (s < K) {
+            col[s] = __ldg(R.dst_to_col + t * K + s);
+            w[s] = __ldg(R.weights + t * K + s);
+        }
+    pdl_trigger();
+    pdl_wait();
+    if (h >= H) return;
+    float2 acc = *reinterpret_cast<const float2*>(residual + (size_t)t * H + h);
+    float2 d[MAX_TOP_K];
+#pragma unroll
+    for (int s = 0; s < MAX_TOP_K; ++s)
+        if (s < K) d[s] = __ldcg(reinterpret_cast<const float2*>(d32 + (size_t)col[s] * H + h));
+#pragma unroll
+    for (int s = 0; s < MAX_TOP_K; ++s)
+        if (s < K) {
+            acc.x = __fadd_rn(acc.x, __fmul_rn(w[s], d[s].x));
+            acc.y = __fadd_rn(acc.y, __fmul_rn(w[s], d[s].y));
+        }
+    *reinterpret_cast<float2*>(out + (size_t)t * H + h) = acc;
+}
+
+template <int Q, int MODE>
 cudaError_t launch_t(const Args& a, int sms, cudaStream_t st) {
-    constexpr size_t smem = (size_t)Cfg<Q>::WARPS * (DOWN ? Cfg<Q>::RING_DN : Cfg<Q>::RING_GU) * (DOWN ? 1 : 2) * Cfg<Q>::GRP * Raw<Q>::bytes;
     static SmemOptIn optin;
-    const cudaError_t e = ensure_dyn_smem(stream_kernel<Q, TERMS, DOWN>, smem, optin);
+    const cudaError_t e = ensure_dyn_smem(stream_kernel<Q, MODE>, Shape<Q, MODE>::smem, optin);
     if (e != cudaSuccess) return e;
     count_launch();
-    return launch_dep(stream_kernel<Q, TERMS, DOWN>, dim3(sms), dim3(Cfg<Q>::WARPS * 32), smem, st, a);
+    return launch_dep(stream_kernel<Q, MODE>, dim3(sms), dim3(Cfg<Q>::WARPS * 32), Shape<Q, MODE>::smem, st, a);
 }
 
-template <int TERMS, bool DOWN>
+template <int MODE>
 cudaError_t launch_q(const Args& a, int sms, cudaStream_t st) {
     switch (a.L.quant) {
-        case Q4_0: return launch_t<Q4_0, TERMS, DOWN>(a, sms, st);
-        case Q8_0: return launch_t<Q8_0, TERMS, DOWN>(a, sms, st);
-        default: return launch_t<BF16, TERMS, DOWN>(a, sms, st);
+        case Q4_0: return launch_t<Q4_0, MODE>(a, sms, st);
+        case Q8_0: return launch_t<Q8_0, MODE>(a, sms, st);
+        default: return launch_t<BF16, MODE>(a, sms, st);
     }
+}
+
+// decode batches: the router's work records are the chunks (an expert has at most sixteen columns)
+static Args decode_args(const DecodeArgs& p) {
+    Args g{};
+    g.L = p.L;
+    g.chunks = p.R.work;
+    g.chunk_stride = 2;
+    g.n_chunks = p.R.n_uexp;
+    return g;
 }
 
 }  // namespace stream
 
-// Activation rows of a prompt for both products: x16 rows by token (planes' element order), s16 by column.
+// gate/up of a decode batch: hi + lo activation fragments by token, SwiGLU fragments for the down product
+cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st) {
+    stream::Args g = stream::decode_args(p);
+    g.col_src_tok = p.R.col_src_tok;
+    g.b = p.xf;
+    g.b_row = (size_t)p.L.kg_h * 16;
+    g.sf = p.sf;
+    return stream::launch_q<stream::GATE_UP_2>(g, p.sms, st);
+}
+
+// down + combine of a decode batch; int8: the SwiGLU outputs are in p.sq (Q4_0), else fragments in p.sf
+cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, cudaStream_t st) {
+    stream::Args d = stream::decode_args(p);
+    d.b = int8 ? reinterpret_cast<const uint4*>(p.sq) : p.sf;
+    d.b_row = (size_t)p.L.kg_i * 16;
+    d.d32 = p.d32;
+    const cudaError_t e = int8 ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st) : stream::launch_q<stream::DOWN_2>(d, p.sms, st);
+    if (e != cudaSuccess) return e;
+    count_launch();
+    return launch_dep(stream::combine_f32_kernel, dim3(p.T, (p.L.H / 2 + 127) / 128), dim3(128), 0, st, (const float*)p.d32, p.R,
+                      p.residual, p.out, p.L.H, p.K);
+}
+
+// Expert products of a short prompt: x16 rows by token (planes' element order), s16 by column.
 cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __half* out16_rows, cudaStream_t st,
                                   const TcPeerOut* peer) {
     stream::Args g{};
     g.L = p.L;
     g.chunks = p.tiles;
+    g.chunk_stride = 1;
     g.n_chunks = p.n_tiles;
     g.starts = p.stream_starts;
     g.col_src_tok = p.R.col_src_tok;
     g.b = reinterpret_cast<const uint4*>(x16);
     g.b_row = (size_t)p.L.H / 8;
     g.out16 = p.s16;
-    g.status = p.status;
-    g.status_host = p.status_host;
-    g.wait_limit_ns = p.wait_limit_us ? (uint64_t)p.wait_limit_us * 1000ull : tc::WAIT_LIMIT_NS;
-    g.debug_extra_tx = p.debug_extra_tx;
-    cudaError_t e = stream::launch_q<1, false>(g, p.sms, st);
+    const cudaError_t e = stream::launch_q<stream::GATE_UP_1>(g, p.sms, st);
     if (e != cudaSuccess) return e;
     stream::Args d = g;
-    d.debug_extra_tx = 0;  // the hook applies to the first kernel of the pair
     d.starts = p.stream_starts ? p.stream_starts + p.sms + 1 : nullptr;
     d.b = reinterpret_cast<const uint4*>(p.s16);
     d.b_row = (size_t)p.L.I / 8;
     d.out16 = out16_rows ? out16_rows : p.d16;
-    if (peer) d.peer = *peer;
     d.out_row_map = out16_rows ? p.R.col_src_tok : nullptr;
-    return stream::launch_q<1, true>(d, p.sms, st);
+    if (peer) d.peer = *peer;
+    return stream::launch_q<stream::DOWN_1>(d, p.sms, st);
 }
 
 }  // namespace lumen
