@@ -564,7 +564,9 @@ cudaError_t launch_decode_phase(const DecodeArgs& a_in, int phase, cudaStream_t 
     DecodeArgs a = a_in;
     // Q4_0 layers that gate_up_stream_kernel takes: int8 activations for both products; every other format and shape:
     // hi + lo fragments and the general streaming kernel
-    const bool int8 = decode_stream_applicable(a);
+    // (up to three tokens only where the context asks for the chain: the fused kernel, which such a batch takes
+    // otherwise, gives the down product the finer activations)
+    const bool int8 = decode_stream_applicable(a) && (a.T >= 4 || a.bar == nullptr);
     if (!int8) a.xq = a.sq = nullptr;
     if (phase == 0) return launch_route_small(a, st);
     if (phase == 1) return int8 ? launch_gate_up_stream(a, st) : launch_stream_gate_up(a, st);
@@ -574,12 +576,21 @@ cudaError_t launch_decode_phase(const DecodeArgs& a_in, int phase, cudaStream_t 
 bool decode_fused_applicable(const DecodeArgs& a);
 cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st);
 
-// Which form a decode call takes. The persistent fused kernel wins up to three tokens; at four
-// tokens on a Q4_0 layer the chain with the streaming gate/up kernel and the int8 down product is
-// faster (35.5 against 38.1 us per layer call; 31.9 / 30.6 at three, 26.1 / 23.9 at two).
+// Which form a decode call takes: the persistent fused kernel (two grid barriers, no boundary between kernels) is ahead
+// while the weights of the selected experts are so few that boundaries cost more than streaming them; the chain's
+// kernels stream faster. Measured us per call, fused / chain (H = 2048, I = 768, E = 128, top-8; 21 MB Q4_0, 40 MB Q8_0,
+// 75 MB BF16 per token): Q4_0 18.6 / 27.5 at one token, 25.8 / 25.1 at two, 32.8 / 29.3 at three; Q8_0 32.8 / 33.7 at two,
+// 41.2 / 39.7 at three; BF16 32.6 / 29.7 at one, 66 / 38 at two. (H = 1024, I = 512, top-6, 5 MB Q4_0 per token: 16.6 / 18.0
+// at two, 20.6 / 18.7 at three.) Both do the same arithmetic for Q8_0 and BF16; the Q4_0 chain's down product takes
+// two-term int8 activations.
 bool decode_uses_fused(const DecodeArgs& a) {
     if (!decode_fused_applicable(a)) return false;
-    return !(a.T >= 4 && decode_stream_applicable(a));
+    const double weights = 3.0 * a.T * a.K * a.L.I * a.L.H;
+    switch (a.L.quant) {
+        case Q4_0: return a.T < 2 || weights * (18.0 / 32) < 14e6;
+        case Q8_0: return a.T < 3 || weights * (34.0 / 32) < 28e6;
+        default: return weights * 2 < (a.T < 2 ? 60e6 : 36e6);
+    }
 }
 
 cudaError_t launch_decode(const DecodeArgs& a, cudaStream_t st) {

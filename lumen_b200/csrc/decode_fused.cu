@@ -228,7 +228,8 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
         if (a.trace != nullptr && tid == 0) a.trace[(size_t)blockIdx.x * 12 + i] = global_ns();
     };
     stamp(0);
-    if (tid < 32) ts.tab[tid] = lumen_exact::exp2_tab_entry(tid);
+    // (the exp table is only needed after barrier 1: the load is in flight until then)
+    const unsigned long long tab_entry = (tid < 32) ? lumen_exact::exp2_tab_entry(tid) : 0ull;
     if (tid == 0) {
         fail_s = 0;
         for (int i = 0; i < 8; ++i) mbar_init(&mbar[i], 1);
@@ -427,6 +428,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
             raise_status(a.status, a.status_host, 4);  // LUMEN_MOE_TIMEOUT
             fail_s = 1;
         }
+        if (tid < 32) ts.tab[tid] = tab_entry;
         __syncthreads();
         if (fail_s) return;
     }

@@ -53,6 +53,9 @@ namespace lumen_exact {
 
 #if defined(__CUDACC__)
 static __device__ __constant__ uint64_t exp2_tab_dev[32] = LUMEN_EXP2_TAB_INIT;
+// the same in global memory, for filling a shared-memory copy: one coalesced load, where the constant cache would
+// serve 32 different addresses one after the other (~0.5 us at the head of a kernel)
+static __device__ const uint64_t exp2_tab_gmem[32] = LUMEN_EXP2_TAB_INIT;
 #endif
 static const uint64_t exp2_tab_host[32] = LUMEN_EXP2_TAB_INIT;
 
@@ -112,6 +115,12 @@ LUMEN_HD float expf_libm_tab(float x, Tab tab) {
 
 LUMEN_HD float expf_libm(float x) { return expf_libm_tab(x, Exp2TabDefault()); }
 
-LUMEN_HD uint64_t exp2_tab_entry(int i) { return exp2_tab(i); }
+LUMEN_HD uint64_t exp2_tab_entry(int i) {
+#if defined(__CUDA_ARCH__)
+    return __ldg(reinterpret_cast<const unsigned long long*>(exp2_tab_gmem) + i);
+#else
+    return exp2_tab(i);
+#endif
+}
 
 }  // namespace lumen_exact
