@@ -578,16 +578,15 @@ cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st);
 
 // Which form a decode call takes: the persistent fused kernel (two grid barriers, no boundary between kernels) is ahead
 // while the weights of the selected experts are so few that boundaries cost more than streaming them; the chain's
-// kernels stream faster. Measured us per call, fused / chain (H = 2048, I = 768, E = 128, top-8; 21 MB Q4_0, 40 MB Q8_0,
-// 75 MB BF16 per token): Q4_0 18.6 / 27.5 at one token, 25.8 / 25.1 at two, 32.8 / 29.3 at three; Q8_0 32.8 / 33.7 at two,
-// 41.2 / 39.7 at three; BF16 32.6 / 29.7 at one, 66 / 38 at two. (H = 1024, I = 512, top-6, 5 MB Q4_0 per token: 16.6 / 18.0
-// at two, 20.6 / 18.7 at three.) Both do the same arithmetic for Q8_0 and BF16; the Q4_0 chain's down product takes
-// two-term int8 activations.
+// kernels stream faster. Measured us per call, fused / chain, at H = 2048, I = 768, E = 128, top-8 (40 MB Q8_0, 75 MB
+// BF16 per token): Q8_0 32.8 / 33.7 at two tokens, 41.2 / 39.7 at three; BF16 32.6 / 29.7 at one, 66 / 38 at two; at
+// H = 1024, I = 512, top-6: Q8_0 24.0 / 23.6 at three, BF16 24.8 / 22.1 at two. Q4_0: fused up to three tokens (32.8 us
+// at three; with activations as fine as its own the chain takes 33.7), the int8 chain from four (38 / 31 us).
 bool decode_uses_fused(const DecodeArgs& a) {
     if (!decode_fused_applicable(a)) return false;
     const double weights = 3.0 * a.T * a.K * a.L.I * a.L.H;
     switch (a.L.quant) {
-        case Q4_0: return a.T < 2 || weights * (18.0 / 32) < 14e6;
+        case Q4_0: return a.T < 4 || !decode_stream_applicable(a);
         case Q8_0: return a.T < 3 || weights * (34.0 / 32) < 28e6;
         default: return weights * 2 < (a.T < 2 ? 60e6 : 36e6);
     }
