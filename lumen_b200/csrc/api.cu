@@ -106,7 +106,7 @@ lumen_moe_status_t lumen_moe_layer_prepare(lumen_moe_ctx* ctx, const void* d_lay
             lumen::Status rs = lumen::aligned_router(d_layer_blob, router_off, sc.E, sc.H, st, &r->layer.repacked,
                                                      &r->layer.dev.router_w);
             if (rs.ok())
-                rs = lumen::build_router_w16(r->layer.dev.router_w, sc.E, sc.H, st, &r->layer.repacked,
+                rs = lumen::build_router_w16(r->layer.dev.router_w, sc.E, sc.H, false, st, &r->layer.repacked,
                                              &r->layer.dev.router_w16);
             if (rs.ok() && cudaStreamSynchronize(st) != cudaSuccess) rs = lumen::Status::Err(LUMEN_MOE_CUDA_ERROR, "copy of the router weight failed");
             if (!rs.ok()) {
@@ -410,11 +410,10 @@ lumen_moe_status_t lumen_moe_stack_prefill(lumen_moe_ctx* ctx, const lumen_moe_l
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     for (int l = 0; l < n_layers; ++l) {
         if (!layers[l] || !d_gammas[l]) return fail(LUMEN_MOE_INVALID_ARG, "null layer or gamma");
-        cudaError_t e = lumen::launch_rmsnorm(d_x, d_gammas[l], d_normed, tokens, ctx->scratch.H, eps, st);
-        if (e != cudaSuccess) return fail(LUMEN_MOE_CUDA_ERROR, cudaGetErrorString(e));
         // residual and output are the same buffer: the combine reads and writes each element in one thread
+        const lumen::NormIn norm{d_x, d_gammas[l], eps};
         lumen::Status s = lumen::encode_moe_ffn_prefill_grouped(&ctx->scratch, layers[l]->layer, d_normed, 0, d_x, d_x,
-                                                                tokens, st, nullptr, nullptr, nullptr);
+                                                                tokens, st, nullptr, nullptr, nullptr, &norm);
         if (!s.ok()) return done(s);
     }
     return LUMEN_MOE_OK;
@@ -506,7 +505,7 @@ lumen_moe_status_t lumen_moe_ep_layer_prepare(lumen_moe_ctx* ctx, const void* d_
         l->layer.repacked.router_w16 = nullptr;
         s = lumen::aligned_router(d_layer_blob, router_off, sc.E, sc.H, st, &l->layer.repacked, &l->layer.dev.router_w);
         if (s.ok())
-            s = lumen::build_router_w16(l->layer.dev.router_w, sc.E, sc.H, st, &l->layer.repacked, &l->layer.dev.router_w16);
+            s = lumen::build_router_w16(l->layer.dev.router_w, sc.E, sc.H, l->layer.dev.planes_natural, st, &l->layer.repacked, &l->layer.dev.router_w16);
     }
     if (s.ok()) {
         cudaError_t e = cudaStreamSynchronize(st);

@@ -14,8 +14,7 @@ cudaError_t launch_scatter_accum(const __half* d16, const float* residual, const
                                  int T, int H, int K, cudaStream_t st);
 cudaError_t launch_build_xf(const void* x, int act_dtype, int T, int H, int nblk_pad, bool bf16_mode,
                             uint4* xf, cudaStream_t st);
-cudaError_t launch_gather_permute_x16(const void* x, int act_dtype, const int32_t* col_src_tok, int C, int H, void* out,
-                                      cudaStream_t st, bool natural);
+cudaError_t launch_gather_rows(const __half* plane, const int32_t* col_src_tok, int C, int H, void* out, cudaStream_t st);
 cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, cudaStream_t st, __half* out16_rows,
                               const TcPlan* plan = nullptr, const TcPeerOut* peer = nullptr);
 cudaError_t launch_rows_from_cols(const __half* d16, const int32_t* dst_to_col, __half* out16, int T, int H, cudaStream_t st);
@@ -104,7 +103,9 @@ Status build_repacked(const CudaMoeScratch& sc, const void* layer_buf, size_t bl
     L.blob = static_cast<const uint8_t*>(layer_buf);
     {
         Status rs = aligned_router(layer_buf, meta.router_weight_off, E, H, st, out, &L.router_w);
-        if (rs.ok()) rs = build_router_w16(L.router_w, E, H, st, out, &L.router_w16);
+        // (layers whose prefill weights are plain f16 matrices multiply in the natural element order)
+        L.planes_natural = (quant == BF16 || (sc.flags & 0x8)) && H % 256 == 0 && I % 128 == 0;
+        if (rs.ok()) rs = build_router_w16(L.router_w, E, H, L.planes_natural, st, out, &L.router_w16);
         if (!rs.ok()) return rs;
     }
     L.quant = quant;
@@ -308,11 +309,11 @@ Status aligned_router(const void* layer_buf, uint64_t router_off, int E, int H, 
 }
 
 // f16 high / low planes of the router weight, once per layer (the batched router multiplies on tcgen05)
-Status build_router_w16(const float* router_w, int E, int H, cudaStream_t st, CudaMoeRepacked* out, const __half** w16) {
+Status build_router_w16(const float* router_w, int E, int H, bool natural, cudaStream_t st, CudaMoeRepacked* out, const __half** w16) {
     *w16 = nullptr;
     if (H % 64 != 0) return Status::Ok();  // the tcgen05 router does not take this shape
     CUDA_TRY(cudaMalloc(&out->router_w16, (size_t)2 * E * H * sizeof(__half)));
-    CUDA_TRY(launch_split_router_w16(router_w, out->router_w16, E, H, st));
+    CUDA_TRY(launch_split_router_w16(router_w, out->router_w16, E, H, natural, st));
     *w16 = out->router_w16;
     return Status::Ok();
 }
@@ -480,7 +481,7 @@ static bool prefill_streams(int columns, int E, int H, int I, int quant, const v
 // cuda/moe.rs:1900-2760
 Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, const void* normed, int act_dtype,
                                       const float* residual, float* output, int batch, cudaStream_t st,
-                                      const uint32_t* ids_in, const float* weights_in, __half* out16_rows) {
+                                      const uint32_t* ids_in, const float* weights_in, __half* out16_rows, const NormIn* norm) {
     if (batch < 1) return Status::Err(1, "batch must be positive");
     if (out16_rows) {
         if (s->K != 1 || !ids_in) return Status::Err(1, "f16 row output needs top_k = 1 and caller-supplied ids");
@@ -532,16 +533,30 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
         p.stream_starts = reinterpret_cast<int32_t*>(s->R.work);  // (decode's work records: 8 KB, unused by a prefill)
     }
     const bool own_router = ids_in == nullptr && s->logits_override == nullptr;
+    // Activation planes of the tcgen05 router (f16 high and low parts): the high one is also what the expert products
+    // of both tensor-core paths read. The RMSNorm of a stack layer goes into their pass where nothing else reads the
+    // normed activations.
+    const bool router_planes = own_router && layer.dev.router_w16 != nullptr && router_tc_applicable(batch, s->E, s->H, normed);
+    if (norm != nullptr) {
+        if (router_planes && p.impl != 1 && norm_split_applicable(s->H, norm->x, norm->gamma)) {
+            p.x = norm->x;
+            p.gamma = norm->gamma;
+            p.eps = norm->eps;
+        } else {
+            CUDA_TRY(launch_rmsnorm(norm->x, norm->gamma, static_cast<float*>(const_cast<void*>(normed)), batch, s->H, norm->eps, st));
+        }
+    }
     CUDA_TRY(launch_route_large(p, st));
+    // planes that the router has not left, or not in the order the streaming kernels read
+    if (p.impl != 1 && (!router_planes || (p.impl == 2 && layer.dev.planes_natural)))
+        CUDA_TRY(p.gamma ? launch_norm_split(norm->x, p.gamma, p.eps, batch, s->H, p.impl == 0 && layer.dev.planes_natural, s->xr16, nullptr, st)
+                         : launch_split_x16(normed, act_dtype, batch, s->H, p.impl == 0 && layer.dev.planes_natural, s->xr16, nullptr, st));
     const bool bf16_mode = (layer.dev.quant == BF16);
     if (p.impl == 2) {
-        // the router has left the activations' f16 planes; with routing from elsewhere they are made here
-        if (!own_router) CUDA_TRY(launch_split_x16(normed, act_dtype, batch, s->H, s->xr16, nullptr, st));
         CUDA_TRY(launch_stream_prefill(p, s->xr16, out16_rows, st));
         if (out16_rows) return Status::Ok();
     } else if (p.impl == 0) {
-        CUDA_TRY(launch_gather_permute_x16(normed, act_dtype, s->R.col_src_tok, batch * s->K, s->H, s->x16, st,
-                                           layer.dev.gu16 != nullptr));
+        CUDA_TRY(launch_gather_rows(s->xr16, s->R.col_src_tok, batch * s->K, s->H, s->x16, st));
         // persistent grid, one CTA per SM; LUMEN_MOE_FLAG_TC_CTAS leaves some SMs to kernels that run beside it
         int sms = s->sms;
         if (s->tc_ctas > 0 && s->tc_ctas < sms) sms = s->tc_ctas;

@@ -88,7 +88,7 @@ struct CudaMoeRepacked {
 // else a copy owned by `out` (enqueued on `st`).
 Status aligned_router(const void* layer_buf, uint64_t router_off, int E, int H, cudaStream_t st,
                       CudaMoeRepacked* out, const float** router_w);
-Status build_router_w16(const float* router_w, int E, int H, cudaStream_t st, CudaMoeRepacked* out, const __half** w16);
+Status build_router_w16(const float* router_w, int E, int H, bool natural, cudaStream_t st, CudaMoeRepacked* out, const __half** w16);
 
 // CudaMoeScratch + CudaMoePrefillGrouped, cuda/moe.rs:101-210.
 struct CudaMoeScratch {
@@ -160,10 +160,18 @@ Status encode_moe_ffn_decode(CudaMoeScratch* scratch, const MoeLayer& layer, con
 Status encode_moe_ffn_decode_fused_norm(CudaMoeScratch* scratch, const MoeLayer& layer,
                                         const float* attn_proj, const float* ffn_norm, float* normed_x,
                                         float* output_x, float eps, int tokens, cudaStream_t st);
+// activations that are rmsnorm(x; gamma, eps) of an f32 residual stream: `normed` is then scratch of the same size, written
+// only where the norm cannot be folded into the pass that prepares the operands
+struct NormIn {
+    const float* x;
+    const float* gamma;
+    float eps;
+};
 Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* scratch, const MoeLayer& layer, const void* normed,
                                       int act_dtype, const float* residual, float* output, int batch,
                                       cudaStream_t st, const uint32_t* ids_in = nullptr,
-                                      const float* weights_in = nullptr, __half* out16_rows = nullptr);
+                                      const float* weights_in = nullptr, __half* out16_rows = nullptr,
+                                      const NormIn* norm = nullptr);
 Status encode_route_only(CudaMoeScratch* scratch, const MoeLayer* layer, const float* normed,
                          const float* logits_in, int tokens, uint32_t* d_ids, float* d_weights,
                          float* d_logits_out, cudaStream_t st);

@@ -334,9 +334,31 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
     for (int i = tid; i < H; i += 256) out[(size_t)t * H + i] = xr[i] * sc * gamma[i];
 }
 
+// 16-byte form for rows of whole 32-blocks
+__global__ void __launch_bounds__(256) rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
+                                                          float* __restrict__ out, int H, float eps) {
+    __shared__ float red[8];
+    const int t = blockIdx.x, tid = threadIdx.x, n8 = H >> 3;
+    const float* xr = x + (size_t)t * H;
+    float ss = 0.0f;
+    for (int i = tid; i < n8; i += 256) {
+        const int oa = (i >> 2) * 32 + (i & 3) * 4;
+        ss = norm_sq_chunk(ss, *reinterpret_cast<const float4*>(xr + oa), *reinterpret_cast<const float4*>(xr + oa + 16));
+    }
+    const float sc = norm_scale(ss, red, H, eps);
+    for (int i = tid; i < H / 4; i += 256) {
+        const float4 v = reinterpret_cast<const float4*>(xr)[i], g = __ldg(reinterpret_cast<const float4*>(gamma) + i);
+        reinterpret_cast<float4*>(out + (size_t)t * H)[i] = make_float4(v.x * sc * g.x, v.y * sc * g.y, v.z * sc * g.z, v.w * sc * g.w);
+    }
+}
+
 cudaError_t launch_rmsnorm(const float* x, const float* gamma, float* out, int T, int H, float eps,
                            cudaStream_t st) {
     count_launch();
+    if (H % 32 == 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(out)) % 16 == 0) {
+        rmsnorm_vec_kernel<<<T, 256, 0, st>>>(x, gamma, out, H, eps);
+        return cudaGetLastError();
+    }
     rmsnorm_kernel<<<T, 256, 0, st>>>(x, gamma, out, H, eps);
     return cudaGetLastError();
 }

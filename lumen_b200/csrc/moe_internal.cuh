@@ -42,6 +42,7 @@ struct LayerDev {
     const uint8_t* blob;
     const float* router_w;  // blob + router_off, [E,H] f32
     const __half* router_w16;  // [2][E][H] f16 high / low parts of router_w (batched router on tcgen05), or null
+    bool planes_natural;       // element order of these planes and of the activations' (see route_tc.cu)
     const uint4* q;         // all experts' quant planes
     const uint4* s;         // all experts' scale planes (unused for BF16)
     // optional plain f16 matrices of all experts (scale folded in) for the TMA-fed prefill products:
@@ -118,6 +119,24 @@ __device__ __forceinline__ void raise_status(int32_t* status, int32_t* status_ho
     }
 }
 
+// Sum of squares of a row and its RMSNorm scale by a CTA of 256 threads, each with chunks of inputs 4t.. and 16+4t.. of
+// 32-blocks: one order of summation for the norm alone and for the norm fused with what follows it.
+__device__ __forceinline__ float norm_sq_chunk(float ss, const float4& p, const float4& q) {
+    ss += p.x * p.x + p.y * p.y + p.z * p.z + p.w * p.w;
+    ss += q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+    return ss;
+}
+__device__ __forceinline__ float norm_scale(float ss, float* red8, int H, float eps) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((threadIdx.x & 31) == 0) red8[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float s = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s += red8[w];
+    return 1.0f / sqrtf(s / (float)H + eps);
+}
+
 // Programmatic dependent launch for the chains of small kernels around the grouped products. A
 // kernel launched with launch_dep() may be scheduled while the kernel before it in the stream
 // is still running; it calls grid_dep_sync() as its first statement (every thread, before any
@@ -172,6 +191,8 @@ struct PrefillArgs {
     RouteDev R;
     const void* x;          // normed [T,H], f32 or bf16
     int act_dtype;          // 0 f32, 1 bf16
+    const float* gamma;     // non-null: x is the raw residual stream (f32), the activations are rmsnorm(x; gamma, eps)
+    float eps;
     const float* residual;
     float* out;
     const float* logits_override;
@@ -200,14 +221,17 @@ struct PrefillArgs {
 };
 cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st);
 // tcgen05 router (route_tc.cu)
-cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, cudaStream_t st);
-// f16 planes of the activations in the weight planes' element order (see route_tc.cu); any_lo null = high plane only
-cudaError_t launch_split_x16(const void* x, int act_dtype, int T, int H, __half* x16, int32_t* any_lo, cudaStream_t st);
+cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, bool natural, cudaStream_t st);
+// f16 planes of the activations (see route_tc.cu); any_lo null = high plane only
+cudaError_t launch_split_x16(const void* x, int act_dtype, int T, int H, bool natural, __half* x16, int32_t* any_lo, cudaStream_t st);
+// the planes of rmsnorm(x; gamma, eps)
+bool norm_split_applicable(int H, const void* x, const void* gamma);
+cudaError_t launch_norm_split(const float* x, const float* gamma, float eps, int T, int H, bool natural, __half* x16, int32_t* any_lo,
+                              cudaStream_t st);
 int router_tc_ksplit(int T, int E, int H, int sms);
 bool router_tc_applicable(int T, int E, int H, const void* x);
-cudaError_t launch_router_logits_tc(const void* x, int act_dtype, const __half* w16, int T, int E, int H, int ksplit,
-                                    __half* x16, int32_t* any_lo, float* part, int32_t* status, int32_t* status_host,
-                                    unsigned wait_limit_us, cudaStream_t st);
+cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int ksplit, const __half* x16, int32_t* any_lo,
+                                    float* part, int32_t* status, int32_t* status_host, unsigned wait_limit_us, cudaStream_t st);
 constexpr int ROUTER_TC_MAX_KSPLIT = 4;
 
 // Expert-parallel form of the grouped products: the rows of the activation operand are not this

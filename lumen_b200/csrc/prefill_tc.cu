@@ -32,9 +32,9 @@
 // Stages are handed over with mbarriers; every wait is bounded (on expiry the
 // kernel raises a status word, drains and frees its TMEM instead of hanging).
 //
-// Inputs are 16-bit: activations pre-converted to f16, gathered into compact-column order
-// and pre-permuted within each 32-block to the order the dequantiser emits
-// (gather_permute_x16_kernel; natural order for TMA-fed weights); the SwiGLU output is
+// Inputs are 16-bit: activations pre-converted to f16 and
+// pre-permuted within each 32-block to the order the dequantiser emits (route_tc.cu; natural order for TMA-fed
+// weights), gathered into compact-column order (gather_rows_kernel); the SwiGLU output is
 // written in the same order so the down product reads it back without any shuffle.
 #include "mma_frag.cuh"
 #include "tc_common.cuh"
@@ -795,81 +795,35 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
     if (tid == 0 && abort_s) raise_status(a.status, a.status_host, 4);  // LUMEN_MOE_TIMEOUT
 }
 
-// activations -> f16, gathered into compact-column order (row c = token
-// col_src_tok[c]) and permuted within each 32-block: the grouped GEMM then reads
-// plain 2-D boxes of it with TMA
-template <typename XT, bool IS_F16 = false, bool NATURAL = false>
+// rows of the activations' high plane (f16, already in the operand's element order) in compact-column order (row c =
+// token col_src_tok[c]): the grouped GEMM then reads plain 2-D boxes of it with TMA. Bound by its writes; eight rows per CTA
+// step, their source rows known first and all loads of a thread in flight together. (Converting from the caller's
+// f32 rows here instead, after the router's pre-pass had done it already, took 89 us at 8192 tokens, H = 2048, against
+// 50.)
 __global__ void __launch_bounds__(256)
-gather_permute_x16_kernel(const XT* __restrict__ x, const int32_t* __restrict__ col_src_tok, int C, int H,
-                          uint16_t* __restrict__ out) {
+gather_rows_kernel(const uint4* __restrict__ plane, const int32_t* __restrict__ col_src_tok, int C, int H8, uint4* __restrict__ out) {
     grid_dep_sync();
-    // one thread per output chunk of 8 values (16 bytes): chunk t of a 32-block holds inputs
-    // (4t, 4t+2, 16+4t, 16+4t+2, 4t+1, 4t+3, 16+4t+1, 16+4t+3), i.e. perm_pos of two runs of four.
-    // Four rows per step: their source rows are known first, then all eight loads of a thread are
-    // in flight together (one row per CTA was a chain of dependent latencies: 43 us for 134 MB).
-    auto to_h = [](XT v) -> uint16_t {
-        if (sizeof(XT) == 4) return __half_as_ushort(__float2half_rn(*reinterpret_cast<const float*>(&v)));
-        if (IS_F16) return *reinterpret_cast<const uint16_t*>(&v);
-        return __half_as_ushort(__float2half_rn(__bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(&v))));
-    };
-    struct __align__(4 * sizeof(XT)) Run { XT v[4]; };
-    constexpr int R = 4;
-    for (int c0 = blockIdx.x * R; c0 < C; c0 += gridDim.x * R) {
-        int tok[R];
+    constexpr int R = 8;
+    const int c0 = blockIdx.x * R;
+    int tok[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) tok[r] = col_src_tok[min(c0 + r, C - 1)];
-        for (int ch = threadIdx.x; ch < H / 8; ch += 256) {
-            const int blk = ch >> 2, t = ch & 3;
-            // NATURAL (TMA-fed weights): chunk ch holds inputs 8 ch .. 8 ch + 7 as they are
-            const int oa = NATURAL ? ch * 8 : blk * 32 + 4 * t, ob = NATURAL ? ch * 8 + 4 : blk * 32 + 16 + 4 * t;
-            Run a[R], b[R];
+    for (int r = 0; r < R; ++r) tok[r] = col_src_tok[min(c0 + r, C - 1)];
+    for (int i = threadIdx.x; i < H8; i += 256) {
+        uint4 v[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const XT* src = x + (size_t)tok[r] * H;
-                a[r] = *reinterpret_cast<const Run*>(src + oa);
-                b[r] = *reinterpret_cast<const Run*>(src + ob);
-            }
+        for (int r = 0; r < R; ++r) v[r] = __ldg(plane + (size_t)tok[r] * H8 + i);
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if (c0 + r < C) {
-                    __align__(16) uint16_t o[8];
-                    if (NATURAL) {
-                        o[0] = to_h(a[r].v[0]); o[1] = to_h(a[r].v[1]); o[2] = to_h(a[r].v[2]); o[3] = to_h(a[r].v[3]);
-                        o[4] = to_h(b[r].v[0]); o[5] = to_h(b[r].v[1]); o[6] = to_h(b[r].v[2]); o[7] = to_h(b[r].v[3]);
-                    } else {
-                        o[0] = to_h(a[r].v[0]); o[1] = to_h(a[r].v[2]); o[2] = to_h(b[r].v[0]); o[3] = to_h(b[r].v[2]);
-                        o[4] = to_h(a[r].v[1]); o[5] = to_h(a[r].v[3]); o[6] = to_h(b[r].v[1]); o[7] = to_h(b[r].v[3]);
-                    }
-                    *reinterpret_cast<uint4*>(out + (size_t)(c0 + r) * H + blk * 32 + t * 8) = *reinterpret_cast<const uint4*>(o);
-                }
-            }
-        }
+        for (int r = 0; r < R; ++r)
+            if (c0 + r < C) out[(size_t)(c0 + r) * H8 + i] = v[r];
     }
 }
 
 }  // namespace tc
 
-cudaError_t launch_gather_permute_x16(const void* x, int act_dtype, const int32_t* col_src_tok, int C, int H, void* out,
-                                      cudaStream_t st, bool natural) {
+cudaError_t launch_gather_rows(const __half* plane, const int32_t* col_src_tok, int C, int H, void* out, cudaStream_t st) {
     count_launch();
-    if (C <= 0) return cudaSuccess;
-    const int ggrid = (C + 3) / 4;  // four rows per CTA step; every CTA takes one step at these sizes
-    cudaError_t lerr = cudaSuccess;
-#define LUMEN_GATHER(XT, F16, NAT) \
-    lerr = launch_dep(tc::gather_permute_x16_kernel<XT, F16, NAT>, dim3(ggrid), dim3(256), 0, st, (const XT*)x, col_src_tok, C, \
-                      H, (uint16_t*)out)
-    if (act_dtype == 0) {
-        if (natural) LUMEN_GATHER(float, false, true);
-        else LUMEN_GATHER(float, false, false);
-    } else if (act_dtype == 2) {
-        if (natural) LUMEN_GATHER(__half, true, true);
-        else LUMEN_GATHER(__half, true, false);
-    } else {
-        if (natural) LUMEN_GATHER(__nv_bfloat16, false, true);
-        else LUMEN_GATHER(__nv_bfloat16, false, false);
-    }
-#undef LUMEN_GATHER
-    return lerr;
+    return launch_dep(tc::gather_rows_kernel, dim3((C + 7) / 8), dim3(256), 0, st, reinterpret_cast<const uint4*>(plane), col_src_tok, C,
+                      H / 8, reinterpret_cast<uint4*>(out));
 }
 
 cudaError_t make_tmap_f16(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out) {

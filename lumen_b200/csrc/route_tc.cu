@@ -176,14 +176,57 @@ router_logits_tc_kernel(const __grid_constant__ Args a) {
     if (tid == 0 && abort_s) raise_status(a.status, a.status_host, 4);  // LUMEN_MOE_TIMEOUT
 }
 
-// x [T, H] (f32, bf16 or f16) -> f16 planes [2][T][H] in the weight planes' element order: high part, low
-// part; *any_lo |= (some low part != 0). The high plane is also the activation operand of the expert
-// products of short prompts. any_lo null: no low plane wanted (routing supplied by the caller).
-// One thread per 16-byte output chunk: chunk t of a 32-block holds inputs
-// (4t, 4t+2, 16+4t, 16+4t+2, 4t+1, 4t+3, 16+4t+1, 16+4t+3).
+// x [T, H] (f32, bf16 or f16) -> f16 planes [2][T][H] in the element order of the router weight's planes: high
+// part, low part; *any_lo |= (some low part != 0). The high plane is also the activation operand of the expert
+// products. any_lo null: no low plane wanted (routing supplied by the caller).
+//
+// Element order. Permuted (layers whose weights are dequantised): the order the dequantiser emits, 16-byte chunk t of a
+// 32-block holding inputs (4t, 4t+2, 16+4t, 16+4t+2, 4t+1, 4t+3, 16+4t+1, 16+4t+3). Natural (weights copied by
+// TMA from plain f16 matrices). A thread has inputs 4t.. (p) and 16+4t.. (q) of chunk i = 4 * block + t in both.
+struct PlaneOut {
+    __half* out;      // high plane, the low one `plane` elements on
+    size_t plane;
+    int32_t* any_lo;  // or null
+    bool natural;
+};
+__device__ __forceinline__ unsigned store_planes(const PlaneOut& o, size_t i, const float4& p, const float4& q) {
+    unsigned nz = 0u;
+    const float f[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+    uint32_t hi[8], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const __half h = __float2half_rn(f[j]);
+        const __half l = __float2half_rn(f[j] - __half2float(h));
+        hi[j] = __half_as_ushort(h);
+        lo[j] = __half_as_ushort(l);
+        nz |= lo[j] & 0x7fffu;
+    }
+    auto pair = [](const uint32_t (&v)[8], int a, int b) { return v[a] | (v[b] << 16); };
+#pragma unroll
+    for (int pl = 0; pl < 2; ++pl) {
+        if (pl == 1 && o.any_lo == nullptr) break;
+        const uint32_t(&v)[8] = pl ? lo : hi;
+        __half* dst = o.out + (pl ? o.plane : 0);
+        if (o.natural) {
+            const size_t oa = (i >> 2) * 32 + (i & 3) * 4;
+            *reinterpret_cast<uint2*>(dst + oa) = make_uint2(pair(v, 0, 1), pair(v, 2, 3));
+            *reinterpret_cast<uint2*>(dst + oa + 16) = make_uint2(pair(v, 4, 5), pair(v, 6, 7));
+        } else {
+            reinterpret_cast<uint4*>(dst)[i] = make_uint4(pair(v, 0, 2), pair(v, 4, 6), pair(v, 1, 3), pair(v, 5, 7));
+        }
+    }
+    return nz;
+}
+__device__ __forceinline__ void note_low_parts(const PlaneOut& o, unsigned nz) {
+    // one warp's finding is enough: the word is read first, so that thousands of atomics do not queue on it
+    if (o.any_lo != nullptr && __any_sync(0xffffffffu, nz != 0u) && (threadIdx.x & 31) == 0 &&
+        *reinterpret_cast<volatile int32_t*>(o.any_lo) == 0)
+        atomicOr(o.any_lo, 1);
+}
+
 template <typename XT>
 __global__ void __launch_bounds__(256)
-split_x16_kernel(const XT* __restrict__ x, size_t n8, size_t plane, __half* __restrict__ out, int32_t* any_lo) {
+split_x16_kernel(const XT* __restrict__ x, size_t n8, const PlaneOut o) {
     grid_dep_sync();
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
     unsigned nz = 0u;
@@ -207,39 +250,68 @@ split_x16_kernel(const XT* __restrict__ x, size_t n8, size_t plane, __half* __re
                                 __uint_as_float(v.y & 0xffff0000u));
             }
         }
-        const float f[8] = {p.x, p.z, q.x, q.z, p.y, p.w, q.y, q.w};
-        __align__(16) __half hi[8], lo[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            hi[j] = __float2half_rn(f[j]);
-            lo[j] = __float2half_rn(f[j] - __half2float(hi[j]));
-            nz |= (unsigned)(__half_as_ushort(lo[j]) & 0x7fffu);
-        }
-        reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(hi);
-        if (any_lo != nullptr) reinterpret_cast<uint4*>(out + plane)[i] = *reinterpret_cast<const uint4*>(lo);
+        nz = store_planes(o, i, p, q);
     }
-    if (any_lo != nullptr && __any_sync(0xffffffffu, nz != 0u) && (threadIdx.x & 31) == 0 && *reinterpret_cast<volatile int32_t*>(any_lo) == 0)
-        atomicOr(any_lo, 1);  // (one warp's finding is enough: the word is read first, so that thousands of atomics do not queue on it)
+    note_low_parts(o, nz);
+}
+
+// RMSNorm (cuda/shaders/norm.cu:28-76) and the planes of its result in one pass over a layer stack's residual stream: one
+// CTA per row, the row held in registers (H <= 8192). The squares are summed in the order of rmsnorm_kernel. At 8192
+// tokens, H = 2048: 72 us as two kernels with the f32 result in between, 26 us (bytes: 128 MB, 20 us at the copy peak).
+constexpr int NORM_MAX_CHUNKS = 4;
+template <int NCH>  // NCH * 2048 >= H
+__global__ void __launch_bounds__(256)
+norm_split_kernel(const float* __restrict__ x, const float* __restrict__ gamma, float eps, int H, const PlaneOut o) {
+    grid_dep_sync();
+    __shared__ float red[8];
+    const int t = blockIdx.x, tid = threadIdx.x, n8 = H >> 3;
+    const float* xr = x + (size_t)t * H;
+    float4 p[NCH], q[NCH];
+    float ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < NCH; ++j) {
+        const int i = tid + j * 256;
+        if (i < n8) {
+            const int oa = (i >> 2) * 32 + (i & 3) * 4;
+            p[j] = *reinterpret_cast<const float4*>(xr + oa);
+            q[j] = *reinterpret_cast<const float4*>(xr + oa + 16);
+            ss = norm_sq_chunk(ss, p[j], q[j]);
+        }
+    }
+    const float sc = norm_scale(ss, red, H, eps);
+    unsigned nz = 0u;
+#pragma unroll
+    for (int j = 0; j < NCH; ++j) {
+        const int i = tid + j * 256;
+        if (i < n8) {
+            const int oa = (i >> 2) * 32 + (i & 3) * 4;
+            const float4 g = __ldg(reinterpret_cast<const float4*>(gamma + oa)), h = __ldg(reinterpret_cast<const float4*>(gamma + oa + 16));
+            const float4 np = make_float4(p[j].x * sc * g.x, p[j].y * sc * g.y, p[j].z * sc * g.z, p[j].w * sc * g.w);
+            const float4 nq = make_float4(q[j].x * sc * h.x, q[j].y * sc * h.y, q[j].z * sc * h.z, q[j].w * sc * h.w);
+            nz |= store_planes(o, (size_t)t * n8 + i, np, nq);
+        }
+    }
+    note_low_parts(o, nz);
 }
 
 }  // namespace rtc
 
 // W_r [E, H] f32 -> f16 planes [2][E][H] (high, low) in the same element order as x: once per layer
-__global__ void split_router_w16_kernel(const float* __restrict__ w, __half* __restrict__ w16, size_t n) {
+__global__ void split_router_w16_kernel(const float* __restrict__ w, __half* __restrict__ w16, size_t n, bool natural) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float v = w[i];
     const __half hi = __float2half_rn(v);
     const int el = (int)(i & 31), t = (el & 15) >> 2, m = el & 3;
-    const size_t o = (i & ~(size_t)31) + t * 8 + ((m & 1) ? 4 : 0) + ((el >> 4) ? 2 : 0) + (m >> 1);
+    const size_t o = natural ? i : (i & ~(size_t)31) + t * 8 + ((m & 1) ? 4 : 0) + ((el >> 4) ? 2 : 0) + (m >> 1);
     w16[o] = hi;
     w16[n + o] = __float2half_rn(v - __half2float(hi));
 }
 
-cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, cudaStream_t st) {
+cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, bool natural, cudaStream_t st) {
     const size_t n = (size_t)E * H;
     count_launch();
-    split_router_w16_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w, w16, n);
+    split_router_w16_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w, w16, n, natural);
     return cudaGetLastError();
 }
 
@@ -260,13 +332,26 @@ bool router_tc_applicable(int T, int E, int H, const void* x) {
     return H % 64 == 0 && E >= 1 && E <= 256 && T >= 1 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
 }
 
-cudaError_t launch_split_x16(const void* x, int act_dtype, int T, int H, __half* x16, int32_t* any_lo, cudaStream_t st) {
-    const size_t n8 = (size_t)T * H / 8, plane = (size_t)T * H;
+cudaError_t launch_split_x16(const void* x, int act_dtype, int T, int H, bool natural, __half* x16, int32_t* any_lo, cudaStream_t st) {
+    const size_t n8 = (size_t)T * H / 8;
+    const rtc::PlaneOut o{x16, (size_t)T * H, any_lo, natural};
     const dim3 grid((unsigned)((n8 + 255) / 256));
     count_launch();
-    if (act_dtype == 0) return launch_dep(rtc::split_x16_kernel<float>, grid, dim3(256), 0, st, (const float*)x, n8, plane, x16, any_lo);
-    if (act_dtype == 2) return launch_dep(rtc::split_x16_kernel<__half>, grid, dim3(256), 0, st, (const __half*)x, n8, plane, x16, any_lo);
-    return launch_dep(rtc::split_x16_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, (const __nv_bfloat16*)x, n8, plane, x16, any_lo);
+    if (act_dtype == 0) return launch_dep(rtc::split_x16_kernel<float>, grid, dim3(256), 0, st, (const float*)x, n8, o);
+    if (act_dtype == 2) return launch_dep(rtc::split_x16_kernel<__half>, grid, dim3(256), 0, st, (const __half*)x, n8, o);
+    return launch_dep(rtc::split_x16_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, (const __nv_bfloat16*)x, n8, o);
+}
+
+bool norm_split_applicable(int H, const void* x, const void* gamma) {
+    return H % 32 == 0 && H <= rtc::NORM_MAX_CHUNKS * 2048 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma)) % 16 == 0;
+}
+
+cudaError_t launch_norm_split(const float* x, const float* gamma, float eps, int T, int H, bool natural, __half* x16, int32_t* any_lo,
+                              cudaStream_t st) {
+    const rtc::PlaneOut o{x16, (size_t)T * H, any_lo, natural};
+    count_launch();
+    auto kern = H <= 2048 ? rtc::norm_split_kernel<1> : H <= 4096 ? rtc::norm_split_kernel<2> : rtc::norm_split_kernel<rtc::NORM_MAX_CHUNKS>;
+    return launch_dep(kern, dim3(T), dim3(256), 0, st, x, gamma, eps, H, o);
 }
 
 template <int BN>
@@ -279,16 +364,14 @@ static cudaError_t launch_rtc(const rtc::Args& a, cudaStream_t st) {
     return launch_dep(rtc::router_logits_tc_kernel<BN>, dim3(grid), dim3(rtc::THREADS), (size_t)smem, st, a);
 }
 
-// logits partials of the whole batch; x16 / any_lo / part are scratch of the context
-cudaError_t launch_router_logits_tc(const void* x, int act_dtype, const __half* w16, int T, int E, int H, int ksplit,
-                                    __half* x16, int32_t* any_lo, float* part, int32_t* status, int32_t* status_host,
+// logits partials of the whole batch from its planes (launch_split_x16 or launch_norm_split); part is scratch of the context
+cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int ksplit,
+                                    const __half* x16, int32_t* any_lo, float* part, int32_t* status, int32_t* status_host,
                                     unsigned wait_limit_us, cudaStream_t st) {
-    cudaError_t e = launch_split_x16(x, act_dtype, T, H, x16, any_lo, st);
-    if (e != cudaSuccess) return e;
     count_launch();
     rtc::Args a{};
     a.m_tiles = (E + 127) / 128;
-    e = make_tmap_f16(w16, (uint64_t)2 * E, (uint64_t)H, 128, &a.tmap_w);
+    cudaError_t e = make_tmap_f16(w16, (uint64_t)2 * E, (uint64_t)H, 128, &a.tmap_w);
     if (e != cudaSuccess) return e;
     const bool narrow = (T + 127) / 128 * a.m_tiles * ksplit < 148 / 2;
     const int bn = narrow ? 32 : 128;
