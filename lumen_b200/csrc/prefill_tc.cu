@@ -57,6 +57,16 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
     asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
+// SwiGLU (cuda/shaders/moe_expert.cu:47-50), g / (1 + e^-g) * u, on the approximate exp2 and reciprocal units: their error
+// (~2^-21) is far below the f16 rounding of the result that follows. The epilogue of a wide tile is exposed, so its
+// instructions count; the range fix-ups of the library forms are not needed here (e^-g = inf gives 0, as it should; a
+// reciprocal below 2^-126 may flush to 0).
+__device__ __forceinline__ float swiglu_fast(float g, float u) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return g * r * u;
+}
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
@@ -420,17 +430,17 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
             // 8-column pieces of this warp's 16-column chunks, the TMEM loads of the next piece issued
             // before the current one is worked on
             auto piece_col = [&](int p) { return part * 16 + (p >> 1) * nparts * 16 + (p & 1) * 8; };
+            __half* const dst0 = a.out16 + (size_t)tile.y * a.out_ld + off0;
+            const uint32_t ld = (uint32_t)a.out_ld;
             auto work = [&](int col, const uint32_t (&g)[8], const uint32_t (&u)[8]) {
-                __half* dst = a.out16 + (size_t)(tile.y + col) * a.out_ld + off0;
+                __half* dst = dst0 + (size_t)((uint32_t)col * ld);
+                if (col + 8 <= ncols) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (col + j < ncols) {
-                        const float gt = __uint_as_float(g[j]);
-                        // SwiGLU (cuda/shaders/moe_expert.cu:47-50) with the fast exp and divide: their
-                        // error (~2^-21) is far below the f16 rounding of the result that follows
-                        dst[(size_t)j * a.out_ld] =
-                            __float2half_rn(__fdividef(gt, 1.0f + __expf(-gt)) * __uint_as_float(u[j]));
-                    }
+                    for (int j = 0; j < 8; ++j, dst += ld) *dst = __float2half_rn(swiglu_fast(__uint_as_float(g[j]), __uint_as_float(u[j])));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j, dst += ld)
+                        if (col + j < ncols) *dst = __float2half_rn(swiglu_fast(__uint_as_float(g[j]), __uint_as_float(u[j])));
                 }
             };
             uint32_t g0[8], u0[8], g1[8], u1[8];
