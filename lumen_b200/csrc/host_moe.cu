@@ -475,7 +475,7 @@ Status encode_route_only(CudaMoeScratch* s, const MoeLayer* layer, const float* 
 // the call is bound by reading the weights, not by multiplying. (BF16 layers have their f16 matrices copied by
 // TMA on the tcgen05 path, which then is bound by HBM as well: 240 against 224 us at 64 tokens.)
 static bool prefill_streams(int columns, int E, int H, int I, int quant, const void* normed) {
-    return quant != BF16 && H % 128 == 0 && I % 128 == 0 && H >= 256 && columns <= STREAM_MAX_COLS * E && reinterpret_cast<uintptr_t>(normed) % 16 == 0;
+    return quant != BF16 && H % 128 == 0 && I % 128 == 0 && H >= 256 && columns <= stream_max_columns(quant, E) && reinterpret_cast<uintptr_t>(normed) % 16 == 0;
 }
 
 // cuda/moe.rs:1900-2760

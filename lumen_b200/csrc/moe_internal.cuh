@@ -254,12 +254,18 @@ struct TcPlan {
 cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_cap, int gu_cols, int4* tiles,
                              int32_t* n_tiles, cudaStream_t st, const int32_t* stream_mode, int4* chunks, int32_t* starts,
                              int sms);
+// Most columns of a prompt that the streaming kernels take. The line lies where the tcgen05 kernels overtake them: Q8_0,
+// whose rows cost twice the bytes, at 10 columns an expert (E = 128, I = 768: 258 us there, 270 streaming; Q4_0 242 and
+// 231, at 12 245 and 248). A lone expert up to one 16-column operand (29 us, 36).
+inline int stream_max_columns(int quant, int experts) {
+    const int n = (quant == Q4_0 ? 12 : 9) * experts;
+    return n > 16 ? n : 16;
+}
 // gate/up of a decode batch, expert products of short prompts (stream.cu)
 cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st);
 cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, cudaStream_t st);
 cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __half* out16_rows, cudaStream_t st,
                                   const TcPeerOut* peer = nullptr);
-constexpr int STREAM_MAX_COLS = 12;
 constexpr int STREAM_SHIFT = 5;
 constexpr int STREAM_CHUNK = 1 << STREAM_SHIFT;  // columns of an expert that one item of the streaming kernels multiplies
 
