@@ -536,7 +536,8 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
     // Activation planes of the tcgen05 router (f16 high and low parts): the high one is also what the expert products
     // of both tensor-core paths read. The RMSNorm of a stack layer goes into their pass where nothing else reads the
     // normed activations.
-    const bool router_planes = own_router && layer.dev.router_w16 != nullptr && router_tc_applicable(batch, s->E, s->H, normed);
+    const bool single = route_single_applicable(p) && norm == nullptr;
+    const bool router_planes = own_router && !single && layer.dev.router_w16 != nullptr && router_tc_applicable(batch, s->E, s->H, normed);
     if (norm != nullptr) {
         if (router_planes && p.impl != 1 && norm_split_applicable(s->H, norm->x, norm->gamma)) {
             p.x = norm->x;
@@ -548,7 +549,7 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
     }
     CUDA_TRY(launch_route_large(p, st));
     // planes that the router has not left, or not in the order the streaming kernels read
-    if (p.impl != 1 && (!router_planes || (p.impl == 2 && layer.dev.planes_natural)))
+    if (p.impl != 1 && !single && (!router_planes || (p.impl == 2 && layer.dev.planes_natural)))
         CUDA_TRY(p.gamma ? launch_norm_split(norm->x, p.gamma, p.eps, batch, s->H, p.impl == 0 && layer.dev.planes_natural, s->xr16, nullptr, st)
                          : launch_split_x16(normed, act_dtype, batch, s->H, p.impl == 0 && layer.dev.planes_natural, s->xr16, nullptr, st));
     const bool bf16_mode = (layer.dev.quant == BF16);
@@ -556,7 +557,7 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
         CUDA_TRY(launch_stream_prefill(p, s->xr16, out16_rows, st));
         if (out16_rows) return Status::Ok();
     } else if (p.impl == 0) {
-        CUDA_TRY(launch_gather_rows(s->xr16, s->R.col_src_tok, batch * s->K, s->H, s->x16, st));
+        if (!single) CUDA_TRY(launch_gather_rows(s->xr16, s->R.col_src_tok, batch * s->K, s->H, s->x16, st));
         // persistent grid, one CTA per SM; LUMEN_MOE_FLAG_TC_CTAS leaves some SMs to kernels that run beside it
         int sms = s->sms;
         if (s->tc_ctas > 0 && s->tc_ctas < sms) sms = s->tc_ctas;
@@ -564,7 +565,7 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
             p.debug_extra_tx = 1;
             s->expire_next[1] = 0;
         }
-        CUDA_TRY(launch_grouped_tc(p, s->x16, sms, st, out16_rows));
+        CUDA_TRY(launch_grouped_tc(p, single ? s->xr16 : s->x16, sms, st, out16_rows));
     } else {
         CUDA_TRY(launch_build_xf(normed, act_dtype, batch, s->H, layer.dev.kg_h * 4, bf16_mode, s->xf, st));
         DecodeArgs a = make_decode_args(s, layer, batch);

@@ -14,8 +14,13 @@ enum Quant : int { Q8_0 = 0, Q4_0 = 1, BF16 = 2 };
 constexpr int MAX_EXPERTS = 256;  // cuda/shaders/moe_router.cu:33
 // Columns per tile of the tcgen05 gate/up product (the down tiles of a one-GPU call follow it): 256 once the
 // experts average more than 128 columns (each dequantised weight tile then serves twice the
-// columns), else 128 (fewer empty columns in ragged tiles, epilogue overlapped).
-inline int tc_gu_tile_cols(int columns, int experts) { return (columns > 128 * experts) ? 256 : 128; }
+// columns), else 128 (fewer empty columns in ragged tiles, epilogue overlapped); 128 too where its tiles are one wave
+// of both products, whose time is then that of one tile (a shared expert alone, 2048 x 512: 300 tokens 47 -> 41 us,
+// 1024 49 -> 46; at 4096, two waves down, 67 us with 256 and 73 with 128).
+inline int tc_gu_tile_cols(int columns, int experts, int hidden, int inter, int sms) {
+    const int mt = inter / 128 > hidden / 256 ? inter / 128 : hidden / 256;
+    return (columns > 128 * experts && columns / 128 * mt > sms) ? 256 : 128;
+}
 constexpr int MAX_TOP_K = 16;     // cuda/shaders/moe_router.cu:34
 constexpr int DECODE_MAX_TOKENS = 16;
 
@@ -220,6 +225,7 @@ struct PrefillArgs {
     const float* weights_in; // [T,K] or null (= 1)
 };
 cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st);
+bool route_single_applicable(const PrefillArgs& a);  // one expert: launch_route_large leaves the operand plane in xr16, columns = tokens
 // tcgen05 router (route_tc.cu)
 cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, bool natural, cudaStream_t st);
 // f16 planes of the activations (see route_tc.cu); any_lo null = high plane only

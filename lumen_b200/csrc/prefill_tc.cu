@@ -878,7 +878,7 @@ static cudaError_t launch_tc_one(const tc::Args& a, int grid, cudaStream_t st) {
 cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, cudaStream_t st, __half* out16_rows,
                               const TcPlan* plan, const TcPeerOut* peer) {
     const int C = plan ? plan->rows : p.T * p.K;
-    const int gu_cols = plan ? plan->gu_cols : tc_gu_tile_cols(C, p.L.E);  // as the tile lists were built
+    const int gu_cols = plan ? plan->gu_cols : tc_gu_tile_cols(C, p.L.E, p.L.H, p.L.I, p.sms);  // as the tile lists were built
     const int max_ct = C / gu_cols + p.L.E;
     // Down tiles: up to 256 tokens (two accumulator sets at once, no epilogue overlap between such
     // tiles) when the gate/up tiles are 256 wide, except with a tile plan of an expert-parallel call,
