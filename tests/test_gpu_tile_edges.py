@@ -1,0 +1,159 @@
+"""The kernels of the prompt and batch paths at the sizes where they can go wrong: edges of column chunks and
+tiles, remainders, the first and last size on each side of a dispatch rule. Against the CPU reference."""
+import numpy as np
+import pytest
+import torch
+
+from lumen_b200 import moe, synth
+from oracle import oracle
+from tests.gpu_util import TOL_REL_L2, make_layer, oracle_layer, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def logits_for_counts(counts, K):
+    """Logits under which expert e is the choice of counts[e] consecutive (token, slot) pairs (K distinct experts a token)."""
+    E = len(counts)
+    left = np.asarray(counts).copy()
+    rows = []
+    while left.max() > 0:
+        pick = np.argsort(-left, kind="stable")[:K]
+        row = np.full(E, -20.0, np.float32)
+        row[pick] = np.linspace(1.0, 0.0, K)
+        left[pick] -= 1
+        rows.append(row)
+    return torch.from_numpy(np.stack(rows)).cuda()
+
+
+def check_prefill(H, I, E, K, quant, lg, act=torch.float32):
+    T = lg.shape[0]
+    lay, meta, blob_np, sc, layer = make_layer(H, I, E, K, quant, seed=T, max_tokens=T)
+    g = torch.Generator("cuda").manual_seed(T + 1)
+    x = torch.randn((T, H), generator=g, device="cuda").to(act)
+    res = torch.randn((T, H), generator=g, device="cuda")
+    sc.set_logits_override(lg)
+    out = sc.prefill(layer, x, res)
+    r = sc.get_routing(T)
+    o_out, o_ids, o_w = oracle_layer(blob_np, meta, lay, K, x.float().cpu().numpy(), res.cpu().numpy(), logits=lg.cpu().numpy())
+    assert np.array_equal(r["ids"], o_ids)
+    assert rel_l2((out - res).cpu().numpy(), o_out - res.cpu().numpy()) < TOL_REL_L2
+    assert torch.equal(out, sc.prefill(layer, x, res))
+
+
+# streaming kernels: chunks of 32 columns, operands of 8; experts with none, one, one more than an operand or a chunk
+@pytest.mark.parametrize("quant", [0, 1])
+@pytest.mark.parametrize("H,I", [(256, 128), (640, 384)])
+def test_streaming_prefill_chunk_edges(cuda_lib, quant, H, I):
+    counts = [0, 1, 7, 8, 9, 16, 17, 31, 0, 33, 2, 0, 1, 1, 1, 1]  # 128 columns: below the limit of 16 experts
+    check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1))
+
+
+# the last batch on the streaming kernels and the first on the tcgen05 ones (9 | 12 columns an expert)
+@pytest.mark.parametrize("quant,T", [(0, 36), (0, 37), (1, 48), (1, 49)])
+def test_prefill_on_both_sides_of_the_streaming_limit(cuda_lib, quant, T):
+    check_prefill(384, 256, 16, 4, quant, synth.zipf_logits(T, 16, 3), torch.bfloat16)
+
+
+# tcgen05 rings and claims: contractions of a few stages, tiles of 128 and of 256 columns (one wave of tiles: 128)
+@pytest.mark.parametrize("quant", [0, 1, 2])
+@pytest.mark.parametrize("H,I,E,T", [(512, 512, 8, 257), (256, 1024, 8, 640), (768, 128, 4, 6200)])
+def test_tcgen05_tiles_of_short_contractions(cuda_lib, quant, H, I, E, T):
+    check_prefill(H, I, E, 2, quant, synth.uniform_logits(T, E, 7))
+
+
+# batches of the decode chain for each format, at contractions with a remainder against the ring's chunk
+@pytest.mark.parametrize("quant,T", [(0, 3), (0, 16), (1, 5), (1, 16), (2, 5), (2, 9), (2, 16)])
+def test_decode_chain_wide_layer(cuda_lib, quant, T):
+    H, I, E, K = 4096, 1408, 8, 2
+    lay, meta, blob_np, sc, layer = make_layer(H, I, E, K, quant, seed=T)
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=g, device="cuda")
+    gamma = 1 + 0.1 * torch.randn(H, generator=g, device="cuda")
+    normed = torch.empty_like(x)
+    out = sc.decode_fused_norm(layer, x, gamma, 1e-6, normed)
+    r = sc.get_routing(T)
+    o_normed = oracle.rmsnorm(x.cpu().numpy(), gamma.cpu().numpy(), 1e-6)
+    np.testing.assert_allclose(normed.cpu().numpy(), o_normed, rtol=2e-6, atol=1e-7)
+    o_out, _, _ = oracle.moe_layer(blob_np, 0, meta.expert_gate_offs, meta.expert_up_offs, meta.expert_down_offs, quant, H, I,
+                                   E, K, o_normed, x.cpu().numpy(), ids=r["ids"], weights=r["weights"], threads=8)
+    assert rel_l2((out - x).cpu().numpy(), o_out - x.cpu().numpy()) < TOL_REL_L2
+
+
+# the small router with one and with two rows of experts a warp, at widths with a remainder
+@pytest.mark.parametrize("E,H,T", [(256, 1024, 5), (256, 2080, 16), (128, 4096, 7), (8, 320, 16)])
+def test_small_router_rows(cuda_lib, E, H, T):
+    K = min(8, E)
+    lay, meta, blob_np, sc, layer = make_layer(H, 128, E, K, 1, seed=E, max_tokens=T)
+    x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(T), device="cuda")
+    ids, w, lg = sc.route_only(layer, x, want_logits=True)
+    router = blob_np[:lay.router_bytes].view(np.float32).reshape(E, H)
+    np.testing.assert_allclose(lg.cpu().numpy(), x.cpu().numpy().astype(np.float64) @ router.T.astype(np.float64), rtol=0, atol=5e-5)
+    o_ids, o_w = oracle.topk_from_logits(lg.cpu().numpy(), K, 0)
+    assert np.array_equal(ids.cpu().numpy().astype(np.uint32), o_ids)
+    assert np.array_equal(w.cpu().numpy().view(np.uint32), o_w.view(np.uint32))
+
+
+# one CTA sorts up to 2048 pairs, the general chain more; experts beyond one warp's 128
+@pytest.mark.parametrize("T,E,K", [(256, 128, 8), (257, 128, 8), (2048, 16, 1), (2049, 16, 1), (129, 256, 16), (700, 33, 5)])
+def test_sorting_on_both_sides_of_one_cta(cuda_lib, T, E, K):
+    lg = synth.zipf_logits(T, E, T)
+    sc = moe.allocate_moe_scratch(256, 128, E, K, T)
+    ids, w = sc.topk_from_logits(lg)
+    r = sc.get_routing(T)
+    o_ids, o_w = oracle.topk_from_logits(lg.cpu().numpy(), K, 0)
+    assert np.array_equal(ids.cpu().numpy().astype(np.uint32), o_ids)
+    assert np.array_equal(w.cpu().numpy().view(np.uint32), o_w.view(np.uint32))
+    ce, cst, d2c, bounds = oracle.counting_sort(o_ids, E)
+    assert np.array_equal(r["dst_to_col"], d2c) and np.array_equal(r["col_src_tok"], cst) and np.array_equal(r["expert_bounds"], bounds)
+
+
+# tcgen05 router: a token's logits are the same in tiles of 32 and of 128 tokens
+@pytest.mark.parametrize("E", [128, 256])
+def test_router_tiles_of_32_and_128_tokens_agree(cuda_lib, E):
+    H, T = 512, 6100
+    lay = synth.LayerLayout(H, 128, E, 1)
+    sc = moe.allocate_moe_scratch(H, 128, E, 8, T)
+    layer = sc.prepare_router_only(synth.make_layer_blob(lay, 9), lay.meta().router_weight_off)
+    x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(1), device="cuda")
+    _, _, big = sc.route_only(layer, x, want_logits=True)
+    for lo, hi in ((0, 31), (33, 98), (6000, 6100)):
+        _, _, lg = sc.route_only(layer, x[lo:hi].contiguous(), want_logits=True)
+        assert torch.equal(lg, big[lo:hi])
+
+
+# the norm that is folded into the operand planes: one to four register chunks a row, whole and partial
+@pytest.mark.parametrize("H", [512, 2048, 2304, 4096, 6400, 8192])
+def test_norm_folded_into_the_planes_matches_the_norm_kernel(cuda_lib, H):
+    T, E, K = 33, 16, 2
+    lay = synth.LayerLayout(H, 128, E, 1)
+    sc = moe.allocate_moe_scratch(H, 128, E, K, T)
+    layers = [sc.prepare_layer(synth.make_layer_blob(lay, s), lay.meta()) for s in (1, 2)]
+    g = torch.Generator("cuda").manual_seed(H)
+    gammas = [1 + 0.1 * torch.randn(H, generator=g, device="cuda") for _ in layers]
+    x0 = torch.randn((T, H), generator=g, device="cuda")
+    x = x0.clone()
+    sc.stack_prefill(layers, gammas, x, 1e-6)
+    y = x0
+    for layer, gamma in zip(layers, gammas):
+        y = sc.prefill(layer, moe.rmsnorm(y, gamma, 1e-6), y)
+    assert torch.equal(x, y)
+
+
+# a context of one expert: routing, operand plane and plan in one kernel of 8 tokens a CTA, then streaming up to 16
+# columns, tiles of 128 in one wave, tiles of 256 beyond
+@pytest.mark.parametrize("quant", [0, 1, 2])
+@pytest.mark.parametrize("T,act,gating", [(1, torch.float32, 2), (9, torch.bfloat16, 2), (16, torch.float32, 3), (17, torch.bfloat16, 2),
+                                          (129, torch.float32, 3), (9500, torch.bfloat16, 2)])
+def test_single_expert_prefill(cuda_lib, quant, T, act, gating):
+    H, I = 768, 256
+    lay, meta, blob_np, sc, layer = make_layer(H, I, 1, 1, quant, seed=T, max_tokens=T, gating=gating)
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=g, device="cuda").to(act)
+    res = torch.randn((T, H), generator=g, device="cuda")
+    out = sc.prefill(layer, x, res)
+    o_out, _, _ = oracle.moe_layer(blob_np, int(meta.router_weight_off), meta.expert_gate_offs, meta.expert_up_offs, meta.expert_down_offs,
+                                   quant, H, I, 1, 1, x.float().cpu().numpy(), res.cpu().numpy(), gating=gating,
+                                   threads=oracle.hardware_threads())
+    assert rel_l2((out - res).cpu().numpy(), o_out - res.cpu().numpy()) < TOL_REL_L2
+    r = sc.get_routing(T)
+    assert (r["ids"] == 0).all() and np.array_equal(r["dst_to_col"].ravel(), np.arange(T))
