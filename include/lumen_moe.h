@@ -76,7 +76,7 @@ typedef struct {
 /* Kernel selection is part of the configuration, never of the environment (the reference
  * selects its kernel generations through ~30 environment variables, cuda/moe.rs:1304-1561;
  * this library reads none).
- * DECODE_SPLIT: 1..4-token decode on the three-kernel chain instead of the persistent
+ * DECODE_SPLIT: 1..4-token decode on the kernel chain instead of the persistent
  *   cooperative kernel (for a process that cannot give the kernel every SM of the device).
  * PREFILL_MMA: grouped products on mma.sync instead of tcgen05 (values outside f16 range).
  * SHORT_WAITS: device-side bounded waits give up after 2 ms instead of 1-2 s (tests).
@@ -465,7 +465,7 @@ LUMEN_MOE_API lumen_moe_status_t lumen_moe_debug_decode_phase(lumen_moe_ctx* ctx
  * done, 9 end, 10 weight tiles requested (predicted expert set), 11 last staged
  * gate/up tile arrived. d_trace: [SM count][12] uint64 on the device, zeroed by the
  * caller.
- * LUMEN_MOE_UNSUPPORTED when the call's shape takes the three-kernel chain. */
+ * LUMEN_MOE_UNSUPPORTED when the call's shape takes the kernel chain. */
 LUMEN_MOE_API lumen_moe_status_t lumen_moe_debug_decode_trace(lumen_moe_ctx* ctx, const lumen_moe_layer* layer,
                                                               uint64_t* d_trace, void* stream);
 

@@ -1,7 +1,8 @@
-// Decode path (1..16 tokens) of the MoE FFN: three kernels chained with
-// programmatic dependent launch.
+// Decode path (1..16 tokens) of the MoE FFN as a chain of kernels launched as programmatic dependents: the
+// router here, the expert products in decode_small.cu and stream.cu; the rule between chain and fused kernel; and
+// the gate/up and down kernels of the mma.sync prefill path.
 //
-//   router_small_kernel   one CTA per expert: router logit(s) W_r[e]·x[t]
+//   router_small_kernel   one or two expert rows per CTA: router logit(s) W_r[e]·x[t]
 //                         (moe_router_logits_v2, cuda/shaders/moe_batched.cu:708),
 //                         optional fused FFN RMSNorm (cuda/shaders/norm.cu:28-76),
 //                         activation fragments; the last CTA to finish (fence +
@@ -13,15 +14,10 @@
 //                         (cuda/shaders/moe_expert_q4_0.cu:58-108, moe_expert.cu:62-97).
 //                         The form of the mma.sync prefill path; decode batches take
 //                         gate_up_stream_kernel (decode_small.cu) or the kernel of stream.cu.
-//   down_combine_kernel   per 16 rows of H: down rows of every selected expert
-//                         (moe_expert_q4_0.cu:118-151; integer tensor cores on int8 SwiGLU
-//                         values after gate_up_stream_kernel) and the weighted combine
-//                         out = residual + sum_k w_k d_k in slot order
-//                         (cuda/shaders/moe_accum.cu:22-46, cuda/moe.rs:6508-6524).
+//   down_general_kernel   its down product (moe_expert_q4_0.cu:118-151).
 //
-// All three are HBM-bound: each weight byte is read exactly once with 128-bit
-// streaming loads, every load of a warp's share is in flight before the first
-// use, and the arithmetic runs on the tensor cores (mma_frag.cuh).
+// The products are HBM-bound: each weight byte is read once with 128-bit loads, and the
+// arithmetic runs on the tensor cores (mma_frag.cuh).
 #include "decode_common.cuh"
 #include <type_traits>
 #include "router.cuh"

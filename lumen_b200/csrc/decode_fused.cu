@@ -1,6 +1,6 @@
 // One persistent kernel for a whole MoE layer call at decode batches of 1..4 tokens.
 //
-// The three-kernel chain (router -> gate/up -> down) pays a kernel boundary twice;
+// The kernel chain (router -> gate/up -> down) pays a kernel boundary twice;
 // at batch 1 a layer is only ~22 MB of weights, so those boundaries cost more than
 // the streaming itself. Here one CTA per SM stays resident and the two boundaries
 // become grid barriers:

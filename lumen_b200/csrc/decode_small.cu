@@ -10,7 +10,7 @@ using namespace dcommon;
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// gate/up + SwiGLU for decode batches of 5..16 tokens, Q4_0 with int8 activations: streaming form.
+// gate/up + SwiGLU for decode batches, Q4_0 with int8 activations: streaming form.
 //
 // One CTA per (16 rows of I, expert) is a chain of a few microseconds (descriptor, weights, products, a
 // reduction across its warps, SwiGLU) and 13 waves of them at 16 tokens. Here a WARP owns a whole item
@@ -197,7 +197,7 @@ static size_t gate_up_stream_smem(const DecodeArgs& a) {
 }
 
 // The streaming gate/up kernel and the int8 down product that consumes its output: Q4_0 layers,
-// 2..16 tokens (whenever the three-kernel chain runs; from four tokens on it is also faster than the
+// 2..16 tokens (whenever the kernel chain runs; from four tokens on it is also faster than the
 // fused kernel), batch activations + rings within shared memory.
 bool decode_stream_applicable(const DecodeArgs& a) {
     return a.L.quant == Q4_0 && a.xq != nullptr && a.sq != nullptr && a.T >= 2 && a.T <= DECODE_MAX_TOKENS &&

@@ -97,8 +97,8 @@ struct CudaMoeScratch {
     int cap_tokens = 0;  // capacity of the token-sized buffers below
     RouteDev R{};
     uint4* xf = nullptr;    // decode activation fragments
-    unsigned* xq = nullptr; // decode activations as two-term int8 blocks (Q4_0 gate/up of the three-kernel chain)
-    unsigned* sq = nullptr; // SwiGLU outputs of a 5..16-token Q4_0 decode in the same form, per compact column
+    unsigned* xq = nullptr; // decode activations as two-term int8 blocks (Q4_0 gate/up of the kernel chain)
+    unsigned* sq = nullptr; // SwiGLU outputs of a Q4_0 decode chain in the same form, per compact column
     uint4* sf = nullptr;    // decode SwiGLU fragments
     float* d32 = nullptr;   // decode down outputs by compact column
     float* s_f32 = nullptr; // optional debug copy
@@ -126,7 +126,7 @@ struct CudaMoeScratch {
     DecodeArgs last_decode{};   // arguments of the most recent decode call (instrumentation)
     bool has_last_decode = false;
     int prefill_impl = 0;
-    int decode_impl = 0;            // 0 = fused persistent kernel where it applies, 1 = three-kernel chain
+    int decode_impl = 0;            // 0 = fused persistent kernel where it applies, 1 = kernel chain
     unsigned int* bar = nullptr;    // grid barrier words of the fused decode kernel
     void* arena = nullptr;       // one allocation for the fixed-size part
     void* arena_tok = nullptr;   // one allocation for the token-sized part

@@ -100,14 +100,14 @@ struct DecodeArgs {
     float* out;             // [T,H]
     const float* logits_override;  // [T,E] or null
     uint4* xf;              // activation fragments [T][2][kg_h*4][4]
-    unsigned* xq;           // two-term int8 activations [T][xq_tok_words] of the three-kernel chain's Q4_0 gate/up (null = f16 fragments in xf)
-    unsigned* sq;           // two-term int8 SwiGLU outputs [C][xq_tok_words(kg_i*4)]: down operand of the 5..16-token Q4_0 chain (null = f16 fragments in sf)
+    unsigned* xq;           // two-term int8 activations [T][xq_tok_words] of the kernel chain's Q4_0 gate/up (null = f16 fragments in xf)
+    unsigned* sq;           // two-term int8 SwiGLU outputs [C][xq_tok_words(kg_i*4)]: down operand of the Q4_0 chain (null = f16 fragments in sf)
     uint4* sf;              // SwiGLU fragments     [C][2][kg_i*4][4]
     float* s_f32;           // optional [C,I] f32 copy of the SwiGLU output (null = skip)
     int T, K, gating;
     int sms;                // multiprocessors of the device
-    float* d32;             // [C,H] unweighted down outputs by compact column (three-kernel chain)
-    unsigned int* bar;      // grid barrier of the fused kernel: arrival counter + per-CTA barrier counts (1024 words); null = three-kernel chain
+    float* d32;             // [C,H] unweighted down outputs by compact column (kernel chain)
+    unsigned int* bar;      // grid barrier of the fused kernel: arrival counter + per-CTA barrier counts (1024 words); null = kernel chain
     int32_t* status;        // context status word (non-zero after a bounded wait expired)
     int32_t* status_host;   // the same code for the host: a word of mapped pinned host memory (null = none)
     unsigned wait_limit_us; // limit of every device-side wait of this launch (0 = one second)
@@ -184,7 +184,7 @@ cudaError_t launch_route_small(const DecodeArgs& a, cudaStream_t st);  // router
 bool decode_fused_applicable(const DecodeArgs& a);
 bool decode_uses_fused(const DecodeArgs& a);  // whether launch_decode takes the fused kernel for this call
 cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st);
-cudaError_t launch_decode_phase(const DecodeArgs& a, int phase, cudaStream_t st);  // one kernel of the three-kernel chain: 0 router, 1 gate/up, 2 down
+cudaError_t launch_decode_phase(const DecodeArgs& a, int phase, cudaStream_t st);  // one kernel of the kernel chain: 0 router, 1 gate/up, 2 down
 cudaError_t launch_quantize(const float* src, int64_t n, int quant, void* dst, cudaStream_t st);
 cudaError_t launch_rmsnorm(const float* x, const float* gamma, float* out, int T, int H, float eps,
                            cudaStream_t st);

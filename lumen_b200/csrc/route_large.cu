@@ -6,7 +6,8 @@
 //   router_logits_large_kernel  logits[T,E] = X[T,H] W_r[E,H]^T, f32 accumulate
 //                               (moe_router_logits_batched, cuda/shaders/moe_grouped.cu:79)
 //   topk_large_kernel           one warp per token (router.cuh)
-//   sort_hist / sort_scan / sort_place
+//   route_single_kernel         contexts of one expert: everything up to the plan in one pass
+//   sort_one_kernel (up to 2048 pairs), sort_hist / sort_rowscan / sort_scan / sort_place
 //                               stable counting sort of (token, slot) pairs by
 //                               expert, tokens ascending then slots ascending:
 //                               expert_bounds, col_expert, col_src_tok, dst_to_col
