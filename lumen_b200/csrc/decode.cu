@@ -577,9 +577,11 @@ cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st);
 // kernels stream faster. Measured us per call, fused / chain, at H = 2048, I = 768, E = 128, top-8 (40 MB Q8_0, 75 MB
 // BF16 per token): Q8_0 32.8 / 33.7 at two tokens, 41.2 / 39.7 at three; BF16 32.6 / 29.7 at one, 66 / 38 at two; at
 // H = 1024, I = 512, top-6: Q8_0 24.0 / 23.6 at three, BF16 24.8 / 22.1 at two. Q4_0: fused up to three tokens (32.8 us
-// at three; with activations as fine as its own the chain takes 33.7), the int8 chain from four (38 / 31 us).
+// at three; with activations as fine as its own the chain takes 33.7), the int8 chain from four (38 / 31 us). One expert:
+// always fused where it applies (four tokens of Q4_0 13.2 us, the chain 19.4).
 bool decode_uses_fused(const DecodeArgs& a) {
     if (!decode_fused_applicable(a)) return false;
+    if (a.L.E == 1) return true;
     const double weights = 3.0 * a.T * a.K * a.L.I * a.L.H;
     switch (a.L.quant) {
         case Q4_0: return a.T < 4 || !decode_stream_applicable(a);

@@ -202,6 +202,10 @@ struct RouteSm {
 // block's precomputed 8 * sx * sum(q0 + q1 / 254).
 constexpr bool kInt8GateUp = true;
 
+__host__ __device__ inline bool single_expert(const DecodeArgs& a) {
+    return a.L.E == 1 && a.K == 1 && a.gating >= 2 && a.logits_override == nullptr;
+}
+
 struct TopkSm {
     float lg[FMAX_T][MAX_EXPERTS];
     float p[FMAX_T][MAX_EXPERTS];
@@ -210,7 +214,7 @@ struct TopkSm {
 
 }  // namespace
 
-template <int Q>
+template <int Q, bool SINGLE>
 __global__ void __launch_bounds__(FT, 1)
 decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, const int gs_slots, const int gs_alias) {
     extern __shared__ uint4 dyn[];
@@ -267,11 +271,62 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
     };
     const SmallDiv div_kgi(kg_i), div_rti(a.L.rt_i), div_g(G);
 
+    const int rt_i = a.L.rt_i;
+    const int it0 = G - 1 - cta;  // work items of this CTA: G-1-cta, then every G-th (CTAs without down rows first)
+    const bool has_down = cta < a.L.rt_h;
+    // Requests every byte this CTA needs for the experts ue[0..nu), called by ONE warp: the
+    // tiles of its first gs_slots gate/up items (all input groups of a matrix are contiguous:
+    // one bulk copy for the quants, one for the scales; barrier j counts item j's bytes), then
+    // the down tiles of its 16 output rows for the first pf_experts experts (barrier 7).
+    // copy r of work item j (its j-th for this CTA) into ring slot sl: r = matrix * PER + {quants, scales}
+    auto copy_gu = [&](int j, int sl, int r, const int* ue) {
+        constexpr int PER_ = (Q != BF16) ? 2 : 1;
+        const int mat = r / PER_, is_s = r - mat * PER_;
+        const int it = it0 + j * G;
+        const int u = div_rti.div(it), rt = it - u * rt_i;
+        const int e = ue[u];
+        uint4* dst = gs_slot(sl) + (size_t)mat * kg_h * TU4 + (is_s ? kg_h * NQ32 : 0);
+        const uint4* src = is_s ? (mat ? a.L.up_s(e) : a.L.gate_s(e)) + (size_t)rt * kg_h * 8
+                                : (mat ? a.L.up_q(e) : a.L.gate_q(e)) + (size_t)rt * kg_h * NQ32;
+        bulk_copy(dst, src, is_s ? (unsigned)kg_h * 128 : (unsigned)kg_h * NQ32 * 16, &mbar[sl]);
+    };
+    auto stage_all = [&](const int* ue, int nu) {
+        const int n_items_ = nu * rt_i;
+        const int n_my_ = (it0 < n_items_) ? div_g.div(n_items_ - it0 + G - 1) : 0;
+        const int n_st_ = min(n_my_, gs_slots);
+        const int n_pf_ = has_down ? min(nu, pf_experts) : 0;
+        const unsigned q_gu = (unsigned)kg_h * NQ32 * 16, s_gu = (Q != BF16) ? (unsigned)kg_h * 128 : 0u;
+        const unsigned q_dn = (unsigned)kg_i * NQ32 * 16, s_dn = (Q != BF16) ? (unsigned)kg_i * 128 : 0u;
+        if (lane < n_st_) mbar_expect_tx(&mbar[lane], 2u * (q_gu + s_gu));
+        if (lane == 7) mbar_expect_tx(&mbar[7], (unsigned)n_pf_ * (q_dn + s_dn));
+        __syncwarp();
+        constexpr int PER = (Q != BF16) ? 2 : 1;  // copies per matrix: quants, scales
+#pragma unroll 1
+        for (int c = lane; c < n_st_ * 2 * PER; c += 32) copy_gu(c / (2 * PER), c / (2 * PER), c % (2 * PER), ue);
+#pragma unroll 1
+        for (int c = lane; c < n_pf_ * PER; c += 32) {
+            const int uu = c / PER, is_s = c - uu * PER;
+            const int ee = ue[uu];
+            uint4* dst = pf + ((size_t)uu * kg_i) * TU4 + (is_s ? kg_i * NQ32 : 0);
+            const uint4* src = is_s ? a.L.down_s(ee) + (size_t)cta * kg_i * 8 : a.L.down_q(ee) + (size_t)cta * kg_i * NQ32;
+            bulk_copy(dst, src, is_s ? s_dn : q_dn, &mbar[7]);
+        }
+    };
+    // SINGLE: one expert (the shared expert): its tiles are requested right away, before the wait for the previous kernel; every
+    // CTA works out the gate logit itself and there is nothing to rank or sort, so barrier 1 falls away. 2048 x 512, three
+    // tokens: 14.5 -> 12.5 us in any format. (As a branch of the general kernel instead of an instance, every other call took
+    // 0.5 us longer: the instruction stream is what bounds them.)
+    if (SINGLE && warp == 0) {
+        if (lane == 0) rs.ue[0] = 0;
+        __syncwarp();
+        stage_all(rs.ue, 1);
+    }
+
     // ---------------- phase A ----------------
     // first router row in registers before waiting on the previous kernel (weights are static)
     float4 wv = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (want_logits && cta < E && tid < H4)
-        wv = __ldg(reinterpret_cast<const float4*>(a.L.router_w + (size_t)cta * H) + tid);
+    if (want_logits && (SINGLE || cta < E) && tid < H4)
+        wv = __ldg(reinterpret_cast<const float4*>(a.L.router_w + (SINGLE ? 0 : (size_t)cta * H)) + tid);
     pdl_wait();
     stamp(1);
     // Thread i holds inputs 4i..4i+3 of every token (H <= 4 * FT): they feed the router
@@ -283,7 +338,14 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
         xv[t] = (t < T && tid < H4) ? reinterpret_cast<const float4*>(a.x)[t * H4 + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int status_now = *reinterpret_cast<volatile int*>(a.status);
     unsigned epoch = *reinterpret_cast<volatile unsigned*>(a.bar + 1 + cta);  // barriers this CTA has passed so far
-    if (status_now != 0) return;  // an earlier launch gave up: do not touch the barrier
+    if (status_now != 0) {  // an earlier launch gave up: do not touch the barrier
+        if (SINGLE) {       // (nor leave with copies in flight)
+            __syncthreads();
+            for (int j = 0; j < gs_slots && it0 + j * G < rt_i; ++j) mbar_wait(&mbar[j], 0, wc);
+            mbar_wait(&mbar[7], 0, wc);
+        }
+        return;
+    }
 
     // normalised activations of all tokens, f32, in shared memory for the fragment build (the
     // region is reused for the SwiGLU fragments and partial sums, written only after the routing)
@@ -326,7 +388,51 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
     for (int t = 0; t < FMAX_T; ++t)
         if (t < T && tid < H4) xn4[t * H4 + tid] = xv[t];
 
-    if (want_logits) {
+    if (SINGLE) {
+#pragma unroll
+        for (int t = 0; t < FMAX_T; ++t) {
+            if (t < T) {
+                float acc = wv.x * xv[t].x + wv.y * xv[t].y + wv.z * xv[t].z + wv.w * xv[t].w;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                if (lane == 0) red_a[warp][t] = acc;
+            }
+        }
+        if (tid < 32) ts.tab[tid] = tab_entry;
+        __syncthreads();
+        if (tid < T) {
+            float v = 0.0f;
+#pragma unroll
+            for (int w = 0; w < FW; ++w) v += red_a[w][tid];
+            float wt = 1.0f;  // gating 3
+            if (a.gating == 2) {
+                const float ex = lumen_exact::expf_libm_tab(-v, lumen_exact::Exp2TabPtr{reinterpret_cast<const uint64_t*>(ts.tab)});
+                wt = __fdiv_rn(1.0f, __fadd_rn(1.0f, ex));
+            }
+            rs.w[tid] = wt;
+            rs.d2c[tid] = tid;
+            rs.col_u[tid] = 0;
+            rs.col_tok[tid] = tid;
+            if (cta == 0) {
+                a.R.ids[tid] = 0u;
+                a.R.weights[tid] = wt;
+                a.R.dst_to_col[tid] = tid;
+                a.R.col_expert[tid] = 0;
+                a.R.col_src_tok[tid] = tid;
+            }
+        }
+        if (tid == 0) {
+            rs.uc0[0] = 0;
+            rs.uncol[0] = T;
+            rs.U = 1;
+            if (cta == 0) {
+                a.R.uexp[0] = 0;
+                *a.R.n_uexp = 1;
+                a.R.expert_bounds[0] = 0;
+                a.R.expert_bounds[1] = T;
+            }
+        }
+    } else if (want_logits) {
 #pragma unroll 1
         for (int e = cta; e < E; e += G) {
             float4 w4 = wv;
@@ -396,7 +502,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
     }
     stamp(2);
     // barrier 1: wait for (and fetch) every logit of this launch
-    {
+    if (!SINGLE) {
         const float* lg = a.logits_override;
         bool ok = true;
 #pragma unroll 1
@@ -442,48 +548,9 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
     // needs. So: rank the raw logits, request every tile for the predicted set, run the
     // exact gating while the tiles stream, then check the prediction and, if it was wrong,
     // drain and request again.
-    const int rt_i = a.L.rt_i;
-    const int it0 = G - 1 - cta;  // work items of this CTA: G-1-cta, then every G-th (CTAs without down rows first)
-    const bool has_down = cta < a.L.rt_h;
-    // Requests every byte this CTA needs for the experts ue[0..nu), called by ONE warp: the
-    // tiles of its first gs_slots gate/up items (all input groups of a matrix are contiguous:
-    // one bulk copy for the quants, one for the scales; barrier j counts item j's bytes), then
-    // the down tiles of its 16 output rows for the first pf_experts experts (barrier 7).
-    // copy r of work item j (its j-th for this CTA) into ring slot sl: r = matrix * PER + {quants, scales}
-    auto copy_gu = [&](int j, int sl, int r, const int* ue) {
-        constexpr int PER_ = (Q != BF16) ? 2 : 1;
-        const int mat = r / PER_, is_s = r - mat * PER_;
-        const int it = it0 + j * G;
-        const int u = div_rti.div(it), rt = it - u * rt_i;
-        const int e = ue[u];
-        uint4* dst = gs_slot(sl) + (size_t)mat * kg_h * TU4 + (is_s ? kg_h * NQ32 : 0);
-        const uint4* src = is_s ? (mat ? a.L.up_s(e) : a.L.gate_s(e)) + (size_t)rt * kg_h * 8
-                                : (mat ? a.L.up_q(e) : a.L.gate_q(e)) + (size_t)rt * kg_h * NQ32;
-        bulk_copy(dst, src, is_s ? (unsigned)kg_h * 128 : (unsigned)kg_h * NQ32 * 16, &mbar[sl]);
-    };
-    auto stage_all = [&](const int* ue, int nu) {
-        const int n_items_ = nu * rt_i;
-        const int n_my_ = (it0 < n_items_) ? div_g.div(n_items_ - it0 + G - 1) : 0;
-        const int n_st_ = min(n_my_, gs_slots);
-        const int n_pf_ = has_down ? min(nu, pf_experts) : 0;
-        const unsigned q_gu = (unsigned)kg_h * NQ32 * 16, s_gu = (Q != BF16) ? (unsigned)kg_h * 128 : 0u;
-        const unsigned q_dn = (unsigned)kg_i * NQ32 * 16, s_dn = (Q != BF16) ? (unsigned)kg_i * 128 : 0u;
-        if (lane < n_st_) mbar_expect_tx(&mbar[lane], 2u * (q_gu + s_gu));
-        if (lane == 7) mbar_expect_tx(&mbar[7], (unsigned)n_pf_ * (q_dn + s_dn));
-        __syncwarp();
-        constexpr int PER = (Q != BF16) ? 2 : 1;  // copies per matrix: quants, scales
-#pragma unroll 1
-        for (int c = lane; c < n_st_ * 2 * PER; c += 32) copy_gu(c / (2 * PER), c / (2 * PER), c % (2 * PER), ue);
-#pragma unroll 1
-        for (int c = lane; c < n_pf_ * PER; c += 32) {
-            const int uu = c / PER, is_s = c - uu * PER;
-            const int ee = ue[uu];
-            uint4* dst = pf + ((size_t)uu * kg_i) * TU4 + (is_s ? kg_i * NQ32 : 0);
-            const uint4* src = is_s ? a.L.down_s(ee) + (size_t)cta * kg_i * 8 : a.L.down_q(ee) + (size_t)cta * kg_i * NQ32;
-            bulk_copy(dst, src, is_s ? s_dn : q_dn, &mbar[7]);
-        }
-    };
-    {
+    if (SINGLE) {
+        __syncthreads();
+    } else {
         // Four warps per token share the exps; then warp 0 of the four finishes the token
         // exactly while another warp ranks the raw logits and requests the tiles.
         const int tok = warp >> 2, sub = warp & 3;
@@ -569,29 +636,26 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
         __syncthreads();
     }
     stamp(4);
+    unsigned par = 0;  // bit i: parity of the phase that barrier i is in
     const int U = rs.U;
     const int n_items = U * rt_i;
     const int n_down = U * kg_i;
-    {
+    if (!SINGLE) {
         bool same = (U == rs.pr_U);
         if (same && tid < U) same = (rs.ue[tid] == rs.pr_ue[tid]);
         if (__syncthreads_or(same ? 0 : 1)) {
-            // wrong prediction: let its copies land (they target the same slots), start the
-            // barriers afresh and request the right tiles
+            // wrong prediction: let its copies land (they target the same slots) and request the right
+            // tiles for the barriers' next phase (barriers set up afresh here lost arrivals now and then)
             const int n_items_p = rs.pr_U * rt_i;
             const int n_my_p = (it0 < n_items_p) ? div_g.div(n_items_p - it0 + G - 1) : 0;
             bool ok = true;
-            for (int j = 0; j < min(n_my_p, gs_slots) && ok; ++j) ok = mbar_wait(&mbar[j], 0, wc);
-            ok = ok && mbar_wait(&mbar[7], 0, wc);
-            if (__syncthreads_or(ok ? 0 : 1)) return;
-            if (tid == 0) {
-                for (int i = 0; i < 8; ++i) {
-                    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(&mbar[i])) : "memory");
-                    mbar_init(&mbar[i], 1);
-                }
-                asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            for (int j = 0; j < min(n_my_p, gs_slots) && ok; ++j) {
+                ok = mbar_wait(&mbar[j], 0, wc);
+                par |= 1u << j;
             }
-            __syncthreads();
+            ok = ok && mbar_wait(&mbar[7], 0, wc);
+            par |= 1u << 7;
+            if (__syncthreads_or(ok ? 0 : 1)) return;
             if (warp == 0) stage_all(rs.ue, U);
         }
     }
@@ -675,11 +739,11 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
         __syncthreads();
     };
     int sl = 0;          // ring slot of item j: j % gs_slots
-    unsigned ring_ph = 0;  // parity of (j / gs_slots): how often the slot has been filled
 #pragma unroll 1
     for (int j = 0; j < n_my; ++j) {
         if (gs_slots > 0) {
-            if (!mbar_wait(&mbar[sl], ring_ph, wc)) return;  // all threads give up together
+            if (!mbar_wait(&mbar[sl], (par >> sl) & 1u, wc)) return;  // all threads give up together
+            par ^= 1u << sl;
             if (a.trace != nullptr && tid == 0 && j == n_my - 1) a.trace[(size_t)blockIdx.x * 12 + 11] = global_ns();
             if (warp < kg_h) {
                 const uint4* gq_ = gs_slot(sl);
@@ -700,10 +764,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
             mbar_expect_tx(&mbar[sl], 2u * ((unsigned)kg_h * NQ32 * 16 + ((Q != BF16) ? (unsigned)kg_h * 128 : 0u)));
             for (int r = 0; r < 2 * PER_; ++r) copy_gu(j + gs_slots, sl, r, rs.ue);
         }
-        if (++sl == gs_slots) {
-            sl = 0;
-            ring_ph ^= 1u;
-        }
+        if (++sl == gs_slots) sl = 0;
     }
     // residual of this CTA's output rows, requested before the barrier
     float resid = 0.0f;
@@ -712,7 +773,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
     __syncthreads();
     grid_arrive(a.bar);
     if (!grid_wait(a.bar, wc, G, ++epoch, a.debug_extra_arrivals, &fail_s)) {
-        mbar_wait(&mbar[7], 0, wc);  // bounded: do not leave with the down copies in flight
+        mbar_wait(&mbar[7], par >> 7, wc);  // bounded: do not leave with the down copies in flight
         return;
     }
     if (tid == 0) a.bar[1 + cta] = epoch;
@@ -722,7 +783,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
     if (!has_down) return;  // (no down tiles were requested for this CTA)
     for (int i = tid; i < C * per_col_i; i += FT) cp_async16(&ss[i], a.sf + i);
     cp_async_wait_all();
-    if (!mbar_wait(&mbar[7], 0, wc)) return;
+    if (!mbar_wait(&mbar[7], par >> 7, wc)) return;
     __syncthreads();
     stamp(7);
     {
@@ -844,7 +905,7 @@ bool decode_fused_applicable(const DecodeArgs& a) {
     return fused_smem_bytes(a, tile_u4_of(a.L.quant), 0) + static_smem <= (size_t)d.smem_optin;
 }
 
-template <int Q>
+template <int Q, bool SINGLE>
 static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t st) {
     const FusedDeviceInfo& d = fused_device_info(device);
     const size_t static_smem = 20 * 1024;
@@ -858,6 +919,7 @@ static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t 
     const size_t item_bytes = (size_t)2 * a.L.kg_h * TileU4<Q>::value * 16;
     int alias = (int)(fused_mid_bytes(a) / item_bytes);
     if (alias > ring) alias = ring;
+    if (SINGLE) alias = 0;  // (tiles arrive while phase A still uses that region)
     while (ring > alias && fused_smem_bytes(a, TileU4<Q>::value, 0, ring - alias) + static_smem > (size_t)d.smem_optin) --ring;
     const int gs = ring - alias;  // slots with storage of their own
     int pf = nu_max;  // experts whose down tiles are staged
@@ -865,7 +927,7 @@ static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t 
     const size_t smem = fused_smem_bytes(a, TileU4<Q>::value, pf, gs);
     static size_t attr_smem[64] = {};
     if (smem > attr_smem[device & 63]) {
-        cudaError_t e = cudaFuncSetAttribute(decode_fused_kernel<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(decode_fused_kernel<Q, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return e;
         attr_smem[device & 63] = smem;
@@ -886,17 +948,18 @@ static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t 
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     count_launch();
-    return cudaLaunchKernelEx(&cfg, decode_fused_kernel<Q>, a, pf, ring, alias);
+    return cudaLaunchKernelEx(&cfg, decode_fused_kernel<Q, SINGLE>, a, pf, ring, alias);
 }
 
 cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
+    const bool one = single_expert(a);
     switch (a.L.quant) {
-        case Q4_0: return launch_fused_t<Q4_0>(a, device, st);
-        case Q8_0: return launch_fused_t<Q8_0>(a, device, st);
-        default: return launch_fused_t<BF16>(a, device, st);
+        case Q4_0: return one ? launch_fused_t<Q4_0, true>(a, device, st) : launch_fused_t<Q4_0, false>(a, device, st);
+        case Q8_0: return one ? launch_fused_t<Q8_0, true>(a, device, st) : launch_fused_t<Q8_0, false>(a, device, st);
+        default: return one ? launch_fused_t<BF16, true>(a, device, st) : launch_fused_t<BF16, false>(a, device, st);
     }
 }
 

@@ -157,3 +157,21 @@ def test_single_expert_prefill(cuda_lib, quant, T, act, gating):
     assert rel_l2((out - res).cpu().numpy(), o_out - res.cpu().numpy()) < TOL_REL_L2
     r = sc.get_routing(T)
     assert (r["ids"] == 0).all() and np.array_equal(r["dst_to_col"].ravel(), np.arange(T))
+
+
+# the fused decode kernel on one expert: no router exchange; items on some CTAs, on all, more than one each, ragged groups
+@pytest.mark.parametrize("quant", [0, 1, 2])
+@pytest.mark.parametrize("H,I,T,gating", [(2048, 512, 3, 2), (96, 160, 1, 2), (1024, 2816, 4, 3), (256, 4800, 2, 2)])
+def test_single_expert_fused_decode(cuda_lib, quant, H, I, T, gating):
+    lay, meta, blob_np, sc, layer = make_layer(H, I, 1, 1, quant, seed=T, gating=gating)
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=g, device="cuda")
+    res = torch.randn((T, H), generator=g, device="cuda")
+    o_out, _, o_w = oracle.moe_layer(blob_np, int(meta.router_weight_off), meta.expert_gate_offs, meta.expert_up_offs, meta.expert_down_offs,
+                                     quant, H, I, 1, 1, x.cpu().numpy(), res.cpu().numpy(), gating=gating, threads=oracle.hardware_threads())
+    outs = [sc.decode(layer, x, res).clone() for _ in range(10)]
+    assert rel_l2((outs[0] - res).cpu().numpy(), o_out - res.cpu().numpy()) < TOL_REL_L2
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    r = sc.get_routing(T)
+    assert (r["ids"] == 0).all() and np.array_equal(r["dst_to_col"].ravel(), np.arange(T)) and np.array_equal(r["expert_bounds"], [0, T])
+    np.testing.assert_allclose(r["weights"], o_w, rtol=1e-4)
