@@ -214,7 +214,7 @@ struct TopkSm {
 
 }  // namespace
 
-template <int Q, bool SINGLE>
+template <int Q, bool SINGLE, bool ONE>
 __global__ void __launch_bounds__(FT, 1)
 decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, const int gs_slots, const int gs_alias) {
     extern __shared__ uint4 dyn[];
@@ -241,7 +241,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
     }
     const int gq = lane >> 2, t4 = lane & 3;
     const int cta = blockIdx.x, G = gridDim.x;
-    const int H = a.L.H, I = a.L.I, E = a.L.E, T = a.T, K = a.K;
+    const int H = a.L.H, I = a.L.I, E = a.L.E, T = ONE ? 1 : a.T, K = a.K;
     const int C = T * K;
     const int H4 = H >> 2;
     const int kg_h = a.L.kg_h, kg_i = a.L.kg_i;
@@ -905,7 +905,7 @@ bool decode_fused_applicable(const DecodeArgs& a) {
     return fused_smem_bytes(a, tile_u4_of(a.L.quant), 0) + static_smem <= (size_t)d.smem_optin;
 }
 
-template <int Q, bool SINGLE>
+template <int Q, bool SINGLE, bool ONE>
 static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t st) {
     const FusedDeviceInfo& d = fused_device_info(device);
     const size_t static_smem = 20 * 1024;
@@ -927,7 +927,7 @@ static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t 
     const size_t smem = fused_smem_bytes(a, TileU4<Q>::value, pf, gs);
     static size_t attr_smem[64] = {};
     if (smem > attr_smem[device & 63]) {
-        cudaError_t e = cudaFuncSetAttribute(decode_fused_kernel<Q, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute((decode_fused_kernel<Q, SINGLE, ONE>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return e;
         attr_smem[device & 63] = smem;
@@ -948,18 +948,25 @@ static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t 
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     count_launch();
-    return cudaLaunchKernelEx(&cfg, decode_fused_kernel<Q, SINGLE>, a, pf, ring, alias);
+    return cudaLaunchKernelEx(&cfg, (decode_fused_kernel<Q, SINGLE, ONE>), a, pf, ring, alias);
 }
 
 cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
-    const bool one = single_expert(a);
+    const bool one = (a.T == 1);
+    if (single_expert(a)) {
+        switch (a.L.quant) {
+            case Q4_0: return launch_fused_t<Q4_0, true, false>(a, device, st);
+            case Q8_0: return launch_fused_t<Q8_0, true, false>(a, device, st);
+            default: return launch_fused_t<BF16, true, false>(a, device, st);
+        }
+    }
     switch (a.L.quant) {
-        case Q4_0: return one ? launch_fused_t<Q4_0, true>(a, device, st) : launch_fused_t<Q4_0, false>(a, device, st);
-        case Q8_0: return one ? launch_fused_t<Q8_0, true>(a, device, st) : launch_fused_t<Q8_0, false>(a, device, st);
-        default: return one ? launch_fused_t<BF16, true>(a, device, st) : launch_fused_t<BF16, false>(a, device, st);
+        case Q4_0: return one ? launch_fused_t<Q4_0, false, true>(a, device, st) : launch_fused_t<Q4_0, false, false>(a, device, st);
+        case Q8_0: return one ? launch_fused_t<Q8_0, false, true>(a, device, st) : launch_fused_t<Q8_0, false, false>(a, device, st);
+        default: return one ? launch_fused_t<BF16, false, true>(a, device, st) : launch_fused_t<BF16, false, false>(a, device, st);
     }
 }
 
