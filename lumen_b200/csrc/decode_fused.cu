@@ -37,7 +37,7 @@ using namespace dcommon;
 
 constexpr int FW = 16;        // warps per CTA
 constexpr int FT = FW * 32;   // threads per CTA
-constexpr int FMAX_T = 4;     // tokens
+constexpr int FMAX_T = FUSED_MAX_TOKENS;
 constexpr int FMAX_C = 32;    // (token, slot) pairs
 
 // n / d for 0 <= n < 2^20 and a divisor known when the kernel starts: one multiply by the
@@ -131,6 +131,23 @@ __device__ __forceinline__ bool grid_wait(unsigned* bar, const WaitCtl& wc, int 
     return *fail_s == 0;
 }
 
+// Four adjacent tagged words, polled until all carry the tag; false when the wait expired.
+__device__ __forceinline__ bool ld_tagged4(const float* slot, unsigned tag, const WaitCtl& wc, float4& v) {
+    unsigned long long t0 = 0;
+    for (unsigned spins = 0;;) {
+        const uint2 p = ld_tagged(slot), q = ld_tagged(slot + 2), r = ld_tagged(slot + 4), s = ld_tagged(slot + 6);
+        v = make_float4(__uint_as_float(p.x), __uint_as_float(q.x), __uint_as_float(r.x), __uint_as_float(s.x));
+        if (p.y == tag && q.y == tag && r.y == tag && s.y == tag) return true;
+        if ((++spins & 63u) == 0) {
+            if (t0 == 0) t0 = global_ns();
+            if (global_ns() - t0 > wc.limit_ns || *reinterpret_cast<volatile int*>(wc.status) != 0) {
+                raise_status(wc.status, wc.status_host, 4);  // LUMEN_MOE_TIMEOUT
+                return false;
+            }
+        }
+    }
+}
+
 // mbarrier + bulk-copy helpers: a weight tile range is contiguous in the fragment planes, so
 // one cp.async.bulk moves all input groups of a work item's matrix at once.
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -206,6 +223,32 @@ __host__ __device__ inline bool single_expert(const DecodeArgs& a) {
     return a.L.E == 1 && a.K == 1 && a.gating >= 2 && a.logits_override == nullptr;
 }
 
+// The layers of a stack that one launch runs through (STACK), or nothing.
+template <bool STACK>
+struct LayerList {
+    __device__ __forceinline__ int n() const { return 1; }
+    __device__ __forceinline__ float* xt() const { return nullptr; }
+    __device__ __forceinline__ const float* router(int) const { return nullptr; }
+    __device__ __forceinline__ const float* gamma(int) const { return nullptr; }
+    __device__ __forceinline__ const uint4* q_of(int) const { return nullptr; }
+    __device__ __forceinline__ const uint4* s_of(int) const { return nullptr; }
+};
+template <>
+struct LayerList<true> {
+    int layers;
+    float* x_tagged;  // [T][H] {value, tag}: a layer's output on its way to the next
+    const float* router_w[FUSED_MAX_LAYERS];
+    const float* gammas[FUSED_MAX_LAYERS];
+    const uint4* q[FUSED_MAX_LAYERS];
+    const uint4* s[FUSED_MAX_LAYERS];
+    __device__ __forceinline__ int n() const { return layers; }
+    __device__ __forceinline__ float* xt() const { return x_tagged; }
+    __device__ __forceinline__ const float* router(int l) const { return router_w[l]; }
+    __device__ __forceinline__ const float* gamma(int l) const { return gammas[l]; }
+    __device__ __forceinline__ const uint4* q_of(int l) const { return q[l]; }
+    __device__ __forceinline__ const uint4* s_of(int l) const { return s[l]; }
+};
+
 struct TopkSm {
     float lg[FMAX_T][MAX_EXPERTS];
     float p[FMAX_T][MAX_EXPERTS];
@@ -214,9 +257,9 @@ struct TopkSm {
 
 }  // namespace
 
-template <int Q, bool SINGLE, bool ONE>
+template <int Q, bool SINGLE, bool ONE, bool STACK>
 __global__ void __launch_bounds__(FT, 1)
-decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, const int gs_slots, const int gs_alias) {
+decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ LayerList<STACK> ls, const int pf_experts, const int gs_slots, const int gs_alias) {
     extern __shared__ uint4 dyn[];
     __shared__ __align__(16) TopkSm ts;
     __shared__ float red_a[FW][FMAX_T];
@@ -227,6 +270,12 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
     __shared__ __align__(8) unsigned long long mbar[8];  // 0..6: staged gate/up items, 7: staged down tiles
 
     pdl_trigger();
+    int layer = 0;
+    // of the layers of a stack only these pointers differ
+    auto router_w = [&]() { return STACK ? ls.router(layer) : a.L.router_w; };
+    auto gamma = [&]() { return STACK ? ls.gamma(layer) : a.gamma; };
+    auto plane_q = [&](int e) { return (STACK ? ls.q_of(layer) : a.L.q) + (size_t)e * a.L.q_exp; };
+    auto plane_s = [&](int e) { return (STACK ? ls.s_of(layer) : a.L.s) + (size_t)e * a.L.s_exp; };
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto stamp = [&](int i) {
         if (a.trace != nullptr && tid == 0) a.trace[(size_t)blockIdx.x * 12 + i] = global_ns();
@@ -286,8 +335,8 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
         const int u = div_rti.div(it), rt = it - u * rt_i;
         const int e = ue[u];
         uint4* dst = gs_slot(sl) + (size_t)mat * kg_h * TU4 + (is_s ? kg_h * NQ32 : 0);
-        const uint4* src = is_s ? (mat ? a.L.up_s(e) : a.L.gate_s(e)) + (size_t)rt * kg_h * 8
-                                : (mat ? a.L.up_q(e) : a.L.gate_q(e)) + (size_t)rt * kg_h * NQ32;
+        const uint4* src = is_s ? (mat ? plane_s(e) + a.L.s_gu : plane_s(e)) + (size_t)rt * kg_h * 8
+                                : (mat ? plane_q(e) + a.L.q_gu : plane_q(e)) + (size_t)rt * kg_h * NQ32;
         bulk_copy(dst, src, is_s ? (unsigned)kg_h * 128 : (unsigned)kg_h * NQ32 * 16, &mbar[sl]);
     };
     auto stage_all = [&](const int* ue, int nu) {
@@ -308,7 +357,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
             const int uu = c / PER, is_s = c - uu * PER;
             const int ee = ue[uu];
             uint4* dst = pf + ((size_t)uu * kg_i) * TU4 + (is_s ? kg_i * NQ32 : 0);
-            const uint4* src = is_s ? a.L.down_s(ee) + (size_t)cta * kg_i * 8 : a.L.down_q(ee) + (size_t)cta * kg_i * NQ32;
+            const uint4* src = is_s ? plane_s(ee) + 2 * a.L.s_gu + (size_t)cta * kg_i * 8 : plane_q(ee) + 2 * a.L.q_gu + (size_t)cta * kg_i * NQ32;
             bulk_copy(dst, src, is_s ? s_dn : q_dn, &mbar[7]);
         }
     };
@@ -324,9 +373,17 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
 
     // ---------------- phase A ----------------
     // first router row in registers before waiting on the previous kernel (weights are static)
-    float4 wv = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (want_logits && (SINGLE || cta < E) && tid < H4)
-        wv = __ldg(reinterpret_cast<const float4*>(a.L.router_w + (SINGLE ? 0 : (size_t)cta * H)) + tid);
+    auto router_row = [&]() {
+        return (want_logits && (SINGLE || cta < E) && tid < H4)
+                   ? __ldg(reinterpret_cast<const float4*>(router_w() + (SINGLE ? 0 : (size_t)cta * H)) + tid)
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    float4 wv = router_row();
+    const bool norm = STACK || a.gamma != nullptr;
+    auto gamma_row = [&]() {
+        return (norm && tid < H4) ? __ldg(reinterpret_cast<const float4*>(gamma()) + tid) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    float4 gv = gamma_row();
     pdl_wait();
     stamp(1);
     // Thread i holds inputs 4i..4i+3 of every token (H <= 4 * FT): they feed the router
@@ -346,11 +403,16 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
         }
         return;
     }
+    unsigned par = 0;    // bit i: parity of the phase that copy barrier i is in
+    float carry = 0.0f;  // STACK: this thread's element of the layer's output = residual of the next layer
+
+#pragma unroll 1
+    for (;;) {
 
     // normalised activations of all tokens, f32, in shared memory for the fragment build (the
     // region is reused for the SwiGLU fragments and partial sums, written only after the routing)
     float4* xn4 = reinterpret_cast<float4*>(ss);
-    if (a.gamma != nullptr) {
+    if (norm) {
 #pragma unroll
         for (int t = 0; t < FMAX_T; ++t) {
             if (t < T) {
@@ -361,6 +423,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
             }
         }
         __syncthreads();
+        if (STACK && fail_s) return;  // (the wait for this layer's input expired)
         if (tid < T) {
             float sq = 0.0f;
 #pragma unroll
@@ -369,7 +432,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
         }
         __syncthreads();
         if (tid < H4) {
-            const float4 g = __ldg(reinterpret_cast<const float4*>(a.gamma) + tid);
+            const float4 g = gv;
 #pragma unroll
             for (int t = 0; t < FMAX_T; ++t) {
                 if (t < T) {
@@ -436,7 +499,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
 #pragma unroll 1
         for (int e = cta; e < E; e += G) {
             float4 w4 = wv;
-            if (e != cta && tid < H4) w4 = __ldg(reinterpret_cast<const float4*>(a.L.router_w + (size_t)e * H) + tid);
+            if (e != cta && tid < H4) w4 = __ldg(reinterpret_cast<const float4*>(router_w() + (size_t)e * H) + tid);
 #pragma unroll
             for (int t = 0; t < FMAX_T; ++t) {
                 if (t < T) {
@@ -636,7 +699,6 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
         __syncthreads();
     }
     stamp(4);
-    unsigned par = 0;  // bit i: parity of the phase that barrier i is in
     const int U = rs.U;
     const int n_items = U * rt_i;
     const int n_down = U * kg_i;
@@ -650,11 +712,11 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
             const int n_my_p = (it0 < n_items_p) ? div_g.div(n_items_p - it0 + G - 1) : 0;
             bool ok = true;
             for (int j = 0; j < min(n_my_p, gs_slots) && ok; ++j) {
-                ok = mbar_wait(&mbar[j], 0, wc);
-                par |= 1u << j;
+                ok = mbar_wait(&mbar[j], (par >> j) & 1u, wc);
+                par ^= 1u << j;
             }
-            ok = ok && mbar_wait(&mbar[7], 0, wc);
-            par |= 1u << 7;
+            ok = ok && mbar_wait(&mbar[7], (par >> 7) & 1u, wc);
+            par ^= 1u << 7;
             if (__syncthreads_or(ok ? 0 : 1)) return;
             if (warp == 0) stage_all(rs.ue, U);
         }
@@ -663,8 +725,8 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
         const int u = div_rti.div(it), rt = it - u * rt_i;
         const int e = rs.ue[u];
         if (warp < kg_h) {
-            load_wtile<Q>(g, a.L.gate_q(e), a.L.gate_s(e), rt * kg_h + warp, lane);
-            load_wtile<Q>(up, a.L.up_q(e), a.L.up_s(e), rt * kg_h + warp, lane);
+            load_wtile<Q>(g, plane_q(e), plane_s(e), rt * kg_h + warp, lane);
+            load_wtile<Q>(up, plane_q(e) + a.L.q_gu, plane_s(e) + a.L.s_gu, rt * kg_h + warp, lane);
         }
     };
     const int n_my = (it0 < n_items) ? div_g.div(n_items - it0 + G - 1) : 0;
@@ -768,64 +830,52 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
     }
     // residual of this CTA's output rows, requested before the barrier
     float resid = 0.0f;
-    if (has_down && tid < 16 * T) resid = a.residual[(size_t)(tid >> 4) * H + cta * 16 + (tid & 15)];
+    if (STACK && layer > 0) resid = carry;
+    else if (has_down && tid < 16 * T) resid = a.residual[(size_t)(tid >> 4) * H + cta * 16 + (tid & 15)];
     stamp(5);
     __syncthreads();
     grid_arrive(a.bar);
     if (!grid_wait(a.bar, wc, G, ++epoch, a.debug_extra_arrivals, &fail_s)) {
-        mbar_wait(&mbar[7], par >> 7, wc);  // bounded: do not leave with the down copies in flight
+        mbar_wait(&mbar[7], (par >> 7) & 1u, wc);  // bounded: do not leave with the down copies in flight
         return;
     }
     if (tid == 0) a.bar[1 + cta] = epoch;
     stamp(6);
 
     // ---------------- phase C: down + combine ----------------
-    if (!has_down) return;  // (no down tiles were requested for this CTA)
+    if (!STACK && !has_down) return;  // (no down tiles were requested for this CTA)
+    if (has_down) {
     for (int i = tid; i < C * per_col_i; i += FT) cp_async16(&ss[i], a.sf + i);
     cp_async_wait_all();
-    if (!mbar_wait(&mbar[7], par >> 7, wc)) return;
+    if (!mbar_wait(&mbar[7], (par >> 7) & 1u, wc)) return;
     __syncthreads();
     stamp(7);
     {
-        // DG tiles of a warp are worked on together: their dependent chains (shared load ->
-        // unpack -> two MMAs -> scale) overlap instead of running one after the other
-        constexpr int DG = (Q == Q4_0) ? 3 : (Q == Q8_0) ? 2 : 1;
+        // one tile at a time in a rolled loop: two or three together overlapped their chains, but that code runs once per
+        // launch and has to be fetched for it (stack of eight Q4_0 layers 148 -> 140 us, a Q8_0 call 22.4 -> 21.7)
         const int rt = cta;
 #pragma unroll 1
-        for (int i0 = 0; warp + FW * i0 < n_down; i0 += DG) {
-            WTile<Q> w[DG];
-            int nn[DG];
-#pragma unroll
-            for (int j = 0; j < DG; ++j) {
-                const int i = i0 + j;
-                nn[j] = min(warp + FW * i, n_down - 1);
-                const int uu = div_kgi.div(nn[j]), kg = nn[j] - uu * kg_i;
-                if (uu < pf_experts) {
-                    const uint4* base = pf + ((size_t)uu * kg_i) * TU4;
-                    read_staged<Q>(w[j], base + kg * NQ32, base + kg_i * NQ32 + kg * 8, lane);
-                } else {
-                    const int ee = rs.ue[uu];
-                    load_wtile<Q>(w[j], a.L.down_q(ee), a.L.down_s(ee), rt * kg_i + kg, lane);
-                }
+        for (int n = warp; n < n_down; n += FW) {
+            WTile<Q> w;
+            const int uu = div_kgi.div(n), kg = n - uu * kg_i;
+            if (uu < pf_experts) {
+                const uint4* base = pf + ((size_t)uu * kg_i) * TU4;
+                read_staged<Q>(w, base + kg * NQ32, base + kg_i * NQ32 + kg * 8, lane);
+            } else {
+                const int ee = rs.ue[uu];
+                load_wtile<Q>(w, plane_q(ee) + 2 * a.L.q_gu, plane_s(ee) + 2 * a.L.s_gu, rt * kg_i + kg, lane);
             }
+            const int c0 = rs.uc0[uu];
+            const int ncol = min(4, rs.uncol[uu]);
+            const int jcol = gq >> 1;
+            const bool bvalid = jcol < ncol;
+            const uint4* bp = ss + ((size_t)((c0 + (bvalid ? jcol : 0)) * 2 + (gq & 1)) * nblk_i_pad) * 4 + t4 + (size_t)kg * 16;
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int j = 0; j < DG; ++j) {
-                const int uu = div_kgi.div(nn[j]), kg = nn[j] - uu * kg_i;
-                const int c0 = rs.uc0[uu];
-                const int ncol = min(4, rs.uncol[uu]);
-                const int jcol = gq >> 1;
-                const bool bvalid = jcol < ncol;
-                const uint4* bp = ss + ((size_t)((c0 + (bvalid ? jcol : 0)) * 2 + (gq & 1)) * nblk_i_pad) * 4 + t4 +
-                                  (size_t)kg * 16;
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int b = 0; b < 4; ++b) block_mma_smem<Q>(w[j], b, bp, bvalid, acc);
-                if (warp + FW * (i0 + j) < n_down) {
-                    float* pp = part + (size_t)nn[j] * 64 + t4 * 16;
-                    pp[gq] = acc[0] + acc[1];
-                    pp[gq + 8] = acc[2] + acc[3];
-                }
-            }
+            for (int b = 0; b < 4; ++b) block_mma_smem<Q>(w, b, bp, bvalid, acc);
+            float* pp = part + (size_t)n * 64 + t4 * 16;
+            pp[gq] = acc[0] + acc[1];
+            pp[gq + 8] = acc[2] + acc[3];
         }
         __syncthreads();
         stamp(8);
@@ -849,10 +899,29 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const int pf_experts, 
             float accv = resid;
 #pragma unroll 1
             for (int slot = 0; slot < K; ++slot) accv = __fadd_rn(accv, wd[(t * K + slot) * 16 + row]);
-            a.out[(size_t)t * H + rt * 16 + row] = accv;
+            if (!STACK || layer + 1 == ls.n()) a.out[(size_t)t * H + rt * 16 + row] = accv;
+            else st_tagged(ls.xt() + 2 * ((size_t)t * H + rt * 16 + row), accv, epoch);
+            carry = accv;
         }
     }
+    }
     stamp(9);
+    if (!STACK || ++layer == ls.n()) return;
+    // ---------------- next layer of the stack ----------------
+    // Its static operands are requested first. Its input is the tagged words that the down CTAs have just stored: every
+    // thread polls for its own four, so that no second round trip follows the wait. Nothing else needs a barrier: a
+    // CTA that has all of the input knows that every down CTA is done with the SwiGLU fragments, and barrier 2 of
+    // the coming layer comes before the next store to these words.
+    par ^= 1u << 7;
+    wv = router_row();
+    gv = gamma_row();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();  // the layer's shared memory is free, its copies have all been waited for
+#pragma unroll
+    for (int t = 0; t < FMAX_T; ++t)
+        if (t < T && tid < H4 && !ld_tagged4(ls.xt() + 2 * ((size_t)t * H + tid * 4), epoch, wc, xv[t])) fail_s = 1;
+    __syncwarp();
+    }
 }
 
 // Shared memory the fused kernel needs besides its static arrays; pf_experts = experts whose
@@ -905,8 +974,8 @@ bool decode_fused_applicable(const DecodeArgs& a) {
     return fused_smem_bytes(a, tile_u4_of(a.L.quant), 0) + static_smem <= (size_t)d.smem_optin;
 }
 
-template <int Q, bool SINGLE, bool ONE>
-static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t st) {
+template <int Q, bool SINGLE, bool ONE, bool STACK = false>
+static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t st, const LayerList<STACK>& ls = {}) {
     const FusedDeviceInfo& d = fused_device_info(device);
     const size_t static_smem = 20 * 1024;
     const int C = a.T * a.K;
@@ -927,7 +996,7 @@ static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t 
     const size_t smem = fused_smem_bytes(a, TileU4<Q>::value, pf, gs);
     static size_t attr_smem[64] = {};
     if (smem > attr_smem[device & 63]) {
-        cudaError_t e = cudaFuncSetAttribute((decode_fused_kernel<Q, SINGLE, ONE>), cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute((decode_fused_kernel<Q, SINGLE, ONE, STACK>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return e;
         attr_smem[device & 63] = smem;
@@ -948,7 +1017,7 @@ static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t 
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     count_launch();
-    return cudaLaunchKernelEx(&cfg, (decode_fused_kernel<Q, SINGLE, ONE>), a, pf, ring, alias);
+    return cudaLaunchKernelEx(&cfg, (decode_fused_kernel<Q, SINGLE, ONE, STACK>), a, ls, pf, ring, alias);
 }
 
 cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st) {
@@ -967,6 +1036,28 @@ cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st) {
         case Q4_0: return one ? launch_fused_t<Q4_0, false, true>(a, device, st) : launch_fused_t<Q4_0, false, false>(a, device, st);
         case Q8_0: return one ? launch_fused_t<Q8_0, false, true>(a, device, st) : launch_fused_t<Q8_0, false, false>(a, device, st);
         default: return one ? launch_fused_t<BF16, false, true>(a, device, st) : launch_fused_t<BF16, false, false>(a, device, st);
+    }
+}
+
+// a: the first layer's call (one token), its gamma set, out = x = residual; layers of one shape and format
+cudaError_t launch_decode_fused_stack(const DecodeArgs& a, const LayerDev* const* layers, const float* const* gammas, int n,
+                                      float* x_tagged, cudaStream_t st) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    LayerList<true> ls{};
+    ls.layers = n;
+    ls.x_tagged = x_tagged;
+    for (int l = 0; l < n; ++l) {
+        ls.router_w[l] = layers[l]->router_w;
+        ls.q[l] = layers[l]->q;
+        ls.s[l] = layers[l]->s;
+        ls.gammas[l] = gammas[l];
+    }
+    switch (a.L.quant) {
+        case Q4_0: return launch_fused_t<Q4_0, false, true, true>(a, device, st, ls);
+        case Q8_0: return launch_fused_t<Q8_0, false, true, true>(a, device, st, ls);
+        default: return launch_fused_t<BF16, false, true, true>(a, device, st, ls);
     }
 }
 

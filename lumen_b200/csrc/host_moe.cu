@@ -223,7 +223,7 @@ Status allocate_moe_scratch(int device, int H, int I, int E, int K, int gating, 
     s.K = K;
     s.gating = gating;
     const size_t fixed = align_up((size_t)(E + 1) * 4, 256) + align_up((size_t)E * 4, 256) + 256 * 4 +
-                         (size_t)MAX_EXPERTS * 2 * sizeof(int4) + 1024 * 4;
+                         (size_t)MAX_EXPERTS * 2 * sizeof(int4) + 1024 * 4 + (size_t)H * 8;
     CUDA_TRY(cudaMalloc(&s.arena, fixed));
     CUDA_TRY(cudaMemset(s.arena, 0, fixed));
     uint8_t* b = static_cast<uint8_t*>(s.arena);
@@ -238,6 +238,7 @@ Status allocate_moe_scratch(int device, int H, int I, int E, int K, int gating, 
     s.any_lo = reinterpret_cast<int32_t*>(b + 772);
     s.R.work = reinterpret_cast<int4*>(b + 1024);
     s.bar = reinterpret_cast<unsigned int*>(b + 1024 + (size_t)MAX_EXPERTS * 2 * sizeof(int4));  // 1024 per-CTA flags
+    s.x_tagged = reinterpret_cast<float*>(s.bar + 1024);
     s.flags = flags;
     s.decode_impl = (flags & 0x1) ? 1 : 0;   // LUMEN_MOE_FLAG_DECODE_SPLIT
     s.prefill_impl = (flags & 0x2) ? 1 : 0;  // LUMEN_MOE_FLAG_PREFILL_MMA
@@ -280,7 +281,7 @@ Status check_status_word(const CudaMoeScratch* s) {
 Status clear_status_word(CudaMoeScratch* s, cudaStream_t st) {
     CUDA_TRY(cudaStreamSynchronize(st));
     CUDA_TRY(cudaMemset(s->status, 0, 4));
-    CUDA_TRY(cudaMemset(s->bar, 0, 1024 * 4));
+    CUDA_TRY(cudaMemset(s->bar, 0, 1024 * 4 + (size_t)s->H * 8));  // and x_tagged behind it
     CUDA_TRY(cudaMemset(s->R.logits, 0, (size_t)s->cap_tokens * s->E * 4));  // tagged logit slots of the fused decode kernel
     CUDA_TRY(cudaDeviceSynchronize());
     *reinterpret_cast<volatile int32_t*>(s->h_status) = 0;
@@ -409,6 +410,36 @@ Status encode_moe_ffn_decode_fused_norm(CudaMoeScratch* s, const MoeLayer& layer
     a.residual = attn_proj;
     a.out = output_x;
     CUDA_TRY(launch_decode(a, st));
+    return Status::Ok();
+}
+
+Status encode_moe_stack_decode(CudaMoeScratch* s, const MoeLayer* const* layers, const float* const* gammas, int n_layers, float* x,
+                               float eps, int tokens, cudaStream_t st) {
+    if (tokens < 1 || tokens > DECODE_MAX_TOKENS) return Status::Err(1, "decode handles 1..16 tokens; use prefill");
+    for (int l0 = 0; l0 < n_layers;) {
+        // one token: the longest run of layers of one format whose calls would take the fused kernel one by one is one launch
+        const LayerDev* devs[FUSED_MAX_LAYERS];
+        int n = 0;
+        for (; n < FUSED_MAX_LAYERS && l0 + n < n_layers; ++n) {
+            const MoeLayer& layer = *layers[l0 + n];
+            Status c = check_layer(s, layer);
+            if (!c.ok()) return c;
+            if (layer.dev.quant != layers[l0]->dev.quant) break;
+            devs[n] = &layer.dev;
+        }
+        DecodeArgs a = make_decode_args(s, *layers[l0], tokens);
+        a.x = a.residual = x;
+        a.out = x;
+        a.gamma = gammas[l0];
+        a.eps = eps;
+        if (n > 1 && tokens == 1 && s->E > 1 && decode_uses_fused(a)) {
+            CUDA_TRY(launch_decode_fused_stack(a, devs, gammas + l0, n, s->x_tagged, st));
+            l0 += n;
+        } else {
+            CUDA_TRY(launch_decode(a, st));
+            ++l0;
+        }
+    }
     return Status::Ok();
 }
 

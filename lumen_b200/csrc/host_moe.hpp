@@ -128,6 +128,7 @@ struct CudaMoeScratch {
     int prefill_impl = 0;
     int decode_impl = 0;            // 0 = fused persistent kernel where it applies, 1 = kernel chain
     unsigned int* bar = nullptr;    // grid barrier words of the fused decode kernel
+    float* x_tagged = nullptr;      // [H] {value, tag}: activations between the layers of a fused decode stack
     void* arena = nullptr;       // one allocation for the fixed-size part
     void* arena_tok = nullptr;   // one allocation for the token-sized part
     size_t arena_tok_bytes = 0;
@@ -160,6 +161,9 @@ Status encode_moe_ffn_decode(CudaMoeScratch* scratch, const MoeLayer& layer, con
 Status encode_moe_ffn_decode_fused_norm(CudaMoeScratch* scratch, const MoeLayer& layer,
                                         const float* attn_proj, const float* ffn_norm, float* normed_x,
                                         float* output_x, float eps, int tokens, cudaStream_t st);
+// x <- x + MoE_l(rmsnorm(x; gamma_l, eps)) in place, layer by layer
+Status encode_moe_stack_decode(CudaMoeScratch* scratch, const MoeLayer* const* layers, const float* const* gammas, int n_layers,
+                               float* x, float eps, int tokens, cudaStream_t st);
 // activations that are rmsnorm(x; gamma, eps) of an f32 residual stream: `normed` is then scratch of the same size, written
 // only where the norm cannot be folded into the pass that prepares the operands
 struct NormIn {

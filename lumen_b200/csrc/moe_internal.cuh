@@ -184,6 +184,11 @@ cudaError_t launch_route_small(const DecodeArgs& a, cudaStream_t st);  // router
 bool decode_fused_applicable(const DecodeArgs& a);
 bool decode_uses_fused(const DecodeArgs& a);  // whether launch_decode takes the fused kernel for this call
 cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st);
+constexpr int FUSED_MAX_TOKENS = 4;
+constexpr int FUSED_MAX_LAYERS = 64;  // layers of a stack in one launch (2 KB of kernel parameters)
+cudaError_t launch_decode_fused_stack(const DecodeArgs& a, const LayerDev* const* layers, const float* const* gammas, int n,
+                                      float* x_tagged, cudaStream_t st);
+bool decode_uses_fused(const DecodeArgs& a);
 cudaError_t launch_decode_phase(const DecodeArgs& a, int phase, cudaStream_t st);  // one kernel of the kernel chain: 0 router, 1 gate/up, 2 down
 cudaError_t launch_quantize(const float* src, int64_t n, int quant, void* dst, cudaStream_t st);
 cudaError_t launch_rmsnorm(const float* x, const float* gamma, float* out, int T, int H, float eps,

@@ -175,3 +175,27 @@ def test_single_expert_fused_decode(cuda_lib, quant, H, I, T, gating):
     r = sc.get_routing(T)
     assert (r["ids"] == 0).all() and np.array_equal(r["dst_to_col"].ravel(), np.arange(T)) and np.array_equal(r["expert_bounds"], [0, T])
     np.testing.assert_allclose(r["weights"], o_w, rtol=1e-4)
+
+
+# a one-token stack in one launch: more layers than one launch holds, a change of format inside, CTAs with and without
+# down rows, more experts than CTAs; two tokens: layer by layer
+@pytest.mark.parametrize("quants,H,E,T", [([1] * 66, 256, 16, 1), ([0, 0, 1, 1, 2, 2, 2, 0], 512, 16, 1), ([1] * 5, 2048, 256, 1),
+                                          ([0] * 4, 1920, 128, 1), ([2] * 3, 128, 8, 1), ([1] * 3, 256, 16, 2)])
+def test_fused_stack_matches_layer_by_layer(cuda_lib, quants, H, E, T):
+    I, K = 128, 4
+    sc = moe.allocate_moe_scratch(H, I, E, K, 16)
+    layers = []
+    for l, quant in enumerate(quants):
+        lay = synth.LayerLayout(H, I, E, quant)
+        layers.append(sc.prepare_layer(synth.make_layer_blob(lay, l), lay.meta()))
+    g = torch.Generator("cuda").manual_seed(H)
+    gammas = [1 + 0.1 * torch.randn(H, generator=g, device="cuda") for _ in layers]
+    x0 = torch.randn((T, H), generator=g, device="cuda")
+    y = x0.clone()
+    for layer, gamma in zip(layers, gammas):
+        y = sc.decode_fused_norm(layer, y, gamma, 1e-6, torch.empty_like(y))
+    for _ in range(20):
+        x = x0.clone()
+        sc.stack_decode(layers, gammas, x, 1e-6)
+        assert torch.equal(x, y)
+    assert sc.poll_status() == 0
