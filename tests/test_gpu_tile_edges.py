@@ -199,3 +199,11 @@ def test_fused_stack_matches_layer_by_layer(cuda_lib, quants, H, E, T):
         sc.stack_decode(layers, gammas, x, 1e-6)
         assert torch.equal(x, y)
     assert sc.poll_status() == 0
+    graph = torch.cuda.CUDAGraph()  # captured: one launch per layer
+    x.copy_(x0)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        sc.stack_decode(layers, gammas, x, 1e-6)
+    assert torch.equal(x, x0)
+    graph.replay()
+    assert torch.equal(x, y)
