@@ -257,7 +257,7 @@ struct TopkSm {
 
 }  // namespace
 
-template <int Q, bool SINGLE, bool ONE, bool STACK>
+template <int Q, int SINGLE, bool ONE, bool STACK>
 __global__ void __launch_bounds__(FT, 1)
 decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ LayerList<STACK> ls, const int pf_experts, const int gs_slots, const int gs_alias) {
     extern __shared__ uint4 dyn[];
@@ -342,8 +342,8 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     auto stage_all = [&](const int* ue, int nu) {
         const int n_items_ = nu * rt_i;
         const int n_my_ = (it0 < n_items_) ? div_g.div(n_items_ - it0 + G - 1) : 0;
-        const int n_st_ = min(n_my_, gs_slots);
-        const int n_pf_ = has_down ? min(nu, pf_experts) : 0;
+        const int n_st_ = (SINGLE == 2) ? 0 : min(n_my_, gs_slots);
+        const int n_pf_ = (has_down && SINGLE != 1) ? min(nu, pf_experts) : 0;
         const unsigned q_gu = (unsigned)kg_h * NQ32 * 16, s_gu = (Q != BF16) ? (unsigned)kg_h * 128 : 0u;
         const unsigned q_dn = (unsigned)kg_i * NQ32 * 16, s_dn = (Q != BF16) ? (unsigned)kg_i * 128 : 0u;
         if (lane < n_st_) mbar_expect_tx(&mbar[lane], 2u * (q_gu + s_gu));
@@ -361,10 +361,12 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
             bulk_copy(dst, src, is_s ? s_dn : q_dn, &mbar[7]);
         }
     };
-    // SINGLE: one expert (the shared expert): its tiles are requested right away, before the wait for the previous kernel; every
-    // CTA works out the gate logit itself and there is nothing to rank or sort, so barrier 1 falls away. 2048 x 512, three
-    // tokens: 14.5 -> 12.5 us in any format. (As a branch of the general kernel instead of an instance, every other call took
-    // 0.5 us longer: the instruction stream is what bounds them.)
+    // SINGLE: one expert (the shared expert), as two kernels (1: gate/up, 2: down) chained as programmatic dependents. The
+    // expert is known, so each requests its tiles before it waits for the kernel before; every CTA works out the gate
+    // logit itself, nothing is ranked or sorted, and no CTA waits for another: the cooperative launch, which starts
+    // ~2.4 us after its predecessor's end, and both grid barriers fall away. 2048 x 512, three tokens: 14.5 -> 12.5 us without
+    // the router exchange, 10.8 as two kernels. (As a branch of the general kernel instead of an instance, every other
+    // call took 0.5 us longer: the instruction stream is what bounds them.)
     if (SINGLE && warp == 0) {
         if (lane == 0) rs.ue[0] = 0;
         __syncwarp();
@@ -374,12 +376,12 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     // ---------------- phase A ----------------
     // first router row in registers before waiting on the previous kernel (weights are static)
     auto router_row = [&]() {
-        return (want_logits && (SINGLE || cta < E) && tid < H4)
+        return (want_logits && SINGLE != 2 && (SINGLE || cta < E) && tid < H4)
                    ? __ldg(reinterpret_cast<const float4*>(router_w() + (SINGLE ? 0 : (size_t)cta * H)) + tid)
                    : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     float4 wv = router_row();
-    const bool norm = STACK || a.gamma != nullptr;
+    const bool norm = SINGLE != 2 && (STACK || a.gamma != nullptr);
     auto gamma_row = [&]() {
         return (norm && tid < H4) ? __ldg(reinterpret_cast<const float4*>(gamma()) + tid) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
@@ -392,13 +394,13 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     float4 xv[FMAX_T];
 #pragma unroll
     for (int t = 0; t < FMAX_T; ++t)
-        xv[t] = (t < T && tid < H4) ? reinterpret_cast<const float4*>(a.x)[t * H4 + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
+        xv[t] = (SINGLE != 2 && t < T && tid < H4) ? reinterpret_cast<const float4*>(a.x)[t * H4 + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int status_now = *reinterpret_cast<volatile int*>(a.status);
     unsigned epoch = *reinterpret_cast<volatile unsigned*>(a.bar + 1 + cta);  // barriers this CTA has passed so far
     if (status_now != 0) {  // an earlier launch gave up: do not touch the barrier
         if (SINGLE) {       // (nor leave with copies in flight)
             __syncthreads();
-            for (int j = 0; j < gs_slots && it0 + j * G < rt_i; ++j) mbar_wait(&mbar[j], 0, wc);
+            for (int j = 0; SINGLE == 1 && j < gs_slots && it0 + j * G < rt_i; ++j) mbar_wait(&mbar[j], 0, wc);
             mbar_wait(&mbar[7], 0, wc);
         }
         return;
@@ -449,12 +451,12 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     }
 #pragma unroll
     for (int t = 0; t < FMAX_T; ++t)
-        if (t < T && tid < H4) xn4[t * H4 + tid] = xv[t];
+        if (SINGLE != 2 && t < T && tid < H4) xn4[t * H4 + tid] = xv[t];
 
     if (SINGLE) {
 #pragma unroll
         for (int t = 0; t < FMAX_T; ++t) {
-            if (t < T) {
+            if (SINGLE == 1 && t < T) {
                 float acc = wv.x * xv[t].x + wv.y * xv[t].y + wv.z * xv[t].z + wv.w * xv[t].w;
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -465,10 +467,12 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
         __syncthreads();
         if (tid < T) {
             float v = 0.0f;
+            if (SINGLE == 1) {
 #pragma unroll
-            for (int w = 0; w < FW; ++w) v += red_a[w][tid];
-            float wt = 1.0f;  // gating 3
-            if (a.gating == 2) {
+                for (int w = 0; w < FW; ++w) v += red_a[w][tid];
+            }
+            float wt = (SINGLE == 2) ? a.R.weights[tid] : 1.0f;  // gating 3
+            if (SINGLE == 1 && a.gating == 2) {
                 const float ex = lumen_exact::expf_libm_tab(-v, lumen_exact::Exp2TabPtr{reinterpret_cast<const uint64_t*>(ts.tab)});
                 wt = __fdiv_rn(1.0f, __fadd_rn(1.0f, ex));
             }
@@ -476,7 +480,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
             rs.d2c[tid] = tid;
             rs.col_u[tid] = 0;
             rs.col_tok[tid] = tid;
-            if (cta == 0) {
+            if (SINGLE == 1 && cta == 0) {
                 a.R.ids[tid] = 0u;
                 a.R.weights[tid] = wt;
                 a.R.dst_to_col[tid] = tid;
@@ -488,7 +492,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
             rs.uc0[0] = 0;
             rs.uncol[0] = T;
             rs.U = 1;
-            if (cta == 0) {
+            if (SINGLE == 1 && cta == 0) {
                 a.R.uexp[0] = 0;
                 *a.R.n_uexp = 1;
                 a.R.expert_bounds[0] = 0;
@@ -521,6 +525,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     }
     // logits are out: build the activation operand while the other CTAs catch up
     __syncthreads();
+    const int Tb = (SINGLE == 2) ? 0 : T;
     // activation operand of every token, private to this CTA
     // int8 form: per token [2 terms][nblk_pad * 8 + 8 words] then [nblk_pad] {sx, 8 * sx * sum}; inside a block
     // the word pair of lane quad t is adjacent: {inputs 4t..4t+3, inputs 16+4t..16+4t+3}
@@ -529,19 +534,19 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     if (Q == Q4_0 && kInt8GateUp) {
         const int sub = tid & 7;
 #pragma unroll 1
-        for (int item = tid >> 3; item < T * nblk; item += FT / 8) {
+        for (int item = tid >> 3; item < Tb * nblk; item += FT / 8) {
             const int t = item / nblk, b = item - t * nblk;
             build_xq_block(xn4[t * H4 + b * 8 + sub], sub, lane, xq + (size_t)t * xq_tok, nblk_pad, b);
         }
         // padding blocks (kg_h * 4 > H / 32) must read as zero
         const int padw = (nblk_pad - nblk) * 8;
 #pragma unroll 1
-        for (int i = tid; i < T * 2 * padw; i += FT) {
+        for (int i = tid; i < Tb * 2 * padw; i += FT) {
             const int tt = i / padw, r = i - tt * padw;
             xq[(size_t)(tt >> 1) * xq_tok + (tt & 1) * xq_term + nblk * 8 + r] = 0u;
         }
 #pragma unroll 1
-        for (int i = tid; i < T * (nblk_pad - nblk); i += FT) {
+        for (int i = tid; i < Tb * (nblk_pad - nblk); i += FT) {
             const int t = i / (nblk_pad - nblk), b = nblk + i - t * (nblk_pad - nblk);
             reinterpret_cast<float2*>(xq + (size_t)t * xq_tok + 2 * xq_term)[b] = make_float2(0.0f, 0.0f);
         }
@@ -549,7 +554,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
         const bool bf16_mode = (Q == BF16);
         const int sub = tid & 7, hl = sub >> 2, s4 = sub & 3;
 #pragma unroll 1
-        for (int item = tid >> 3; item < T * nblk; item += FT / 8) {
+        for (int item = tid >> 3; item < Tb * nblk; item += FT / 8) {
             const int t = item / nblk, b = item - t * nblk;
             const float4 lo4 = xn4[t * H4 + b * 8 + s4];
             const float4 hi4 = xn4[t * H4 + b * 8 + 4 + s4];
@@ -558,7 +563,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
         // padding blocks (kg_h * 4 > H / 32) must read as zero
         const int per = (nblk_pad - nblk) * 4;
 #pragma unroll 1
-        for (int i = tid; i < T * 2 * per; i += FT) {
+        for (int i = tid; i < Tb * 2 * per; i += FT) {
             const int th = i / per, r = i - th * per;
             xs[(size_t)(th >> 1) * per_col + ((size_t)(th & 1) * nblk_pad + nblk) * 4 + r] = make_uint4(0u, 0u, 0u, 0u);
         }
@@ -729,7 +734,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
             load_wtile<Q>(up, plane_q(e) + a.L.q_gu, plane_s(e) + a.L.s_gu, rt * kg_h + warp, lane);
         }
     };
-    const int n_my = (it0 < n_items) ? div_g.div(n_items - it0 + G - 1) : 0;
+    const int n_my = (SINGLE != 2 && it0 < n_items) ? div_g.div(n_items - it0 + G - 1) : 0;
     WTile<Q> wg0, wu0, wg1, wu1;
     if (gs_slots == 0 && n_my > 0) load_gu(it0, wg1, wu1);  // no ring: tiles go through registers, one item ahead
 
@@ -833,13 +838,14 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     if (STACK && layer > 0) resid = carry;
     else if (has_down && tid < 16 * T) resid = a.residual[(size_t)(tid >> 4) * H + cta * 16 + (tid & 15)];
     stamp(5);
+    if (SINGLE == 1) return;
     __syncthreads();
-    grid_arrive(a.bar);
-    if (!grid_wait(a.bar, wc, G, ++epoch, a.debug_extra_arrivals, &fail_s)) {
+    if (!SINGLE) grid_arrive(a.bar);
+    if (!SINGLE && !grid_wait(a.bar, wc, G, ++epoch, a.debug_extra_arrivals, &fail_s)) {
         mbar_wait(&mbar[7], (par >> 7) & 1u, wc);  // bounded: do not leave with the down copies in flight
         return;
     }
-    if (tid == 0) a.bar[1 + cta] = epoch;
+    if (!SINGLE && tid == 0) a.bar[1 + cta] = epoch;
     stamp(6);
 
     // ---------------- phase C: down + combine ----------------
@@ -989,7 +995,7 @@ bool decode_fused_applicable(const DecodeArgs& a) {
     return fused_smem_bytes(a, tile_u4_of(a.L.quant), 0) + static_smem <= (size_t)d.smem_optin;
 }
 
-template <int Q, bool SINGLE, bool ONE, bool STACK = false>
+template <int Q, int SINGLE, bool ONE, bool STACK = false>
 static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t st, const LayerList<STACK>& ls = {}) {
     const FusedDeviceInfo& d = fused_device_info(device);
     const size_t static_smem = 20 * 1024;
@@ -1029,8 +1035,8 @@ static cudaError_t launch_fused_t(const DecodeArgs& a, int device, cudaStream_t 
     attr[0].val.cooperative = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.attrs = SINGLE ? attr + 1 : attr;  // (the two kernels of a single expert have no grid barrier)
+    cfg.numAttrs = SINGLE ? 1 : 2;
     count_launch();
     return cudaLaunchKernelEx(&cfg, (decode_fused_kernel<Q, SINGLE, ONE, STACK>), a, ls, pf, ring, alias);
 }
@@ -1042,15 +1048,15 @@ cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st) {
     const bool one = (a.T == 1);
     if (single_expert(a)) {
         switch (a.L.quant) {
-            case Q4_0: return launch_fused_t<Q4_0, true, false>(a, device, st);
-            case Q8_0: return launch_fused_t<Q8_0, true, false>(a, device, st);
-            default: return launch_fused_t<BF16, true, false>(a, device, st);
+            case Q4_0: e = launch_fused_t<Q4_0, 1, false>(a, device, st); return e != cudaSuccess ? e : launch_fused_t<Q4_0, 2, false>(a, device, st);
+            case Q8_0: e = launch_fused_t<Q8_0, 1, false>(a, device, st); return e != cudaSuccess ? e : launch_fused_t<Q8_0, 2, false>(a, device, st);
+            default: e = launch_fused_t<BF16, 1, false>(a, device, st); return e != cudaSuccess ? e : launch_fused_t<BF16, 2, false>(a, device, st);
         }
     }
     switch (a.L.quant) {
-        case Q4_0: return one ? launch_fused_t<Q4_0, false, true>(a, device, st) : launch_fused_t<Q4_0, false, false>(a, device, st);
-        case Q8_0: return one ? launch_fused_t<Q8_0, false, true>(a, device, st) : launch_fused_t<Q8_0, false, false>(a, device, st);
-        default: return one ? launch_fused_t<BF16, false, true>(a, device, st) : launch_fused_t<BF16, false, false>(a, device, st);
+        case Q4_0: return one ? launch_fused_t<Q4_0, 0, true>(a, device, st) : launch_fused_t<Q4_0, 0, false>(a, device, st);
+        case Q8_0: return one ? launch_fused_t<Q8_0, 0, true>(a, device, st) : launch_fused_t<Q8_0, 0, false>(a, device, st);
+        default: return one ? launch_fused_t<BF16, 0, true>(a, device, st) : launch_fused_t<BF16, 0, false>(a, device, st);
     }
 }
 
@@ -1070,9 +1076,9 @@ cudaError_t launch_decode_fused_stack(const DecodeArgs& a, const LayerDev* const
         ls.gammas[l] = gammas[l];
     }
     switch (a.L.quant) {
-        case Q4_0: return launch_fused_t<Q4_0, false, true, true>(a, device, st, ls);
-        case Q8_0: return launch_fused_t<Q8_0, false, true, true>(a, device, st, ls);
-        default: return launch_fused_t<BF16, false, true, true>(a, device, st, ls);
+        case Q4_0: return launch_fused_t<Q4_0, 0, true, true>(a, device, st, ls);
+        case Q8_0: return launch_fused_t<Q8_0, 0, true, true>(a, device, st, ls);
+        default: return launch_fused_t<BF16, 0, true, true>(a, device, st, ls);
     }
 }
 
