@@ -1060,7 +1060,7 @@ cudaError_t launch_decode_fused(const DecodeArgs& a, cudaStream_t st) {
     }
 }
 
-// a: the first layer's call (one token), its gamma set, out = x = residual; layers of one shape and format
+// a: the first layer's call (one token), its gamma set, out = x = residual; Q4_0 layers of one shape
 cudaError_t launch_decode_fused_stack(const DecodeArgs& a, const LayerDev* const* layers, const float* const* gammas, int n,
                                       float* x_tagged, cudaStream_t st) {
     int device = 0;
@@ -1075,11 +1075,7 @@ cudaError_t launch_decode_fused_stack(const DecodeArgs& a, const LayerDev* const
         ls.s[l] = layers[l]->s;
         ls.gammas[l] = gammas[l];
     }
-    switch (a.L.quant) {
-        case Q4_0: return launch_fused_t<Q4_0, 0, true, true>(a, device, st, ls);
-        case Q8_0: return launch_fused_t<Q8_0, 0, true, true>(a, device, st, ls);
-        default: return launch_fused_t<BF16, 0, true, true>(a, device, st, ls);
-    }
+    return launch_fused_t<Q4_0, 0, true, true>(a, device, st, ls);
 }
 
 }  // namespace lumen

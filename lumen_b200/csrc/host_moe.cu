@@ -416,20 +416,21 @@ Status encode_moe_ffn_decode_fused_norm(CudaMoeScratch* s, const MoeLayer& layer
 Status encode_moe_stack_decode(CudaMoeScratch* s, const MoeLayer* const* layers, const float* const* gammas, int n_layers, float* x,
                                float eps, int tokens, cudaStream_t st) {
     if (tokens < 1 || tokens > DECODE_MAX_TOKENS) return Status::Err(1, "decode handles 1..16 tokens; use prefill");
-    // In a graph a cooperative launch follows the one before without the gap, and separate launches are the faster form (eight
-    // Q4_0 layers 136 us, in one launch 140); from the host 154 and 145.
+    // One launch for a run of Q4_0 layers at one token. Not in a graph, where a cooperative launch follows the one before
+    // without the gap (eight layers 136 us launched one by one, 140 in one; from the host 154 and 145), and not where the
+    // tiles or the tokens are more (four layers: Q8_0 104 us one by one, 107 in one; three tokens of Q4_0 137 and 147).
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) (void)cudaGetLastError();
     const bool in_one = (tokens == 1 && s->E > 1 && capture == cudaStreamCaptureStatusNone);
     for (int l0 = 0; l0 < n_layers;) {
-        // one token: the longest run of layers of one format whose calls would take the fused kernel one by one is one launch
+        // the longest run of Q4_0 layers whose calls would take the fused kernel one by one
         const LayerDev* devs[FUSED_MAX_LAYERS];
         int n = 0;
-        for (; n < FUSED_MAX_LAYERS && l0 + n < n_layers; ++n) {
+        for (; n < (in_one ? FUSED_MAX_LAYERS : 1) && l0 + n < n_layers; ++n) {
             const MoeLayer& layer = *layers[l0 + n];
             Status c = check_layer(s, layer);
             if (!c.ok()) return c;
-            if (layer.dev.quant != layers[l0]->dev.quant) break;
+            if (layer.dev.quant != Q4_0) break;
             devs[n] = &layer.dev;
         }
         DecodeArgs a = make_decode_args(s, *layers[l0], tokens);

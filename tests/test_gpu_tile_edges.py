@@ -177,10 +177,10 @@ def test_single_expert_fused_decode(cuda_lib, quant, H, I, T, gating):
     np.testing.assert_allclose(r["weights"], o_w, rtol=1e-4)
 
 
-# a one-token stack in one launch: more layers than one launch holds, a change of format inside, CTAs with and without
-# down rows, more experts than CTAs; two tokens: layer by layer
+# a one-token stack of Q4_0 layers in one launch: more layers than one launch holds, other formats in between, CTAs with
+# and without down rows, more experts than CTAs; other formats, more tokens, a captured stream: layer by layer
 @pytest.mark.parametrize("quants,H,E,T", [([1] * 66, 256, 16, 1), ([0, 0, 1, 1, 2, 2, 2, 0], 512, 16, 1), ([1] * 5, 2048, 256, 1),
-                                          ([0] * 4, 1920, 128, 1), ([2] * 3, 128, 8, 1), ([1] * 3, 256, 16, 2)])
+                                          ([1] * 4, 1920, 128, 1), ([0, 2, 1, 1], 128, 8, 1), ([1] * 5, 2048, 16, 3), ([0] * 4, 1920, 256, 2), ([1] * 3, 256, 16, 5)])
 def test_fused_stack_matches_layer_by_layer(cuda_lib, quants, H, E, T):
     I, K = 128, 4
     sc = moe.allocate_moe_scratch(H, I, E, K, 16)
