@@ -400,8 +400,12 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     if (status_now != 0) {  // an earlier launch gave up: do not touch the barrier
         if (SINGLE) {       // (nor leave with copies in flight)
             __syncthreads();
-            for (int j = 0; SINGLE == 1 && j < gs_slots && it0 + j * G < rt_i; ++j) mbar_wait(&mbar[j], 0, wc);
-            mbar_wait(&mbar[7], 0, wc);
+            auto landed = [&](int i) {
+                for (int n = 0; n < (1 << 20) && !mbar_try(&mbar[i], 0); ++n) {
+                }
+            };
+            for (int j = 0; SINGLE == 1 && j < gs_slots && it0 + j * G < rt_i; ++j) landed(j);
+            landed(7);
         }
         return;
     }
