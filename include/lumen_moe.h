@@ -143,7 +143,8 @@ LUMEN_MOE_API lumen_moe_status_t lumen_moe_shared_expert_prefill(lumen_moe_ctx* 
 /* Replaces encode_moe_ffn_decode (cuda/moe.rs:1119): out[t] = residual[t] +
  * sum_k w[t,k] * Down_e(silu(Gate_e x[t]) * Up_e x[t]), f32 [T,H] in and out,
  * 1 <= T <= 16. d_out may alias d_residual (the backend passes the same buffer,
- * cuda/backend_impl.rs:3570-3573) but not d_normed. */
+ * cuda/backend_impl.rs:3570-3573) but not d_normed. d_residual and d_out may lie on any
+ * 4-byte boundary. */
 LUMEN_MOE_API lumen_moe_status_t lumen_moe_decode(lumen_moe_ctx* ctx, const lumen_moe_layer* layer,
                                     const float* d_normed, const float* d_residual, float* d_out,
                                     int32_t tokens, void* stream);

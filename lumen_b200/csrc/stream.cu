@@ -412,7 +412,10 @@ stream_kernel(const __grid_constant__ Args a) {
     }
 }
 
-// out[t] = residual[t] + sum_slot w * d32[column of the slot], in slot order (cuda/shaders/moe_accum.cu:22-46)
+// out[t] = residual[t] + sum_slot w * d32[column of the slot], in slot order (cuda/shaders/moe_accum.cu:22-46). Two outputs
+// a thread. PAIRS: residual and out, the caller's rows of f32, lie on 8-byte boundaries; else they are read and written
+// one by one (d32 is the context's own and always aligned).
+template <bool PAIRS>
 __global__ void __launch_bounds__(128)
 combine_f32_kernel(const float* __restrict__ d32, RouteDev R, const float* residual, float* out, int H, int K) {
     const int t = blockIdx.x, h = (blockIdx.y * 128 + threadIdx.x) * 2;
@@ -428,7 +431,8 @@ combine_f32_kernel(const float* __restrict__ d32, RouteDev R, const float* resid
     pdl_trigger();
     pdl_wait();
     if (h >= H) return;
-    float2 acc = *reinterpret_cast<const float2*>(residual + (size_t)t * H + h);
+    const float* res = residual + (size_t)t * H + h;
+    float2 acc = PAIRS ? *reinterpret_cast<const float2*>(res) : make_float2(res[0], res[1]);
     float2 d[MAX_TOP_K];
 #pragma unroll
     for (int s = 0; s < MAX_TOP_K; ++s)
@@ -439,7 +443,13 @@ combine_f32_kernel(const float* __restrict__ d32, RouteDev R, const float* resid
             acc.x = __fadd_rn(acc.x, __fmul_rn(w[s], d[s].x));
             acc.y = __fadd_rn(acc.y, __fmul_rn(w[s], d[s].y));
         }
-    *reinterpret_cast<float2*>(out + (size_t)t * H + h) = acc;
+    float* dst = out + (size_t)t * H + h;
+    if (PAIRS) {
+        *reinterpret_cast<float2*>(dst) = acc;
+    } else {
+        dst[0] = acc.x;
+        dst[1] = acc.y;
+    }
 }
 
 template <int Q, int MODE>
@@ -491,7 +501,9 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, cudaStream_t st) 
     const cudaError_t e = int8 ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st) : stream::launch_q<stream::DOWN_2>(d, p.sms, st);
     if (e != cudaSuccess) return e;
     count_launch();
-    return launch_dep(stream::combine_f32_kernel, dim3(p.T, (p.L.H / 2 + 127) / 128), dim3(128), 0, st, (const float*)p.d32, p.R,
+    // (H is a multiple of 32, so every row lies on the boundary that the first one does)
+    const bool pairs = (reinterpret_cast<uintptr_t>(p.residual) | reinterpret_cast<uintptr_t>(p.out)) % 8 == 0;
+    return launch_dep(pairs ? stream::combine_f32_kernel<true> : stream::combine_f32_kernel<false>, dim3(p.T, (p.L.H / 2 + 127) / 128), dim3(128), 0, st, (const float*)p.d32, p.R,
                       p.residual, p.out, p.L.H, p.K);
 }
 

@@ -258,3 +258,26 @@ def test_streaming_chain_experts_with_many_columns(cuda_lib, K):
     # determinism
     out2 = sc.decode(layer, x, res)
     assert torch.equal(out, out2)
+
+
+# residual and output on a 4-byte boundary, in the fused kernel (one token) and in each form of the kernel chain
+@pytest.mark.parametrize("quant,T", [(1, 1), (1, 4), (1, 16), (0, 1), (0, 5), (2, 1), (2, 16)])
+def test_residual_and_output_on_a_4_byte_boundary(cuda_lib, quant, T):
+    H, I, E, K = 2048, 512, 32, 4
+    lay, meta, blob_np, sc, layer = make_layer(H, I, E, K, quant, seed=T)
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=g, device="cuda")
+    res = torch.randn((T, H), generator=g, device="cuda")
+    aligned = sc.decode(layer, x, res).clone()
+    r = sc.get_routing(T)
+    pad = torch.full((2, T * H + 2), 7.0, device="cuda")  # a word in front, one behind
+    res_odd, out_odd = (p[1:-1].view(T, H) for p in pad)
+    res_odd.copy_(res)
+    for res_, out_ in ((res_odd, out_odd), (res, out_odd), (res_odd, torch.empty_like(res))):
+        assert res_.data_ptr() % 8 == 4 or out_.data_ptr() % 8 == 4
+        assert torch.equal(sc.decode(layer, x, res_, out_), aligned)
+    sc.decode(layer, x, res_odd, res_odd)  # in place
+    assert torch.equal(res_odd, aligned) and (pad[:, 0] == 7.0).all() and (pad[:, -1] == 7.0).all()
+    o_out, _, _ = oracle.moe_layer(blob_np, 0, meta.expert_gate_offs, meta.expert_up_offs, meta.expert_down_offs, quant, H, I, E, K,
+                                   x.cpu().numpy(), res.cpu().numpy(), ids=r["ids"], weights=r["weights"], threads=8)
+    assert rel_l2((aligned - res).cpu().numpy(), o_out - res.cpu().numpy()) < TOL_REL_L2
