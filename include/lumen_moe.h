@@ -264,12 +264,14 @@ LUMEN_MOE_API lumen_moe_status_t lumen_moe_get_routing_ids_stride_e(lumen_moe_ct
 LUMEN_MOE_API lumen_moe_status_t lumen_moe_poll_status(const lumen_moe_ctx* ctx);
 LUMEN_MOE_API lumen_moe_status_t lumen_moe_clear_status(lumen_moe_ctx* ctx, void* stream);
 
-/* Test hook for the give-up paths, without faulting or hanging anything: the NEXT kernel of
- * the given kind launched on this context waits for something that cannot happen (which = 0:
- * the grid barrier of the persistent decode kernel expects one arrival more than there are
- * CTAs; which = 1: a stage barrier of the tcgen05 grouped GEMM expects one byte more than the
- * copies deliver), so its bounded wait runs out, the kernel records LUMEN_MOE_TIMEOUT, releases
- * what it holds and returns. Use with LUMEN_MOE_FLAG_SHORT_WAITS. */
+/* Test hook for the give-up paths, without faulting or hanging anything: a kernel of the NEXT
+ * call of the given kind on this context waits for something that cannot happen (which = 0,
+ * lumen_moe_decode: the grid barrier of the persistent kernel expects one arrival more than there
+ * are CTAs, the first streaming kernel of the chain one byte more than its copies deliver; which =
+ * 1, lumen_moe_prefill: the first kernel of the expert products, streaming or tcgen05, one byte
+ * more than its copies deliver), so its bounded wait runs out, the kernel records
+ * LUMEN_MOE_TIMEOUT, releases what it holds and returns. A call without such a wait (a shared
+ * expert's decode, mma.sync products) leaves the hook set. Use with LUMEN_MOE_FLAG_SHORT_WAITS. */
 LUMEN_MOE_API lumen_moe_status_t lumen_moe_debug_expire_next_wait(lumen_moe_ctx* ctx, int32_t which);
 
 /* Device-to-device copy of the sort tables of the most recent routing call (no

@@ -219,10 +219,6 @@ struct RouteSm {
 // block's precomputed 8 * sx * sum(q0 + q1 / 254).
 constexpr bool kInt8GateUp = true;
 
-__host__ __device__ inline bool single_expert(const DecodeArgs& a) {
-    return a.L.E == 1 && a.K == 1 && a.gating >= 2 && a.logits_override == nullptr;
-}
-
 // The layers of a stack that one launch runs through (STACK), or nothing.
 template <bool STACK>
 struct LayerList {
@@ -845,7 +841,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     if (SINGLE == 1) return;
     __syncthreads();
     if (!SINGLE) grid_arrive(a.bar);
-    if (!SINGLE && !grid_wait(a.bar, wc, G, ++epoch, a.debug_extra_arrivals, &fail_s)) {
+    if (!SINGLE && !grid_wait(a.bar, wc, G, ++epoch, a.debug_expire, &fail_s)) {
         mbar_wait(&mbar[7], (par >> 7) & 1u, wc);  // bounded: do not leave with the down copies in flight
         return;
     }

@@ -367,7 +367,7 @@ static DecodeArgs make_decode_args(CudaMoeScratch* s, const MoeLayer& layer, int
     a.status = s->status;
     a.status_host = s->status_host;
     a.wait_limit_us = s->wait_limit_us;
-    a.debug_extra_arrivals = 0;
+    a.debug_expire = 0;
     a.trace = nullptr;
     return a;
 }
@@ -386,8 +386,8 @@ Status encode_moe_ffn_decode(CudaMoeScratch* s, const MoeLayer& layer, const flo
     a.out = output_x;
     s->last_decode = a;
     s->has_last_decode = true;
-    if (s->expire_next[0] && decode_uses_fused(a)) {
-        a.debug_extra_arrivals = 1;
+    if (s->expire_next[0] && !(single_expert(a) && decode_uses_fused(a))) {
+        a.debug_expire = 1;
         s->expire_next[0] = 0;
     }
     CUDA_TRY(launch_decode(a, st));
@@ -564,8 +564,7 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
     const bool tc_ok = (s->H % 256 == 0) && (s->I % 128 == 0) && (reinterpret_cast<uintptr_t>(normed) % 16 == 0) &&
                        (reinterpret_cast<uintptr_t>(out16_rows) % 32 == 0);
     p.impl = (s->prefill_impl == 1 || !tc_ok) ? 1 : 0;
-    // (the streaming kernels wait for nothing that could fail to come: the test hook takes the tcgen05 path)
-    if (s->prefill_impl == 0 && !s->expire_next[1] && prefill_streams(batch * s->K, s->E, s->H, s->I, layer.dev.quant, normed)) {
+    if (s->prefill_impl == 0 && prefill_streams(batch * s->K, s->E, s->H, s->I, layer.dev.quant, normed)) {
         p.impl = 2;
         p.stream_starts = reinterpret_cast<int32_t*>(s->R.work);  // (decode's work records: 8 KB, unused by a prefill)
     }
@@ -590,6 +589,10 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
         CUDA_TRY(p.gamma ? launch_norm_split(norm->x, p.gamma, p.eps, batch, s->H, p.impl == 0 && layer.dev.planes_natural, s->xr16, nullptr, st)
                          : launch_split_x16(normed, act_dtype, batch, s->H, p.impl == 0 && layer.dev.planes_natural, s->xr16, nullptr, st));
     const bool bf16_mode = (layer.dev.quant == BF16);
+    if (s->expire_next[1] && p.impl != 1) {
+        p.debug_extra_tx = 1;
+        s->expire_next[1] = 0;
+    }
     if (p.impl == 2) {
         CUDA_TRY(launch_stream_prefill(p, s->xr16, out16_rows, st));
         if (out16_rows) return Status::Ok();
@@ -598,10 +601,6 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
         // persistent grid, one CTA per SM; LUMEN_MOE_FLAG_TC_CTAS leaves some SMs to kernels that run beside it
         int sms = s->sms;
         if (s->tc_ctas > 0 && s->tc_ctas < sms) sms = s->tc_ctas;
-        if (s->expire_next[1]) {
-            p.debug_extra_tx = 1;
-            s->expire_next[1] = 0;
-        }
         CUDA_TRY(launch_grouped_tc(p, single ? s->xr16 : s->x16, sms, st, out16_rows));
     } else {
         CUDA_TRY(launch_build_xf(normed, act_dtype, batch, s->H, layer.dev.kg_h * 4, bf16_mode, s->xf, st));

@@ -121,7 +121,7 @@ struct CudaMoeScratch {
     unsigned wait_limit_us = 0;        // 0 = the kernels' defaults (1-2 s); 2000 with LUMEN_MOE_FLAG_SHORT_WAITS
     int tc_ctas = 0;                   // cap of the persistent tcgen05 grid (0 = every SM)
     int sms = 0;                       // multiprocessors of the device
-    int expire_next[2] = {0, 0};       // test hook (lumen_moe_debug_expire_next_wait): one-shot per kernel kind
+    int expire_next[2] = {0, 0};       // test hook (lumen_moe_debug_expire_next_wait): one-shot per kind of call
     const float* logits_override = nullptr;
     DecodeArgs last_decode{};   // arguments of the most recent decode call (instrumentation)
     bool has_last_decode = false;

@@ -111,9 +111,15 @@ struct DecodeArgs {
     int32_t* status;        // context status word (non-zero after a bounded wait expired)
     int32_t* status_host;   // the same code for the host: a word of mapped pinned host memory (null = none)
     unsigned wait_limit_us; // limit of every device-side wait of this launch (0 = one second)
-    int debug_extra_arrivals;  // test hook: the grid barrier expects this many arrivals more than there are CTAs
+    int debug_expire;       // test hook: the fused kernel's grid barrier expects this many arrivals more than there are CTAs, the
+                            // first copy barrier of the chain this many bytes more than arrive
     unsigned long long* trace;  // optional [grid][12] globaltimer stamps of the fused kernel's phases (null = off)
 };
+
+// A decode call of the always-on shared expert: known without a router, so nothing is ranked
+__host__ __device__ inline bool single_expert(const DecodeArgs& a) {
+    return a.L.E == 1 && a.K == 1 && a.gating >= 2 && a.logits_override == nullptr;
+}
 
 #ifdef __CUDACC__
 // A kernel that gives up records why: the first code wins; the host copy is written once.
@@ -188,7 +194,6 @@ constexpr int FUSED_MAX_TOKENS = 4;
 constexpr int FUSED_MAX_LAYERS = 64;  // layers of a stack in one launch (2 KB of kernel parameters)
 cudaError_t launch_decode_fused_stack(const DecodeArgs& a, const LayerDev* const* layers, const float* const* gammas, int n,
                                       float* x_tagged, cudaStream_t st);
-bool decode_uses_fused(const DecodeArgs& a);
 cudaError_t launch_decode_phase(const DecodeArgs& a, int phase, cudaStream_t st);  // one kernel of the kernel chain: 0 router, 1 gate/up, 2 down
 cudaError_t launch_quantize(const float* src, int64_t n, int quant, void* dst, cudaStream_t st);
 cudaError_t launch_rmsnorm(const float* x, const float* gamma, float* out, int T, int H, float eps,
@@ -223,7 +228,7 @@ struct PrefillArgs {
     int32_t* status;        // [1] device-side error flag (bounded waits, invalid caller-supplied ids)
     int32_t* status_host;   // the same code in mapped pinned host memory (null = none)
     unsigned wait_limit_us; // limit of the device-side waits (0 = two seconds)
-    int debug_extra_tx;     // test hook: the first stage barrier expects this many bytes more than arrive
+    int debug_extra_tx;     // test hook: the first copy barrier of the expert products expects this many bytes more than arrive
     int tc_ctas;            // cap of the persistent tcgen05 grid (0 = every SM)
     int impl;               // 0 = tcgen05 path, 1 = mma.sync grouped fallback, 2 = streaming kernels (few columns per expert)
     const uint32_t* ids_in;  // caller-supplied routing [T,K] (null = route here)

@@ -80,7 +80,24 @@ struct Args {
     float* d32;                 // DOWN_2(I): [C, H]
     const int32_t* out_row_map; // DOWN_1: output row of compact column c (null = c itself)
     TcPeerOut peer;             // DOWN_1, expert parallel: output rows go to other ranks' buffers (ret_map null = off)
+    int32_t* status;            // the context's status word and its copy for the host
+    int32_t* status_host;
+    uint32_t wait_limit_ns;     // limit of a warp's wait for a copy of its own
+    int debug_extra_tx;         // test hook: the first slot of a CTA's first warp expects this many bytes more than arrive
 };
+
+// A lane's wait for one of its warp's copies; false once the limit is over.
+__device__ __forceinline__ bool wait_copy(uint32_t bar, uint32_t parity, uint32_t limit_ns) {
+    for (uint32_t i = 1, t0 = 0; !tc::mbar_try(bar, parity); ++i) {
+        if ((i & 63u) == 0u) {
+            const uint32_t t = (uint32_t)tc::globaltimer_ns();
+            if (i == 64u) t0 = t;
+            else if (t - t0 > limit_ns) return false;
+        }
+    }
+    return true;
+}
+constexpr uint32_t DRAIN_NS = 1000000;  // a warp that gives up waits this long for each copy still on its way
 
 // b fragments of the block's two MMAs out of one 16-byte chunk (the two layouts order them differently)
 template <int TERMS>
@@ -223,6 +240,10 @@ stream_kernel(const __grid_constant__ Args a) {
             pi += WARPS;
         }
     };
+    if (a.debug_extra_tx != 0 && warp == 0) {
+        if (lane == 0) tc::mbar_expect_more(bar0, a.debug_extra_tx);
+        __syncwarp();
+    }
 #pragma unroll 1
     for (int i = 0; i < RING; ++i) request();
     if (DOWN) {
@@ -280,9 +301,21 @@ stream_kernel(const __grid_constant__ Args a) {
         int sub = 0;
 #pragma unroll 1
         for (int kg = 0; kg < kg_n; ++kg) {
-            if (sub == 0) {
-                // (the warp's own copies: they arrive; the limit only keeps a broken launch from spinning for good)
-                for (int k = 0; k < (1 << 22) && !tc::mbar_try(bar0 + rslot * 8, rphase); ++k) {}
+            if (sub == 0 && !wait_copy(bar0 + rslot * 8, rphase, a.wait_limit_ns)) {
+                // The copy has not come within the limit: the lanes raise the status word, wait (with a limit again) for
+                // the copies still on their way into this shared memory, and end without storing anything more. They all
+                // watch one barrier, whose phase cannot move on before they have passed it, so they come to the same end
+                // without a vote; one vote per slot made a 77-token prompt take 2 % longer.
+                raise_status(a.status, a.status_host, 4);  // LUMEN_MOE_TIMEOUT
+                do {
+                    wait_copy(bar0 + rslot * 8, rphase, DRAIN_NS);
+                    if (++rslot == RING) {
+                        rslot = 0;
+                        rphase ^= 1u;
+                    }
+                } while (rslot != wslot);
+                asm volatile("exit;");
+                __builtin_unreachable();
             }
             WTile<Q> w[NM];
             const uint32_t src = ring + rslot * S::slot;
@@ -294,13 +327,13 @@ stream_kernel(const __grid_constant__ Args a) {
             }
             if (GRP == 1 || ++sub == GRP || kg + 1 == kg_n) {
                 sub = 0;
+                // every lane's reads of the slot are ordered before the bulk copy that fills it again
+                tc::fence_proxy_async();
+                __syncwarp();
                 if (++rslot == RING) {
                     rslot = 0;
                     rphase ^= 1u;
                 }
-                // every lane's reads of the slot are ordered before the bulk copy that fills it again
-                tc::fence_proxy_async();
-                __syncwarp();
                 request();
             }
 #pragma unroll
@@ -470,9 +503,14 @@ cudaError_t launch_q(const Args& a, int sms, cudaStream_t st) {
     }
 }
 
+static uint32_t limit_ns(unsigned wait_limit_us) { return wait_limit_us ? wait_limit_us * 1000u : (uint32_t)tc::WAIT_LIMIT_NS; }
+
 // decode batches: the router's work records are the chunks (an expert has at most sixteen columns)
 static Args decode_args(const DecodeArgs& p) {
     Args g{};
+    g.status = p.status;
+    g.status_host = p.status_host;
+    g.wait_limit_ns = limit_ns(p.wait_limit_us);
     g.L = p.L;
     g.chunks = p.R.work;
     g.chunk_stride = 2;
@@ -489,6 +527,7 @@ cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st) {
     g.b = p.xf;
     g.b_row = (size_t)p.L.kg_h * 16;
     g.sf = p.sf;
+    g.debug_extra_tx = p.debug_expire;
     return stream::launch_q<stream::GATE_UP_2>(g, p.sms, st);
 }
 
@@ -498,6 +537,7 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, cudaStream_t st) 
     d.b = int8 ? reinterpret_cast<const uint4*>(p.sq) : p.sf;
     d.b_row = (size_t)p.L.kg_i * 16;
     d.d32 = p.d32;
+    d.debug_extra_tx = int8 ? p.debug_expire : 0;  // (the chain's first streaming kernel)
     const cudaError_t e = int8 ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st) : stream::launch_q<stream::DOWN_2>(d, p.sms, st);
     if (e != cudaSuccess) return e;
     count_launch();
@@ -520,9 +560,14 @@ cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __hal
     g.b = reinterpret_cast<const uint4*>(x16);
     g.b_row = (size_t)p.L.H / 8;
     g.out16 = p.s16;
+    g.status = p.status;
+    g.status_host = p.status_host;
+    g.wait_limit_ns = stream::limit_ns(p.wait_limit_us);
+    g.debug_extra_tx = p.debug_extra_tx;
     const cudaError_t e = stream::launch_q<stream::GATE_UP_1>(g, p.sms, st);
     if (e != cudaSuccess) return e;
     stream::Args d = g;
+    d.debug_extra_tx = 0;  // the hook applies to the first kernel of the pair
     d.starts = p.stream_starts ? p.stream_starts + p.sms + 1 : nullptr;
     d.b = reinterpret_cast<const uint4*>(p.s16);
     d.b_row = (size_t)p.L.I / 8;

@@ -69,6 +69,32 @@ def test_grouped_gemm_stage_barrier_that_runs_out_is_reported_and_recoverable(cu
     assert torch.equal(again, good)
 
 
+# the streaming kernels: decode chains on int8 (Q4_0) and hi + lo operands, short prompts
+@pytest.mark.parametrize("call,quant,T", [("decode", 1, 16), ("decode", 0, 5), ("decode", 2, 9), ("prefill", 1, 40), ("prefill", 0, 30)])
+def test_streaming_copy_that_never_comes_is_reported_and_recoverable(cuda_lib, call, quant, T):
+    H, I, E, K = 512, 256, 16, 4
+    lay = synth.LayerLayout(H, I, E, quant)
+    blob = synth.make_layer_blob(lay, 0)
+    sc = moe.allocate_moe_scratch(H, I, E, K, 64, flags=_lib.FLAG_SHORT_WAITS)
+    layer = sc.prepare_layer(blob, lay.meta())
+    x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(T), device="cuda")
+    run = sc.decode if call == "decode" else sc.prefill
+    good = run(layer, x, x.clone()).clone()
+    torch.cuda.synchronize()
+    assert sc.poll_status() == _lib.OK
+    sc.debug_expire_next_wait(0 if call == "decode" else 1)
+    run(layer, x, x.clone())
+    torch.cuda.synchronize()
+    assert sc.poll_status() == _lib.TIMEOUT
+    with pytest.raises(moe.LumenMoeError) as ei:
+        run(layer, x, x.clone())
+    assert ei.value.code == _lib.TIMEOUT
+    sc.clear_status()
+    again = run(layer, x, x.clone())
+    torch.cuda.synchronize()
+    assert sc.poll_status() == _lib.OK and torch.equal(again, good)
+
+
 def test_expert_id_out_of_range_is_an_error_code_not_a_fault(cuda_lib):
     # caller-supplied routing (what an expert-parallel rank receives over the wire): an id >= E must
     # never index a table; the pair is dropped (expert 0, weight 0) and the context reports INVALID_ARG
