@@ -53,6 +53,34 @@ def test_one_rank_window_equals_plain_prefill(cuda_lib, T, act, routing, quant):
     assert np.linalg.norm(got - want) / np.linalg.norm(want) < 1e-3
 
 
+# layers kept as f16 matrices too (rows in the natural order), short batches on the streaming kernels (rows in the planes'
+# order): the last batch of one form and the first of the other
+@pytest.mark.parametrize("quant,T", [(1, 10), (1, 96), (1, 97), (0, 72), (0, 73)])
+def test_one_rank_window_with_f16_weights_equals_plain_prefill(cuda_lib, quant, T):
+    from lumen_b200 import _lib, ep, moe, synth
+    from oracle import oracle
+    H, I, E, K = 512, 256, 32, 4
+    lay = synth.LayerLayout(H, I, E, quant)
+    blob = synth.make_layer_blob(lay, 3)
+    meta = lay.meta()
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=g, device="cuda")
+    res = torch.randn((T, H), generator=g, device="cuda")
+    sc = moe.allocate_moe_scratch(H, I, E, K, T, flags=_lib.FLAG_PREFILL_F16_WEIGHTS)
+    ref = sc.prefill(sc.prepare_layer(blob, meta), x, res)
+    r = sc.get_routing(T)
+    pe = ep.PushExpertParallel(H, I, E, K, T, 0, 1, 0, flags=_lib.FLAG_PREFILL_F16_WEIGHTS)
+    layer = pe.prepare_layer(blob, meta)
+    outs = [pe.forward(layer, x, res).clone() for _ in range(2)]
+    torch.cuda.synchronize()
+    assert pe.sc.poll_status() == _lib.OK
+    assert torch.equal(outs[0], ref) and torch.equal(outs[1], ref)
+    o_out, _, _ = oracle.moe_layer(blob.cpu().numpy(), 0, meta.expert_gate_offs, meta.expert_up_offs, meta.expert_down_offs, quant, H, I,
+                                   E, K, x.cpu().numpy(), res.cpu().numpy(), ids=r["ids"], weights=r["weights"], threads=8)
+    want = o_out - res.cpu().numpy()
+    assert np.linalg.norm((ref - res).cpu().numpy() - want) / np.linalg.norm(want) < 1e-3
+
+
 def test_expert_parallel_call_replayed_from_a_cuda_graph(cuda_lib):
     # the call number that tags the flags lives in device memory: a captured call can be replayed
     from lumen_b200 import ep, moe, synth
