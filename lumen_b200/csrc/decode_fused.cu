@@ -188,6 +188,17 @@ __device__ __forceinline__ bool mbar_wait(void* bar, unsigned parity, const Wait
     }
 }
 
+// A CTA that gives up does not leave while copies are on their way into its shared memory: waits, with a limit of its own,
+// for the barriers in `mask` (bit i: barrier i, whose phase at hand has parity bit i of `par`).
+static __device__ __noinline__ void let_land(unsigned long long* bars, unsigned mask, unsigned par) {
+    const unsigned long long t0 = global_ns();
+    for (; mask != 0u; mask &= mask - 1u) {
+        const int i = __ffs(mask) - 1;
+        while (!mbar_try(&bars[i], (par >> i) & 1u) && global_ns() - t0 < 10000000ull) {
+        }
+    }
+}
+
 // One lane's share of a staged tile: q words of the tile at qp (lane-major), scale words at sp.
 template <int Q>
 __device__ __forceinline__ void read_staged(WTile<Q>& w, const uint4* qp, const uint4* sp, int lane) {
@@ -396,12 +407,9 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     if (status_now != 0) {  // an earlier launch gave up: do not touch the barrier
         if (SINGLE) {       // (nor leave with copies in flight)
             __syncthreads();
-            auto landed = [&](int i) {
-                for (int n = 0; n < (1 << 20) && !mbar_try(&mbar[i], 0); ++n) {
-                }
-            };
-            for (int j = 0; SINGLE == 1 && j < gs_slots && it0 + j * G < rt_i; ++j) landed(j);
-            landed(7);
+            unsigned mask = 1u << 7;
+            for (int j = 0; SINGLE == 1 && j < gs_slots && it0 + j * G < rt_i; ++j) mask |= 1u << j;
+            let_land(mbar, mask, 0u);
         }
         return;
     }
@@ -715,14 +723,15 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
             // tiles for the barriers' next phase (barriers set up afresh here lost arrivals now and then)
             const int n_items_p = rs.pr_U * rt_i;
             const int n_my_p = (it0 < n_items_p) ? div_g.div(n_items_p - it0 + G - 1) : 0;
+            const unsigned asked = (1u << min(n_my_p, gs_slots)) - 1u | 1u << 7;  // barriers of those copies
             bool ok = true;
-            for (int j = 0; j < min(n_my_p, gs_slots) && ok; ++j) {
-                ok = mbar_wait(&mbar[j], (par >> j) & 1u, wc);
-                par ^= 1u << j;
+            for (int j = 0; j < 8 && ok; ++j)
+                if ((asked >> j) & 1u) ok = mbar_wait(&mbar[j], (par >> j) & 1u, wc);
+            if (__syncthreads_or(ok ? 0 : 1)) {
+                let_land(mbar, asked, par);
+                return;
             }
-            ok = ok && mbar_wait(&mbar[7], (par >> 7) & 1u, wc);
-            par ^= 1u << 7;
-            if (__syncthreads_or(ok ? 0 : 1)) return;
+            par ^= asked;
             if (warp == 0) stage_all(rs.ue, U);
         }
     }
@@ -809,7 +818,12 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
 #pragma unroll 1
     for (int j = 0; j < n_my; ++j) {
         if (gs_slots > 0) {
-            if (!mbar_wait(&mbar[sl], (par >> sl) & 1u, wc)) return;  // all threads give up together
+            if (!mbar_wait(&mbar[sl], (par >> sl) & 1u, wc)) {  // all threads give up together
+                unsigned mask = 1u << 7;
+                for (int i = 0; i < gs_slots && j + i < n_my; ++i) mask |= 1u << (j + i) % gs_slots;
+                let_land(mbar, mask, par);
+                return;
+            }
             par ^= 1u << sl;
             if (a.trace != nullptr && tid == 0 && j == n_my - 1) a.trace[(size_t)blockIdx.x * 12 + 11] = global_ns();
             if (warp < kg_h) {
@@ -842,7 +856,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     __syncthreads();
     if (!SINGLE) grid_arrive(a.bar);
     if (!SINGLE && !grid_wait(a.bar, wc, G, ++epoch, a.debug_expire, &fail_s)) {
-        mbar_wait(&mbar[7], (par >> 7) & 1u, wc);  // bounded: do not leave with the down copies in flight
+        let_land(mbar, 1u << 7, par);
         return;
     }
     if (!SINGLE && tid == 0) a.bar[1 + cta] = epoch;
@@ -853,7 +867,10 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     if (has_down) {
     for (int i = tid; i < C * per_col_i; i += FT) cp_async16(&ss[i], a.sf + i);
     cp_async_wait_all();
-    if (!mbar_wait(&mbar[7], (par >> 7) & 1u, wc)) return;
+    if (!mbar_wait(&mbar[7], (par >> 7) & 1u, wc)) {
+        let_land(mbar, 1u << 7, par);
+        return;
+    }
     __syncthreads();
     stamp(7);
     {

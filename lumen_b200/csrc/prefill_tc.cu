@@ -668,8 +668,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
             const uint64_t tmap_a_addr = reinterpret_cast<uint64_t>(&a.tmap_a);
             int row0 = 0, nbox = 1, arow0 = 0;
             bool ok = true;
-            int tn = 0;
-            for (int n = 0; ok; ++n) {
+            int tn = 0, n = 0;
+            for (; ok; ++n) {
                 const int kh = n % khs;
                 if (kh == 0) {
                     int4 tile;
@@ -703,6 +703,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                         "l"(tmap_addr), "r"(kh * 64), "r"(row0 + q * BBOX), "r"(bar)
                         : "memory");
             }
+            if (*abort_flag.flag) let_land(smem_u32(&full_bar[0]), STAGES, n);
         }
         __syncwarp();
     } else if (warp == MMA_WARP) {

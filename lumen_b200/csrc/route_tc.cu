@@ -108,7 +108,8 @@ router_logits_tc_kernel(const __grid_constant__ Args a) {
     if (warp == 0) {
         if (lane == 0) {
             bool ok = true;
-            for (int n = 0; ok && n < kh_per; ++n) {
+            int n = 0;
+            for (; ok && n < kh_per; ++n) {
                 const int s = n % STAGES, ph = (n / STAGES) & 1;
                 if (n >= STAGES) {
                     ok = mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag);
@@ -121,6 +122,7 @@ router_logits_tc_kernel(const __grid_constant__ Args a) {
                 tma_load_2d(base, &a.tmap_x, k, t0, bar);
                 if (use_lo) tma_load_2d(base + X_BYTES, &a.tmap_x, k, a.T + t0, bar);
             }
+            if (!ok) let_land(smem_u32(&full_bar[0]), STAGES, n);
         }
         __syncwarp();
     } else if (warp == 1) {

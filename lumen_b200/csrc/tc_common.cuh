@@ -54,6 +54,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const A
     }
 }
 
+// A role that gives up does not leave while its copies are on their way into shared memory: the last `stages` of the n
+// phases it has asked for on the ring of barriers at bar0, each complete or the limit over (a phase that other roles
+// have a part in may stay incomplete for good).
+__device__ __forceinline__ void let_land(uint32_t bar0, int stages, int n) {
+    const uint64_t t0 = globaltimer_ns();
+    for (int q = n > stages ? n - stages : 0; q < n; ++q)
+        while (!mbar_try(bar0 + (q % stages) * 8, (q / stages) & 1) && globaltimer_ns() - t0 < 1000000ull) {
+        }
+}
+
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
