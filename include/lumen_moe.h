@@ -160,7 +160,8 @@ LUMEN_MOE_API lumen_moe_status_t lumen_moe_decode_fused_norm(lumen_moe_ctx* ctx,
 /* Replaces encode_moe_ffn_prefill_grouped (cuda/moe.rs:1900) without its host
  * round trip: routing, the stable counting sort (:2115-2147), the grouped expert
  * products and the scatter-accumulate all run on the device. d_normed is
- * [T,H] of act_dtype; d_residual and d_out are f32 [T,H]. */
+ * [T,H] of act_dtype; d_residual and d_out are f32 [T,H] (any 4-byte boundary; the fast forms need
+ * all three on 16 bytes). */
 LUMEN_MOE_API lumen_moe_status_t lumen_moe_prefill(lumen_moe_ctx* ctx, const lumen_moe_layer* layer,
                                      const void* d_normed, const float* d_residual, float* d_out,
                                      int32_t tokens, int32_t act_dtype, void* stream);
@@ -182,7 +183,8 @@ LUMEN_MOE_API lumen_moe_status_t lumen_moe_prefill_routed(lumen_moe_ctx* ctx, co
  * d_ids[r]; output f16 [rows, H] in the caller's row order, unweighted.
  * lumen_moe_combine_f16: out[t] = residual[t] + sum_slot w[t,slot] * D[dst_to_col[t*K+slot]]
  * in slot order (moe_grouped_scatter_accum_q8_0, cuda/shaders/moe_grouped.cu:493-517) on
- * f16 rows D, e.g. those returned by the combine all-to-all. Needs no context. */
+ * f16 rows D, e.g. those returned by the combine all-to-all. Needs no context. hidden_dim: any even
+ * number (multiples of 8 with all buffers on 16-byte boundaries are the fast form). */
 LUMEN_MOE_API lumen_moe_status_t lumen_moe_experts_routed_f16(lumen_moe_ctx* ctx, const lumen_moe_layer* layer,
                                                               const void* d_rows, const uint32_t* d_ids,
                                                               void* d_out16, int32_t rows, int32_t act_dtype,

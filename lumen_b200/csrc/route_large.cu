@@ -766,9 +766,29 @@ scatter_accum_kernel(const __half* __restrict__ d16, const float* residual,
     *reinterpret_cast<float4*>(out + o + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
 }
 
+// The same, one output a thread, for what the 16-byte accesses above cannot take: rows that are no whole number of them
+// (lumen_moe_combine_f16 takes any even hidden_dim) or a caller's buffer that lies between two such boundaries.
+__global__ void __launch_bounds__(256)
+scatter_accum_scalar_kernel(const __half* __restrict__ d16, const float* residual, const float* __restrict__ weights,
+                            const int32_t* __restrict__ dst_to_col, float* out, int T, int H, int K) {
+    grid_dep_sync();
+    const int t = blockIdx.x, h = blockIdx.y * 256 + threadIdx.x;
+    if (h >= H) return;
+    float acc = residual[(size_t)t * H + h];
+    for (int s = 0; s < K; ++s) {
+        const size_t p = (size_t)t * K + s;
+        acc = __fadd_rn(acc, __fmul_rn(weights[p], __half2float(d16[(size_t)dst_to_col[p] * H + h])));
+    }
+    out[(size_t)t * H + h] = acc;
+}
+
 cudaError_t launch_scatter_accum(const __half* d16, const float* residual, const RouteDev& R, float* out,
                                  int T, int H, int K, cudaStream_t st) {
     count_launch();
+    const bool vec = H % 8 == 0 && (reinterpret_cast<uintptr_t>(d16) | reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+    if (!vec)
+        return launch_dep(scatter_accum_scalar_kernel, dim3(T, (H + 255) / 256), dim3(256), 0, st, d16, residual, R.weights, R.dst_to_col, out,
+                          T, H, K);
     return launch_dep(T <= 512 ? scatter_accum_kernel<8> : scatter_accum_kernel<4>, dim3(T, (H / 8 + 255) / 256), dim3(256), 0, st, d16, residual, R.weights,
                       R.dst_to_col, out, T, H, K);
 }

@@ -207,3 +207,40 @@ def test_fused_stack_matches_layer_by_layer(cuda_lib, quants, H, E, T):
     assert torch.equal(x, x0)
     graph.replay()
     assert torch.equal(x, y)
+
+
+# weighted sum of the expert outputs: rows of no whole number of 16-byte words, buffers between two 16-byte boundaries
+@pytest.mark.parametrize("H", [2, 6, 8, 36, 514, 2048])
+@pytest.mark.parametrize("off", [0, 1])
+def test_combine_of_any_even_width_and_4_byte_boundary(cuda_lib, H, off):
+    T, K = 5, 3
+    g = torch.Generator("cuda").manual_seed(H)
+    d16 = torch.randn((T * K, H), generator=g, device="cuda").half()
+    w = torch.rand((T, K), generator=g, device="cuda")
+    d2c = torch.randperm(T * K, generator=g, device="cuda").int()
+    pad = torch.full((2, T * H + 8), 7.0, device="cuda")  # words around the rows that no thread may touch
+    res, out = (p[off:off + T * H].view(T, H) for p in pad)
+    res.copy_(torch.randn((T, H), generator=g, device="cuda"))
+    want = res.clone()
+    for s in range(K):  # slot order, product and sum rounded apart
+        want = want + w[:, s:s + 1] * d16[d2c.view(T, K)[:, s].long()].float()
+    moe.combine_f16(d16, res, w, d2c, out)
+    assert torch.equal(out, want)
+    assert (pad[:, :off] == 7.0).all() and (pad[:, off + T * H:] == 7.0).all()
+
+
+# prompts whose residual and output lie on a 4-byte boundary: streaming, tcgen05 and mma.sync products
+@pytest.mark.parametrize("H,I,T", [(512, 256, 20), (512, 256, 200), (160, 96, 50)])
+def test_prefill_residual_and_output_on_a_4_byte_boundary(cuda_lib, H, I, T):
+    E, K = 16, 4
+    _, _, _, sc, layer = make_layer(H, I, E, K, 1, seed=T, max_tokens=T)
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=g, device="cuda")
+    res = torch.randn((T, H), generator=g, device="cuda")
+    aligned = sc.prefill(layer, x, res)
+    pad = torch.full((2, T * H + 2), 7.0, device="cuda")
+    res_odd, out_odd = (p[1:-1].view(T, H) for p in pad)
+    res_odd.copy_(res)
+    assert torch.equal(sc.prefill(layer, x, res_odd, out_odd), aligned)
+    sc.prefill(layer, x, res_odd, res_odd)
+    assert torch.equal(res_odd, aligned) and (pad[:, 0] == 7.0).all() and (pad[:, -1] == 7.0).all()
