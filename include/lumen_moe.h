@@ -6,6 +6,10 @@
  * replaces (paths relative to the reference project's root). All pointers named
  * d_* are device pointers; `stream` is a cudaStream_t passed as void*. Calls are
  * asynchronous on that stream and never synchronise it, except where stated.
+ * Alignment: a device pointer lies on a boundary of its element type at least. Decode activations,
+ * norm weights and normed outputs (lumen_moe_decode, _decode_fused_norm, _stack_decode, _route_only
+ * up to 16 tokens, the shared expert's decode), f16 and 16-bit output rows and the source of
+ * lumen_moe_quantize lie on 16 bytes: LUMEN_MOE_INVALID_ARG otherwise.
  * No exceptions cross this boundary; every function returns a status code and
  * lumen_moe_last_error() gives the text of the last failure on the calling thread.
  *

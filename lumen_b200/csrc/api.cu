@@ -363,6 +363,7 @@ lumen_moe_status_t lumen_moe_ep_prepare(lumen_moe_ctx* ctx, const void* d_normed
         return fail(LUMEN_MOE_INVALID_ARG, "experts_per_rank must divide num_experts");
     if (s.H % 8 != 0) return fail(LUMEN_MOE_UNSUPPORTED, "hidden_dim must be a multiple of 8");
     if (act_dtype != 0 && act_dtype != 1) return fail(LUMEN_MOE_INVALID_ARG, "unknown activation dtype");
+    if (reinterpret_cast<uintptr_t>(d_rows16) % 16) return fail(LUMEN_MOE_INVALID_ARG, "the 16-bit rows must lie on a 16-byte boundary");
     cudaError_t e = lumen::launch_ep_prepare(d_normed, act_dtype, s.R, tokens * s.K, s.H, s.E, experts_per_rank, d_rows16,
                                              d_local_ids, reinterpret_cast<long long*>(d_send_counts),
                                              static_cast<cudaStream_t>(stream));
@@ -375,6 +376,7 @@ lumen_moe_status_t lumen_moe_quantize(const float* d_src, int64_t n_elements, in
     if (!d_src || !d_dst) return fail(LUMEN_MOE_INVALID_ARG, "null argument");
     if (n_elements <= 0 || n_elements % 32) return fail(LUMEN_MOE_INVALID_ARG, "n_elements must be a positive multiple of 32");
     if (quant < 0 || quant > 2) return fail(LUMEN_MOE_UNSUPPORTED, "unsupported quant scheme");
+    if (quant != LUMEN_MOE_BF16 && reinterpret_cast<uintptr_t>(d_src) % 16) return fail(LUMEN_MOE_INVALID_ARG, "the source must lie on a 16-byte boundary");
     cudaError_t e = lumen::launch_quantize(d_src, n_elements, quant, d_dst, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(LUMEN_MOE_CUDA_ERROR, cudaGetErrorString(e));
     return LUMEN_MOE_OK;

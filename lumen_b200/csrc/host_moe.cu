@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 
 namespace lumen {
 
@@ -348,6 +349,13 @@ static Status check_layer(const CudaMoeScratch* s, const MoeLayer& layer) {
     return Status::Ok();
 }
 
+// Pointers that the kernels read or write 16 bytes at a time (null passes): an address in between would be a fault.
+static Status on_16_bytes(std::initializer_list<const void*> ptrs, const char* what) {
+    for (const void* p : ptrs)
+        if (reinterpret_cast<uintptr_t>(p) % 16) return Status::Err(1, std::string(what) + " must lie on a 16-byte boundary");
+    return Status::Ok();
+}
+
 static DecodeArgs make_decode_args(CudaMoeScratch* s, const MoeLayer& layer, int tokens) {
     DecodeArgs a{};
     a.L = layer.dev;
@@ -378,7 +386,8 @@ Status encode_moe_ffn_decode(CudaMoeScratch* s, const MoeLayer& layer, const flo
     if (tokens < 1 || tokens > DECODE_MAX_TOKENS) return Status::Err(1, "decode handles 1..16 tokens; use prefill");
     if (!normed_x || !residual || !output_x) return Status::Err(1, "null activation pointer");
     if (normed_x == output_x) return Status::Err(1, "output must not alias the normed input");
-    Status c = check_layer(s, layer);
+    Status c = on_16_bytes({normed_x}, "the activations");
+    if (c.ok()) c = check_layer(s, layer);
     if (!c.ok()) return c;
     DecodeArgs a = make_decode_args(s, layer, tokens);
     a.x = normed_x;
@@ -400,7 +409,8 @@ Status encode_moe_ffn_decode_fused_norm(CudaMoeScratch* s, const MoeLayer& layer
                                         int tokens, cudaStream_t st) {
     if (tokens < 1 || tokens > DECODE_MAX_TOKENS) return Status::Err(1, "decode handles 1..16 tokens; use prefill");
     if (!attn_proj || !ffn_norm || !output_x) return Status::Err(1, "null activation pointer");
-    Status c = check_layer(s, layer);
+    Status c = on_16_bytes({attn_proj, ffn_norm, normed_x}, "the activations, the norm weight and the normed output");
+    if (c.ok()) c = check_layer(s, layer);
     if (!c.ok()) return c;
     DecodeArgs a = make_decode_args(s, layer, tokens);
     a.x = attn_proj;
@@ -416,6 +426,10 @@ Status encode_moe_ffn_decode_fused_norm(CudaMoeScratch* s, const MoeLayer& layer
 Status encode_moe_stack_decode(CudaMoeScratch* s, const MoeLayer* const* layers, const float* const* gammas, int n_layers, float* x,
                                float eps, int tokens, cudaStream_t st) {
     if (tokens < 1 || tokens > DECODE_MAX_TOKENS) return Status::Err(1, "decode handles 1..16 tokens; use prefill");
+    for (int l = 0; l < n_layers; ++l) {
+        Status c = on_16_bytes({x, gammas[l]}, "the activations and the norm weights");
+        if (!c.ok()) return c;
+    }
     // One launch for a run of Q4_0 layers at one token. Not in a graph, where a cooperative launch follows the one before
     // without the gap (eight layers 136 us launched one by one, 140 in one; from the host 154 and 145), and not where the
     // tiles or the tokens are more (four layers: Q8_0 104 us one by one, 107 in one; three tokens of Q4_0 137 and 147).
@@ -461,6 +475,8 @@ Status encode_route_only(CudaMoeScratch* s, const MoeLayer* layer, const float* 
     if (!g.ok()) return g;
     const size_t C = (size_t)tokens * s->K;
     if (tokens <= DECODE_MAX_TOKENS) {
+        Status al = on_16_bytes({normed}, "the activations");
+        if (!al.ok()) return al;
         DecodeArgs a{};
         if (layer) a.L = layer->dev;
         a.L.H = s->H;
@@ -568,6 +584,9 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
         p.impl = 2;
         p.stream_starts = reinterpret_cast<int32_t*>(s->R.work);  // (decode's work records: 8 KB, unused by a prefill)
     }
+    // f16 output rows: stored in pairs by the streaming kernels, 16 bytes at a time by the others
+    if (reinterpret_cast<uintptr_t>(out16_rows) % (p.impl == 2 ? 4 : 16))
+        return Status::Err(1, "the f16 output rows must lie on a 16-byte boundary");
     const bool own_router = ids_in == nullptr && s->logits_override == nullptr;
     // Activation planes of the tcgen05 router (f16 high and low parts): the high one is also what the expert products
     // of both tensor-core paths read. The RMSNorm of a stack layer goes into their pass where nothing else reads the

@@ -145,6 +145,35 @@ def test_ids_in_the_reference_stride_e_layout(cuda_lib):
     assert np.array_equal(r["expert_bounds"], bounds)
 
 
+def test_pointers_between_16_byte_boundaries_are_refused_where_kernels_need_them(cuda_lib):
+    H, I, E, K, T = 512, 256, 16, 4, 3
+    _, blob, sc, layer = _ctx(H, I, E, K, 64)
+    one = _ctx(H, I, E, 1, 64)
+    x, off = torch.randn((T, H), device="cuda"), torch.zeros(T * H + 1, device="cuda")[1:].view(T, H)
+    gamma, gamma_off = torch.ones(H, device="cuda"), torch.ones(H + 1, device="cuda")[1:]
+    ids = torch.zeros(200, device="cuda", dtype=torch.int32)
+    rows16, out16 = torch.zeros((200, H), device="cuda"), torch.zeros(200 * H + 1, device="cuda", dtype=torch.float16)[1:]
+    sc.route_only(layer, x)  # leaves the tables ep_prepare needs
+    lib = _lib.lib()
+    calls = [
+        lambda: sc.decode(layer, off, x),
+        lambda: sc.decode_fused_norm(layer, off, gamma, 1e-6),
+        lambda: sc.decode_fused_norm(layer, x, gamma_off, 1e-6),
+        lambda: sc.decode_fused_norm(layer, x, gamma, 1e-6, off),
+        lambda: sc.stack_decode([layer], [gamma], off, 1e-6),
+        lambda: sc.stack_decode([layer, layer], [gamma, gamma_off], x, 1e-6),
+        lambda: sc.route_only(layer, off),
+        lambda: moe.quantize(off.view(-1), 1),
+        lambda: _lib.check(lib.lumen_moe_experts_routed_f16(one[2]._h, one[3]._h, rows16.data_ptr(), ids.data_ptr(), out16.data_ptr(), 200, 0, 0)),
+        lambda: _lib.check(lib.lumen_moe_ep_prepare(sc._h, x.data_ptr(), 0, T, 4, out16.data_ptr(), ids.data_ptr(), ids.data_ptr(), 0)),
+    ]
+    for call in calls:
+        with pytest.raises(moe.LumenMoeError) as ei:
+            call()
+        assert ei.value.code == _lib.INVALID_ARG and "16-byte" in str(ei.value)
+    assert torch.isfinite(sc.decode(layer, x, off, off)).all() and sc.poll_status() == _lib.OK
+
+
 def test_unknown_config_flags_are_rejected(cuda_lib):
     with pytest.raises(moe.LumenMoeError):
         moe.allocate_moe_scratch(256, 128, 8, 2, 16, flags=0x10)
