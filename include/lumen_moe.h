@@ -461,9 +461,11 @@ LUMEN_MOE_API lumen_moe_status_t lumen_moe_debug_expf(const float* d_in, float* 
 
 /* Instrumentation: re-launch ONE kernel of the most recent lumen_moe_decode call
  * on `layer` with the routing tables that call left in the context (phase 0 =
- * router, 1 = gate/up + SwiGLU, 2 = down + combine), so that a benchmark can time
- * a single kernel with CUDA events. No counterpart in the reference (its
- * profiler brackets whole stages, cuda/profiler.rs:1-80). */
+ * router, 1 = gate/up + SwiGLU, 2 = down + combine) of the kernel chain, so that a benchmark can time
+ * a single kernel with CUDA events. Phases 1 and 2 need the chain's tables: the most recent call on
+ * the context was a lumen_moe_decode that took the chain, or phase 0 (LUMEN_MOE_INVALID_ARG
+ * otherwise). No counterpart in the reference (its profiler brackets whole stages,
+ * cuda/profiler.rs:1-80). */
 LUMEN_MOE_API lumen_moe_status_t lumen_moe_debug_decode_phase(lumen_moe_ctx* ctx, const lumen_moe_layer* layer,
                                                               int32_t phase, void* stream);
 

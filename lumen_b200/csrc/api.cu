@@ -428,13 +428,23 @@ lumen_moe_status_t lumen_moe_debug_expf(const float* d_in, float* d_out, int64_t
     return LUMEN_MOE_OK;
 }
 
+static bool fits(const lumen_moe_ctx* ctx, const lumen_moe_layer* layer) {
+    const lumen::LayerDev& d = layer->layer.dev;
+    return d.H == ctx->scratch.H && d.I == ctx->scratch.I && d.E == ctx->scratch.E && d.quant >= 0;
+}
+
 lumen_moe_status_t lumen_moe_debug_decode_phase(lumen_moe_ctx* ctx, const lumen_moe_layer* layer, int32_t phase,
                                                 void* stream) {
     if (!ctx || !layer || phase < 0 || phase > 2) return fail(LUMEN_MOE_INVALID_ARG, "bad argument");
     if (!ctx->scratch.has_last_decode) return fail(LUMEN_MOE_INVALID_ARG, "no decode call has been made yet");
+    if (!fits(ctx, layer)) return fail(LUMEN_MOE_INVALID_ARG, "layer shape does not match the context");
+    // (the products follow the chain's work records: nothing else in the context may have overwritten them)
+    if (phase == 0) ctx->scratch.chain_tables = true;
+    if (!ctx->scratch.chain_tables)
+        return fail(LUMEN_MOE_INVALID_ARG, "the most recent call on this context did not take the decode chain; run phase 0 first");
     lumen::DecodeArgs a = ctx->scratch.last_decode;
     a.L = layer->layer.dev;
-    cudaError_t e = lumen::launch_decode_phase(a, phase, static_cast<cudaStream_t>(stream));
+    cudaError_t e = lumen::launch_decode_phase(a, phase, true, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(LUMEN_MOE_CUDA_ERROR, cudaGetErrorString(e));
     return LUMEN_MOE_OK;
 }
@@ -443,6 +453,7 @@ lumen_moe_status_t lumen_moe_debug_decode_trace(lumen_moe_ctx* ctx, const lumen_
                                                 uint64_t* d_trace, void* stream) {
     if (!ctx || !layer) return fail(LUMEN_MOE_INVALID_ARG, "bad argument");
     if (!ctx->scratch.has_last_decode) return fail(LUMEN_MOE_INVALID_ARG, "no decode call has been made yet");
+    if (!fits(ctx, layer)) return fail(LUMEN_MOE_INVALID_ARG, "layer shape does not match the context");
     lumen::DecodeArgs a = ctx->scratch.last_decode;
     a.L = layer->layer.dev;
     a.trace = reinterpret_cast<unsigned long long*>(d_trace);

@@ -556,7 +556,7 @@ cudaError_t launch_route_small(const DecodeArgs& a, cudaStream_t st) {
 bool decode_stream_applicable(const DecodeArgs& a);
 cudaError_t launch_gate_up_stream(const DecodeArgs& a, cudaStream_t st);
 
-cudaError_t launch_decode_phase(const DecodeArgs& a_in, int phase, cudaStream_t st) {
+cudaError_t launch_decode_phase(const DecodeArgs& a_in, int phase, bool alone, cudaStream_t st) {
     DecodeArgs a = a_in;
     // Q4_0 layers that gate_up_stream_kernel takes: int8 activations for both products; every other format and shape:
     // hi + lo fragments and the general streaming kernel
@@ -566,7 +566,7 @@ cudaError_t launch_decode_phase(const DecodeArgs& a_in, int phase, cudaStream_t 
     if (!int8) a.xq = a.sq = nullptr;
     if (phase == 0) return launch_route_small(a, st);
     if (phase == 1) return int8 ? launch_gate_up_stream(a, st) : launch_stream_gate_up(a, st);
-    return launch_stream_down(a, int8, st);
+    return launch_stream_down(a, int8, !alone, st);
 }
 
 bool decode_fused_applicable(const DecodeArgs& a);
@@ -593,7 +593,7 @@ bool decode_uses_fused(const DecodeArgs& a) {
 cudaError_t launch_decode(const DecodeArgs& a, cudaStream_t st) {
     if (decode_uses_fused(a)) return launch_decode_fused(a, st);
     for (int phase = 0; phase < 3; ++phase) {
-        const cudaError_t err = launch_decode_phase(a, phase, st);
+        const cudaError_t err = launch_decode_phase(a, phase, false, st);
         if (err != cudaSuccess) return err;
     }
     return cudaSuccess;

@@ -357,6 +357,7 @@ static Status on_16_bytes(std::initializer_list<const void*> ptrs, const char* w
 }
 
 static DecodeArgs make_decode_args(CudaMoeScratch* s, const MoeLayer& layer, int tokens) {
+    s->chain_tables = false;
     DecodeArgs a{};
     a.L = layer.dev;
     a.R = s->R;
@@ -395,6 +396,7 @@ Status encode_moe_ffn_decode(CudaMoeScratch* s, const MoeLayer& layer, const flo
     a.out = output_x;
     s->last_decode = a;
     s->has_last_decode = true;
+    s->chain_tables = !decode_uses_fused(a);
     if (s->expire_next[0] && !(single_expert(a) && decode_uses_fused(a))) {
         a.debug_expire = 1;
         s->expire_next[0] = 0;
@@ -474,6 +476,7 @@ Status encode_route_only(CudaMoeScratch* s, const MoeLayer* layer, const float* 
     Status g = ensure_prefill_grouped(s, tokens);
     if (!g.ok()) return g;
     const size_t C = (size_t)tokens * s->K;
+    s->chain_tables = false;
     if (tokens <= DECODE_MAX_TOKENS) {
         Status al = on_16_bytes({normed}, "the activations");
         if (!al.ok()) return al;
@@ -548,6 +551,7 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
     if (!c.ok()) return c;
     Status g = ensure_prefill_grouped(s, batch);
     if (!g.ok()) return g;
+    s->chain_tables = false;
     PrefillArgs p{};
     p.L = layer.dev;
     p.R = s->R;

@@ -125,6 +125,7 @@ struct CudaMoeScratch {
     const float* logits_override = nullptr;
     DecodeArgs last_decode{};   // arguments of the most recent decode call (instrumentation)
     bool has_last_decode = false;
+    bool chain_tables = false;      // the routing tables and work records are those of a call of the decode chain
     int prefill_impl = 0;
     int decode_impl = 0;            // 0 = fused persistent kernel where it applies, 1 = kernel chain
     unsigned int* bar = nullptr;    // grid barrier words of the fused decode kernel

@@ -194,7 +194,8 @@ constexpr int FUSED_MAX_TOKENS = 4;
 constexpr int FUSED_MAX_LAYERS = 64;  // layers of a stack in one launch (2 KB of kernel parameters)
 cudaError_t launch_decode_fused_stack(const DecodeArgs& a, const LayerDev* const* layers, const float* const* gammas, int n,
                                       float* x_tagged, cudaStream_t st);
-cudaError_t launch_decode_phase(const DecodeArgs& a, int phase, cudaStream_t st);  // one kernel of the kernel chain: 0 router, 1 gate/up, 2 down
+// one step of the kernel chain: 0 router, 1 gate/up, 2 down + combine. alone: any other step may be in front of it in the stream
+cudaError_t launch_decode_phase(const DecodeArgs& a, int phase, bool alone, cudaStream_t st);
 cudaError_t launch_quantize(const float* src, int64_t n, int quant, void* dst, cudaStream_t st);
 cudaError_t launch_rmsnorm(const float* x, const float* gamma, float* out, int T, int H, float eps,
                            cudaStream_t st);
@@ -279,7 +280,7 @@ inline int stream_max_columns(int quant, int experts) {
 }
 // gate/up of a decode batch, expert products of short prompts (stream.cu)
 cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st);
-cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, cudaStream_t st);
+cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_up, cudaStream_t st);
 cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __half* out16_rows, cudaStream_t st,
                                   const TcPeerOut* peer = nullptr);
 constexpr int STREAM_SHIFT = 5;

@@ -485,21 +485,26 @@ combine_f32_kernel(const float* __restrict__ d32, RouteDev R, const float* resid
     }
 }
 
+// chained: the kernel in front in the stream waits for the routing kernels before it lets this one start (see above)
 template <int Q, int MODE>
-cudaError_t launch_t(const Args& a, int sms, cudaStream_t st) {
+cudaError_t launch_t(const Args& a, int sms, cudaStream_t st, bool chained = true) {
     static SmemOptIn optin;
     const cudaError_t e = ensure_dyn_smem(stream_kernel<Q, MODE>, Shape<Q, MODE>::smem, optin);
     if (e != cudaSuccess) return e;
     count_launch();
+    if (!chained) {
+        stream_kernel<Q, MODE><<<sms, Cfg<Q>::WARPS * 32, Shape<Q, MODE>::smem, st>>>(a);
+        return cudaGetLastError();
+    }
     return launch_dep(stream_kernel<Q, MODE>, dim3(sms), dim3(Cfg<Q>::WARPS * 32), Shape<Q, MODE>::smem, st, a);
 }
 
 template <int MODE>
-cudaError_t launch_q(const Args& a, int sms, cudaStream_t st) {
+cudaError_t launch_q(const Args& a, int sms, cudaStream_t st, bool chained = true) {
     switch (a.L.quant) {
-        case Q4_0: return launch_t<Q4_0, MODE>(a, sms, st);
-        case Q8_0: return launch_t<Q8_0, MODE>(a, sms, st);
-        default: return launch_t<BF16, MODE>(a, sms, st);
+        case Q4_0: return launch_t<Q4_0, MODE>(a, sms, st, chained);
+        case Q8_0: return launch_t<Q8_0, MODE>(a, sms, st, chained);
+        default: return launch_t<BF16, MODE>(a, sms, st, chained);
     }
 }
 
@@ -531,14 +536,16 @@ cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st) {
     return stream::launch_q<stream::GATE_UP_2>(g, p.sms, st);
 }
 
-// down + combine of a decode batch; int8: the SwiGLU outputs are in p.sq (Q4_0), else fragments in p.sf
-cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, cudaStream_t st) {
+// down + combine of a decode batch; int8: the SwiGLU outputs are in p.sq (Q4_0), else fragments in p.sf. after_gate_up: the
+// gate/up kernel is in front of it in the stream
+cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_up, cudaStream_t st) {
     stream::Args d = stream::decode_args(p);
     d.b = int8 ? reinterpret_cast<const uint4*>(p.sq) : p.sf;
     d.b_row = (size_t)p.L.kg_i * 16;
     d.d32 = p.d32;
     d.debug_extra_tx = int8 ? p.debug_expire : 0;  // (the chain's first streaming kernel)
-    const cudaError_t e = int8 ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st) : stream::launch_q<stream::DOWN_2>(d, p.sms, st);
+    const cudaError_t e = int8 ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st, after_gate_up)
+                               : stream::launch_q<stream::DOWN_2>(d, p.sms, st, after_gate_up);
     if (e != cudaSuccess) return e;
     count_launch();
     // (H is a multiple of 32, so every row lies on the boundary that the first one does)

@@ -281,3 +281,28 @@ def test_residual_and_output_on_a_4_byte_boundary(cuda_lib, quant, T):
     o_out, _, _ = oracle.moe_layer(blob_np, 0, meta.expert_gate_offs, meta.expert_up_offs, meta.expert_down_offs, quant, H, I, E, K,
                                    x.cpu().numpy(), res.cpu().numpy(), ids=r["ids"], weights=r["weights"], threads=8)
     assert rel_l2((aligned - res).cpu().numpy(), o_out - res.cpu().numpy()) < TOL_REL_L2
+
+
+# the steps of the chain one by one: in any order on tables that the chain left, refused on tables of another call
+@pytest.mark.parametrize("quant", [0, 1, 2])
+def test_chain_phases_run_alone_on_the_chain_s_tables_only(cuda_lib, quant):
+    H, I, E, K, T = 512, 256, 32, 4, 16
+    _, _, _, sc, layer = make_layer(H, I, E, K, quant, seed=5, max_tokens=64)
+    x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(5), device="cuda")
+    out, one = torch.empty_like(x), torch.empty_like(x[:1])
+    good = sc.decode(layer, x, x, out).clone()
+    for order in ((2,), (0, 2), (1, 2), (2, 0, 2), (0, 1, 2)):
+        out.zero_()
+        for phase in order:
+            sc.debug_decode_phase(layer, phase)
+        assert torch.equal(out, good), order
+    sc.prefill(layer, x[:9].contiguous(), x[:9].contiguous())  # its shares lie where the chain's work records were
+    for phase in (1, 2):
+        with pytest.raises(moe.LumenMoeError):
+            sc.debug_decode_phase(layer, phase)
+    for phase in (0, 1, 2):
+        sc.debug_decode_phase(layer, phase)
+    assert torch.equal(out, good)
+    sc.decode(layer, x[:1], x[:1], one)  # the fused kernel keeps no work records
+    with pytest.raises(moe.LumenMoeError):
+        sc.debug_decode_phase(layer, 2)
