@@ -3,7 +3,6 @@
 #include "../../include/lumen_moe.h"
 #include "host_moe.hpp"
 #include <new>
-#include <vector>
 
 namespace lumen {
 long long read_launch_count(bool reset);
@@ -394,14 +393,13 @@ lumen_moe_status_t lumen_moe_stack_decode(lumen_moe_ctx* ctx, const lumen_moe_la
                                           const float* const* d_gammas, int32_t n_layers, float* d_x, float eps,
                                           int32_t tokens, void* stream) {
     if (!ctx || !layers || !d_gammas || !d_x || n_layers < 1) return fail(LUMEN_MOE_INVALID_ARG, "bad argument");
-    std::vector<const lumen::MoeLayer*> l(n_layers);
-    for (int i = 0; i < n_layers; ++i) {
+    for (int i = 0; i < n_layers; ++i)
         if (!layers[i] || !d_gammas[i]) return fail(LUMEN_MOE_INVALID_ARG, "null layer or gamma");
-        l[i] = &layers[i]->layer;
-    }
     // x <- x + MoE(rmsnorm(x)); residual and output are the same buffer (cuda/backend_impl.rs:3570-3573)
-    return done(lumen::encode_moe_stack_decode(&ctx->scratch, l.data(), d_gammas, n_layers, d_x, eps, tokens,
-                                               static_cast<cudaStream_t>(stream)));
+    const lumen::LayersOf list{layers, [](const void* handles, int i) -> const lumen::MoeLayer& {
+                                   return static_cast<const lumen_moe_layer* const*>(handles)[i]->layer;
+                               }};
+    return done(lumen::encode_moe_stack_decode(&ctx->scratch, list, d_gammas, n_layers, d_x, eps, tokens, static_cast<cudaStream_t>(stream)));
 }
 
 lumen_moe_status_t lumen_moe_stack_prefill(lumen_moe_ctx* ctx, const lumen_moe_layer* const* layers,

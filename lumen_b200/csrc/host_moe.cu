@@ -425,7 +425,7 @@ Status encode_moe_ffn_decode_fused_norm(CudaMoeScratch* s, const MoeLayer& layer
     return Status::Ok();
 }
 
-Status encode_moe_stack_decode(CudaMoeScratch* s, const MoeLayer* const* layers, const float* const* gammas, int n_layers, float* x,
+Status encode_moe_stack_decode(CudaMoeScratch* s, const LayersOf& layers, const float* const* gammas, int n_layers, float* x,
                                float eps, int tokens, cudaStream_t st) {
     if (tokens < 1 || tokens > DECODE_MAX_TOKENS) return Status::Err(1, "decode handles 1..16 tokens; use prefill");
     for (int l = 0; l < n_layers; ++l) {
@@ -443,13 +443,13 @@ Status encode_moe_stack_decode(CudaMoeScratch* s, const MoeLayer* const* layers,
         const LayerDev* devs[FUSED_MAX_LAYERS];
         int n = 0;
         for (; n < (in_one ? FUSED_MAX_LAYERS : 1) && l0 + n < n_layers; ++n) {
-            const MoeLayer& layer = *layers[l0 + n];
+            const MoeLayer& layer = layers[l0 + n];
             Status c = check_layer(s, layer);
             if (!c.ok()) return c;
             if (layer.dev.quant != Q4_0) break;
             devs[n] = &layer.dev;
         }
-        DecodeArgs a = make_decode_args(s, *layers[l0], tokens);
+        DecodeArgs a = make_decode_args(s, layers[l0], tokens);
         a.x = a.residual = x;
         a.out = x;
         a.gamma = gammas[l0];

@@ -163,7 +163,13 @@ Status encode_moe_ffn_decode_fused_norm(CudaMoeScratch* scratch, const MoeLayer&
                                         const float* attn_proj, const float* ffn_norm, float* normed_x,
                                         float* output_x, float eps, int tokens, cudaStream_t st);
 // x <- x + MoE_l(rmsnorm(x; gamma_l, eps)) in place, layer by layer
-Status encode_moe_stack_decode(CudaMoeScratch* scratch, const MoeLayer* const* layers, const float* const* gammas, int n_layers,
+// (the caller's array of handles is read in place: a copy would be an allocation that can throw, on a path behind a C entry)
+struct LayersOf {
+    const void* handles;
+    const MoeLayer& (*at)(const void* handles, int i);
+    const MoeLayer& operator[](int i) const { return at(handles, i); }
+};
+Status encode_moe_stack_decode(CudaMoeScratch* scratch, const LayersOf& layers, const float* const* gammas, int n_layers,
                                float* x, float eps, int tokens, cudaStream_t st);
 // activations that are rmsnorm(x; gamma, eps) of an f32 residual stream: `normed` is then scratch of the same size, written
 // only where the norm cannot be folded into the pass that prepares the operands
