@@ -24,8 +24,8 @@
 
 namespace lumen {
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+using dcommon::pdl_trigger;
+using dcommon::pdl_wait;
 
 constexpr int RS_THREADS = 512;  // 16 warps: the last CTA gates one token per warp at batches up to 16
 constexpr int RS_WARPS = RS_THREADS / 32;
@@ -51,7 +51,7 @@ __device__ __forceinline__ float warp_sum16(float (&v)[16]) {
 // experts with work and their work records. A pair's column is the number of pairs in front of it, which its
 // threads count directly (a scan over 256 experts was most of the time of this step).
 __device__ __forceinline__ void decode_tables(const RouteDev& R, const int* ids_s, int C, int E, int K, unsigned* mask_s, int* c0_s) {
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x;
     if (tid < MAX_EXPERTS / 32) mask_s[tid] = 0u;
     __syncthreads();
     // four threads per pair at up to 128 pairs, two above; each takes every 4th (2nd) quadruple of pairs
@@ -111,7 +111,6 @@ __device__ __forceinline__ void decode_tables(const RouteDev& R, const int* ids_
         const int u = (tid < MAX_EXPERTS) ? rank_of(tid) : U;
         R.expert_bounds[tid] = (u < U) ? c0_s[u] : C;
     }
-    (void)lane;
 }
 
 // Router of a decode batch. The first CTAs: the logits of an expert row (or two) for all tokens; the CTAs after them: the
@@ -341,13 +340,6 @@ __device__ __forceinline__ void tile_mma_pair(const WTile<Q>& wg, const WTile<Q>
     }
 }
 
-// Position of element r (0..15 within a half block) inside the 8-half fragment
-// vector: quad t = r/4, order within the quad (v0, v2, v1, v3).
-__device__ __forceinline__ int frag_pos(int r) {
-    const int m = r & 3;
-    return (m == 0) ? 0 : (m == 2) ? 1 : (m == 1) ? 2 : 3;
-}
-
 template <int Q>
 __global__ void __launch_bounds__(GU_THREADS)
 gate_up_kernel(const __grid_constant__ DecodeArgs a) {
@@ -431,26 +423,7 @@ gate_up_kernel(const __grid_constant__ DecodeArgs a) {
                 const int col = chunk + tokc;
                 const int irow = rt * 16 + row;
                 if (a.s_f32 != nullptr) a.s_f32[(size_t)col * I + irow] = sv;
-                const bool bf16_mode = (Q == BF16);
-                const int blk = irow >> 5, within = irow & 31, j = within >> 4, r16 = within & 15;
-                unsigned short hi_bits, lo_bits;
-                if (!bf16_mode) {
-                    const __half h = __float2half_rn(sv);
-                    const __half l = __float2half_rn(sv - __half2float(h));
-                    hi_bits = __half_as_ushort(h);
-                    lo_bits = __half_as_ushort(l);
-                } else {
-                    const __nv_bfloat16 h = __float2bfloat16_rn(sv);
-                    const __nv_bfloat16 l = __float2bfloat16_rn(sv - __bfloat162float(h));
-                    hi_bits = __bfloat16_as_ushort(h);
-                    lo_bits = __bfloat16_as_ushort(l);
-                }
-                unsigned short* sf16 = reinterpret_cast<unsigned short*>(a.sf);
-                const size_t in_vec = (size_t)j * 4 + frag_pos(r16);
-                const size_t v_hi = (((size_t)(col * 2 + 0) * nblk_i_pad + blk) * 4 + (r16 >> 2)) * 8 + in_vec;
-                const size_t v_lo = (((size_t)(col * 2 + 1) * nblk_i_pad + blk) * 4 + (r16 >> 2)) * 8 + in_vec;
-                sf16[v_hi] = hi_bits;
-                sf16[v_lo] = lo_bits;
+                dcommon::store_swiglu_frag<Q>(a.sf, col, irow, nblk_i_pad, sv);
             }
         }
         __syncthreads();

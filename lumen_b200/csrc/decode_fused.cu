@@ -228,7 +228,6 @@ struct RouteSm {
 // x ~ sx * (q0 + q1 / 254) with one f32 scale per 32-block (|error| <= amax_block * 1.6e-5),
 // q0 and q1 in adjacent MMA columns; the -8 offset of the nibbles is taken out with the
 // block's precomputed 8 * sx * sum(q0 + q1 / 254).
-constexpr bool kInt8GateUp = true;
 
 // The layers of a stack that one launch runs through (STACK), or nothing.
 template <bool STACK>
@@ -539,7 +538,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     // the word pair of lane quad t is adjacent: {inputs 4t..4t+3, inputs 16+4t..16+4t+3}
     const int xq_term = xq_term_words(nblk_pad), xq_tok = xq_tok_words(nblk_pad);  // in 32-bit words
     unsigned* xq = reinterpret_cast<unsigned*>(xs);
-    if (Q == Q4_0 && kInt8GateUp) {
+    if (Q == Q4_0) {
         const int sub = tid & 7;
 #pragma unroll 1
         for (int item = tid >> 3; item < Tb * nblk; item += FT / 8) {
@@ -756,7 +755,7 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
         const bool bvalid = jcol < ncol;
         const int tok = bvalid ? rs.col_tok[c0 + jcol] : 0;
         float acc_g[4] = {0.f, 0.f, 0.f, 0.f}, acc_u[4] = {0.f, 0.f, 0.f, 0.f};
-        if (Q == Q4_0 && kInt8GateUp) {
+        if (Q == Q4_0) {
             // acc[0] / acc[2]: rows gq / gq + 8 of the lane's token column t4 (acc[1], acc[3] stay zero)
             if (warp < kg_h) {
                 const unsigned* bq = xq + (size_t)tok * xq_tok + (gq & 1) * xq_term + (warp * 4) * 8 + t4 * 2;

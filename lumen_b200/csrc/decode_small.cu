@@ -1,13 +1,9 @@
-// gate/up + SwiGLU of the three-kernel decode chain for Q4_0 layers, on the integer tensor cores.
+// gate/up + SwiGLU of the decode chain for Q4_0 layers, on the integer tensor cores.
 #include "decode_common.cuh"
 
 namespace lumen {
 
-namespace {
-
 using namespace dcommon;
-
-}  // namespace
 
 // ---------------------------------------------------------------------------
 // gate/up + SwiGLU for decode batches, Q4_0 with int8 activations: streaming form.
@@ -175,23 +171,6 @@ gate_up_stream_kernel(const __grid_constant__ DecodeArgs a) {
     }
 }
 
-template <typename Kern>
-static cudaError_t launch_pdl_smem(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                                   const DecodeArgs& a) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    count_launch();
-    return cudaLaunchKernelEx(&cfg, kern, a);
-}
-
 static size_t gate_up_stream_smem(const DecodeArgs& a) {
     return (size_t)GS_WARPS * GS_RING * 2 * GS_TU4 * 16 + (size_t)a.T * xq_tok_words(a.L.kg_h * 4) * 4;
 }
@@ -209,7 +188,8 @@ cudaError_t launch_gate_up_stream(const DecodeArgs& a, cudaStream_t st) {
     static SmemOptIn optin;
     const cudaError_t e = ensure_dyn_smem(gate_up_stream_kernel, smem, optin);
     if (e != cudaSuccess) return e;
-    return launch_pdl_smem(gate_up_stream_kernel, dim3(a.sms), dim3(GS_WARPS * 32), smem, st, a);
+    count_launch();
+    return launch_dep(gate_up_stream_kernel, dim3(a.sms), dim3(GS_WARPS * 32), smem, st, a);
 }
 
 }  // namespace lumen

@@ -136,10 +136,8 @@ Status build_repacked(const CudaMoeScratch& sc, const void* layer_buf, size_t bl
     // Q4_0 / Q8_0 when the context asks to trade memory for prefill speed
     // (LUMEN_MOE_FLAG_PREFILL_F16_WEIGHTS: 2 bytes per weight more per layer).
     if ((quant == BF16 || (sc.flags & 0x8)) && H % 256 == 0 && I % 128 == 0) {
-        const size_t n = (size_t)E * 3 * I * H;
         CUDA_TRY(cudaMalloc(&out->gu16, (size_t)E * 2 * I * H * sizeof(__half)));
         CUDA_TRY(cudaMalloc(&out->dn16, (size_t)E * H * I * sizeof(__half)));
-        (void)n;
         CUDA_TRY(launch_dequant_f16(L.blob, offs.gate_offsets, offs.up_offsets, offs.down_offsets, L, out->gu16, out->dn16, st));
         L.gu16 = out->gu16;
         L.dn16 = out->dn16;

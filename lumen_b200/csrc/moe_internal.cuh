@@ -245,9 +245,9 @@ cudaError_t launch_split_x16(const void* x, int act_dtype, int T, int H, bool na
 bool norm_split_applicable(int H, const void* x, const void* gamma);
 cudaError_t launch_norm_split(const float* x, const float* gamma, float eps, int T, int H, bool natural, __half* x16, int32_t* any_lo,
                               cudaStream_t st);
-int router_tc_ksplit(int T, int E, int H, int sms);
+int router_tc_ksplit(int H);
 bool router_tc_applicable(int T, int E, int H, const void* x);
-cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int ksplit, const __half* x16, int32_t* any_lo,
+cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int ksplit, int sms, const __half* x16, int32_t* any_lo,
                                     float* part, int32_t* status, int32_t* status_host, unsigned wait_limit_us, cudaStream_t st);
 constexpr int ROUTER_TC_MAX_KSPLIT = 4;
 

@@ -85,10 +85,8 @@ struct Args {
     int a_rows_exp;              // rows per expert there: 2 I (gate rows then up rows) or H (down)
     int a_row1;                  // second operand's rows relative to the first: I (up) or 128 (next row tile of down)
     LayerDev L;
-    const int32_t* col_src_tok;  // unused by the GEMM (rows are pre-gathered); kept for diagnostics
     const int4* tiles;
     int32_t* n_tiles;            // [0..1] tiles of the gate/up and the down list, [2..3] the kernels' tile counters (zero at launch)
-    const void* b_src;      // 16-bit activations [rows, kdim], permuted order
     __half* out16;          // gate/up: S16 [C, I] permuted order; down: D16 [C, H] natural order
     int32_t* status;
     int32_t* status_host;   // mapped pinned copy of the status word for the host (null = none)
@@ -207,8 +205,8 @@ struct RawTile {  // bytes of one 16-row x 128-input tile: quants, then scales
 constexpr int STG_ROW_BYTES = 256 + 16;                 // 128 f16 outputs of one token + padding (bank spread)
 constexpr int STG_BYTES = 2 * 128 * STG_ROW_BYTES;      // two warp groups x 128 tokens
 
-// Debug aid (compile with -DLUMEN_TC_TRACE): per CTA, the cycles the MMA thread and the first
-// producer warp spend in their waits, read back with lumen_debug_tc_trace.
+// Debug aid (compile with -DLUMEN_TC_TRACE): per CTA, the MMA warp's cycles: [2] waiting for full stages, [3] waiting for a
+// free accumulator, [4] in all, and [5] its tiles, read back with lumen_debug_tc_trace.
 #ifdef LUMEN_TC_TRACE
 __device__ unsigned long long g_tc_trace[2][160][8];
 #define TRACE_WAIT(acc, expr) ([&] { const long long t0_ = clock64(); const bool r_ = (expr); (acc) += clock64() - t0_; return r_; }())
@@ -314,8 +312,6 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
     const int ntiles = a.n_tiles[MODE];
     const int kgs = a.kdim >> 7;   // 128-input groups (weight tile granularity)
     const int khs = kgs * 2;       // 64-input pipeline stages per tile
-    // every operand is f16 here: BF16 weights are converted exactly (see dequant_store)
-    const bool bf16_mode = false;
     // The n-th tile of this CTA (n counted by the caller): false when the list is exhausted or the
     // kernel gives up. The descriptor is copied and its ring slot released at once. WARP: the whole
     // warp takes it together (one arrival for all lanes), else one thread does.
@@ -721,7 +717,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                 // down: D[128 tokens, 256 output rows] = X[128, k] W[256, k]^T, the two adjacent 128-row
                 // weight operands of a stage forming one 256-row N operand; a tile of more than 128
                 // tokens is two such products per 16 inputs, into two accumulator sets
-                const uint32_t idesc = make_idesc(MODE == 1 ? 256 : n16, bf16_mode);
+                const uint32_t idesc = make_idesc(MODE == 1 ? 256 : n16, false);  // (every operand is f16)
                 const int nh = (tile.z > 128) ? 2 : 1;  // accumulator sets of the tile
                 for (int h = 0; ok && h < nh; ++h) {
                     const int ab = (v + h) % NACC, use = (v + h) / NACC;
@@ -893,10 +889,8 @@ cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, c
     cudaError_t te = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, tc::bbox_rows(gu_cols), &gu.tmap);
     if (te != cudaSuccess) return te;
     gu.L = p.L;
-    gu.col_src_tok = p.R.col_src_tok;
     gu.tiles = p.tiles;
     gu.n_tiles = p.n_tiles;
-    gu.b_src = x16;
     gu.out16 = p.s16;
     gu.status = p.status;
     gu.status_host = p.status_host;
@@ -907,10 +901,8 @@ cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, c
     tc::Args dn = gu;
     te = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, tc::bbox_rows(dn256 ? 256 : 128), &dn.tmap);
     if (te != cudaSuccess) return te;
-    dn.col_src_tok = nullptr;
     dn.debug_extra_tx = 0;  // the hook applies to the first kernel of the pair
     dn.tiles = p.tiles + (size_t)max_ct * (mt_gu > 0 ? mt_gu : 1);  // as laid out by launch_route_large
-    dn.b_src = p.s16;
     // out16_rows: write the down product straight into caller rows (row = col_src_tok[column])
     dn.out16 = out16_rows ? out16_rows : p.d16;
     dn.out_row_map = out16_rows ? p.R.col_src_tok : nullptr;

@@ -901,12 +901,12 @@ cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st) {
     } else if (lg == nullptr && a.L.router_w16 != nullptr && a.xr16 != nullptr && a.rpart != nullptr &&
                router_tc_applicable(T, E, H, a.x)) {
         // tcgen05 router: partial logits per k range, summed by the top-k kernel
-        nparts = router_tc_ksplit(T, E, H, a.sms > 0 ? a.sms : 148);
+        nparts = router_tc_ksplit(H);
         if (a.gamma != nullptr)
             CUDA_RET(launch_norm_split(static_cast<const float*>(a.x), a.gamma, a.eps, T, H, a.L.planes_natural, a.xr16, a.any_lo, st));
         else
             CUDA_RET(launch_split_x16(a.x, a.act_dtype, T, H, a.L.planes_natural, a.xr16, a.any_lo, st));
-        CUDA_RET(launch_router_logits_tc(a.L.router_w16, T, E, H, nparts, a.xr16, a.any_lo, a.rpart, a.status, a.status_host,
+        CUDA_RET(launch_router_logits_tc(a.L.router_w16, T, E, H, nparts, a.sms, a.xr16, a.any_lo, a.rpart, a.status, a.status_host,
                                          a.wait_limit_us, st));
         lg = a.rpart;
     } else if (lg == nullptr) {

@@ -322,10 +322,7 @@ cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, b
 // routed with: an expert-parallel rank routing its shard must get the bits one GPU gets for the
 // whole batch. Four ranges of whole 64-input stages when H allows (a few thousand tokens then
 // fill the machine), else two, else one.
-int router_tc_ksplit(int T, int E, int H, int sms) {
-    (void)T;
-    (void)E;
-    (void)sms;
+int router_tc_ksplit(int H) {
     const int stages = H / 64;
     return (stages % 4 == 0) ? 4 : (stages % 2 == 0) ? 2 : 1;
 }
@@ -367,7 +364,7 @@ static cudaError_t launch_rtc(const rtc::Args& a, cudaStream_t st) {
 }
 
 // logits partials of the whole batch from its planes (launch_split_x16 or launch_norm_split); part is scratch of the context
-cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int ksplit,
+cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int ksplit, int sms,
                                     const __half* x16, int32_t* any_lo, float* part, int32_t* status, int32_t* status_host,
                                     unsigned wait_limit_us, cudaStream_t st) {
     count_launch();
@@ -375,7 +372,7 @@ cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int 
     a.m_tiles = (E + 127) / 128;
     cudaError_t e = make_tmap_f16(w16, (uint64_t)2 * E, (uint64_t)H, 128, &a.tmap_w);
     if (e != cudaSuccess) return e;
-    const bool narrow = (T + 127) / 128 * a.m_tiles * ksplit < 148 / 2;
+    const bool narrow = (T + 127) / 128 * a.m_tiles * ksplit < sms / 2;  // tiles of 128 tokens would leave half of the SMs idle
     const int bn = narrow ? 32 : 128;
     e = make_tmap_f16(x16, (uint64_t)2 * T, (uint64_t)H, bn, &a.tmap_x);
     if (e != cudaSuccess) return e;

@@ -108,24 +108,6 @@ __device__ __forceinline__ void b_regs(const uint4& v, uint32_t& l0, uint32_t& l
     h1 = v.w;
 }
 
-// A bf16 pair as an f16 pair (exact for normal f16 magnitudes, as the f16 copies of the tcgen05 path)
-__device__ __forceinline__ uint32_t bf2_to_h2(uint32_t v) {
-    const __half2 h = __floats2half2_rn(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-template <int Q, int TERMS>
-__device__ __forceinline__ void unpack(const WTile<Q>& w, int b, uint32_t (&lo)[4], uint32_t (&hi)[4], const UnpackConst& k) {
-    unpack_block<Q>(w, b, lo, hi, k);
-    if (Q == BF16 && TERMS == 1) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            lo[i] = bf2_to_h2(lo[i]);
-            hi[i] = bf2_to_h2(hi[i]);
-        }
-    }
-}
-
 // acc += scale * (block b of the tile) x (eight columns)
 template <int Q, int TERMS>
 __device__ __forceinline__ void block_mma(const uint32_t (&lo)[4], const uint32_t (&hi)[4], const float2 sc, const uint4& bv,
@@ -133,13 +115,8 @@ __device__ __forceinline__ void block_mma(const uint32_t (&lo)[4], const uint32_
     uint32_t l0, l1, h0, h1;
     b_regs<TERMS>(bv, l0, l1, h0, h1);
     if constexpr (Q == BF16) {
-        if constexpr (TERMS == 1) {
-            mma_f16(acc, lo, l0, l1);
-            mma_f16(acc, hi, h0, h1);
-        } else {
-            mma_bf16(acc, lo, l0, l1);
-            mma_bf16(acc, hi, h0, h1);
-        }
+        mma_bf16(acc, lo, l0, l1);
+        mma_bf16(acc, hi, h0, h1);
     } else {
         float c[4] = {0.f, 0.f, 0.f, 0.f};
         mma_f16(c, lo, l0, l1);
@@ -174,6 +151,7 @@ stream_kernel(const __grid_constant__ Args a) {
     constexpr bool DOWN = S::down, I8 = S::int8;
     constexpr int WARPS = S::warps, RING = S::ring, NM = S::nm, TERMS = S::terms, NQ = QTraits<Q>::NQ, GRP = S::grp;
     static_assert(!I8 || Q == Q4_0, "the integer form is for Q4_0 nibbles");
+    static_assert(Q != BF16 || TERMS == 2, "prompts of BF16 layers take the tcgen05 kernels");
     extern __shared__ __align__(128) uint8_t ring_smem[];  // [WARPS][RING][NM][quants of GRP groups | their scales]
     __shared__ uint64_t bar_s[WARPS * RING];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -365,7 +343,7 @@ stream_kernel(const __grid_constant__ Args a) {
                         }
                     } else {
                         uint32_t lo[4], hi[4];
-                        unpack<Q, TERMS>(w[m], b, lo, hi, kc);
+                        unpack_block<Q>(w[m], b, lo, hi, kc);
 #pragma unroll
                         for (int g = 0; g < NG; ++g) block_mma<Q, TERMS>(lo, hi, sc, bc[g], acc[m][g]);
                     }
@@ -504,7 +482,9 @@ cudaError_t launch_q(const Args& a, int sms, cudaStream_t st, bool chained = tru
     switch (a.L.quant) {
         case Q4_0: return launch_t<Q4_0, MODE>(a, sms, st, chained);
         case Q8_0: return launch_t<Q8_0, MODE>(a, sms, st, chained);
-        default: return launch_t<BF16, MODE>(a, sms, st, chained);
+        default:
+            if constexpr (MODE == GATE_UP_1 || MODE == DOWN_1) return cudaErrorInvalidValue;  // (prefill_streams takes none)
+            else return launch_t<BF16, MODE>(a, sms, st, chained);
     }
 }
 
