@@ -53,7 +53,8 @@ BLK = {0: 34, 1: 18, 2: 64}
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the ncu
 # capture summarised under profiles/ (kernel, quant, tokens) -> bytes
-NCU_DRAM_BYTES_PER_LAUNCH = {("decode_fused_kernel", "q4_0", 1): 22_372_000}
+NCU_DRAM_BYTES_PER_LAUNCH = {("decode_fused_kernel", "q4_0", 1): 22_378_000,
+                             ("gate_up_stream_kernel", "q4_0", 16): 150_562_000}
 
 
 # arithmetic of the decode path per weight format (f32 activations in and out in all cases)
@@ -71,6 +72,13 @@ def algorithmic_bytes(T: int, U: int, quant: int) -> int:
 def gate_up_bytes(T: int, U: int, quant: int) -> int:
     """Compulsory traffic of the gate/up + SwiGLU kernel alone."""
     return U * 2 * (I * H // 32) * BLK[quant] + T * H * 4 + T * K * I * 4
+
+
+def chain_kernels(quant_name: str, T: int):
+    """Expert-product kernels of a decode batch on the kernel chain: gate/up, and down with the weighted sum."""
+    int8 = quant_name == "q4_0" and T >= 4
+    return ("gate_up_stream_kernel" if int8 else "stream_kernel<GATE_UP_2>",
+            ("stream_kernel<DOWN_2I>" if int8 else "stream_kernel<DOWN_2>") + " + combine_f32_kernel")
 
 
 def peaks():
@@ -593,12 +601,12 @@ def run_gpu(args):
 
     for _ in range(max(3, args.warmup)):
         step()
-    # The 3*L launches of a step are replayed from one CUDA graph (the reference's
+    # The launches of a step are replayed from one CUDA graph (the reference's
     # backend enqueues them from Rust; a Python loop would time the interpreter).
     torch.cuda.synchronize()
     moe.launch_count(reset=True)
     step()
-    launches_per_step = moe.launch_count(reset=True)  # L with the fused kernel, 3 L with the three-kernel chain
+    launches_per_step = moe.launch_count(reset=True)  # L with the fused kernel, 4 L with the kernel chain
     step_eager = step
     if not args.no_graph:
         torch.cuda.synchronize()
@@ -657,8 +665,8 @@ def run_gpu(args):
                          "since_kernel_start_us_median": {"tiles_requested": stamps[10], "last_gate_up_tile_arrived": stamps[11],
                                                           "end": stamps[9]}}
         else:
-            # each kernel of the chain alone, one launch per layer blob, CUDA events on the launch stream
-            # (phase 1 = gate/up + SwiGLU is the dominant kernel)
+            # each step of the chain alone, one run per layer blob, CUDA events on the launch stream
+            # (phase 1 = gate/up + SwiGLU is the dominant kernel; phase 2 is two kernels)
             def time_phase(phase, reps=5):
                 def run():
                     for l in range(L):
@@ -681,13 +689,12 @@ def run_gpu(args):
                 torch.cuda.synchronize()
                 return ev0.elapsed_time(ev1) / (reps * L)
             phase_ms = [time_phase(ph) for ph in (0, 1, 2)]
-            k_name = "gate_up_kernel"
+            k_name, down_name = chain_kernels(args.quant, T)
             k_ms = phase_ms[1]
             # routing tables in the context belong to the last layer called: same count of experts for every launch
             k_bytes = gate_up_bytes(T, U[-1], quant)
             achieved = k_bytes / (k_ms / 1e3) / 1e9
-            kernel_us = {"router_small_kernel": phase_ms[0] * 1e3, "gate_up_kernel": phase_ms[1] * 1e3,
-                         "down_combine_kernel": phase_ms[2] * 1e3}
+            kernel_us = {"router_small_kernel": phase_ms[0] * 1e3, k_name: phase_ms[1] * 1e3, down_name: phase_ms[2] * 1e3}
         traffic = NCU_DRAM_BYTES_PER_LAUNCH.get((k_name, args.quant, T))
         cpu = cpu_reference_leg(quant, T, 12.0, blob0)
         one = cpu_reference_leg(quant, T, 3.0, blob0, threads=1)
