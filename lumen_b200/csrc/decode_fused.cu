@@ -370,8 +370,9 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
     // SINGLE: one expert (the shared expert), as two kernels (1: gate/up, 2: down) chained as programmatic dependents. The
     // expert is known, so each requests its tiles before it waits for the kernel before; every CTA works out the gate
     // logit itself, nothing is ranked or sorted, and no CTA waits for another: the cooperative launch, which starts
-    // ~2.4 us after its predecessor's end, and both grid barriers fall away. 2048 x 512, three tokens: 14.5 -> 12.5 us without
-    // the router exchange, 10.8 as two kernels. (As a branch of the general kernel instead of an instance, every other
+    // ~2.4 us after its predecessor's end, and both grid barriers fall away. 2048 x 512, three tokens, called from the host:
+    // 14.4 -> 12.5 us without the router exchange, 11.0 as two kernels; replayed 12.3 -> 11.0, but alternating with a
+    // cooperative routed call in one graph the pair takes 40.4 us where two cooperative launches took 39.0. (As a branch of the general kernel instead of an instance, every other
     // call took 0.5 us longer: the instruction stream is what bounds them.)
     if (SINGLE && warp == 0) {
         if (lane == 0) rs.ue[0] = 0;
