@@ -97,7 +97,7 @@ lumen_moe_status_t lumen_moe_layer_prepare(lumen_moe_ctx* ctx, const void* d_lay
     }
     if (!gate_offs && !up_offs && !down_offs) {
         // router-only layer: nothing is repacked; usable with lumen_moe_route_only
-        if (router_off % 4 != 0 || router_off + (uint64_t)sc.E * sc.H * 4 > blob_bytes)
+        if (router_off % 4 != 0 || !lumen::inside_blob(router_off, (uint64_t)sc.E * sc.H * 4, blob_bytes))
             return fail(LUMEN_MOE_INVALID_ARG, "router weight misaligned or outside the layer blob");
         lumen_moe_layer* r = new (std::nothrow) lumen_moe_layer();
         if (!r) return fail(LUMEN_MOE_CUDA_ERROR, "out of host memory");
@@ -492,7 +492,7 @@ lumen_moe_status_t lumen_moe_ep_layer_prepare(lumen_moe_ctx* ctx, const void* d_
     int cur = -1;
     if (cudaGetDevice(&cur) != cudaSuccess || cur != sc.device)
         return fail(LUMEN_MOE_INVALID_ARG, "the context belongs to another CUDA device than the current one");
-    if (router_off % 4 != 0 || router_off + (uint64_t)sc.E * sc.H * 4 > blob_bytes)
+    if (router_off % 4 != 0 || !lumen::inside_blob(router_off, (uint64_t)sc.E * sc.H * 4, blob_bytes))
         return fail(LUMEN_MOE_INVALID_ARG, "router weight misaligned or outside the layer blob");
     const int epr = lumen::ep_experts_per_rank(ctx->ep), first = lumen::ep_rank(ctx->ep) * epr;
     lumen_moe_layer* l = new (std::nothrow) lumen_moe_layer();

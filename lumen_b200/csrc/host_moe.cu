@@ -92,12 +92,12 @@ Status build_repacked(const CudaMoeScratch& sc, const void* layer_buf, size_t bl
     if ((int)meta.expert_gate_offs.size() != E) return Status::Err(1, "expert count does not match the context");
     // cuda/moe.rs:1258-1271: router offset alignment and bounds
     if (meta.router_weight_off % 4 != 0) return Status::Err(1, "router weight offset is not 4-byte aligned");
-    if (meta.router_weight_off + (uint64_t)E * H * 4 > blob_bytes)
+    if (!inside_blob(meta.router_weight_off, (uint64_t)E * H * 4, blob_bytes))
         return Status::Err(1, "router weight exceeds the layer blob");
     const size_t gu_bytes = (size_t)I * row_bytes(H, quant), dn_bytes = (size_t)H * row_bytes(I, quant);
     for (int e = 0; e < E; ++e) {
-        if (meta.expert_gate_offs[e] + gu_bytes > blob_bytes || meta.expert_up_offs[e] + gu_bytes > blob_bytes ||
-            meta.expert_down_offs[e] + dn_bytes > blob_bytes)
+        if (!inside_blob(meta.expert_gate_offs[e], gu_bytes, blob_bytes) || !inside_blob(meta.expert_up_offs[e], gu_bytes, blob_bytes) ||
+            !inside_blob(meta.expert_down_offs[e], dn_bytes, blob_bytes))
             return Status::Err(1, "expert " + std::to_string(e) + " weight slice exceeds the layer blob");
     }
     LayerDev L{};

@@ -39,6 +39,9 @@ struct Status {
     }
 };
 
+// whether [off, off + bytes) lies inside a blob of `total` bytes, for any 64-bit offset (the sum may wrap)
+inline bool inside_blob(uint64_t off, uint64_t bytes, uint64_t total) { return off <= total && bytes <= total - off; }
+
 // lumen_format::index::TensorSlice / ExpertSlice / SubtensorOffsets restricted to
 // the fields this path reads (crates/lumen-format/src/index.rs).
 struct TensorSlice {

@@ -174,6 +174,28 @@ def test_pointers_between_16_byte_boundaries_are_refused_where_kernels_need_them
     assert torch.isfinite(sc.decode(layer, x, off, off)).all() and sc.poll_status() == _lib.OK
 
 
+@pytest.mark.parametrize("which", ["router_weight_off", "expert_gate_offs", "expert_up_offs", "expert_down_offs"])
+@pytest.mark.parametrize("off", [2**64 - 64, 2**63, "one past the end"])
+def test_layer_offsets_outside_the_blob_are_refused(cuda_lib, which, off):
+    # an offset so large that offset + length wraps round must not pass for a small one
+    H, I, E = 256, 128, 4
+    lay = synth.LayerLayout(H, I, E, 1)
+    blob = synth.make_layer_blob(lay, 0)
+    sc = moe.allocate_moe_scratch(H, I, E, 2, 16)
+    meta = lay.meta()
+    value = off if isinstance(off, int) else blob.numel()
+    if which == "router_weight_off":
+        meta.router_weight_off = value // 4 * 4
+    else:
+        offs = list(getattr(meta, which))
+        offs[2] = value
+        setattr(meta, which, offs)
+    with pytest.raises(moe.LumenMoeError) as ei:
+        sc.prepare_layer(blob, meta)
+    assert ei.value.code == _lib.INVALID_ARG
+    sc.prepare_layer(blob, lay.meta())  # the context is none the worse
+
+
 def test_unknown_config_flags_are_rejected(cuda_lib):
     with pytest.raises(moe.LumenMoeError):
         moe.allocate_moe_scratch(256, 128, 8, 2, 16, flags=0x10)
