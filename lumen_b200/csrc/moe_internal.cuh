@@ -12,14 +12,18 @@ namespace lumen {
 enum Quant : int { Q8_0 = 0, Q4_0 = 1, BF16 = 2 };
 
 constexpr int MAX_EXPERTS = 256;  // cuda/shaders/moe_router.cu:33
-// Columns per tile of the tcgen05 gate/up product (the down tiles of a one-GPU call follow it): 256 once the
-// experts average more than 128 columns (each dequantised weight tile then serves twice the
-// columns), else 128 (fewer empty columns in ragged tiles, epilogue overlapped); 128 too where its tiles are one wave
-// of both products, whose time is then that of one tile (a shared expert alone, 2048 x 512: 300 tokens 47 -> 41 us,
-// 1024 49 -> 46; at 4096, two waves down, 67 us with 256 and 73 with 128).
-inline int tc_gu_tile_cols(int columns, int experts, int hidden, int inter, int sms) {
+// Columns per tile of the tcgen05 gate/up product; the down tiles of a one-GPU call follow it. 512: the CTA-pair kernels
+// (prefill_pair.cu), once the experts average more than 176 columns (4096 tokens, H = 2048, I = 768, E = 128, K = 8:
+// 468 -> 425 us for Q8_0; at 187 columns an expert 338 -> 334, at 150 (H = 4096, I = 1536) 509 -> 524). 256 above 128 (each dequantised weight tile
+// then serves twice the columns), else 128 (fewer empty columns in ragged tiles, epilogue overlapped); 128 too where its
+// tiles are one wave of both products, whose time is then that of one tile (a shared expert alone, 2048 x 512: 300
+// tokens 47 -> 41 us, 1024 49 -> 46; at 4096, two waves down, 67 us with 256 and 73 with 128).
+// ctas: cap of the persistent grid (0 = every SM).
+constexpr int PAIR_TILE_COLS = 512;
+inline int tc_gu_tile_cols(int columns, int experts, int hidden, int inter, int sms, int ctas) {
     const int mt = inter / 128 > hidden / 256 ? inter / 128 : hidden / 256;
-    return (columns > 128 * experts && columns / 128 * mt > sms) ? 256 : 128;
+    if (columns <= 128 * experts || columns / 128 * mt <= sms) return 128;
+    return (columns > 176 * experts && ctas != 1) ? PAIR_TILE_COLS : 256;
 }
 constexpr int MAX_TOP_K = 16;     // cuda/shaders/moe_router.cu:34
 constexpr int DECODE_MAX_TOKENS = 16;
@@ -236,6 +240,8 @@ struct PrefillArgs {
     const float* weights_in; // [T,K] or null (= 1)
 };
 cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st);
+// grouped products on CTA pairs (prefill_pair.cu)
+cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int ctas, cudaStream_t st, __half* out16_rows);
 bool route_single_applicable(const PrefillArgs& a);  // one expert: launch_route_large leaves the operand plane in xr16, columns = tokens
 // tcgen05 router (route_tc.cu)
 cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, bool natural, cudaStream_t st);

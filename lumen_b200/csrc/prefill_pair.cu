@@ -1,0 +1,710 @@
+// Prefill grouped expert products on CTA pairs (tcgen05, cta_group::2): the form of a one-GPU call whose experts have
+// enough columns to be bound by the tensor cores. Smaller batches and expert-parallel calls: prefill_tc.cu. The products
+// are the reference's moe_grouped_gate_up_swiglu / moe_grouped_down kernels (cuda/shaders/moe_grouped.cu:1202-1760,
+// :2183-2598).
+//
+// What bounds it: the tensor cores, if their operands arrive. One CTA alone reads 96 bytes a clock of operands from its
+// shared memory for MMAs of 128 x 256 x 16, next to 32 + 32 written by its producers and its copies; 128 is all there
+// is. A pair multiplies 256 x 256 x 16: each CTA holds 128 rows of the weights and half of the columns, which its partner
+// reads as well, so that 64 bytes a clock are read. A tile has up to 512 columns (two
+// accumulator sets of 256, all of TMEM), so each dequantised weight serves twice as many columns as in the one-CTA form.
+//
+// Weights are the M operand of both products, [128 rows per CTA, k], and the columns the N operand:
+//   gate/up  a tile is 128 rows of I: 64 per CTA, as 64 gate and 64 up rows in groups of eight (eight gate rows, then
+//            the same eight up rows). In the 16 x 256-bit shape of tcgen05.ld a thread then has gate and up of the same
+//            two outputs, and SwiGLU needs no exchange
+//   down     a tile is 256 rows of H: 128 per CTA
+// N is 32..256 in steps of 32 per set, so ragged tiles cost what they hold. Results go through stmatrix (transposed) and a
+// small buffer of the warp, and leave as whole 32- or 64-byte pieces of a column's row.
+//
+// One CTA pair per two SMs, persistent; tiles are claimed from a device-wide counter by the first CTA of the pair.
+// Warps of a CTA: 0-7 epilogue (16 of them for gate/up when the weights come by TMA), then 16 weight producers (none with
+// TMA-fed weights), one thread for the copies, one warp for the MMAs (idle in the second CTA), one thread for the tiles
+// (idle in the second CTA). Every wait is bounded; on expiry the kernel raises the status word, lets its copies and
+// MMAs end, frees its TMEM and returns.
+#include "mma_frag.cuh"
+#include "tc_common.cuh"
+
+namespace lumen {
+
+namespace pair {
+
+using namespace tc;
+
+constexpr int PROD_WARPS = 16;
+constexpr int STAGES = 4;                                // of 64 inputs (one swizzle atom in K)
+constexpr int STAGE_BYTES = SUB_BYTES + 2 * SUB_BYTES;   // 128 weight rows, then this CTA's half of two sets of 256 columns
+constexpr int SCHED_RING = 8;                            // tile descriptors in flight between the scheduler and the roles
+constexpr int MAX_AHEAD = 4;                             // tiles that are claimed ahead of the MMAs at most
+constexpr int SKEW = 2;                                  // stages by which the sets of a wide tile are taken apart at its ends
+constexpr int TMEM_COLS = 512;
+
+template <int MODE, bool ATMA>
+struct Roles {
+    static constexpr int epi = (ATMA && MODE == 0) ? 16 : 8, prod = ATMA ? 0 : PROD_WARPS;
+    static constexpr int prod0 = epi, tma = epi + prod, mma = tma + 1, sched = mma + 1, threads = (sched + 1) * 32;
+    // a warp's output buffer: 32 columns of its 16 (gate/up) or 32 (down) rows, padded so that the eight rows of an
+    // stmatrix hit eight different 16-byte bank groups
+    static constexpr int row_bytes = (MODE == 0) ? 32 : 64, pitch = row_bytes + 16, out_bytes = 32 * pitch;
+    static constexpr size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + (size_t)epi * out_bytes;
+};
+
+struct Args {
+    CUtensorMap tmap_n;   // columns [rows, kdim] f16, box 64 x 32
+    CUtensorMap tmap_w;   // the same, box 64 x 128
+    CUtensorMap tmap_a;   // ATMA: the experts' f16 matrices (gate/up: in groups of eight gate and eight up rows)
+    LayerDev L;
+    const int4* tiles;    // {expert, first column, columns, m-tile}
+    int32_t* n_tiles;     // [0..1] tiles of the gate/up and the down list, [2..3] the kernels' tile counters
+    __half* out16;        // gate/up: S16 [C, I] in the order down reads it; down: D16 [C, H]
+    const int32_t* out_row_map;  // down: output row of compact column c (null = c itself)
+    int32_t* status;
+    int32_t* status_host;
+    uint64_t wait_limit_ns;
+    int debug_extra_tx;   // test hook: the first stage's barrier expects this many bytes too many
+    int kdim;             // H (gate/up) or I (down)
+    int out_ld;           // I or H
+};
+
+// --- pair-wide forms of the building blocks ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cta_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// the address, in the pair's window, of the same shared-memory location of CTA `rank`
+__device__ __forceinline__ uint32_t map_to(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void arrive_at(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void arrive_release_at(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ bool try_acquire(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// mbar_wait for barriers that the other CTA arrives at with something written
+__device__ __forceinline__ bool wait_acquire(uint32_t bar, uint32_t parity, const AbortCtl& ac) {
+    if (try_acquire(bar, parity)) return true;
+    const uint64_t t0 = globaltimer_ns();
+    for (uint32_t i = 0;; ++i) {
+        if (try_acquire(bar, parity)) return true;
+        if ((i & 63u) == 63u) {
+            if (*ac.flag) return false;
+            if (globaltimer_ns() - t0 > ac.limit_ns) {
+                *ac.flag = 1u;
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ void pair_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// D[256, N] (+)= A[256, 16] B[N, 16]^T over the pair: each CTA holds 128 rows of A and N / 2 rows of B at these addresses
+__device__ __forceinline__ void umma2(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+}
+// one arrival at this barrier of both CTAs once the MMAs issued so far are done
+__device__ __forceinline__ void umma2_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"((uint16_t)3)
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t idesc2(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((256u >> 4) << 24); }
+// copies whose bytes count on a barrier of the pair's first CTA
+__device__ __forceinline__ void tma_pair_2d(uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t cluster_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(cluster_bar)
+        : "memory");
+}
+__device__ __forceinline__ void tma_pair_5d(uint32_t dst, const CUtensorMap* m, int x, int c1, int c2, int c3, int c4, uint32_t cluster_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], "
+        "[%7];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(cluster_bar)
+        : "memory");
+}
+// 16 TMEM lanes x 32 columns in the accumulator-fragment shape: v[4j..4j+1] row lane / 4, columns 8j + 2 (lane % 4) and the
+// next, v[4j+2..4j+3] row lane / 4 + 8
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+// four 8 x 8 matrices of 16-bit elements, each stored transposed; lane l gives the address of row l % 8 of matrix l / 8
+__device__ __forceinline__ void stmatrix4_t(uint32_t addr, const uint32_t (&v)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t pack_f16(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// --- dequantisation ---------------------------------------------------------------------------------------------------
+// A producer warp owns 16 rows x 64 inputs (blocks 2 sub, 2 sub + 1 of every 128-input group) of this CTA's operand: eight
+// warps fill a stage, the other eight the next one. What a lane holds of it:
+template <int Q>
+struct Half {
+    uint4 q[Q == Q4_0 ? 1 : 2];
+    uint32_t s_g, s_g8;  // f16 scales of the two blocks, rows g and g + 8
+};
+// groups a warp keeps on the way in registers: 128 rows x 128 inputs are 9 (Q4_0) or 17 KB an SM
+template <int Q>
+struct Prefetch {
+    static constexpr int depth = (Q == Q4_0) ? 4 : 3;
+};
+
+// Where a lane's chunks go in the operand: 16 bytes of row m at (m / 8) 1024 + (m % 8) 128 + ((chunk ^ m % 8) 16).
+// A quarter warp is two rows g of four chunks each. Down: rows in order, the two rows' m % 8 agree in bit 2, and the odd
+// one takes the second block first. Gate/up: rows in the order in which down reads their outputs, their m % 8
+// differ in bit 2, and both take the same block. Either way eight lanes hit eight different bank groups.
+template <int MODE>
+struct Place {
+    uint32_t off[2];  // first / second pass, row g
+    static constexpr uint32_t row8 = (MODE == 0) ? 4096 : 1024;  // row g + 8 from there
+    bool swap;
+    __device__ __forceinline__ Place(int rtl, int lane) {
+        const int g = lane >> 2, t = lane & 3;
+        int m;
+        if (MODE == 0) {
+            const int op = rtl >> 2, rt = rtl & 3, hi = rt & 1, mm = g & 3;
+            const int slot = 4 * (mm & 1) + 2 * hi + (mm >> 1);
+            m = 64 * (rt >> 1) + 16 * (g >> 2) + 8 * op + slot;
+            swap = false;
+        } else {
+            m = 16 * rtl + g;
+            swap = (g & 1) != 0;
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int second = p ^ (swap ? 1 : 0);
+            off[p] = (uint32_t)((m >> 3) * 1024 + (m & 7) * 128 + ((((second << 2) + t) ^ (m & 7)) << 4));
+        }
+    }
+};
+
+__device__ __forceinline__ uint32_t scale_f16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ void store16(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+template <int Q, int MODE>
+__device__ __forceinline__ void dequant(const Half<Q>& w, uint32_t a_base, const Place<MODE>& pl, const UnpackConst& k) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            // (gate/up never swaps: the selections below fold away)
+            const bool second = (MODE == 0) ? (p == 1) : ((p == 1) != pl.swap);
+            const uint32_t sc = prmt(r ? w.s_g8 : w.s_g, 0u, second ? 0x3232u : 0x1010u);
+            uint32_t l0, l1, h0, h1;
+            if constexpr (Q == Q4_0) {
+                const uint32_t a = r ? w.q[0].y : w.q[0].x, b = r ? w.q[0].w : w.q[0].z;
+                const uint32_t x = second ? b : a, y = x >> 8;
+                l0 = hsub2_u32(lop_and_or(x, 0x000F000Fu, k.or_a), k.sub_a);
+                h0 = hsub2_u32(lop_and_or(x, 0x00F000F0u, k.or_b), k.sub_b);
+                l1 = hsub2_u32(lop_and_or(y, 0x000F000Fu, k.or_a), k.sub_a);
+                h1 = hsub2_u32(lop_and_or(y, 0x00F000F0u, k.or_b), k.sub_b);
+            } else {
+                const uint32_t a0 = r ? w.q[0].z : w.q[0].x, a1 = r ? w.q[0].w : w.q[0].y;
+                const uint32_t b0 = r ? w.q[1].z : w.q[1].x, b1 = r ? w.q[1].w : w.q[1].y;
+                const uint32_t x = (second ? b0 : a0) ^ k.or_b, y = (second ? b1 : a1) ^ k.or_b;
+                l0 = hsub2_u32(prmt(x, k.or_a, 0x4240u), k.sub_a);
+                l1 = hsub2_u32(prmt(x, k.or_a, 0x4341u), k.sub_a);
+                h0 = hsub2_u32(prmt(y, k.or_a, 0x4240u), k.sub_a);
+                h1 = hsub2_u32(prmt(y, k.or_a, 0x4341u), k.sub_a);
+            }
+            store16(a_base + pl.off[p] + r * Place<MODE>::row8, scale_f16x2(l0, sc), scale_f16x2(h0, sc), scale_f16x2(l1, sc), scale_f16x2(h1, sc));
+        }
+}
+
+// SwiGLU (cuda/shaders/moe_expert.cu:47-50) as in prefill_tc.cu
+__device__ __forceinline__ float swiglu(float g, float u) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return g * r * u;
+}
+
+// columns of set h of a tile, rounded up to what an MMA of the pair takes
+__device__ __forceinline__ int set_cols(int ncols, int h) { return (min(256, ncols - 256 * h) + 31) & ~31; }
+
+template <int Q, int MODE, bool ATMA>
+__global__ void __launch_bounds__(Roles<MODE, ATMA>::threads, 1)
+grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
+    using R = Roles<MODE, ATMA>;
+    extern __shared__ uint8_t smem_raw[];
+    // "first": used in the pair's first CTA only, which both CTAs' roles arrive at
+    __shared__ uint64_t full_bar[STAGES];      // first: a stage is filled in both CTAs
+    __shared__ uint64_t empty_bar[STAGES];     // a stage has been multiplied
+    __shared__ uint64_t acc_full_bar[2];       // an accumulator set is complete
+    __shared__ uint64_t acc_empty_bar[2];      // first: it has been read in both CTAs
+    __shared__ uint64_t sched_full_bar[SCHED_RING];
+    __shared__ uint64_t sched_empty_bar[SCHED_RING];  // first
+    __shared__ uint64_t go_bar[MAX_AHEAD];     // first: the next tile may be claimed
+    __shared__ uint64_t drain_bar;             // give-up path: the MMAs issued are done
+    __shared__ int4 sched_tile_s[SCHED_RING];
+    __shared__ uint32_t tmem_base_s;
+    __shared__ uint32_t abort_s;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = cta_rank();
+    const uint32_t stage0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const AbortCtl abort_flag{&abort_s, a.wait_limit_ns};
+
+    if (tid == 0) {
+        abort_s = 0u;
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), 1 + 2 * (R::prod / 2));  // the copies' expected bytes, eight producer warps of each CTA
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&acc_full_bar[b]), 1);
+            mbar_init(smem_u32(&acc_empty_bar[b]), 2 * R::epi);
+        }
+        for (int s = 0; s < SCHED_RING; ++s) {
+            mbar_init(smem_u32(&sched_full_bar[s]), 1);
+            mbar_init(smem_u32(&sched_empty_bar[s]), 2 * (R::epi + R::prod + 1) + 1);  // readers: epilogue, producers, copies of both; MMAs
+        }
+        for (int i = 0; i < MAX_AHEAD; ++i) mbar_init(smem_u32(&go_bar[i]), 1);
+        mbar_init(smem_u32(&drain_bar), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == R::mma) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"((uint32_t)TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    pair_sync();  // both CTAs' barriers exist before either arrives at the other's
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_base_s;
+
+    grid_dep_sync();
+    const int ntiles = a.n_tiles[MODE];
+    const int kgs = a.kdim >> 7;  // 128-input groups
+    const int khs = kgs * 2;      // 64-input stages per tile
+    const int cl = blockIdx.x >> 1, ncl = gridDim.x >> 1;
+    const uint32_t sched_empty_first = map_to(smem_u32(&sched_empty_bar[0]), 0);
+
+    // The n-th tile of the pair (n counted by the caller): false when the list is exhausted or the kernel gives up.
+    auto take_tile = [&](bool whole_warp, int& n, int4& tile) -> bool {
+        const int slot = n % SCHED_RING;
+        bool ok = wait_acquire(smem_u32(&sched_full_bar[slot]), (n / SCHED_RING) & 1, abort_flag);
+        if (whole_warp) ok = __all_sync(0xffffffffu, ok);
+        if (!ok) return false;
+        tile = sched_tile_s[slot];
+        if (whole_warp) __syncwarp();
+        if (!whole_warp || lane == 0) arrive_at(sched_empty_first + slot * 8);
+        ++n;
+        return tile.z >= 0;
+    };
+    // How many tiles are claimed ahead of the MMAs, and at which stage of a tile they allow the next claim. Long tiles:
+    // one ahead, late in a wide tile so that the last tiles go to the pairs that are free first (before the producers need
+    // it: they hold up to `depth` groups and four stages beyond the MMAs), at the start of a narrow one, which
+    // is over in about the time of a claim. Short ones: two ahead, so that the producers never run dry; four
+    // where a tile is one group, because the producers' registers hold more than two of them.
+    const int ahead = (khs >= 24) ? 1 : (kgs >= 2) ? 2 : MAX_AHEAD;
+
+    if (warp < R::epi) {
+        // ------------------------------ epilogue ------------------------------
+        constexpr int PARTS = R::epi / 4;
+        const int quad = warp & 3, part = warp >> 2;  // (TMEM lanes 32 quad.. are this warp's by the hardware's rule)
+        const uint32_t buf = stage0 + STAGES * STAGE_BYTES + (uint32_t)warp * R::out_bytes;
+        const uint32_t acc_empty_first = map_to(smem_u32(&acc_empty_bar[0]), 0);
+        const uint32_t st_addr = buf + lane * R::pitch;  // row `lane` of the buffer: column `lane` of the chunk
+        int v = 0, tn = 0;
+        int4 tile;
+        bool ok = true;
+        while (ok && take_tile(true, tn, tile)) {
+            const int nsets = (tile.z > 256) ? 2 : 1;
+            // this warp's first output of a column's row
+            const int o0 = (MODE == 0) ? tile.w * 128 + (int)rank * 64 + quad * 16 : tile.w * 256 + (int)rank * 128 + quad * 32;
+            for (int h = 0; h < nsets; ++h, ++v) {
+                const int set = v & 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_full_bar[set]), (v >> 1) & 1, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+                const int ncols = min(256, tile.z - 256 * h), col0 = tile.y + 256 * h;
+                const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + set * 256;
+                for (int c = part * 32; c < ncols; c += PARTS * 32) {
+                    uint32_t v0[16], v1[16];
+                    tmem_ld_frag32(taddr + c, v0);
+                    tmem_ld_frag32(taddr + (16u << 16) + c, v1);
+                    tmem_ld_wait();
+                    __syncwarp();  // the chunk before has left the buffer
+                    auto rows16 = [&](const uint32_t (&x)[16], int half) {
+                        if (MODE == 0) {
+                            uint32_t o[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                o[j] = pack_f16(swiglu(__uint_as_float(x[4 * j]), __uint_as_float(x[4 * j + 2])),
+                                                swiglu(__uint_as_float(x[4 * j + 1]), __uint_as_float(x[4 * j + 3])));
+                            stmatrix4_t(st_addr + half * 16, o);
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 2; ++q) {
+                                uint32_t o[4];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) o[j] = pack_f16(__uint_as_float(x[4 * j + 2 * q]), __uint_as_float(x[4 * j + 2 * q + 1]));
+                                stmatrix4_t(st_addr + half * 32 + q * 16, o);
+                            }
+                        }
+                    };
+                    rows16(v0, 0);
+                    rows16(v1, 1);
+                    __syncwarp();
+                    constexpr int PIECES = R::row_bytes / 16;  // 16-byte pieces of a column
+#pragma unroll
+                    for (int i = 0; i < PIECES; ++i) {
+                        const int p = i * 32 + lane, cc = p / PIECES, pc = p % PIECES;
+                        const uint4 x = lds128(buf + cc * R::pitch + pc * 16);
+                        if (c + cc < ncols) {
+                            int row = col0 + c + cc;
+                            if (MODE == 1 && a.out_row_map != nullptr) row = a.out_row_map[row];
+                            *reinterpret_cast<uint4*>(a.out16 + (size_t)row * a.out_ld + o0 + pc * 8) = x;
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) arrive_at(acc_empty_first + set * 8);
+            }
+        }
+    } else if (warp < R::tma) {
+        // --------------------------- weight producers --------------------------
+        if constexpr (!ATMA) {
+            const int pw = warp - R::prod0, rtl = pw & 7, sub = pw >> 3;
+            constexpr int PF = Prefetch<Q>::depth, NQH = QTraits<Q>::NQ / 2;
+            const Place<MODE> pl(rtl, lane);
+            const UnpackConst k = unpack_const_pinned<Q>();
+            const uint32_t full_first = map_to(smem_u32(&full_bar[0]), 0);
+            int tn = 0, pkg = kgs;
+            bool more = true;
+            const uint4* qp = nullptr;
+            const uint32_t* sp = nullptr;
+            // the next group of the list into registers; false when there is none. The descriptor of a tile that is still
+            // to be claimed is waited for: it comes without any help from the groups that are held here (see `ahead`)
+            auto load_next = [&](Half<Q>& w) -> bool {
+                if (pkg == kgs) {
+                    int4 tile;
+                    if (more) more = take_tile(true, tn, tile);
+                    if (!more) return false;
+                    const int e = tile.x;
+                    const uint4 *qb, *sb;
+                    int rt;
+                    if (MODE == 0) {
+                        const bool up = rtl >= 4;
+                        qb = up ? a.L.up_q(e) : a.L.gate_q(e);
+                        sb = up ? a.L.up_s(e) : a.L.gate_s(e);
+                        rt = tile.w * 8 + (int)rank * 4 + (rtl & 3);
+                    } else {
+                        qb = a.L.down_q(e);
+                        sb = a.L.down_s(e);
+                        rt = tile.w * 16 + (int)rank * 8 + rtl;
+                    }
+                    const size_t tidx = (size_t)rt * kgs;
+                    qp = qb + (tidx * QTraits<Q>::NQ + sub * NQH) * 32 + lane;
+                    sp = reinterpret_cast<const uint32_t*>(sb + tidx * 8 + (lane >> 2)) + sub;
+                    pkg = 0;
+                }
+#pragma unroll
+                for (int j = 0; j < NQH; ++j) w.q[j] = ldg_stream(qp + j * 32);
+                w.s_g = __ldg(sp);
+                w.s_g8 = __ldg(sp + 2);
+                qp += QTraits<Q>::NQ * 32;
+                sp += 32;
+                ++pkg;
+                return true;
+            };
+            Half<Q> w[PF];
+            bool there[PF];
+#pragma unroll
+            for (int j = 0; j < PF; ++j) there[j] = load_next(w[j]);
+            int s = sub, ph = 0;  // this warp's stages are every second one
+            bool ok = true;
+            while (ok) {
+#pragma unroll
+                for (int j = 0; j < PF; ++j) {
+                    ok = ok && there[j];
+                    if (!ok) break;
+                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag));
+                    if (!ok) break;
+                    dequant<Q, MODE>(w[j], stage0 + s * STAGE_BYTES, pl, k);
+                    fence_proxy_async();  // every lane's own stores, before the warp's one arrival
+                    __syncwarp();
+                    if (lane == 0) arrive_at(full_first + s * 8);
+                    s += 2;
+                    if (s >= STAGES) {
+                        s -= STAGES;
+                        ph ^= 1;
+                    }
+                    there[j] = load_next(w[j]);
+                }
+            }
+        }
+    } else if (warp == R::tma) {
+        // ------------------------------- copies --------------------------------
+        if (lane == 0) {
+            const uint32_t full_first = map_to(smem_u32(&full_bar[0]), 0);
+            int tn = 0, n = 0;
+            bool ok = true;
+            int4 tile;
+            while (ok && take_tile(false, tn, tile)) {
+                const int nsets = (tile.z > 256) ? 2 : 1;
+                int row[2], nbox[2];  // boxes: 0 = one of 128 rows, else of 32
+                uint32_t bytes = 0;
+                for (int h = 0; h < nsets; ++h) {
+                    const int half = set_cols(tile.z, h) / 2;
+                    row[h] = tile.y + 256 * h + (int)rank * half;
+                    nbox[h] = (half == 128) ? 0 : (half + 31) / 32;
+                    bytes += (nbox[h] ? nbox[h] * 32 : 128) * 128;
+                }
+                if (ATMA) bytes += SUB_BYTES;
+                for (int kh = 0; kh < khs; ++kh, ++n) {
+                    const int s = n % STAGES, ph = (n / STAGES) & 1;
+                    ok = mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag);
+                    if (!ok) break;
+                    // both CTAs' bytes (their copies have the same shape) are expected once, by the first CTA
+                    if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * bytes + (n == 0 ? a.debug_extra_tx : 0));
+                    const uint32_t base = stage0 + s * STAGE_BYTES, bar = full_first + s * 8;
+                    if (ATMA) {
+                        if (MODE == 0)
+                            tma_pair_5d(base, &a.tmap_a, kh * 64, 0, 0, tile.w * 16 + (int)rank * 8, tile.x, bar);
+                        else
+                            tma_pair_2d(base, &a.tmap_a, kh * 64, tile.x * a.L.H + tile.w * 256 + (int)rank * 128, bar);
+                    }
+                    for (int h = 0; h < nsets; ++h) {
+                        const uint32_t dst = base + (1 + h) * SUB_BYTES;
+                        if (nbox[h] == 0) {
+                            tma_pair_2d(dst, &a.tmap_w, kh * 64, row[h], bar);
+                        } else {
+                            for (int q = 0; q < nbox[h]; ++q) tma_pair_2d(dst + q * 4096, &a.tmap_n, kh * 64, row[h] + q * 32, bar);
+                        }
+                    }
+                }
+            }
+            if (*abort_flag.flag) {
+                // the copies land before the shared memory goes away. The second CTA cannot watch the first one's barriers:
+                // it waits as long as the first one does at most
+                if (rank == 0) {
+                    let_land(smem_u32(&full_bar[0]), STAGES, n);
+                } else {
+                    const uint64_t t0 = globaltimer_ns();
+                    while (globaltimer_ns() - t0 < STAGES * 1000000ull) {
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == R::mma) {
+        // -------------------------------- MMA ---------------------------------
+        if (rank == 0) {
+            int tl = 0, tn = 0, v = 0, s = 0, ph = 0;
+            bool ok = true;
+            int4 tile;
+            for (; ok && take_tile(true, tn, tile); ++tl) {
+                const int nsets = (tile.z > 256) ? 2 : 1;
+                const int go_kh = (khs >= 24 && tile.z > 128) ? khs / 2 - 4 : 0;
+                const uint32_t id0 = idesc2(set_cols(tile.z, 0)), id1 = idesc2(nsets == 2 ? set_cols(tile.z, 1) : 32);
+                const int set0 = v & 1, set1 = set0 ^ 1;
+                const uint32_t acc0 = tmem_base + set0 * 256, acc1 = tmem_base + set1 * 256;
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_empty_bar[set0]), ((v >> 1) & 1) ^ 1, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+                // A wide tile holds both sets, and its epilogue would leave the tensor cores idle. So its first and its last
+                // SKEW stages are multiplied set by set: the first set is complete, and its epilogue under way, while the
+                // second one's last products run, and the next tile's first products run under the second one's epilogue.
+                const int skew = (nsets == 2 && khs >= 2 * SKEW) ? SKEW : 1;
+                for (int kh = 0; kh < khs;) {
+                    const int nb = (kh == 0 || kh == khs - skew) ? skew : 1;
+                    if (kh <= go_kh && go_kh < kh + nb && lane == 0) mbar_arrive(smem_u32(&go_bar[tl % ahead]));
+                    const int s_first = s;
+                    for (int i = 0; i < nb; ++i) {
+                        ok = __all_sync(0xffffffffu, wait_acquire(smem_u32(&full_bar[s]), ph, abort_flag));
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (elect_one()) {
+                            const uint64_t w0 = make_desc(stage0 + s * STAGE_BYTES), b0 = w0 + (SUB_BYTES >> 4);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) umma2(acc0, w0 + j * 2, b0 + j * 2, id0, (kh + i > 0 || j > 0) ? 1u : 0u);
+                            if (nsets == 1) umma2_commit(smem_u32(&empty_bar[s]));
+                            if (kh + i == khs - 1) umma2_commit(smem_u32(&acc_full_bar[set0]));
+                        }
+                        __syncwarp();
+                        if (++s == STAGES) {
+                            s = 0;
+                            ph ^= 1;
+                        }
+                    }
+                    if (!ok) break;
+                    if (nsets == 2) {
+                        if (kh == 0) {
+                            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_empty_bar[set1]), (((v + 1) >> 1) & 1) ^ 1, abort_flag));
+                            if (!ok) break;
+                            tc_fence_after();
+                        }
+                        if (elect_one()) {
+                            for (int i = 0; i < nb; ++i) {
+                                const int si = (s_first + i) % STAGES;
+                                const uint64_t w0 = make_desc(stage0 + si * STAGE_BYTES), b0 = w0 + (2 * SUB_BYTES >> 4);
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) umma2(acc1, w0 + j * 2, b0 + j * 2, id1, (kh + i > 0 || j > 0) ? 1u : 0u);
+                                umma2_commit(smem_u32(&empty_bar[si]));
+                            }
+                            if (kh + nb == khs) umma2_commit(smem_u32(&acc_full_bar[set1]));
+                        }
+                        __syncwarp();
+                    }
+                    kh += nb;
+                }
+                if (!ok) break;
+                v += nsets;
+            }
+            if (*abort_flag.flag) {
+                // what has been issued reads both CTAs' shared memory: it ends before either goes away
+                if (elect_one()) umma2_commit(smem_u32(&drain_bar));
+                __syncwarp();
+                let_land(smem_u32(&drain_bar), 1, 1);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------ scheduler ------------------------------
+        if (rank == 0 && lane == 0) {
+            const uint32_t tile_other = map_to(smem_u32(&sched_tile_s[0]), 1), full_other = map_to(smem_u32(&sched_full_bar[0]), 1);
+            for (int n = 0;; ++n) {
+                const int slot = n % SCHED_RING, m = n - ahead;
+                // tile n is claimed once the MMAs are far enough into tile n - ahead
+                if (m >= 0 && !mbar_wait(smem_u32(&go_bar[m % ahead]), (m / ahead) & 1, abort_flag)) break;
+                if (!wait_acquire(smem_u32(&sched_empty_bar[slot]), ((n / SCHED_RING) & 1) ^ 1, abort_flag)) break;
+                // the first `ahead` tiles are the pair's by its index
+                const int t = (n < ahead) ? cl + n * ncl : ahead * ncl + atomicAdd(a.n_tiles + 2 + MODE, 1);
+                const int4 d = (t < ntiles) ? a.tiles[t] : make_int4(0, 0, -1, 0);  // columns < 0: no more tiles
+                sched_tile_s[slot] = d;
+                asm volatile("st.shared::cluster.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(tile_other + slot * 16), "r"(d.x), "r"(d.y), "r"(d.z), "r"(d.w)
+                             : "memory");
+                arrive_release_at(full_other + slot * 8);
+                mbar_arrive(smem_u32(&sched_full_bar[slot]));
+                if (t >= ntiles) break;
+            }
+        }
+        __syncwarp();
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    pair_sync();  // neither CTA leaves while the other may still arrive at its barriers or multiply from its shared memory
+    if (warp == R::mma) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS) : "memory");
+    }
+    if (tid == 0 && abort_s) raise_status(a.status, a.status_host, 4);  // LUMEN_MOE_TIMEOUT
+}
+
+template <int Q, int MODE, bool ATMA>
+cudaError_t launch_one(const Args& a, int ctas, cudaStream_t st) {
+    using R = Roles<MODE, ATMA>;
+    auto* kern = grouped_gemm_pair_kernel<Q, MODE, ATMA>;
+    static SmemOptIn optin;
+    const cudaError_t e = ensure_dyn_smem(kern, R::smem, optin);
+    if (e != cudaSuccess) return e;
+    count_launch();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas & ~1);
+    cfg.blockDim = dim3(R::threads);
+    cfg.dynamicSmemBytes = R::smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
+}  // namespace pair
+
+// The experts' gate/up matrices [E][gate rows, up rows][H] f16 as a 5-D array (input, row of eight, gate | up, group of eight
+// rows, expert): a box is 64 inputs of 64 gate and 64 up rows in the order of the pair's operand.
+static cudaError_t make_tmap_gate_up(const __half* gu16, int E, int I, int H, CUtensorMap* out) {
+    const uint64_t dims[5] = {(uint64_t)H, 8, 2, (uint64_t)I / 8, (uint64_t)E};
+    const uint64_t strides[4] = {(uint64_t)H * 2, (uint64_t)I * H * 2, (uint64_t)H * 16, (uint64_t)I * H * 4};
+    const uint32_t box[5] = {64, 8, 2, 8, 1};
+    return make_tmap_f16_nd(gu16, 5, dims, strides, box, out);
+}
+
+// gate/up + SwiGLU, then down. x16: activation rows [columns, H] in the operands' element order
+cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int ctas, cudaStream_t st, __half* out16_rows) {
+    const int C = p.T * p.K, mt_gu = p.L.I / 128;
+    const int max_ct = C / PAIR_TILE_COLS + p.L.E;
+    pair::Args gu{};
+    gu.L = p.L;
+    gu.tiles = p.tiles;
+    gu.n_tiles = p.n_tiles;
+    gu.out16 = p.s16;
+    gu.status = p.status;
+    gu.status_host = p.status_host;
+    gu.wait_limit_ns = p.wait_limit_us ? (uint64_t)p.wait_limit_us * 1000ull : tc::WAIT_LIMIT_NS;
+    gu.debug_extra_tx = p.debug_extra_tx;
+    gu.kdim = p.L.H;
+    gu.out_ld = p.L.I;
+    pair::Args dn = gu;
+    dn.debug_extra_tx = 0;  // the hook applies to the first kernel of the pair
+    dn.tiles = p.tiles + (size_t)max_ct * mt_gu;  // as laid out by launch_route_large
+    dn.out16 = out16_rows ? out16_rows : p.d16;
+    dn.out_row_map = out16_rows ? p.R.col_src_tok : nullptr;
+    dn.kdim = p.L.I;
+    dn.out_ld = p.L.H;
+    cudaError_t e = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, 32, &gu.tmap_n);
+    if (e == cudaSuccess) e = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, 128, &gu.tmap_w);
+    if (e == cudaSuccess) e = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, 32, &dn.tmap_n);
+    if (e == cudaSuccess) e = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, 128, &dn.tmap_w);
+    if (e != cudaSuccess) return e;
+    if (p.L.gu16 != nullptr) {
+        e = make_tmap_gate_up(p.L.gu16, p.L.E, p.L.I, p.L.H, &gu.tmap_a);
+        if (e == cudaSuccess) e = make_tmap_f16(p.L.dn16, (uint64_t)p.L.E * p.L.H, (uint64_t)p.L.I, 128, &dn.tmap_a);
+        if (e == cudaSuccess) e = pair::launch_one<BF16, 0, true>(gu, ctas, st);
+        if (e == cudaSuccess) e = pair::launch_one<BF16, 1, true>(dn, ctas, st);
+        return e;
+    }
+    switch (p.L.quant) {
+        case Q4_0:
+            e = pair::launch_one<Q4_0, 0, false>(gu, ctas, st);
+            return e == cudaSuccess ? pair::launch_one<Q4_0, 1, false>(dn, ctas, st) : e;
+        case Q8_0:
+            e = pair::launch_one<Q8_0, 0, false>(gu, ctas, st);
+            return e == cudaSuccess ? pair::launch_one<Q8_0, 1, false>(dn, ctas, st) : e;
+        default:
+            return cudaErrorInvalidValue;  // BF16 layers always carry their f16 matrices on this path
+    }
+}
+
+}  // namespace lumen

@@ -833,7 +833,7 @@ cudaError_t launch_gather_rows(const __half* plane, const int32_t* col_src_tok, 
                       H / 8, reinterpret_cast<uint4*>(out));
 }
 
-cudaError_t make_tmap_f16(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out) {
+cudaError_t make_tmap_f16_nd(const void* base, int nd, const uint64_t* dims, const uint64_t* strides, const uint32_t* box, CUtensorMap* out) {
     typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -846,14 +846,24 @@ cudaError_t make_tmap_f16(const void* base, uint64_t rows, uint64_t cols, uint32
         if (qres != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
         encode = reinterpret_cast<EncodeFn>(fn);
     }
-    const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols * 2};
-    const cuuint32_t box[2] = {64, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+    cuuint64_t d[5], st[4];
+    cuuint32_t bx[5];
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    for (int i = 0; i < nd; ++i) {
+        d[i] = dims[i];
+        bx[i] = box[i];
+        if (i + 1 < nd) st[i] = strides[i];
+    }
+    const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)nd, const_cast<void*>(base), d, st, bx, estr,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+cudaError_t make_tmap_f16(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out) {
+    const uint64_t dims[2] = {cols, rows}, strides[1] = {cols * 2};
+    const uint32_t box[2] = {64, box_rows};
+    return make_tmap_f16_nd(base, 2, dims, strides, box, out);
 }
 
 template <int Q, int MODE, int BN, bool ATMA = false, bool STG = false>
@@ -875,7 +885,8 @@ static cudaError_t launch_tc_one(const tc::Args& a, int grid, cudaStream_t st) {
 cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, cudaStream_t st, __half* out16_rows,
                               const TcPlan* plan, const TcPeerOut* peer) {
     const int C = plan ? plan->rows : p.T * p.K;
-    const int gu_cols = plan ? plan->gu_cols : tc_gu_tile_cols(C, p.L.E, p.L.H, p.L.I, p.sms);  // as the tile lists were built
+    if (!plan && tc_gu_tile_cols(C, p.L.E, p.L.H, p.L.I, p.sms, p.tc_ctas) == PAIR_TILE_COLS) return launch_grouped_pair(p, x16, grid, st, out16_rows);
+    const int gu_cols = plan ? plan->gu_cols : tc_gu_tile_cols(C, p.L.E, p.L.H, p.L.I, p.sms, p.tc_ctas);  // as the tile lists were built
     const int max_ct = C / gu_cols + p.L.E;
     // Down tiles: up to 256 tokens (two accumulator sets at once, no epilogue overlap between such
     // tiles) when the gate/up tiles are 256 wide, except with a tile plan of an expert-parallel call,

@@ -69,6 +69,25 @@ def test_grouped_gemm_stage_barrier_that_runs_out_is_reported_and_recoverable(cu
     assert torch.equal(again, good)
 
 
+# the same on CTA pairs (both CTAs give up), dequantised and TMA-fed weights
+@pytest.mark.parametrize("quant", [0, 1, 2])
+def test_pair_stage_barrier_that_runs_out_is_reported_and_recoverable(cuda_lib, quant):
+    H, I, E, K, T = 2048, 256, 8, 2, 1500
+    lay = synth.LayerLayout(H, I, E, quant)
+    sc = moe.allocate_moe_scratch(H, I, E, K, T, flags=_lib.FLAG_SHORT_WAITS)
+    layer = sc.prepare_layer(synth.make_layer_blob(lay, 0), lay.meta())
+    x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(4), device="cuda")
+    good = sc.prefill(layer, x, x).clone()
+    torch.cuda.synchronize()
+    assert sc.poll_status() == _lib.OK
+    sc.debug_expire_next_wait(1)
+    sc.prefill(layer, x, x)
+    torch.cuda.synchronize()
+    assert sc.poll_status() == _lib.TIMEOUT
+    sc.clear_status()
+    assert torch.equal(sc.prefill(layer, x, x), good)
+
+
 # the streaming kernels: decode chains on int8 (Q4_0) and hi + lo operands, short prompts
 @pytest.mark.parametrize("call,quant,T", [("decode", 1, 16), ("decode", 0, 5), ("decode", 2, 9), ("prefill", 1, 40), ("prefill", 0, 30)])
 def test_streaming_copy_that_never_comes_is_reported_and_recoverable(cuda_lib, call, quant, T):

@@ -61,6 +61,15 @@ def test_tcgen05_tiles_of_short_contractions(cuda_lib, quant, H, I, E, T):
     check_prefill(H, I, E, 2, quant, synth.uniform_logits(T, E, 7))
 
 
+# products on CTA pairs: sets of 32..256 columns and what is left of them, one and two sets a tile, contractions of one,
+# two, three and many 128-input groups (tiles claimed four, two and one ahead)
+@pytest.mark.parametrize("quant", [0, 1, 2])
+@pytest.mark.parametrize("H,I", [(256, 1024), (2048, 128), (1536, 384), (3072, 256)])
+def test_pair_products_tile_edges(cuda_lib, quant, H, I):
+    counts = [0, 1, 16, 31, 33, 64, 255, 256, 257, 288, 511, 512, 513, 1025, 7, 95]
+    check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1), torch.bfloat16)
+
+
 # batches of the decode chain for each format, at contractions with a remainder against the ring's chunk
 @pytest.mark.parametrize("quant,T", [(0, 3), (0, 16), (1, 5), (1, 16), (2, 5), (2, 9), (2, 16)])
 def test_decode_chain_wide_layer(cuda_lib, quant, T):
