@@ -150,7 +150,7 @@ static size_t tok_arena_bytes(const CudaMoeScratch& s, int cap, size_t* offs) {
     // order: logits, ids, weights, col_expert, col_src_tok, dst_to_col, blk_hist, tiles, s16, d16, x16, xf, sf, w16, xq, xr16, rpart, sq, d32
     const size_t C = (size_t)cap * s.K;
     const size_t nblk_h_pad = (size_t)((s.H / 32 + 3) / 4) * 4, nblk_i_pad = (size_t)((s.I / 32 + 3) / 4) * 4;
-    const size_t max_ct = C / 128 + s.E, max_ct_dn = C / 128 + s.E;  // gate/up tiles of 128 or 256 columns (sized for 128), down tiles of 128
+    const size_t max_ct = C / 128 + s.E, max_ct_dn = C / 128 + s.E;  // tiles of 128 or 512 columns (sized for 128)
     const size_t n_tile_entries = max_ct * ((size_t)s.I / 128 + 1) + max_ct_dn * ((size_t)s.H / 256 + 1);
     size_t sizes[19] = {
         (size_t)cap * s.E * 4, C * 4, C * 4, C * 4, C * 4, C * 4,
@@ -618,11 +618,13 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
         CUDA_TRY(launch_stream_prefill(p, s->xr16, out16_rows, st));
         if (out16_rows) return Status::Ok();
     } else if (p.impl == 0) {
-        if (!single) CUDA_TRY(launch_gather_rows(s->xr16, s->R.col_src_tok, batch * s->K, s->H, s->x16, st));
+        const bool pairs = tc_tile_cols(layer.dev, batch * s->K, s->sms, s->tc_ctas) == PAIR_TILE_COLS;  // gathers by itself
+        if (!single && !pairs) CUDA_TRY(launch_gather_rows(s->xr16, s->R.col_src_tok, batch * s->K, s->H, s->x16, st));
         // persistent grid, one CTA per SM; LUMEN_MOE_FLAG_TC_CTAS leaves some SMs to kernels that run beside it
         int sms = s->sms;
         if (s->tc_ctas > 0 && s->tc_ctas < sms) sms = s->tc_ctas;
-        CUDA_TRY(launch_grouped_tc(p, single ? s->xr16 : s->x16, sms, st, out16_rows));
+        if (pairs) CUDA_TRY(launch_grouped_pair(p, single ? s->xr16 : nullptr, sms, st, out16_rows));
+        else CUDA_TRY(launch_grouped_tc(p, single ? s->xr16 : s->x16, sms, st, out16_rows));
     } else {
         CUDA_TRY(launch_build_xf(normed, act_dtype, batch, s->H, layer.dev.kg_h * 4, bf16_mode, s->xf, st));
         DecodeArgs a = make_decode_args(s, layer, batch);

@@ -12,19 +12,6 @@ namespace lumen {
 enum Quant : int { Q8_0 = 0, Q4_0 = 1, BF16 = 2 };
 
 constexpr int MAX_EXPERTS = 256;  // cuda/shaders/moe_router.cu:33
-// Columns per tile of the tcgen05 gate/up product; the down tiles of a one-GPU call follow it. 512: the CTA-pair kernels
-// (prefill_pair.cu), once the experts average more than 176 columns (4096 tokens, H = 2048, I = 768, E = 128, K = 8:
-// 468 -> 425 us for Q8_0; at 187 columns an expert 338 -> 334, at 150 (H = 4096, I = 1536) 509 -> 524). 256 above 128 (each dequantised weight tile
-// then serves twice the columns), else 128 (fewer empty columns in ragged tiles, epilogue overlapped); 128 too where its
-// tiles are one wave of both products, whose time is then that of one tile (a shared expert alone, 2048 x 512: 300
-// tokens 47 -> 41 us, 1024 49 -> 46; at 4096, two waves down, 67 us with 256 and 73 with 128).
-// ctas: cap of the persistent grid (0 = every SM).
-constexpr int PAIR_TILE_COLS = 512;
-inline int tc_gu_tile_cols(int columns, int experts, int hidden, int inter, int sms, int ctas) {
-    const int mt = inter / 128 > hidden / 256 ? inter / 128 : hidden / 256;
-    if (columns <= 128 * experts || columns / 128 * mt <= sms) return 128;
-    return (columns > 176 * experts && ctas != 1) ? PAIR_TILE_COLS : 256;
-}
 constexpr int MAX_TOP_K = 16;     // cuda/shaders/moe_router.cu:34
 constexpr int DECODE_MAX_TOKENS = 16;
 
@@ -72,6 +59,22 @@ struct LayerDev {
     __host__ __device__ const uint4* up_s(int e) const { return s + (size_t)e * s_exp + s_gu; }
     __host__ __device__ const uint4* down_s(int e) const { return s + (size_t)e * s_exp + 2 * s_gu; }
 };
+
+// Columns per tile of the tcgen05 products of a one-GPU call: 512 = the CTA-pair kernels (prefill_pair.cu), 128 = one CTA a
+// tile (prefill_tc.cu). Pairs from that average of columns an expert on at which they overtake: a pair has half as many weight
+// tiles in flight, which counts while a call is bound by its weights (E = 128, I = 768, us from the host: Q4_0 62 columns
+// 219 and 213 with pairs, 94 columns 247 and 237, 187 columns 376 and 321; Q8_0 111 columns 298 and 286, 78 columns of
+// E = 256 362 and 362; f16 matrices 111 columns 302 and 313, 144 columns 361 and 343). A lone expert (a shared one)
+// fills a few SMs with pairs where tiles of 128 fill four times as many: pairs once those are more than one wave
+// (2048 x 512: 1024 tokens 62 and 64 us, 4096 98 and 91; 900 tokens of 2048 x 1536 64 and 72), and the same for f16
+// matrices (2336 columns of 16 experts, 512 x 384: 62.5 and 63.2).
+// ctas: cap of the persistent grid (0 = every SM).
+constexpr int PAIR_TILE_COLS = 512;
+inline int tc_tile_cols(const LayerDev& L, int columns, int sms, int ctas) {
+    const int least = L.gu16 != nullptr ? 128 : L.quant == Q4_0 ? 88 : 104;
+    const int mt = L.I / 128 > L.H / 256 ? L.I / 128 : L.H / 256;
+    return (columns > least * L.E && ((L.E > 1 && L.gu16 == nullptr) || columns / 128 * mt > sms) && ctas != 1) ? PAIR_TILE_COLS : 128;
+}
 
 // Routing tables of one call (device pointers into the context's scratch).
 struct RouteDev {

@@ -18,9 +18,17 @@
 // small buffer of the warp, and leave as whole 32- or 64-byte pieces of a column's row.
 //
 // One CTA pair per two SMs, persistent; tiles are claimed from a device-wide counter by the first CTA of the pair.
-// Warps of a CTA: 0-7 epilogue (16 of them for gate/up when the weights come by TMA), then 16 weight producers (none with
-// TMA-fed weights), one thread for the copies, one warp for the MMAs (idle in the second CTA), one thread for the tiles
-// (idle in the second CTA). Every wait is bounded; on expiry the kernel raises the status word, lets its copies and
+// Warps of a CTA: 0-7 epilogue (16 of them for gate/up when the weights come by TMA), then 16 weight producers (with
+// TMA-fed weights a copy warp instead), two copy warps for the columns, one for each set, one warp for the MMAs (idle in the
+// second CTA), one thread for the tiles (idle in the second CTA).
+//
+// Operands come through two rings: weights in stages of 128 rows x 128 inputs, columns in units of up to 128 rows x 128
+// inputs, of which a stage takes one per set. A pass multiplies one unit with its stage. What a pass costs the MMA warp
+// besides its products bounds narrow tiles, hence 128 inputs, ONE barrier to wait for (the unit's bytes and, in a stage's
+// first pass, its weights) and ONE commit (unit free, and the stage with its last pass): with two barriers and two commits
+// for every 64 inputs a tile of 60 columns took ~1200 cycles a pass (1000 tokens, 279 us a call).
+// The columns of gate/up are gathered by the copies themselves (tile::gather4 on the token rows): the plane of the tokens
+// stays in L2, where the gathered rows (268 MB at 8192 tokens of 2048, K = 8, 54 us to write) did not. Every wait is bounded; on expiry the kernel raises the status word, lets its copies and
 // MMAs end, frees its TMEM and returns.
 #include "mma_frag.cuh"
 #include "tc_common.cuh"
@@ -32,31 +40,36 @@ namespace pair {
 using namespace tc;
 
 constexpr int PROD_WARPS = 16;
-constexpr int STAGES = 4;                                // of 64 inputs (one swizzle atom in K)
-constexpr int STAGE_BYTES = SUB_BYTES + 2 * SUB_BYTES;   // 128 weight rows, then this CTA's half of two sets of 256 columns
+constexpr int STAGES = 2;                                // weights: 128 rows x 128 inputs, as two swizzle atoms of 64
+constexpr int UNITS = 4;                                 // columns: this CTA's half of a set of 256, x 128 inputs
+constexpr int STAGE_BYTES = 2 * SUB_BYTES;               // of a stage and of a unit
 constexpr int SCHED_RING = 8;                            // tile descriptors in flight between the scheduler and the roles
 constexpr int MAX_AHEAD = 4;                             // tiles that are claimed ahead of the MMAs at most
-constexpr int SKEW = 2;                                  // stages by which the sets of a wide tile are taken apart at its ends
 constexpr int TMEM_COLS = 512;
 
 template <int MODE, bool ATMA>
 struct Roles {
     static constexpr int epi = (ATMA && MODE == 0) ? 16 : 8, prod = ATMA ? 0 : PROD_WARPS;
-    static constexpr int prod0 = epi, tma = epi + prod, mma = tma + 1, sched = mma + 1, threads = (sched + 1) * 32;
+    static constexpr int copies = ATMA ? 3 : 2;  // a set's columns each, the weights
+    static constexpr int prod0 = epi, copy0 = epi + prod, mma = copy0 + copies, sched = mma + 1, threads = (sched + 1) * 32;
+    // arrivals for a stage's weights: every producer warp of both CTAs | the copies' expected bytes
+    static constexpr int weight_arrivals = ATMA ? 1 : 2 * prod;
     // a warp's output buffer: 32 columns of its 16 (gate/up) or 32 (down) rows, padded so that the eight rows of an
     // stmatrix hit eight different 16-byte bank groups
     static constexpr int row_bytes = (MODE == 0) ? 32 : 64, pitch = row_bytes + 16, out_bytes = 32 * pitch;
-    static constexpr size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + (size_t)epi * out_bytes;
+    static constexpr size_t smem = 1024 + (size_t)(STAGES + UNITS) * STAGE_BYTES + (size_t)epi * out_bytes;
 };
 
 struct Args {
-    CUtensorMap tmap_n;   // columns [rows, kdim] f16, box 64 x 32
+    CUtensorMap tmap_n;   // columns [rows, kdim] f16, box 64 x 32 (gathered: token rows, box 64 x 1)
     CUtensorMap tmap_w;   // the same, box 64 x 128
     CUtensorMap tmap_a;   // ATMA: the experts' f16 matrices (gate/up: in groups of eight gate and eight up rows)
     LayerDev L;
     const int4* tiles;    // {expert, first column, columns, m-tile}
     int32_t* n_tiles;     // [0..1] tiles of the gate/up and the down list, [2..3] the kernels' tile counters
     __half* out16;        // gate/up: S16 [C, I] in the order down reads it; down: D16 [C, H]
+    const int32_t* gather;       // gate/up: token row of a compact column (null = the columns are rows of their own)
+    int n_cols;                  // compact columns of the call
     const int32_t* out_row_map;  // down: output row of compact column c (null = c itself)
     int32_t* status;
     int32_t* status_host;
@@ -93,7 +106,7 @@ __device__ __forceinline__ bool try_acquire(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// mbar_wait for barriers that the other CTA arrives at with something written
+// mbar_wait for what the other CTA writes with ordinary stores (tile descriptors)
 __device__ __forceinline__ bool wait_acquire(uint32_t bar, uint32_t parity, const AbortCtl& ac) {
     if (try_acquire(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
@@ -108,6 +121,14 @@ __device__ __forceinline__ bool wait_acquire(uint32_t bar, uint32_t parity, cons
         }
     }
 }
+__device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t n) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+}
+__device__ __forceinline__ void pause_ns(uint64_t ns) {
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < ns) {
+    }
+}
 __device__ __forceinline__ void pair_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -119,6 +140,10 @@ __device__ __forceinline__ void umma2(uint32_t d_tmem, uint64_t adesc, uint64_t 
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
         : "memory");
+}
+// make_desc of an address given in 16-byte units
+__device__ __forceinline__ uint64_t desc_of(uint32_t lo) {
+    return (uint64_t)(lo | (1u << 16)) | ((uint64_t)((1u << 14) | (2u << 29) | 64u) << 32);
 }
 // one arrival at this barrier of both CTAs once the MMAs issued so far are done
 __device__ __forceinline__ void umma2_commit(uint32_t bar) {
@@ -141,6 +166,14 @@ __device__ __forceinline__ void tma_pair_5d(uint32_t dst, const CUtensorMap* m, 
         "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(cluster_bar)
         : "memory");
 }
+// four rows of 64 inputs each, one after the other
+__device__ __forceinline__ void tma_pair_gather4(uint32_t dst, const CUtensorMap* m, int x, const int4& r, uint32_t cluster_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w), "r"(cluster_bar)
+        : "memory");
+}
 // 16 TMEM lanes x 32 columns in the accumulator-fragment shape: v[4j..4j+1] row lane / 4, columns 8j + 2 (lane % 4) and the
 // next, v[4j+2..4j+3] row lane / 4 + 8
 __device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t (&r)[16]) {
@@ -149,6 +182,11 @@ __device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t (&r)[16]
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
+}
+// (see tmem_ld_fence8)
+__device__ __forceinline__ void tmem_ld_fence16(uint32_t (&r)[16]) {
+    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                      "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
 }
 // four 8 x 8 matrices of 16-bit elements, each stored transposed; lane l gives the address of row l % 8 of matrix l / 8
 __device__ __forceinline__ void stmatrix4_t(uint32_t addr, const uint32_t (&v)[4]) {
@@ -161,8 +199,8 @@ __device__ __forceinline__ uint32_t pack_f16(float a, float b) {
 }
 
 // --- dequantisation ---------------------------------------------------------------------------------------------------
-// A producer warp owns 16 rows x 64 inputs (blocks 2 sub, 2 sub + 1 of every 128-input group) of this CTA's operand: eight
-// warps fill a stage, the other eight the next one. What a lane holds of it:
+// A producer warp owns 16 rows x 64 inputs (blocks 2 sub, 2 sub + 1 of every 128-input group) of this CTA's operand. What a
+// lane holds of it:
 template <int Q>
 struct Half {
     uint4 q[Q == Q4_0 ? 1 : 2];
@@ -258,8 +296,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
     using R = Roles<MODE, ATMA>;
     extern __shared__ uint8_t smem_raw[];
     // "first": used in the pair's first CTA only, which both CTAs' roles arrive at
-    __shared__ uint64_t full_bar[STAGES];      // first: a stage is filled in both CTAs
-    __shared__ uint64_t empty_bar[STAGES];     // a stage has been multiplied
+    __shared__ uint64_t full_bar[UNITS];       // first: what a pass multiplies is there in both CTAs
+    __shared__ uint64_t done_bar[UNITS];       // a pass is over
     __shared__ uint64_t acc_full_bar[2];       // an accumulator set is complete
     __shared__ uint64_t acc_empty_bar[2];      // first: it has been read in both CTAs
     __shared__ uint64_t sched_full_bar[SCHED_RING];
@@ -267,6 +305,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
     __shared__ uint64_t go_bar[MAX_AHEAD];     // first: the next tile may be claimed
     __shared__ uint64_t drain_bar;             // give-up path: the MMAs issued are done
     __shared__ int4 sched_tile_s[SCHED_RING];
+    __shared__ int4 rows_s[2][32];             // a tile's token rows in fours, by set
     __shared__ uint32_t tmem_base_s;
     __shared__ uint32_t abort_s;
 
@@ -277,9 +316,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
 
     if (tid == 0) {
         abort_s = 0u;
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(smem_u32(&full_bar[s]), 1 + 2 * (R::prod / 2));  // the copies' expected bytes, eight producer warps of each CTA
-            mbar_init(smem_u32(&empty_bar[s]), 1);
+        for (int i = 0; i < UNITS; ++i) {
+            mbar_init(smem_u32(&full_bar[i]), R::weight_arrivals + 1);  // and the columns' copies
+            mbar_init(smem_u32(&done_bar[i]), 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&acc_full_bar[b]), 1);
@@ -287,7 +326,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
         }
         for (int s = 0; s < SCHED_RING; ++s) {
             mbar_init(smem_u32(&sched_full_bar[s]), 1);
-            mbar_init(smem_u32(&sched_empty_bar[s]), 2 * (R::epi + R::prod + 1) + 1);  // readers: epilogue, producers, copies of both; MMAs
+            mbar_init(smem_u32(&sched_empty_bar[s]), 2 * (R::epi + R::prod + R::copies) + 1);  // readers: epilogue, producers, copies of both; MMAs
         }
         for (int i = 0; i < MAX_AHEAD; ++i) mbar_init(smem_u32(&go_bar[i]), 1);
         mbar_init(smem_u32(&drain_bar), 1);
@@ -306,8 +345,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
 
     grid_dep_sync();
     const int ntiles = a.n_tiles[MODE];
-    const int kgs = a.kdim >> 7;  // 128-input groups
-    const int khs = kgs * 2;      // 64-input stages per tile
+    const int kgs = a.kdim >> 7;  // 128-input groups: stages of a tile
+    auto pass_done = [&](uint32_t n) -> bool { return mbar_wait(smem_u32(&done_bar[n % UNITS]), (n / UNITS) & 1, abort_flag); };
     const int cl = blockIdx.x >> 1, ncl = gridDim.x >> 1;
     const uint32_t sched_empty_first = map_to(smem_u32(&sched_empty_bar[0]), 0);
 
@@ -321,20 +360,20 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
         if (whole_warp) __syncwarp();
         if (!whole_warp || lane == 0) arrive_at(sched_empty_first + slot * 8);
         ++n;
-        return tile.z >= 0;
+        return whole_warp ? __all_sync(0xffffffffu, tile.z >= 0) : tile.z >= 0;
     };
     // How many tiles are claimed ahead of the MMAs, and at which stage of a tile they allow the next claim. Long tiles:
     // one ahead, late in a wide tile so that the last tiles go to the pairs that are free first (before the producers need
-    // it: they hold up to `depth` groups and four stages beyond the MMAs), at the start of a narrow one, which
+    // it: they hold up to `depth` groups and two stages beyond the MMAs), at the start of a narrow one, which
     // is over in about the time of a claim. Short ones: two ahead, so that the producers never run dry; four
     // where a tile is one group, because the producers' registers hold more than two of them.
-    const int ahead = (khs >= 24) ? 1 : (kgs >= 2) ? 2 : MAX_AHEAD;
+    const int ahead = (kgs >= 12) ? 1 : (kgs >= 2) ? 2 : MAX_AHEAD;
 
     if (warp < R::epi) {
         // ------------------------------ epilogue ------------------------------
         constexpr int PARTS = R::epi / 4;
         const int quad = warp & 3, part = warp >> 2;  // (TMEM lanes 32 quad.. are this warp's by the hardware's rule)
-        const uint32_t buf = stage0 + STAGES * STAGE_BYTES + (uint32_t)warp * R::out_bytes;
+        const uint32_t buf = stage0 + (STAGES + UNITS) * STAGE_BYTES + (uint32_t)warp * R::out_bytes;
         const uint32_t acc_empty_first = map_to(smem_u32(&acc_empty_bar[0]), 0);
         const uint32_t st_addr = buf + lane * R::pitch;  // row `lane` of the buffer: column `lane` of the chunk
         int v = 0, tn = 0;
@@ -351,31 +390,37 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                 tc_fence_after();
                 const int ncols = min(256, tile.z - 256 * h), col0 = tile.y + 256 * h;
                 const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + set * 256;
-                for (int c = part * 32; c < ncols; c += PARTS * 32) {
-                    uint32_t v0[16], v1[16];
-                    tmem_ld_frag32(taddr + c, v0);
-                    tmem_ld_frag32(taddr + (16u << 16) + c, v1);
-                    tmem_ld_wait();
-                    __syncwarp();  // the chunk before has left the buffer
-                    auto rows16 = [&](const uint32_t (&x)[16], int half) {
-                        if (MODE == 0) {
+                // 32 columns of 16 rows into the buffer
+                auto rows16 = [&](const uint32_t (&x)[16], int half) {
+                    if (MODE == 0) {
+                        uint32_t o[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            o[j] = pack_f16(swiglu(__uint_as_float(x[4 * j]), __uint_as_float(x[4 * j + 2])),
+                                            swiglu(__uint_as_float(x[4 * j + 1]), __uint_as_float(x[4 * j + 3])));
+                        stmatrix4_t(st_addr + half * 16, o);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
                             uint32_t o[4];
 #pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                                o[j] = pack_f16(swiglu(__uint_as_float(x[4 * j]), __uint_as_float(x[4 * j + 2])),
-                                                swiglu(__uint_as_float(x[4 * j + 1]), __uint_as_float(x[4 * j + 3])));
-                            stmatrix4_t(st_addr + half * 16, o);
-                        } else {
-#pragma unroll
-                            for (int q = 0; q < 2; ++q) {
-                                uint32_t o[4];
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) o[j] = pack_f16(__uint_as_float(x[4 * j + 2 * q]), __uint_as_float(x[4 * j + 2 * q + 1]));
-                                stmatrix4_t(st_addr + half * 32 + q * 16, o);
-                            }
+                            for (int j = 0; j < 4; ++j) o[j] = pack_f16(__uint_as_float(x[4 * j + 2 * q]), __uint_as_float(x[4 * j + 2 * q + 1]));
+                            stmatrix4_t(st_addr + half * 32 + q * 16, o);
                         }
-                    };
+                    }
+                };
+                // the TMEM loads of the next 16 rows are issued before the current ones are worked on
+                uint32_t v0[16], v1[16];
+                if (part * 32 < ncols) tmem_ld_frag32(taddr + part * 32, v0);
+                for (int c = part * 32; c < ncols; c += PARTS * 32) {
+                    tmem_ld_wait();
+                    tmem_ld_fence16(v0);
+                    tmem_ld_frag32(taddr + (16u << 16) + c, v1);
+                    __syncwarp();  // the chunk before has left the buffer
                     rows16(v0, 0);
+                    tmem_ld_wait();
+                    tmem_ld_fence16(v1);
+                    if (c + PARTS * 32 < ncols) tmem_ld_frag32(taddr + c + PARTS * 32, v0);
                     rows16(v1, 1);
                     __syncwarp();
                     constexpr int PIECES = R::row_bytes / 16;  // 16-byte pieces of a column
@@ -395,7 +440,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                 if (lane == 0) arrive_at(acc_empty_first + set * 8);
             }
         }
-    } else if (warp < R::tma) {
+    } else if (warp < R::copy0) {
         // --------------------------- weight producers --------------------------
         if constexpr (!ATMA) {
             const int pw = warp - R::prod0, rtl = pw & 7, sub = pw >> 3;
@@ -409,11 +454,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
             const uint32_t* sp = nullptr;
             // the next group of the list into registers; false when there is none. The descriptor of a tile that is still
             // to be claimed is waited for: it comes without any help from the groups that are held here (see `ahead`)
-            auto load_next = [&](Half<Q>& w) -> bool {
+            int sets = 1;  // accumulator sets of the tile being loaded
+            // (returns the sets of the group's tile, 0 when there is none)
+            auto load_next = [&](Half<Q>& w) -> int {
                 if (pkg == kgs) {
                     int4 tile;
                     if (more) more = take_tile(true, tn, tile);
-                    if (!more) return false;
+                    if (!more) return 0;
+                    sets = (tile.z > 256) ? 2 : 1;
                     const int e = tile.x;
                     const uint4 *qb, *sb;
                     int rt;
@@ -439,151 +487,197 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                 qp += QTraits<Q>::NQ * 32;
                 sp += 32;
                 ++pkg;
-                return true;
+                return sets;
             };
             Half<Q> w[PF];
-            bool there[PF];
+            int there[PF];
 #pragma unroll
             for (int j = 0; j < PF; ++j) there[j] = load_next(w[j]);
-            int s = sub, ph = 0;  // this warp's stages are every second one
+            uint32_t n = 0, u = 0, last_1 = 0, last_2 = 0;  // stages, passes so far; the last passes of the stages before
             bool ok = true;
             while (ok) {
 #pragma unroll
                 for (int j = 0; j < PF; ++j) {
-                    ok = ok && there[j];
+                    ok = ok && there[j] != 0;
                     if (!ok) break;
-                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag));
+                    if (n >= STAGES) ok = __all_sync(0xffffffffu, pass_done(last_2));
                     if (!ok) break;
-                    dequant<Q, MODE>(w[j], stage0 + s * STAGE_BYTES, pl, k);
+                    dequant<Q, MODE>(w[j], stage0 + (n % STAGES) * STAGE_BYTES + sub * SUB_BYTES, pl, k);
                     fence_proxy_async();  // every lane's own stores, before the warp's one arrival
                     __syncwarp();
-                    if (lane == 0) arrive_at(full_first + s * 8);
-                    s += 2;
-                    if (s >= STAGES) {
-                        s -= STAGES;
-                        ph ^= 1;
-                    }
+                    if (lane == 0) arrive_at(full_first + (u % UNITS) * 8);
+                    ++n;
+                    u += there[j];
+                    last_2 = last_1;
+                    last_1 = u - 1;
                     there[j] = load_next(w[j]);
                 }
             }
         }
-    } else if (warp == R::tma) {
-        // ------------------------------- copies --------------------------------
-        if (lane == 0) {
-            const uint32_t full_first = map_to(smem_u32(&full_bar[0]), 0);
-            int tn = 0, n = 0;
-            bool ok = true;
-            int4 tile;
-            while (ok && take_tile(false, tn, tile)) {
-                const int nsets = (tile.z > 256) ? 2 : 1;
-                int row[2], nbox[2];  // boxes: 0 = one of 128 rows, else of 32
-                uint32_t bytes = 0;
-                for (int h = 0; h < nsets; ++h) {
-                    const int half = set_cols(tile.z, h) / 2;
-                    row[h] = tile.y + 256 * h + (int)rank * half;
-                    nbox[h] = (half == 128) ? 0 : (half + 31) / 32;
-                    bytes += (nbox[h] ? nbox[h] * 32 : 128) * 128;
-                }
-                if (ATMA) bytes += SUB_BYTES;
-                for (int kh = 0; kh < khs; ++kh, ++n) {
-                    const int s = n % STAGES, ph = (n / STAGES) & 1;
-                    ok = mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag);
-                    if (!ok) break;
-                    // both CTAs' bytes (their copies have the same shape) are expected once, by the first CTA
-                    if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * bytes + (n == 0 ? a.debug_extra_tx : 0));
-                    const uint32_t base = stage0 + s * STAGE_BYTES, bar = full_first + s * 8;
-                    if (ATMA) {
-                        if (MODE == 0)
-                            tma_pair_5d(base, &a.tmap_a, kh * 64, 0, 0, tile.w * 16 + (int)rank * 8, tile.x, bar);
-                        else
-                            tma_pair_2d(base, &a.tmap_a, kh * 64, tile.x * a.L.H + tile.w * 256 + (int)rank * 128, bar);
+    } else if (warp < R::copy0 + 2) {
+        // ------------------------- copies of the columns -----------------------
+        // Each warp takes every second unit: one set of a wide tile's stages, every second stage of a narrow tile.
+        const uint32_t w = warp - R::copy0;
+        const uint32_t full_first = map_to(smem_u32(&full_bar[0]), 0);
+        const uint32_t units0 = stage0 + STAGES * STAGE_BYTES;
+        const bool gather = (MODE == 0) && a.gather != nullptr;
+        int tn = 0;
+        uint32_t u0 = 0;  // the tile's first unit
+        bool ok = true;
+        // this CTA's rows of the warp's set of a tile that begins at unit u: `half` of them from the returned column on
+        auto rows_of = [&](const int4& t, uint32_t u, int& half) -> int {
+            const int h = (t.z > 256) ? (int)((w ^ u) & 1) : 0;
+            half = set_cols(t.z, h) / 2;
+            return t.y + 256 * h + (int)rank * half;
+        };
+        auto token_rows = [&](const int4& t, uint32_t u) -> int4 {
+            int half;
+            const int c = rows_of(t, u, half) + 4 * lane, last = a.n_cols - 1;
+            if (4 * lane >= half) return make_int4(0, 0, 0, 0);
+            return make_int4(__ldg(a.gather + min(c, last)), __ldg(a.gather + min(c + 1, last)), __ldg(a.gather + min(c + 2, last)),
+                             __ldg(a.gather + min(c + 3, last)));
+        };
+        int4 tile, tile_n = make_int4(0, 0, -1, 0), rows_n = make_int4(0, 0, 0, 0);
+        bool have = take_tile(true, tn, tile);
+        if (have && gather) rows_n = token_rows(tile, 0);
+        const int pre = max(kgs - 4, 0);  // where the next tile's descriptor and token rows are fetched
+        while (ok && have) {
+            const bool wide = tile.z > 256;
+            int half;
+            const int first = rows_of(tile, u0, half);
+            const uint32_t bytes = 2 * (gather ? half * 128 : (half == 128) ? 128 * 128 : ((half + 31) / 32) * 4096);
+            const uint32_t u_next = u0 + (wide ? 2 * kgs : kgs), odd = (w ^ u0) & 1;
+            if (gather) {
+                __syncwarp();
+                rows_s[w][lane] = rows_n;
+                __syncwarp();
+            }
+            bool fetched = false;
+            auto fetch_next = [&]() {
+                have = take_tile(true, tn, tile_n);
+                if (have && gather) rows_n = token_rows(tile_n, u_next);
+                fetched = true;
+            };
+            for (int k = wide ? 0 : (int)odd; k < kgs; k += wide ? 1 : 2) {
+                if (k >= pre && !fetched) fetch_next();
+                const uint32_t unit = u0 + (wide ? 2 * k + odd : k), s = unit % UNITS;
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&done_bar[s]), ((unit / UNITS) & 1) ^ 1, abort_flag));
+                if (!ok) break;
+                if (elect_one()) {
+                    if (rank == 0) {
+                        // both CTAs' bytes (their copies have the same shape) are expected once, by the first CTA; the second
+                        // pass of a stage has no weights of its own to wait for
+                        mbar_expect_tx(smem_u32(&full_bar[s]), 2 * bytes + (unit == 0 ? a.debug_extra_tx : 0));
+                        if (wide && odd) mbar_arrive_n(smem_u32(&full_bar[s]), R::weight_arrivals);
                     }
-                    for (int h = 0; h < nsets; ++h) {
-                        const uint32_t dst = base + (1 + h) * SUB_BYTES;
-                        if (nbox[h] == 0) {
-                            tma_pair_2d(dst, &a.tmap_w, kh * 64, row[h], bar);
-                        } else {
-                            for (int q = 0; q < nbox[h]; ++q) tma_pair_2d(dst + q * 4096, &a.tmap_n, kh * 64, row[h] + q * 32, bar);
+                    const uint32_t dst = units0 + s * STAGE_BYTES, bar = full_first + s * 8;
+                    const int x = k * 128;
+                    if (gather) {
+                        // (sixteen rows' numbers first: a load between two copies would cost its latency each time)
+                        for (int q = 0; q < half / 4; q += 4) {
+                            int4 r[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) r[i] = rows_s[w][q + i];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                tma_pair_gather4(dst + (i & 1) * SUB_BYTES + (q + (i >> 1)) * 512, &a.tmap_n, x + (i & 1) * 64, r[i >> 1], bar);
+                        }
+                    } else if (half == 128) {
+                        tma_pair_2d(dst, &a.tmap_w, x, first, bar);
+                        tma_pair_2d(dst + SUB_BYTES, &a.tmap_w, x + 64, first, bar);
+                    } else {
+                        for (int q = 0; q * 32 < half; ++q) {
+                            tma_pair_2d(dst + q * 4096, &a.tmap_n, x, first + q * 32, bar);
+                            tma_pair_2d(dst + SUB_BYTES + q * 4096, &a.tmap_n, x + 64, first + q * 32, bar);
                         }
                     }
                 }
+                __syncwarp();
+            }
+            if (ok && !fetched) fetch_next();
+            u0 = u_next;
+            tile = tile_n;
+        }
+        // the copies land before the shared memory goes away. The second CTA cannot watch the first one's barriers: it
+        // waits as long as the first one does at most
+        if (lane == 0 && *abort_flag.flag) {
+            if (rank == 0) let_land(smem_u32(&full_bar[0]), UNITS, u0 + 2 * kgs);
+            else pause_ns(UNITS * 1000000ull);
+        }
+        __syncwarp();
+    } else if (ATMA && warp == R::copy0 + 2) {
+        // ------------------------- copies of the weights -----------------------
+        if (lane == 0) {
+            const uint32_t full_first = map_to(smem_u32(&full_bar[0]), 0);
+            int tn = 0;
+            uint32_t n = 0, u = 0, last_1 = 0, last_2 = 0;  // as the producers count
+            bool ok = true;
+            int4 tile;
+            while (ok && take_tile(false, tn, tile)) {
+                for (int k = 0; k < kgs; ++k, ++n) {
+                    ok = n < STAGES || pass_done(last_2);
+                    if (!ok) break;
+                    const uint32_t s = u % UNITS, dst = stage0 + (n % STAGES) * STAGE_BYTES, bar = full_first + s * 8;
+                    if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * STAGE_BYTES);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        if (MODE == 0)
+                            tma_pair_5d(dst + i * SUB_BYTES, &a.tmap_a, k * 128 + i * 64, 0, 0, tile.w * 16 + (int)rank * 8, tile.x, bar);
+                        else
+                            tma_pair_2d(dst + i * SUB_BYTES, &a.tmap_a, k * 128 + i * 64, tile.x * a.L.H + tile.w * 256 + (int)rank * 128, bar);
+                    }
+                    u += (tile.z > 256) ? 2 : 1;
+                    last_2 = last_1;
+                    last_1 = u - 1;
+                }
             }
             if (*abort_flag.flag) {
-                // the copies land before the shared memory goes away. The second CTA cannot watch the first one's barriers:
-                // it waits as long as the first one does at most
-                if (rank == 0) {
-                    let_land(smem_u32(&full_bar[0]), STAGES, n);
-                } else {
-                    const uint64_t t0 = globaltimer_ns();
-                    while (globaltimer_ns() - t0 < STAGES * 1000000ull) {
-                    }
-                }
+                if (rank == 0) let_land(smem_u32(&full_bar[0]), UNITS, u);
+                else pause_ns(UNITS * 1000000ull);
             }
         }
         __syncwarp();
     } else if (warp == R::mma) {
         // -------------------------------- MMA ---------------------------------
         if (rank == 0) {
-            int tl = 0, tn = 0, v = 0, s = 0, ph = 0;
+            // (one warp in order: every instruction of a pass counts. Votes keep what the MMA operands are made of uniform)
+            const uint32_t a_base = ((stage0 >> 4) & 0x3FFFu), b_base = (((stage0 + STAGES * STAGE_BYTES) >> 4) & 0x3FFFu);
+            const uint32_t full0 = smem_u32(&full_bar[0]), done0 = smem_u32(&done_bar[0]);
+            int tl = 0, tn = 0;
+            uint32_t v = 0, u = 0, n = 0;  // accumulator sets, passes, stages so far
             bool ok = true;
             int4 tile;
             for (; ok && take_tile(true, tn, tile); ++tl) {
-                const int nsets = (tile.z > 256) ? 2 : 1;
-                const int go_kh = (khs >= 24 && tile.z > 128) ? khs / 2 - 4 : 0;
-                const uint32_t id0 = idesc2(set_cols(tile.z, 0)), id1 = idesc2(nsets == 2 ? set_cols(tile.z, 1) : 32);
-                const int set0 = v & 1, set1 = set0 ^ 1;
-                const uint32_t acc0 = tmem_base + set0 * 256, acc1 = tmem_base + set1 * 256;
-                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_empty_bar[set0]), ((v >> 1) & 1) ^ 1, abort_flag));
-                if (!ok) break;
-                tc_fence_after();
-                // A wide tile holds both sets, and its epilogue would leave the tensor cores idle. So its first and its last
-                // SKEW stages are multiplied set by set: the first set is complete, and its epilogue under way, while the
+                const uint32_t wide = __any_sync(0xffffffffu, tile.z > 256) ? 1u : 0u;
+                const uint32_t id0 = idesc2(32 * __popc(__ballot_sync(0xffffffffu, lane < set_cols(tile.z, 0) / 32)));
+                const uint32_t id1 = idesc2(32 * max(1, __popc(__ballot_sync(0xffffffffu, lane < set_cols(tile.z, 1) / 32))));
+                const uint32_t passes = (uint32_t)kgs << wide;
+                const uint32_t go = (kgs >= 12 && __any_sync(0xffffffffu, tile.z > 128)) ? (uint32_t)(kgs / 2 - 2) << wide : 0u;
+                // The sets of a wide tile take turns, so that the first one is complete, and its epilogue under way, while the
                 // second one's last products run, and the next tile's first products run under the second one's epilogue.
-                const int skew = (nsets == 2 && khs >= 2 * SKEW) ? SKEW : 1;
-                for (int kh = 0; kh < khs;) {
-                    const int nb = (kh == 0 || kh == khs - skew) ? skew : 1;
-                    if (kh <= go_kh && go_kh < kh + nb && lane == 0) mbar_arrive(smem_u32(&go_bar[tl % ahead]));
-                    const int s_first = s;
-                    for (int i = 0; i < nb; ++i) {
-                        ok = __all_sync(0xffffffffu, wait_acquire(smem_u32(&full_bar[s]), ph, abort_flag));
-                        if (!ok) break;
-                        tc_fence_after();
-                        if (elect_one()) {
-                            const uint64_t w0 = make_desc(stage0 + s * STAGE_BYTES), b0 = w0 + (SUB_BYTES >> 4);
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) umma2(acc0, w0 + j * 2, b0 + j * 2, id0, (kh + i > 0 || j > 0) ? 1u : 0u);
-                            if (nsets == 1) umma2_commit(smem_u32(&empty_bar[s]));
-                            if (kh + i == khs - 1) umma2_commit(smem_u32(&acc_full_bar[set0]));
-                        }
-                        __syncwarp();
-                        if (++s == STAGES) {
-                            s = 0;
-                            ph ^= 1;
-                        }
-                    }
+                for (uint32_t p = 0; p < passes; ++p, ++u) {
+                    const uint32_t h = p & wide, set = (v + h) & 1, c = u % UNITS;
+                    if (p == go && lane == 0) mbar_arrive(smem_u32(&go_bar[tl % ahead]));
+                    if (p <= wide) ok = mbar_wait(smem_u32(&acc_empty_bar[set]), (((v + h) >> 1) & 1) ^ 1, abort_flag);
+                    ok = __all_sync(0xffffffffu, ok && mbar_wait(full0 + c * 8, (u / UNITS) & 1, abort_flag));
                     if (!ok) break;
-                    if (nsets == 2) {
-                        if (kh == 0) {
-                            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_empty_bar[set1]), (((v + 1) >> 1) & 1) ^ 1, abort_flag));
-                            if (!ok) break;
-                            tc_fence_after();
-                        }
-                        if (elect_one()) {
-                            for (int i = 0; i < nb; ++i) {
-                                const int si = (s_first + i) % STAGES;
-                                const uint64_t w0 = make_desc(stage0 + si * STAGE_BYTES), b0 = w0 + (2 * SUB_BYTES >> 4);
+                    tc_fence_after();
+                    const uint32_t w_lo = a_base + (n % STAGES) * (STAGE_BYTES >> 4), c_lo = b_base + c * (STAGE_BYTES >> 4);
+                    const uint32_t acc = tmem_base + set * 256, id = h ? id1 : id0;
+                    if (elect_one()) {
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) umma2(acc1, w0 + j * 2, b0 + j * 2, id1, (kh + i > 0 || j > 0) ? 1u : 0u);
-                                umma2_commit(smem_u32(&empty_bar[si]));
-                            }
-                            if (kh + nb == khs) umma2_commit(smem_u32(&acc_full_bar[set1]));
+                        for (int j = 0; j < 8; ++j) {
+                            const uint32_t o = (j >> 2) * (SUB_BYTES >> 4) + (j & 3) * 2;
+                            umma2(acc, desc_of(w_lo + o), desc_of(c_lo + o), id, (p > wide || j > 0) ? 1u : 0u);
                         }
-                        __syncwarp();
+                        umma2_commit(done0 + c * 8);
+                        if (p + 1 + wide >= passes) umma2_commit(smem_u32(&acc_full_bar[set]));
                     }
-                    kh += nb;
+                    __syncwarp();
+                    n += (h == wide);
                 }
                 if (!ok) break;
-                v += nsets;
+                v += 1 + wide;
             }
             if (*abort_flag.flag) {
                 // what has been issued reads both CTAs' shared memory: it ends before either goes away
@@ -661,7 +755,8 @@ static cudaError_t make_tmap_gate_up(const __half* gu16, int E, int I, int H, CU
     return make_tmap_f16_nd(gu16, 5, dims, strides, box, out);
 }
 
-// gate/up + SwiGLU, then down. x16: activation rows [columns, H] in the operands' element order
+// gate/up + SwiGLU, then down. x16: activation rows [columns, H] in the operands' element order, or null: the columns' rows
+// are taken from the tokens' plane p.xr16
 cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int ctas, cudaStream_t st, __half* out16_rows) {
     const int C = p.T * p.K, mt_gu = p.L.I / 128;
     const int max_ct = C / PAIR_TILE_COLS + p.L.E;
@@ -677,14 +772,19 @@ cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int ctas,
     gu.kdim = p.L.H;
     gu.out_ld = p.L.I;
     pair::Args dn = gu;
+    // the columns are gathered from the tokens' plane, unless they are its rows already (one expert)
+    const bool gathered = x16 == nullptr;
+    gu.gather = gathered ? p.R.col_src_tok : nullptr;
+    gu.n_cols = C;
     dn.debug_extra_tx = 0;  // the hook applies to the first kernel of the pair
     dn.tiles = p.tiles + (size_t)max_ct * mt_gu;  // as laid out by launch_route_large
     dn.out16 = out16_rows ? out16_rows : p.d16;
     dn.out_row_map = out16_rows ? p.R.col_src_tok : nullptr;
     dn.kdim = p.L.I;
     dn.out_ld = p.L.H;
-    cudaError_t e = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, 32, &gu.tmap_n);
-    if (e == cudaSuccess) e = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, 128, &gu.tmap_w);
+    cudaError_t e = gathered ? make_tmap_f16(p.xr16, (uint64_t)p.T, (uint64_t)p.L.H, 1, &gu.tmap_n)
+                             : make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, 32, &gu.tmap_n);
+    if (e == cudaSuccess && !gathered) e = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, 128, &gu.tmap_w);
     if (e == cudaSuccess) e = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, 32, &dn.tmap_n);
     if (e == cudaSuccess) e = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, 128, &dn.tmap_w);
     if (e != cudaSuccess) return e;

@@ -54,7 +54,7 @@ def test_prefill_on_both_sides_of_the_streaming_limit(cuda_lib, quant, T):
     check_prefill(384, 256, 16, 4, quant, synth.zipf_logits(T, 16, 3), torch.bfloat16)
 
 
-# tcgen05 rings and claims: contractions of a few stages, tiles of 128 and of 256 columns (one wave of tiles: 128)
+# tcgen05 rings and claims: contractions of a few stages, tiles of 128 columns and on CTA pairs
 @pytest.mark.parametrize("quant", [0, 1, 2])
 @pytest.mark.parametrize("H,I,E,T", [(512, 512, 8, 257), (256, 1024, 8, 640), (768, 128, 4, 6200)])
 def test_tcgen05_tiles_of_short_contractions(cuda_lib, quant, H, I, E, T):
@@ -64,10 +64,16 @@ def test_tcgen05_tiles_of_short_contractions(cuda_lib, quant, H, I, E, T):
 # products on CTA pairs: sets of 32..256 columns and what is left of them, one and two sets a tile, contractions of one,
 # two, three and many 128-input groups (tiles claimed four, two and one ahead)
 @pytest.mark.parametrize("quant", [0, 1, 2])
-@pytest.mark.parametrize("H,I", [(256, 1024), (2048, 128), (1536, 384), (3072, 256)])
+@pytest.mark.parametrize("H,I", [(256, 1024), (2048, 128), (1536, 384), (3072, 256), (768, 640)])
 def test_pair_products_tile_edges(cuda_lib, quant, H, I):
     counts = [0, 1, 16, 31, 33, 64, 255, 256, 257, 288, 511, 512, 513, 1025, 7, 95]
     check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1), torch.bfloat16)
+
+
+# one CTA a tile | pairs: the last batch of the one and the first of the other; a lone expert, whose columns are the tokens
+@pytest.mark.parametrize("quant,E,T", [(0, 8, 352), (0, 8, 353), (1, 8, 416), (1, 8, 417), (2, 8, 512), (2, 8, 4800)])
+def test_prefill_on_both_sides_of_the_pair_limit(cuda_lib, quant, E, T):
+    check_prefill(512, 256, E, 2, quant, synth.zipf_logits(T, E, 5))
 
 
 # batches of the decode chain for each format, at contractions with a remainder against the ring's chunk
@@ -149,7 +155,7 @@ def test_norm_folded_into_the_planes_matches_the_norm_kernel(cuda_lib, H):
 
 
 # a context of one expert: routing, operand plane and plan in one kernel of 8 tokens a CTA, then streaming up to 16
-# columns, tiles of 128 in one wave, tiles of 256 beyond
+# columns, tiles of 128 in one wave, CTA pairs beyond
 @pytest.mark.parametrize("quant", [0, 1, 2])
 @pytest.mark.parametrize("T,act,gating", [(1, torch.float32, 2), (9, torch.bfloat16, 2), (16, torch.float32, 3), (17, torch.bfloat16, 2),
                                           (129, torch.float32, 3), (9500, torch.bfloat16, 2)])
