@@ -14,8 +14,10 @@
 //            the same eight up rows). In the 16 x 256-bit shape of tcgen05.ld a thread then has gate and up of the same
 //            two outputs, and SwiGLU needs no exchange
 //   down     a tile is 256 rows of H: 128 per CTA
-// N is 32..256 in steps of 32 per set, so ragged tiles cost what they hold. Results go through stmatrix (transposed) and a
-// small buffer of the warp, and leave as whole 32- or 64-byte pieces of a column's row.
+// N is 32..256 in steps of 32 per set, so ragged tiles cost what they hold. Results go through stmatrix (transposed) into one
+// of two small buffers of the warp and leave from there: gate/up 32 bytes of a column at a time by the warp's stores, down 64 bytes of
+// 32 columns as one tiled copy (by stores the waits for a free accumulator of 8192 tokens are 47 instead of 30 us; the
+// 32-byte rows of gate/up lose with tiled copies, 27 and 33 us).
 //
 // One CTA pair per two SMs, persistent; tiles are claimed from a device-wide counter by the first CTA of the pair.
 // Warps of a CTA: 0-7 epilogue (16 of them for gate/up when the weights come by TMA), then 16 weight producers (with
@@ -54,15 +56,16 @@ struct Roles {
     static constexpr int prod0 = epi, copy0 = epi + prod, mma = copy0 + copies, sched = mma + 1, threads = (sched + 1) * 32;
     // arrivals for a stage's weights: every producer warp of both CTAs | the copies' expected bytes
     static constexpr int weight_arrivals = ATMA ? 1 : 2 * prod;
-    // a warp's output buffer: 32 columns of its 16 (gate/up) or 32 (down) rows, padded so that the eight rows of an
-    // stmatrix hit eight different 16-byte bank groups
-    static constexpr int row_bytes = (MODE == 0) ? 32 : 64, pitch = row_bytes + 16, out_bytes = 32 * pitch;
-    static constexpr size_t smem = 1024 + (size_t)(STAGES + UNITS) * STAGE_BYTES + (size_t)epi * out_bytes;
+    // an output buffer: 32 columns of the warp's 16 (gate/up) or 32 (down) rows, in the 32- or 64-byte swizzle of the tiled
+    // copy, with which the eight rows of an stmatrix hit eight different 16-byte bank groups
+    static constexpr int row_bytes = (MODE == 0) ? 32 : 64, out_bytes = 32 * row_bytes;
+    static constexpr size_t smem = 1024 + (size_t)(STAGES + UNITS) * STAGE_BYTES + (size_t)epi * 2 * out_bytes;
 };
 
 struct Args {
     CUtensorMap tmap_n;   // columns [rows, kdim] f16, box 64 x 32 (gathered: token rows, box 64 x 1)
     CUtensorMap tmap_w;   // the same, box 64 x 128
+    CUtensorMap tmap_o;   // down: results [columns, H] f16, box 32 x 32
     CUtensorMap tmap_a;   // ATMA: the experts' f16 matrices (gate/up: in groups of eight gate and eight up rows)
     LayerDev L;
     const int4* tiles;    // {expert, first column, columns, m-tile}
@@ -373,9 +376,13 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
         // ------------------------------ epilogue ------------------------------
         constexpr int PARTS = R::epi / 4;
         const int quad = warp & 3, part = warp >> 2;  // (TMEM lanes 32 quad.. are this warp's by the hardware's rule)
-        const uint32_t buf = stage0 + (STAGES + UNITS) * STAGE_BYTES + (uint32_t)warp * R::out_bytes;
+        const uint32_t buf0 = stage0 + (STAGES + UNITS) * STAGE_BYTES + (uint32_t)warp * 2 * R::out_bytes;
+        // 16-byte piece pc of row (column) cc of a buffer
+        auto piece = [&](int cc, int pc) -> uint32_t {
+            return (MODE == 0) ? cc * 32 + ((pc ^ ((cc >> 2) & 1)) << 4) : cc * 64 + ((pc ^ ((cc >> 1) & 3)) << 4);
+        };
+        int chunk = 0;  // this warp's so far: its parity is the buffer
         const uint32_t acc_empty_first = map_to(smem_u32(&acc_empty_bar[0]), 0);
-        const uint32_t st_addr = buf + lane * R::pitch;  // row `lane` of the buffer: column `lane` of the chunk
         int v = 0, tn = 0;
         int4 tile;
         bool ok = true;
@@ -391,47 +398,61 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                 const int ncols = min(256, tile.z - 256 * h), col0 = tile.y + 256 * h;
                 const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + set * 256;
                 // 32 columns of 16 rows into the buffer
-                auto rows16 = [&](const uint32_t (&x)[16], int half) {
+                auto rows16 = [&](const uint32_t (&x)[16], int half, uint32_t buf) {
                     if (MODE == 0) {
                         uint32_t o[4];
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
                             o[j] = pack_f16(swiglu(__uint_as_float(x[4 * j]), __uint_as_float(x[4 * j + 2])),
                                             swiglu(__uint_as_float(x[4 * j + 1]), __uint_as_float(x[4 * j + 3])));
-                        stmatrix4_t(st_addr + half * 16, o);
+                        stmatrix4_t(buf + piece(lane, half), o);
                     } else {
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
                             uint32_t o[4];
 #pragma unroll
                             for (int j = 0; j < 4; ++j) o[j] = pack_f16(__uint_as_float(x[4 * j + 2 * q]), __uint_as_float(x[4 * j + 2 * q + 1]));
-                            stmatrix4_t(st_addr + half * 32 + q * 16, o);
+                            stmatrix4_t(buf + piece(lane, 2 * half + q), o);
                         }
                     }
                 };
                 // the TMEM loads of the next 16 rows are issued before the current ones are worked on
                 uint32_t v0[16], v1[16];
                 if (part * 32 < ncols) tmem_ld_frag32(taddr + part * 32, v0);
-                for (int c = part * 32; c < ncols; c += PARTS * 32) {
+                for (int c = part * 32; c < ncols; c += PARTS * 32, ++chunk) {
+                    const uint32_t buf = buf0 + (chunk & 1) * R::out_bytes;
                     tmem_ld_wait();
                     tmem_ld_fence16(v0);
                     tmem_ld_frag32(taddr + (16u << 16) + c, v1);
-                    __syncwarp();  // the chunk before has left the buffer
-                    rows16(v0, 0);
+                    if (MODE == 1 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the copy before the last has left its buffer
+                    __syncwarp();
+                    rows16(v0, 0, buf);
                     tmem_ld_wait();
                     tmem_ld_fence16(v1);
                     if (c + PARTS * 32 < ncols) tmem_ld_frag32(taddr + c + PARTS * 32, v0);
-                    rows16(v1, 1);
+                    rows16(v1, 1, buf);
+                    if (MODE == 1) fence_proxy_async();
                     __syncwarp();
-                    constexpr int PIECES = R::row_bytes / 16;  // 16-byte pieces of a column
+                    const bool whole = MODE == 1 && c + 32 <= ncols && a.out_row_map == nullptr;
+                    if (MODE == 1 && lane == 0) {
+                        if (whole)
+                            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                                             reinterpret_cast<uint64_t>(&a.tmap_o)),
+                                         "r"(o0), "r"(col0 + c), "r"(buf)
+                                         : "memory");
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");  // (one group a chunk, an empty one too)
+                    }
+                    if (!whole) {
+                        constexpr int PIECES = R::row_bytes / 16;
 #pragma unroll
-                    for (int i = 0; i < PIECES; ++i) {
-                        const int p = i * 32 + lane, cc = p / PIECES, pc = p % PIECES;
-                        const uint4 x = lds128(buf + cc * R::pitch + pc * 16);
-                        if (c + cc < ncols) {
-                            int row = col0 + c + cc;
-                            if (MODE == 1 && a.out_row_map != nullptr) row = a.out_row_map[row];
-                            *reinterpret_cast<uint4*>(a.out16 + (size_t)row * a.out_ld + o0 + pc * 8) = x;
+                        for (int i = 0; i < PIECES; ++i) {
+                            const int p = i * 32 + lane, cc = p / PIECES, pc = p % PIECES;
+                            const uint4 x = lds128(buf + piece(cc, pc));
+                            if (c + cc < ncols) {
+                                int row = col0 + c + cc;
+                                if (MODE == 1 && a.out_row_map != nullptr) row = a.out_row_map[row];
+                                *reinterpret_cast<uint4*>(a.out16 + (size_t)row * a.out_ld + o0 + pc * 8) = x;
+                            }
                         }
                     }
                 }
@@ -440,6 +461,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                 if (lane == 0) arrive_at(acc_empty_first + set * 8);
             }
         }
+        if (MODE == 1 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // every result has been written
+        __syncwarp();
     } else if (warp < R::copy0) {
         // --------------------------- weight producers --------------------------
         if constexpr (!ATMA) {
@@ -785,6 +808,11 @@ cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int ctas,
     cudaError_t e = gathered ? make_tmap_f16(p.xr16, (uint64_t)p.T, (uint64_t)p.L.H, 1, &gu.tmap_n)
                              : make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, 32, &gu.tmap_n);
     if (e == cudaSuccess && !gathered) e = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, 128, &gu.tmap_w);
+    if (e == cudaSuccess) {
+        const uint64_t dims[2] = {(uint64_t)p.L.H, (uint64_t)C}, strides[1] = {(uint64_t)p.L.H * 2};
+        const uint32_t box[2] = {32, 32};
+        e = make_tmap_f16_nd(p.d16, 2, dims, strides, box, &dn.tmap_o, CU_TENSOR_MAP_SWIZZLE_64B);
+    }
     if (e == cudaSuccess) e = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, 32, &dn.tmap_n);
     if (e == cudaSuccess) e = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, 128, &dn.tmap_w);
     if (e != cudaSuccess) return e;

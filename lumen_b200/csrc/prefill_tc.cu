@@ -825,7 +825,7 @@ cudaError_t launch_gather_rows(const __half* plane, const int32_t* col_src_tok, 
                       H / 8, reinterpret_cast<uint4*>(out));
 }
 
-cudaError_t make_tmap_f16_nd(const void* base, int nd, const uint64_t* dims, const uint64_t* strides, const uint32_t* box, CUtensorMap* out) {
+cudaError_t make_tmap_f16_nd(const void* base, int nd, const uint64_t* dims, const uint64_t* strides, const uint32_t* box, CUtensorMap* out, CUtensorMapSwizzle swizzle) {
     typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -847,7 +847,7 @@ cudaError_t make_tmap_f16_nd(const void* base, int nd, const uint64_t* dims, con
         if (i + 1 < nd) st[i] = strides[i];
     }
     const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)nd, const_cast<void*>(base), d, st, bx, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }

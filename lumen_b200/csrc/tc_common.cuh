@@ -155,6 +155,7 @@ __device__ __forceinline__ void mbar_expect_more(uint32_t bar, uint32_t bytes) {
 // x (the column) of every copy is a multiple of 64 elements = 128 bytes.
 cudaError_t make_tmap_f16(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out);
 // the same for an f16 array of nd <= 5 dimensions (innermost first; strides in bytes, from the second dimension on)
-cudaError_t make_tmap_f16_nd(const void* base, int nd, const uint64_t* dims, const uint64_t* strides, const uint32_t* box, CUtensorMap* out);
+cudaError_t make_tmap_f16_nd(const void* base, int nd, const uint64_t* dims, const uint64_t* strides, const uint32_t* box, CUtensorMap* out,
+                             CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
 }  // namespace lumen
