@@ -618,12 +618,13 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
         CUDA_TRY(launch_stream_prefill(p, s->xr16, out16_rows, st));
         if (out16_rows) return Status::Ok();
     } else if (p.impl == 0) {
-        const bool pairs = tc_tile_cols(layer.dev, batch * s->K, s->sms, s->tc_ctas) == PAIR_TILE_COLS;  // gathers by itself
-        if (!single && !pairs) CUDA_TRY(launch_gather_rows(s->xr16, s->R.col_src_tok, batch * s->K, s->H, s->x16, st));
+        const TcForm form = tc_form(layer.dev, batch * s->K, s->sms, s->tc_ctas);
+        if (!single && !form.pairs)  // (pairs gather by themselves)
+             CUDA_TRY(launch_gather_rows(s->xr16, s->R.col_src_tok, batch * s->K, s->H, s->x16, st));
         // persistent grid, one CTA per SM; LUMEN_MOE_FLAG_TC_CTAS leaves some SMs to kernels that run beside it
         int sms = s->sms;
         if (s->tc_ctas > 0 && s->tc_ctas < sms) sms = s->tc_ctas;
-        if (pairs) CUDA_TRY(launch_grouped_pair(p, single ? s->xr16 : nullptr, sms, st, out16_rows));
+        if (form.pairs) CUDA_TRY(launch_grouped_pair(p, single ? s->xr16 : nullptr, form.cols, sms, st, out16_rows));
         else CUDA_TRY(launch_grouped_tc(p, single ? s->xr16 : s->x16, sms, st, out16_rows));
     } else {
         CUDA_TRY(launch_build_xf(normed, act_dtype, batch, s->H, layer.dev.kg_h * 4, bf16_mode, s->xf, st));

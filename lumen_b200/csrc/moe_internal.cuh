@@ -60,20 +60,22 @@ struct LayerDev {
     __host__ __device__ const uint4* down_s(int e) const { return s + (size_t)e * s_exp + 2 * s_gu; }
 };
 
-// Columns per tile of the tcgen05 products of a one-GPU call: 512 = the CTA-pair kernels (prefill_pair.cu), 128 = one CTA a
-// tile (prefill_tc.cu). Pairs from that average of columns an expert on at which they overtake: a pair has half as many weight
-// tiles in flight, which counts while a call is bound by its weights (E = 128, I = 768, us from the host: Q4_0 62 columns
-// 219 and 213 with pairs, 94 columns 247 and 237, 187 columns 376 and 321; Q8_0 111 columns 298 and 286, 78 columns of
-// E = 256 362 and 362; f16 matrices 111 columns 302 and 313, 144 columns 361 and 343). A lone expert (a shared one)
-// fills a few SMs with pairs where tiles of 128 fill four times as many: pairs once those are more than one wave
-// (2048 x 512: 1024 tokens 62 and 64 us, 4096 98 and 91; 900 tokens of 2048 x 1536 64 and 72), and the same for f16
-// matrices (2336 columns of 16 experts, 512 x 384: 62.5 and 63.2).
+// Form of the tcgen05 products of a one-GPU call: columns per tile, and whether CTA pairs work them (prefill_pair.cu: 512 or
+// 128 columns) or single CTAs (prefill_tc.cu: 128; only where the grid is capped at one).
+// 512: once the experts average so many columns that tiles of 128 would be cut often (E = 128, I = 768, us from the host, tiles of
+// 128 and of 512: Q4_0 112 columns 249 and 261, 128 columns 301 and 275; f16 matrices, whose weights come through the
+// ring as they are, 128 columns 320 and 332, 144 columns 360 and 345), and its tiles give half of the pairs work (a lone expert of
+// 2048 x 512: 2048 tokens 65 and 80, 4096 90 and 90; four experts of 1024 x 512 with 200 columns 37 and 41, sixteen with
+// 150 48 and 44).
 // ctas: cap of the persistent grid (0 = every SM).
-constexpr int PAIR_TILE_COLS = 512;
-inline int tc_tile_cols(const LayerDev& L, int columns, int sms, int ctas) {
-    const int least = L.gu16 != nullptr ? 128 : L.quant == Q4_0 ? 88 : 104;
-    const int mt = L.I / 128 > L.H / 256 ? L.I / 128 : L.H / 256;
-    return (columns > least * L.E && ((L.E > 1 && L.gu16 == nullptr) || columns / 128 * mt > sms) && ctas != 1) ? PAIR_TILE_COLS : 128;
+struct TcForm {
+    int cols;
+    bool pairs;
+};
+inline TcForm tc_form(const LayerDev& L, int columns, int sms, int ctas) {
+    if (ctas == 1) return TcForm{128, false};
+    const int least = L.gu16 != nullptr ? 136 : 120, tiles = (columns / 512 > L.E ? columns / 512 : L.E) * (L.I / 128);
+    return TcForm{columns > least * L.E && 4 * tiles >= sms ? 512 : 128, true};
 }
 
 // Routing tables of one call (device pointers into the context's scratch).
@@ -244,7 +246,7 @@ struct PrefillArgs {
 };
 cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st);
 // grouped products on CTA pairs (prefill_pair.cu)
-cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int ctas, cudaStream_t st, __half* out16_rows);
+cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int tile_cols, int ctas, cudaStream_t st, __half* out16_rows);
 bool route_single_applicable(const PrefillArgs& a);  // one expert: launch_route_large leaves the operand plane in xr16, columns = tokens
 // tcgen05 router (route_tc.cu)
 cudaError_t launch_split_router_w16(const float* w, __half* w16, int E, int H, bool natural, cudaStream_t st);
@@ -280,11 +282,11 @@ struct TcPlan {
 cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_cap, int gu_cols, int4* tiles,
                              int32_t* n_tiles, cudaStream_t st, const int32_t* stream_mode, int4* chunks, int32_t* starts,
                              int sms);
-// Most columns of a prompt that the streaming kernels take. The line lies where the tcgen05 kernels overtake them: Q8_0,
-// whose rows cost twice the bytes, at 10 columns an expert (E = 128, I = 768: 258 us there, 270 streaming; Q4_0 242 and
-// 231, at 12 245 and 248). A lone expert up to one 16-column operand (29 us, 36).
+// Most columns of a prompt that the streaming kernels take. The line lies where the tcgen05 kernels overtake them (E = 128,
+// I = 768, us, streaming and pairs: Q4_0 8 columns an expert 148 and 171, 10 columns 174 and 172; Q8_0, whose rows cost twice
+// the bytes, 8 columns 178 and 184, 9 columns 197 and 184). A lone expert up to one 16-column operand (29 us, 36).
 inline int stream_max_columns(int quant, int experts) {
-    const int n = (quant == Q4_0 ? 12 : 9) * experts;
+    const int n = (quant == Q4_0 ? 20 : 17) * experts / 2;
     return n > 16 ? n : 16;
 }
 // gate/up of a decode batch, expert products of short prompts (stream.cu)

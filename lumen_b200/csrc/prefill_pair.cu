@@ -1,6 +1,5 @@
-// Prefill grouped expert products on CTA pairs (tcgen05, cta_group::2): the form of a one-GPU call whose experts have
-// enough columns to be bound by the tensor cores. Smaller batches and expert-parallel calls: prefill_tc.cu. The products
-// are the reference's moe_grouped_gate_up_swiglu / moe_grouped_down kernels (cuda/shaders/moe_grouped.cu:1202-1760,
+// Prefill grouped expert products on CTA pairs (tcgen05, cta_group::2), the form of a one-GPU call. Expert-parallel calls:
+// prefill_tc.cu. The products are the reference's moe_grouped_gate_up_swiglu / moe_grouped_down kernels (cuda/shaders/moe_grouped.cu:1202-1760,
 // :2183-2598).
 //
 // What bounds it: the tensor cores, if their operands arrive. One CTA alone reads 96 bytes a clock of operands from its
@@ -42,14 +41,23 @@ namespace pair {
 using namespace tc;
 
 constexpr int PROD_WARPS = 16;
-constexpr int STAGES = 2;                                // weights: 128 rows x 128 inputs, as two swizzle atoms of 64
-constexpr int UNITS = 4;                                 // columns: this CTA's half of a set of 256, x 128 inputs
-constexpr int STAGE_BYTES = 2 * SUB_BYTES;               // of a stage and of a unit
+constexpr int UNITS = 4;                                 // of the columns' ring
+constexpr int STAGE_BYTES = 2 * SUB_BYTES;               // weights: 128 rows x 128 inputs, as two swizzle atoms of 64
+// The two forms. Wide: tiles of up to 512 columns; two stages of weights, units of 128 rows (this CTA's half of a set of 256).
+// Narrow: tiles of up to 128 columns; four stages, units of 64 rows. A stage comes back to its producers after ~1500
+// cycles (dequantised, announced, multiplied, committed): with two stages that is what a narrow tile waits for, not the
+// dequantisation (62 columns an expert: 1190 cycles a pass, 1000 without it).
+template <bool NARROW>
+struct Form {
+    static constexpr int cols = NARROW ? 128 : 512, stages = NARROW ? 4 : 2;
+    static constexpr int unit_rows = NARROW ? 64 : 128, atom_bytes = unit_rows * 128, unit_bytes = 2 * atom_bytes;
+    static constexpr int ring_bytes = stages * STAGE_BYTES + UNITS * unit_bytes;  // 192 KB both
+};
 constexpr int SCHED_RING = 8;                            // tile descriptors in flight between the scheduler and the roles
 constexpr int MAX_AHEAD = 4;                             // tiles that are claimed ahead of the MMAs at most
 constexpr int TMEM_COLS = 512;
 
-template <int MODE, bool ATMA>
+template <int MODE, bool ATMA, bool NARROW>
 struct Roles {
     static constexpr int epi = (ATMA && MODE == 0) ? 16 : 8, prod = ATMA ? 0 : PROD_WARPS;
     static constexpr int copies = ATMA ? 3 : 2;  // a set's columns each, the weights
@@ -59,7 +67,7 @@ struct Roles {
     // an output buffer: 32 columns of the warp's 16 (gate/up) or 32 (down) rows, in the 32- or 64-byte swizzle of the tiled
     // copy, with which the eight rows of an stmatrix hit eight different 16-byte bank groups
     static constexpr int row_bytes = (MODE == 0) ? 32 : 64, out_bytes = 32 * row_bytes;
-    static constexpr size_t smem = 1024 + (size_t)(STAGES + UNITS) * STAGE_BYTES + (size_t)epi * 2 * out_bytes;
+    static constexpr size_t smem = 1024 + (size_t)Form<NARROW>::ring_bytes + (size_t)epi * 2 * out_bytes;
 };
 
 struct Args {
@@ -293,10 +301,12 @@ __device__ __forceinline__ float swiglu(float g, float u) {
 // columns of set h of a tile, rounded up to what an MMA of the pair takes
 __device__ __forceinline__ int set_cols(int ncols, int h) { return (min(256, ncols - 256 * h) + 31) & ~31; }
 
-template <int Q, int MODE, bool ATMA>
-__global__ void __launch_bounds__(Roles<MODE, ATMA>::threads, 1)
+template <int Q, int MODE, bool ATMA, bool NARROW>
+__global__ void __launch_bounds__(Roles<MODE, ATMA, NARROW>::threads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
-    using R = Roles<MODE, ATMA>;
+    using R = Roles<MODE, ATMA, NARROW>;
+    using F = Form<NARROW>;
+    constexpr int STAGES = F::stages, UNIT_BYTES = F::unit_bytes;
     extern __shared__ uint8_t smem_raw[];
     // "first": used in the pair's first CTA only, which both CTAs' roles arrive at
     __shared__ uint64_t full_bar[UNITS];       // first: what a pass multiplies is there in both CTAs
@@ -370,13 +380,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
     // it: they hold up to `depth` groups and two stages beyond the MMAs), at the start of a narrow one, which
     // is over in about the time of a claim. Short ones: two ahead, so that the producers never run dry; four
     // where a tile is one group, because the producers' registers hold more than two of them.
-    const int ahead = (kgs >= 12) ? 1 : (kgs >= 2) ? 2 : MAX_AHEAD;
+    // (Narrow form: two more stages beyond the MMAs, passes of less than half the time.)
+    const int ahead = NARROW ? (kgs >= 8 ? 2 : MAX_AHEAD) : (kgs >= 12) ? 1 : (kgs >= 2) ? 2 : MAX_AHEAD;
 
     if (warp < R::epi) {
         // ------------------------------ epilogue ------------------------------
         constexpr int PARTS = R::epi / 4;
         const int quad = warp & 3, part = warp >> 2;  // (TMEM lanes 32 quad.. are this warp's by the hardware's rule)
-        const uint32_t buf0 = stage0 + (STAGES + UNITS) * STAGE_BYTES + (uint32_t)warp * 2 * R::out_bytes;
+        const uint32_t buf0 = stage0 + F::ring_bytes + (uint32_t)warp * 2 * R::out_bytes;
         // 16-byte piece pc of row (column) cc of a buffer
         auto piece = [&](int cc, int pc) -> uint32_t {
             return (MODE == 0) ? cc * 32 + ((pc ^ ((cc >> 2) & 1)) << 4) : cc * 64 + ((pc ^ ((cc >> 1) & 3)) << 4);
@@ -387,7 +398,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
         int4 tile;
         bool ok = true;
         while (ok && take_tile(true, tn, tile)) {
-            const int nsets = (tile.z > 256) ? 2 : 1;
+            const int nsets = (!NARROW && tile.z > 256) ? 2 : 1;
             // this warp's first output of a column's row
             const int o0 = (MODE == 0) ? tile.w * 128 + (int)rank * 64 + quad * 16 : tile.w * 256 + (int)rank * 128 + quad * 32;
             for (int h = 0; h < nsets; ++h, ++v) {
@@ -484,7 +495,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                     int4 tile;
                     if (more) more = take_tile(true, tn, tile);
                     if (!more) return 0;
-                    sets = (tile.z > 256) ? 2 : 1;
+                    sets = (!NARROW && tile.z > 256) ? 2 : 1;
                     const int e = tile.x;
                     const uint4 *qb, *sb;
                     int rt;
@@ -523,7 +534,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                 for (int j = 0; j < PF; ++j) {
                     ok = ok && there[j] != 0;
                     if (!ok) break;
-                    if (n >= STAGES) ok = __all_sync(0xffffffffu, pass_done(last_2));
+                    // the last pass of the stage that was here
+                    if (n >= STAGES) ok = __all_sync(0xffffffffu, pass_done(NARROW ? n - STAGES : last_2));
                     if (!ok) break;
                     dequant<Q, MODE>(w[j], stage0 + (n % STAGES) * STAGE_BYTES + sub * SUB_BYTES, pl, k);
                     fence_proxy_async();  // every lane's own stores, before the warp's one arrival
@@ -549,7 +561,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
         bool ok = true;
         // this CTA's rows of the warp's set of a tile that begins at unit u: `half` of them from the returned column on
         auto rows_of = [&](const int4& t, uint32_t u, int& half) -> int {
-            const int h = (t.z > 256) ? (int)((w ^ u) & 1) : 0;
+            const int h = (!NARROW && t.z > 256) ? (int)((w ^ u) & 1) : 0;
             half = set_cols(t.z, h) / 2;
             return t.y + 256 * h + (int)rank * half;
         };
@@ -565,7 +577,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
         if (have && gather) rows_n = token_rows(tile, 0);
         const int pre = max(kgs - 4, 0);  // where the next tile's descriptor and token rows are fetched
         while (ok && have) {
-            const bool wide = tile.z > 256;
+            const bool wide = !NARROW && tile.z > 256;
             int half;
             const int first = rows_of(tile, u0, half);
             const uint32_t bytes = 2 * (gather ? half * 128 : (half == 128) ? 128 * 128 : ((half + 31) / 32) * 4096);
@@ -593,7 +605,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                         mbar_expect_tx(smem_u32(&full_bar[s]), 2 * bytes + (unit == 0 ? a.debug_extra_tx : 0));
                         if (wide && odd) mbar_arrive_n(smem_u32(&full_bar[s]), R::weight_arrivals);
                     }
-                    const uint32_t dst = units0 + s * STAGE_BYTES, bar = full_first + s * 8;
+                    const uint32_t dst = units0 + s * UNIT_BYTES, bar = full_first + s * 8;
                     const int x = k * 128;
                     if (gather) {
                         // (sixteen rows' numbers first: a load between two copies would cost its latency each time)
@@ -603,15 +615,15 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                             for (int i = 0; i < 4; ++i) r[i] = rows_s[w][q + i];
 #pragma unroll
                             for (int i = 0; i < 8; ++i)
-                                tma_pair_gather4(dst + (i & 1) * SUB_BYTES + (q + (i >> 1)) * 512, &a.tmap_n, x + (i & 1) * 64, r[i >> 1], bar);
+                                tma_pair_gather4(dst + (i & 1) * F::atom_bytes + (q + (i >> 1)) * 512, &a.tmap_n, x + (i & 1) * 64, r[i >> 1], bar);
                         }
-                    } else if (half == 128) {
+                    } else if (!NARROW && half == 128) {
                         tma_pair_2d(dst, &a.tmap_w, x, first, bar);
-                        tma_pair_2d(dst + SUB_BYTES, &a.tmap_w, x + 64, first, bar);
+                        tma_pair_2d(dst + F::atom_bytes, &a.tmap_w, x + 64, first, bar);
                     } else {
                         for (int q = 0; q * 32 < half; ++q) {
                             tma_pair_2d(dst + q * 4096, &a.tmap_n, x, first + q * 32, bar);
-                            tma_pair_2d(dst + SUB_BYTES + q * 4096, &a.tmap_n, x + 64, first + q * 32, bar);
+                            tma_pair_2d(dst + F::atom_bytes + q * 4096, &a.tmap_n, x + 64, first + q * 32, bar);
                         }
                     }
                 }
@@ -638,7 +650,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
             int4 tile;
             while (ok && take_tile(false, tn, tile)) {
                 for (int k = 0; k < kgs; ++k, ++n) {
-                    ok = n < STAGES || pass_done(last_2);
+                    ok = n < STAGES || pass_done(NARROW ? n - STAGES : last_2);
                     if (!ok) break;
                     const uint32_t s = u % UNITS, dst = stage0 + (n % STAGES) * STAGE_BYTES, bar = full_first + s * 8;
                     if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * STAGE_BYTES);
@@ -649,7 +661,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                         else
                             tma_pair_2d(dst + i * SUB_BYTES, &a.tmap_a, k * 128 + i * 64, tile.x * a.L.H + tile.w * 256 + (int)rank * 128, bar);
                     }
-                    u += (tile.z > 256) ? 2 : 1;
+                    u += (!NARROW && tile.z > 256) ? 2 : 1;
                     last_2 = last_1;
                     last_1 = u - 1;
                 }
@@ -664,18 +676,18 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
         // -------------------------------- MMA ---------------------------------
         if (rank == 0) {
             // (one warp in order: every instruction of a pass counts. Votes keep what the MMA operands are made of uniform)
-            const uint32_t a_base = ((stage0 >> 4) & 0x3FFFu), b_base = (((stage0 + STAGES * STAGE_BYTES) >> 4) & 0x3FFFu);
+            const uint32_t a_base = (stage0 >> 4) & 0x3FFFu, b_base = ((stage0 + STAGES * STAGE_BYTES) >> 4) & 0x3FFFu;
             const uint32_t full0 = smem_u32(&full_bar[0]), done0 = smem_u32(&done_bar[0]);
             int tl = 0, tn = 0;
             uint32_t v = 0, u = 0, n = 0;  // accumulator sets, passes, stages so far
             bool ok = true;
             int4 tile;
             for (; ok && take_tile(true, tn, tile); ++tl) {
-                const uint32_t wide = __any_sync(0xffffffffu, tile.z > 256) ? 1u : 0u;
+                const uint32_t wide = (!NARROW && __any_sync(0xffffffffu, tile.z > 256)) ? 1u : 0u;
                 const uint32_t id0 = idesc2(32 * __popc(__ballot_sync(0xffffffffu, lane < set_cols(tile.z, 0) / 32)));
                 const uint32_t id1 = idesc2(32 * max(1, __popc(__ballot_sync(0xffffffffu, lane < set_cols(tile.z, 1) / 32))));
                 const uint32_t passes = (uint32_t)kgs << wide;
-                const uint32_t go = (kgs >= 12 && __any_sync(0xffffffffu, tile.z > 128)) ? (uint32_t)(kgs / 2 - 2) << wide : 0u;
+                const uint32_t go = (!NARROW && kgs >= 12 && __any_sync(0xffffffffu, tile.z > 128)) ? (uint32_t)(kgs / 2 - 2) << wide : 0u;
                 // The sets of a wide tile take turns, so that the first one is complete, and its epilogue under way, while the
                 // second one's last products run, and the next tile's first products run under the second one's epilogue.
                 for (uint32_t p = 0; p < passes; ++p, ++u) {
@@ -685,13 +697,13 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                     ok = __all_sync(0xffffffffu, ok && mbar_wait(full0 + c * 8, (u / UNITS) & 1, abort_flag));
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t w_lo = a_base + (n % STAGES) * (STAGE_BYTES >> 4), c_lo = b_base + c * (STAGE_BYTES >> 4);
+                    const uint32_t w_lo = a_base + (n % STAGES) * (STAGE_BYTES >> 4), c_lo = b_base + c * (UNIT_BYTES >> 4);
                     const uint32_t acc = tmem_base + set * 256, id = h ? id1 : id0;
                     if (elect_one()) {
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
-                            const uint32_t o = (j >> 2) * (SUB_BYTES >> 4) + (j & 3) * 2;
-                            umma2(acc, desc_of(w_lo + o), desc_of(c_lo + o), id, (p > wide || j > 0) ? 1u : 0u);
+                            const uint32_t ow = (j >> 2) * (SUB_BYTES >> 4) + (j & 3) * 2, oc = (j >> 2) * (F::atom_bytes >> 4) + (j & 3) * 2;
+                            umma2(acc, desc_of(w_lo + ow), desc_of(c_lo + oc), id, (p > wide || j > 0) ? 1u : 0u);
                         }
                         umma2_commit(done0 + c * 8);
                         if (p + 1 + wide >= passes) umma2_commit(smem_u32(&acc_full_bar[set]));
@@ -743,10 +755,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
     if (tid == 0 && abort_s) raise_status(a.status, a.status_host, 4);  // LUMEN_MOE_TIMEOUT
 }
 
-template <int Q, int MODE, bool ATMA>
+template <int Q, int MODE, bool ATMA, bool NARROW>
 cudaError_t launch_one(const Args& a, int ctas, cudaStream_t st) {
-    using R = Roles<MODE, ATMA>;
-    auto* kern = grouped_gemm_pair_kernel<Q, MODE, ATMA>;
+    using R = Roles<MODE, ATMA, NARROW>;
+    auto* kern = grouped_gemm_pair_kernel<Q, MODE, ATMA, NARROW>;
     static SmemOptIn optin;
     const cudaError_t e = ensure_dyn_smem(kern, R::smem, optin);
     if (e != cudaSuccess) return e;
@@ -767,6 +779,12 @@ cudaError_t launch_one(const Args& a, int ctas, cudaStream_t st) {
     return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
+template <int Q, bool ATMA, bool NARROW>
+cudaError_t launch_both(const Args& gu, const Args& dn, int ctas, cudaStream_t st) {
+    const cudaError_t e = launch_one<Q, 0, ATMA, NARROW>(gu, ctas, st);
+    return e == cudaSuccess ? launch_one<Q, 1, ATMA, NARROW>(dn, ctas, st) : e;
+}
+
 }  // namespace pair
 
 // The experts' gate/up matrices [E][gate rows, up rows][H] f16 as a 5-D array (input, row of eight, gate | up, group of eight
@@ -780,9 +798,10 @@ static cudaError_t make_tmap_gate_up(const __half* gu16, int E, int I, int H, CU
 
 // gate/up + SwiGLU, then down. x16: activation rows [columns, H] in the operands' element order, or null: the columns' rows
 // are taken from the tokens' plane p.xr16
-cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int ctas, cudaStream_t st, __half* out16_rows) {
+cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int tile_cols, int ctas, cudaStream_t st, __half* out16_rows) {
+    const bool narrow = tile_cols == pair::Form<true>::cols;
     const int C = p.T * p.K, mt_gu = p.L.I / 128;
-    const int max_ct = C / PAIR_TILE_COLS + p.L.E;
+    const int max_ct = C / tile_cols + p.L.E;
     pair::Args gu{};
     gu.L = p.L;
     gu.tiles = p.tiles;
@@ -819,17 +838,12 @@ cudaError_t launch_grouped_pair(const PrefillArgs& p, const void* x16, int ctas,
     if (p.L.gu16 != nullptr) {
         e = make_tmap_gate_up(p.L.gu16, p.L.E, p.L.I, p.L.H, &gu.tmap_a);
         if (e == cudaSuccess) e = make_tmap_f16(p.L.dn16, (uint64_t)p.L.E * p.L.H, (uint64_t)p.L.I, 128, &dn.tmap_a);
-        if (e == cudaSuccess) e = pair::launch_one<BF16, 0, true>(gu, ctas, st);
-        if (e == cudaSuccess) e = pair::launch_one<BF16, 1, true>(dn, ctas, st);
-        return e;
+        if (e != cudaSuccess) return e;
+        return narrow ? pair::launch_both<BF16, true, true>(gu, dn, ctas, st) : pair::launch_both<BF16, true, false>(gu, dn, ctas, st);
     }
     switch (p.L.quant) {
-        case Q4_0:
-            e = pair::launch_one<Q4_0, 0, false>(gu, ctas, st);
-            return e == cudaSuccess ? pair::launch_one<Q4_0, 1, false>(dn, ctas, st) : e;
-        case Q8_0:
-            e = pair::launch_one<Q8_0, 0, false>(gu, ctas, st);
-            return e == cudaSuccess ? pair::launch_one<Q8_0, 1, false>(dn, ctas, st) : e;
+        case Q4_0: return narrow ? pair::launch_both<Q4_0, false, true>(gu, dn, ctas, st) : pair::launch_both<Q4_0, false, false>(gu, dn, ctas, st);
+        case Q8_0: return narrow ? pair::launch_both<Q8_0, false, true>(gu, dn, ctas, st) : pair::launch_both<Q8_0, false, false>(gu, dn, ctas, st);
         default:
             return cudaErrorInvalidValue;  // BF16 layers always carry their f16 matrices on this path
     }

@@ -1,6 +1,6 @@
 // Prefill grouped expert products on the 5th-generation tensor cores (tcgen05,
-// accumulators in TMEM), one CTA a tile: for experts of a few dozen columns, a lone expert and expert-parallel calls (more
-// columns: prefill_pair.cu). Replaces the reference's tiled prefill kernels
+// accumulators in TMEM), one CTA a tile: for expert-parallel calls, and where the grid is capped at one CTA (all other
+// calls: prefill_pair.cu). Replaces the reference's tiled prefill kernels
 // (moe_grouped_gate_up_swiglu_q4_0_tiled_f32act / moe_grouped_down_q4_0_tiled_f32act,
 // cuda/shaders/moe_grouped.cu:1202-1510; the Q8_0 dp4a / mma.sync variants :566-1170,
 // :2183-2598; the BF16 variants :1523-1760).

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from lumen_b200 import moe, synth
+from lumen_b200 import _lib, moe, synth
 from oracle import oracle
 from tests.gpu_util import TOL_REL_L2, make_layer, oracle_layer, rel_l2
 
@@ -48,8 +48,8 @@ def test_streaming_prefill_chunk_edges(cuda_lib, quant, H, I):
     check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1))
 
 
-# the last batch on the streaming kernels and the first on the tcgen05 ones (9 | 12 columns an expert)
-@pytest.mark.parametrize("quant,T", [(0, 36), (0, 37), (1, 48), (1, 49)])
+# the last batch on the streaming kernels and the first on the tcgen05 ones (8.5 | 10 columns an expert), and batches between
+@pytest.mark.parametrize("quant,T", [(0, 34), (0, 35), (0, 36), (0, 37), (1, 40), (1, 41), (1, 48), (1, 49)])
 def test_prefill_on_both_sides_of_the_streaming_limit(cuda_lib, quant, T):
     check_prefill(384, 256, 16, 4, quant, synth.zipf_logits(T, 16, 3), torch.bfloat16)
 
@@ -61,19 +61,42 @@ def test_tcgen05_tiles_of_short_contractions(cuda_lib, quant, H, I, E, T):
     check_prefill(H, I, E, 2, quant, synth.uniform_logits(T, E, 7))
 
 
-# products on CTA pairs: sets of 32..256 columns and what is left of them, one and two sets a tile, contractions of one,
-# two, three and many 128-input groups (tiles claimed four, two and one ahead)
+# products on CTA pairs, tiles of up to 512 columns: sets of 32..256 columns and what is left of them, one and two sets a
+# tile, contractions of one, two, three and many 128-input groups (tiles claimed four, two and one ahead)
 @pytest.mark.parametrize("quant", [0, 1, 2])
-@pytest.mark.parametrize("H,I", [(256, 1024), (2048, 128), (1536, 384), (3072, 256), (768, 640)])
-def test_pair_products_tile_edges(cuda_lib, quant, H, I):
+@pytest.mark.parametrize("H,I", [(256, 1024), (2048, 384), (1536, 384), (3072, 512), (768, 640)])
+def test_pair_products_wide_tile_edges(cuda_lib, quant, H, I):
     counts = [0, 1, 16, 31, 33, 64, 255, 256, 257, 288, 511, 512, 513, 1025, 7, 95]
     check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1), torch.bfloat16)
 
 
-# one CTA a tile | pairs: the last batch of the one and the first of the other; a lone expert, whose columns are the tokens
-@pytest.mark.parametrize("quant,E,T", [(0, 8, 352), (0, 8, 353), (1, 8, 416), (1, 8, 417), (2, 8, 512), (2, 8, 4800)])
-def test_prefill_on_both_sides_of_the_pair_limit(cuda_lib, quant, E, T):
-    check_prefill(512, 256, E, 2, quant, synth.zipf_logits(T, E, 5))
+# tiles of up to 128 columns: operands of 32..128 columns, several tiles an expert, contractions of one group and more
+@pytest.mark.parametrize("quant", [0, 1, 2])
+@pytest.mark.parametrize("H,I", [(256, 1024), (2048, 128), (1536, 384), (3072, 256), (768, 640)])
+def test_pair_products_narrow_tile_edges(cuda_lib, quant, H, I):
+    counts = [0, 1, 16, 31, 32, 33, 63, 65, 96, 97, 127, 128, 129, 257, 7, 400]
+    check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1), torch.bfloat16)
+
+
+# tiles of 128 | 512: the last batch of the one and the first of the other; few experts; a grid capped at one CTA and at three
+@pytest.mark.parametrize("quant,E,I,T", [(0, 16, 384, 960), (0, 16, 384, 961), (1, 16, 384, 961), (2, 16, 384, 1088), (2, 16, 384, 1089), (1, 4, 256, 600)])
+def test_prefill_on_both_sides_of_the_wide_tiles(cuda_lib, quant, E, I, T):
+    check_prefill(512, I, E, 2, quant, synth.zipf_logits(T, E, 5))
+
+
+@pytest.mark.parametrize("quant", [0, 1, 2])
+@pytest.mark.parametrize("ctas,T", [(1, 300), (3, 300), (3, 1100)])
+def test_prefill_on_a_capped_grid(cuda_lib, quant, ctas, T):
+    H, I, E, K = 512, 384, 16, 2
+    lay = synth.LayerLayout(H, I, E, quant)
+    blob = synth.make_layer_blob(lay, 3)
+    x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(T), device="cuda")
+    outs = []
+    for flags in (0, _lib.flag_tc_ctas(ctas)):
+        sc = moe.allocate_moe_scratch(H, I, E, K, T, flags=flags)
+        outs.append(sc.prefill(sc.prepare_layer(blob, lay.meta()), x, x))
+        assert sc.poll_status() == _lib.OK
+    assert torch.equal(*outs)
 
 
 # batches of the decode chain for each format, at contractions with a remainder against the ring's chunk
