@@ -62,8 +62,8 @@ struct Roles {
     static constexpr int epi = (ATMA && MODE == 0) ? 16 : 8, prod = ATMA ? 0 : PROD_WARPS;
     static constexpr int copies = ATMA ? 3 : 2;  // a set's columns each, the weights
     static constexpr int prod0 = epi, copy0 = epi + prod, mma = copy0 + copies, sched = mma + 1, threads = (sched + 1) * 32;
-    // arrivals for a stage's weights: every producer warp of both CTAs | the copies' expected bytes
-    static constexpr int weight_arrivals = ATMA ? 1 : 2 * prod;
+    // arrivals for a stage's weights: half of the producer warps of both CTAs | the copies' expected bytes
+    static constexpr int weight_arrivals = ATMA ? 1 : prod;
     // an output buffer: 32 columns of the warp's 16 (gate/up) or 32 (down) rows, in the 32- or 64-byte swizzle of the tiled
     // copy, with which the eight rows of an stmatrix hit eight different 16-byte bank groups
     static constexpr int row_bytes = (MODE == 0) ? 32 : 64, out_bytes = 32 * row_bytes;
@@ -131,6 +131,16 @@ __device__ __forceinline__ bool wait_acquire(uint32_t bar, uint32_t parity, cons
             }
         }
     }
+}
+// whether the phase is over, without waiting for it
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
 }
 __device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t n) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
@@ -210,18 +220,10 @@ __device__ __forceinline__ uint32_t pack_f16(float a, float b) {
 }
 
 // --- dequantisation ---------------------------------------------------------------------------------------------------
-// A producer warp owns 16 rows x 64 inputs (blocks 2 sub, 2 sub + 1 of every 128-input group) of this CTA's operand. What a
-// lane holds of it:
-template <int Q>
-struct Half {
-    uint4 q[Q == Q4_0 ? 1 : 2];
-    uint32_t s_g, s_g8;  // f16 scales of the two blocks, rows g and g + 8
-};
-// groups a warp keeps on the way in registers: 128 rows x 128 inputs are 9 (Q4_0) or 17 KB an SM
-template <int Q>
-struct Prefetch {
-    static constexpr int depth = (Q == Q4_0) ? 4 : 3;
-};
+// A producer warp owns 16 rows x 128 inputs of this CTA's operand in every second stage: eight warps fill a stage, the other
+// eight the next one, so that each has the time of two passes for one wait, one fence and one arrival. It keeps this many of its
+// tiles on the way in registers (9 or 17 KB an SM and stage):
+constexpr int PREFETCH = 2;
 
 // Where a lane's chunks go in the operand: 16 bytes of row m at (m / 8) 1024 + (m % 8) 128 + ((chunk ^ m % 8) 16).
 // A quarter warp is two rows g of four chunks each. Down: rows in order, the two rows' m % 8 agree in bit 2, and the odd
@@ -260,26 +262,28 @@ __device__ __forceinline__ uint32_t scale_f16x2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ void store16(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
+// half a tile (16 rows x 64 inputs): q words of blocks 2 sub, 2 sub + 1, the blocks' f16 scales of rows g and g + 8
 template <int Q, int MODE>
-__device__ __forceinline__ void dequant(const Half<Q>& w, uint32_t a_base, const Place<MODE>& pl, const UnpackConst& k) {
+__device__ __forceinline__ void dequant(const uint4& q0, const uint4& q1, uint32_t s_g, uint32_t s_g8, uint32_t a_base, const Place<MODE>& pl,
+                                        const UnpackConst& k) {
 #pragma unroll
     for (int p = 0; p < 2; ++p)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             // (gate/up never swaps: the selections below fold away)
             const bool second = (MODE == 0) ? (p == 1) : ((p == 1) != pl.swap);
-            const uint32_t sc = prmt(r ? w.s_g8 : w.s_g, 0u, second ? 0x3232u : 0x1010u);
+            const uint32_t sc = prmt(r ? s_g8 : s_g, 0u, second ? 0x3232u : 0x1010u);
             uint32_t l0, l1, h0, h1;
             if constexpr (Q == Q4_0) {
-                const uint32_t a = r ? w.q[0].y : w.q[0].x, b = r ? w.q[0].w : w.q[0].z;
+                const uint32_t a = r ? q0.y : q0.x, b = r ? q0.w : q0.z;
                 const uint32_t x = second ? b : a, y = x >> 8;
                 l0 = hsub2_u32(lop_and_or(x, 0x000F000Fu, k.or_a), k.sub_a);
                 h0 = hsub2_u32(lop_and_or(x, 0x00F000F0u, k.or_b), k.sub_b);
                 l1 = hsub2_u32(lop_and_or(y, 0x000F000Fu, k.or_a), k.sub_a);
                 h1 = hsub2_u32(lop_and_or(y, 0x00F000F0u, k.or_b), k.sub_b);
             } else {
-                const uint32_t a0 = r ? w.q[0].z : w.q[0].x, a1 = r ? w.q[0].w : w.q[0].y;
-                const uint32_t b0 = r ? w.q[1].z : w.q[1].x, b1 = r ? w.q[1].w : w.q[1].y;
+                const uint32_t a0 = r ? q0.z : q0.x, a1 = r ? q0.w : q0.y;
+                const uint32_t b0 = r ? q1.z : q1.x, b1 = r ? q1.w : q1.y;
                 const uint32_t x = (second ? b0 : a0) ^ k.or_b, y = (second ? b1 : a1) ^ k.or_b;
                 l0 = hsub2_u32(prmt(x, k.or_a, 0x4240u), k.sub_a);
                 l1 = hsub2_u32(prmt(x, k.or_a, 0x4341u), k.sub_a);
@@ -477,24 +481,35 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
     } else if (warp < R::copy0) {
         // --------------------------- weight producers --------------------------
         if constexpr (!ATMA) {
-            const int pw = warp - R::prod0, rtl = pw & 7, sub = pw >> 3;
-            constexpr int PF = Prefetch<Q>::depth, NQH = QTraits<Q>::NQ / 2;
+            const int pw = warp - R::prod0, rtl = pw & 7;
+            constexpr int NQ = QTraits<Q>::NQ;
             const Place<MODE> pl(rtl, lane);
             const UnpackConst k = unpack_const_pinned<Q>();
             const uint32_t full_first = map_to(smem_u32(&full_bar[0]), 0);
-            int tn = 0, pkg = kgs;
-            bool more = true;
-            const uint4* qp = nullptr;
-            const uint32_t* sp = nullptr;
-            // the next group of the list into registers; false when there is none. The descriptor of a tile that is still
-            // to be claimed is waited for: it comes without any help from the groups that are held here (see `ahead`)
-            int sets = 1;  // accumulator sets of the tile being loaded
-            // (returns the sets of the group's tile, 0 when there is none)
-            auto load_next = [&](Half<Q>& w) -> int {
-                if (pkg == kgs) {
+            // load cursor: this warp's next stage is group kg of the tile at hand, whose first pass is number u0
+            int tn = 0, kg = (pw >> 3) - kgs;
+            uint32_t u0 = 0;
+            bool more = true;               // the list may hold further tiles
+            int sets = 0, sets_before = 0;  // accumulator sets of the tile at hand and of the one before (0: none)
+            const uint4 *qt = nullptr, *st = nullptr;
+            WTile<Q> w[PREFETCH];
+            uint32_t pass[PREFETCH];   // a slot's first pass
+            uint32_t before[PREFETCH]; // the passes over which its stage is free
+            bool there[PREFETCH];
+            // the warp's next tile into registers; false when there is none. The descriptor of a tile that is still to be
+            // claimed is waited for: it comes without any help from the tiles that are held here (see `ahead`)
+            auto load_next = [&](int j) {
+                kg += (sets == 0) ? kgs : 2;  // (the first call starts at the warp's own first group)
+                while (sets == 0 || kg >= kgs) {
+                    if (sets != 0) kg -= kgs;
                     int4 tile;
-                    if (more) more = take_tile(true, tn, tile);
-                    if (!more) return 0;
+                    more = more && take_tile(true, tn, tile);
+                    if (!more) {
+                        there[j] = false;
+                        return;
+                    }
+                    u0 += (uint32_t)(kgs * sets);
+                    sets_before = sets;
                     sets = (!NARROW && tile.z > 256) ? 2 : 1;
                     const int e = tile.x;
                     const uint4 *qb, *sb;
@@ -510,42 +525,39 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                         rt = tile.w * 16 + (int)rank * 8 + rtl;
                     }
                     const size_t tidx = (size_t)rt * kgs;
-                    qp = qb + (tidx * QTraits<Q>::NQ + sub * NQH) * 32 + lane;
-                    sp = reinterpret_cast<const uint32_t*>(sb + tidx * 8 + (lane >> 2)) + sub;
-                    pkg = 0;
+                    qt = qb + tidx * (NQ * 32) + lane;
+                    st = sb + tidx * 8 + (lane >> 2);
                 }
+                const uint4* qp = qt + kg * (NQ * 32);
 #pragma unroll
-                for (int j = 0; j < NQH; ++j) w.q[j] = ldg_stream(qp + j * 32);
-                w.s_g = __ldg(sp);
-                w.s_g8 = __ldg(sp + 2);
-                qp += QTraits<Q>::NQ * 32;
-                sp += 32;
-                ++pkg;
-                return sets;
+                for (int i = 0; i < NQ; ++i) w[j].q[i] = ldg_stream(qp + i * 32);
+                w[j].s = ldg_stream(st + kg * 8);
+                pass[j] = u0 + (uint32_t)(kg * sets);
+                // stage n - 2 is over with the pass in front of stage n - 1's first
+                if (!NARROW) before[j] = pass[j] - (uint32_t)(kg > 0 ? sets : sets_before);
+                there[j] = true;
             };
-            Half<Q> w[PF];
-            int there[PF];
 #pragma unroll
-            for (int j = 0; j < PF; ++j) there[j] = load_next(w[j]);
-            uint32_t n = 0, u = 0, last_1 = 0, last_2 = 0;  // stages, passes so far; the last passes of the stages before
+            for (int j = 0; j < PREFETCH; ++j) load_next(j);
+            uint32_t n = pw >> 3;  // stage
             bool ok = true;
             while (ok) {
 #pragma unroll
-                for (int j = 0; j < PF; ++j) {
-                    ok = ok && there[j] != 0;
+                for (int j = 0; j < PREFETCH; ++j) {
+                    ok = ok && there[j];
                     if (!ok) break;
-                    // the last pass of the stage that was here
-                    if (n >= STAGES) ok = __all_sync(0xffffffffu, pass_done(NARROW ? n - STAGES : last_2));
+                    if (n >= STAGES) ok = __all_sync(0xffffffffu, pass_done((NARROW ? n - STAGES + 1 : before[j]) - 1));
                     if (!ok) break;
-                    dequant<Q, MODE>(w[j], stage0 + (n % STAGES) * STAGE_BYTES + sub * SUB_BYTES, pl, k);
+                    const uint32_t base = stage0 + (n % STAGES) * STAGE_BYTES;
+#pragma unroll
+                    for (int sub = 0; sub < 2; ++sub)
+                        dequant<Q, MODE>(w[j].q[Q == Q4_0 ? sub : (2 * sub) % NQ], w[j].q[Q == Q4_0 ? sub : (2 * sub + 1) % NQ], sub ? w[j].s.y : w[j].s.x,
+                                         sub ? w[j].s.w : w[j].s.z, base + sub * SUB_BYTES, pl, k);
                     fence_proxy_async();  // every lane's own stores, before the warp's one arrival
                     __syncwarp();
-                    if (lane == 0) arrive_at(full_first + (u % UNITS) * 8);
-                    ++n;
-                    u += there[j];
-                    last_2 = last_1;
-                    last_1 = u - 1;
-                    there[j] = load_next(w[j]);
+                    if (lane == 0) arrive_at(full_first + ((NARROW ? n : pass[j]) % UNITS) * 8);
+                    n += 2;
+                    load_next(j);
                 }
             }
         }
@@ -680,7 +692,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
             const uint32_t full0 = smem_u32(&full_bar[0]), done0 = smem_u32(&done_bar[0]);
             int tl = 0, tn = 0;
             uint32_t v = 0, u = 0, n = 0;  // accumulator sets, passes, stages so far
-            bool ok = true;
+            bool ok = true, ready = false;  // ready: the next pass's operands are known to be there
             int4 tile;
             for (; ok && take_tile(true, tn, tile); ++tl) {
                 const uint32_t wide = (!NARROW && __any_sync(0xffffffffu, tile.z > 256)) ? 1u : 0u;
@@ -694,8 +706,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                     const uint32_t h = p & wide, set = (v + h) & 1, c = u % UNITS;
                     if (p == go && lane == 0) mbar_arrive(smem_u32(&go_bar[tl % ahead]));
                     if (p <= wide) ok = mbar_wait(smem_u32(&acc_empty_bar[set]), (((v + h) >> 1) & 1) ^ 1, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok && mbar_wait(full0 + c * 8, (u / UNITS) & 1, abort_flag));
+                    ok = __all_sync(0xffffffffu, ok && (ready || mbar_wait(full0 + c * 8, (u / UNITS) & 1, abort_flag)));
                     if (!ok) break;
+                    ready = mbar_test(full0 + ((u + 1) % UNITS) * 8, ((u + 1) / UNITS) & 1);  // (its answer comes under the products' issue)
                     tc_fence_after();
                     const uint32_t w_lo = a_base + (n % STAGES) * (STAGE_BYTES >> 4), c_lo = b_base + c * (UNIT_BYTES >> 4);
                     const uint32_t acc = tmem_base + set * 256, id = h ? id1 : id0;
