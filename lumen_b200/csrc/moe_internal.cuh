@@ -282,13 +282,12 @@ struct TcPlan {
 cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_cap, int gu_cols, int4* tiles,
                              int32_t* n_tiles, cudaStream_t st, const int32_t* stream_mode, int4* chunks, int32_t* starts,
                              int sms);
-// Most columns of a prompt that the streaming kernels take. The line lies where the tcgen05 kernels overtake them (E = 128,
-// I = 768, us, streaming and pairs: Q4_0 8 columns an expert 148 and 171, 10 columns 174 and 172; Q8_0, whose rows cost twice
-// the bytes, 8 columns 178 and 184, 9 columns 197 and 184). A lone expert up to one 16-column operand (29 us, 36).
-inline int stream_max_columns(int quant, int experts) {
-    const int n = (quant == Q4_0 ? 20 : 17) * experts / 2;
-    return n > 16 ? n : 16;
-}
+// Most columns of a prompt that the streaming kernels take. The line lies where the CTA-pair kernels overtake them (E = 128,
+// I = 768, us from the host, streaming and pairs): Q4_0 7.2 columns an expert 132 and 144, 8.1 columns 147 and 146; Q8_0,
+// whose rows cost twice the bytes, 7.2 columns 162 and 174, 8.1 columns 175 and 176, 9 columns 197 and 184; a lone expert of
+// 2048 x 512 with 8 columns 35 and 36, with 12 columns 38 and 35. The same line for an expert-parallel call, whose results
+// are one GPU's to the bit (its one-CTA tiles would overtake later, Q4_0 at 12 columns).
+inline int stream_max_columns(int quant, int experts) { return (quant == Q4_0 ? 16 : 17) * experts / 2; }
 // gate/up of a decode batch, expert products of short prompts (stream.cu)
 cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st);
 cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_up, cudaStream_t st);

@@ -686,33 +686,33 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
         __syncwarp();
     } else if (warp == R::mma) {
         // -------------------------------- MMA ---------------------------------
-        if (rank == 0) {
-            // (one warp in order: every instruction of a pass counts. Votes keep what the MMA operands are made of uniform)
+        if (rank == 0 && elect_one()) {
+            // (one thread in order: every instruction of a pass counts)
             const uint32_t a_base = (stage0 >> 4) & 0x3FFFu, b_base = ((stage0 + STAGES * STAGE_BYTES) >> 4) & 0x3FFFu;
             const uint32_t full0 = smem_u32(&full_bar[0]), done0 = smem_u32(&done_bar[0]);
             int tl = 0, tn = 0;
             uint32_t v = 0, u = 0, n = 0;  // accumulator sets, passes, stages so far
             bool ok = true, ready = false;  // ready: the next pass's operands are known to be there
             int4 tile;
-            for (; ok && take_tile(true, tn, tile); ++tl) {
-                const uint32_t wide = (!NARROW && __any_sync(0xffffffffu, tile.z > 256)) ? 1u : 0u;
-                const uint32_t id0 = idesc2(32 * __popc(__ballot_sync(0xffffffffu, lane < set_cols(tile.z, 0) / 32)));
-                const uint32_t id1 = idesc2(32 * max(1, __popc(__ballot_sync(0xffffffffu, lane < set_cols(tile.z, 1) / 32))));
+            for (; ok && take_tile(false, tn, tile); ++tl) {
+                const uint32_t wide = (!NARROW && (tile.z > 256)) ? 1u : 0u;
+                const uint32_t id0 = idesc2(set_cols(tile.z, 0));
+                const uint32_t id1 = idesc2(max(32, set_cols(tile.z, 1)));
                 const uint32_t passes = (uint32_t)kgs << wide;
-                const uint32_t go = (!NARROW && kgs >= 12 && __any_sync(0xffffffffu, tile.z > 128)) ? (uint32_t)(kgs / 2 - 2) << wide : 0u;
+                const uint32_t go = (!NARROW && kgs >= 12 && (tile.z > 128)) ? (uint32_t)(kgs / 2 - 2) << wide : 0u;
                 // The sets of a wide tile take turns, so that the first one is complete, and its epilogue under way, while the
                 // second one's last products run, and the next tile's first products run under the second one's epilogue.
                 for (uint32_t p = 0; p < passes; ++p, ++u) {
                     const uint32_t h = p & wide, set = (v + h) & 1, c = u % UNITS;
-                    if (p == go && lane == 0) mbar_arrive(smem_u32(&go_bar[tl % ahead]));
+                    if (p == go) mbar_arrive(smem_u32(&go_bar[tl % ahead]));
                     if (p <= wide) ok = mbar_wait(smem_u32(&acc_empty_bar[set]), (((v + h) >> 1) & 1) ^ 1, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok && (ready || mbar_wait(full0 + c * 8, (u / UNITS) & 1, abort_flag)));
+                    ok = (ok && (ready || mbar_wait(full0 + c * 8, (u / UNITS) & 1, abort_flag)));
                     if (!ok) break;
                     ready = mbar_test(full0 + ((u + 1) % UNITS) * 8, ((u + 1) / UNITS) & 1);  // (its answer comes under the products' issue)
                     tc_fence_after();
                     const uint32_t w_lo = a_base + (n % STAGES) * (STAGE_BYTES >> 4), c_lo = b_base + c * (UNIT_BYTES >> 4);
                     const uint32_t acc = tmem_base + set * 256, id = h ? id1 : id0;
-                    if (elect_one()) {
+                    {
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
                             const uint32_t ow = (j >> 2) * (SUB_BYTES >> 4) + (j & 3) * 2, oc = (j >> 2) * (F::atom_bytes >> 4) + (j & 3) * 2;
@@ -721,7 +721,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                         umma2_commit(done0 + c * 8);
                         if (p + 1 + wide >= passes) umma2_commit(smem_u32(&acc_full_bar[set]));
                     }
-                    __syncwarp();
                     n += (h == wide);
                 }
                 if (!ok) break;
@@ -729,8 +728,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
             }
             if (*abort_flag.flag) {
                 // what has been issued reads both CTAs' shared memory: it ends before either goes away
-                if (elect_one()) umma2_commit(smem_u32(&drain_bar));
-                __syncwarp();
+                umma2_commit(smem_u32(&drain_bar));
                 let_land(smem_u32(&drain_bar), 1, 1);
             }
         }
