@@ -142,9 +142,9 @@ __device__ __forceinline__ void raise_status(int32_t* status, int32_t* status_ho
 // Sum of squares of a row and its RMSNorm scale by a CTA of 256 threads, each with chunks of inputs 4t.. and 16+4t.. of
 // 32-blocks: one order of summation for the norm alone and for the norm fused with what follows it.
 __device__ __forceinline__ float norm_sq_chunk(float ss, const float4& p, const float4& q) {
-    ss += p.x * p.x + p.y * p.y + p.z * p.z + p.w * p.w;
-    ss += q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
-    return ss;
+    // (written out: left to the compiler, the contractions differ from kernel to kernel)
+    auto sq4 = [](const float4& v) { return __fmaf_rn(v.w, v.w, __fmaf_rn(v.z, v.z, __fmaf_rn(v.y, v.y, __fmul_rn(v.x, v.x)))); };
+    return __fadd_rn(__fadd_rn(ss, sq4(p)), sq4(q));
 }
 __device__ __forceinline__ float norm_scale(float ss, float* red8, int H, float eps) {
 #pragma unroll
@@ -223,7 +223,7 @@ struct PrefillArgs {
     const float* logits_override;
     int T, K, gating;
     // scratch
-    int32_t* blk_hist;      // [nchunks, E]
+    int32_t* blk_hist;      // [E, nchunks], then [E] totals
     __half* w16;            // [2, E, H] router weight split into f16 high and low planes (per call, when the layer has none)
     __half* xr16;           // [2, T, H] activations split into f16 high and low planes (tcgen05 router)
     float* rpart;           // [ksplit, T, E] partial logits of the tcgen05 router

@@ -7,13 +7,13 @@
 //                               (moe_router_logits_batched, cuda/shaders/moe_grouped.cu:79)
 //   topk_large_kernel           one warp per token (router.cuh)
 //   route_single_kernel         contexts of one expert: everything up to the plan in one pass
-//   sort_one_kernel (up to 2048 pairs), sort_hist / sort_rowscan / sort_scan / sort_place
+//   sort_one_kernel (up to 2048 pairs), sort_hist / sort_rowscan / sort_place
 //                               stable counting sort of (token, slot) pairs by
 //                               expert, tokens ascending then slots ascending:
 //                               expert_bounds, col_expert, col_src_tok, dst_to_col
-//                               exactly as cuda/moe.rs:2115-2147; sort_scan also
-//                               emits the list of experts with work and the tile
-//                               lists of the grouped GEMMs (cuda/moe.rs:2188-2207).
+//                               exactly as cuda/moe.rs:2115-2147; and
+//                               the list of experts with work and the tile lists
+//                               of the grouped GEMMs (cuda/moe.rs:2188-2207).
 //   scatter_accum_kernel        out[t] = residual[t] + sum_slot w[t,slot] * D[dst_to_col[t,slot]]
 //                               in slot order (moe_grouped_scatter_accum_q8_0,
 //                               cuda/shaders/moe_grouped.cu:493-517).
@@ -329,14 +329,14 @@ sort_hist_kernel(const uint32_t* __restrict__ ids, int T, int K, int E, int32_t*
     const int n = min(SORT_TOK, T - t0) * K;
     for (int p = tid; p < n; p += 256) atomicAdd(&h[ids[(size_t)t0 * K + p]], 1);
     __syncthreads();
-    // layout [expert][chunk]: a warp of sort_scan then scans one expert's row with coalesced loads
+    // layout [expert][chunk]: a warp of sort_rowscan then scans one expert's row with coalesced loads
     for (int e = tid; e < E; e += 256) blk_hist[(size_t)e * gridDim.x + blockIdx.x] = h[e];
 }
 
 // One warp per expert: exclusive scan over the chunk counts of the expert's row (in place);
-// the row total goes to expert_bounds[e] for sort_scan_kernel.
+// the row total goes behind the rows.
 __global__ void __launch_bounds__(32)
-sort_rowscan_kernel(int32_t* __restrict__ blk_hist, int nchunks, RouteDev R) {
+sort_rowscan_kernel(int32_t* __restrict__ blk_hist, int nchunks) {
     grid_dep_sync();
     const int e = blockIdx.x, lane = threadIdx.x;
     int32_t* rowp = blk_hist + (size_t)e * nchunks;
@@ -361,7 +361,7 @@ sort_rowscan_kernel(int32_t* __restrict__ blk_hist, int nchunks, RouteDev R) {
             run += __shfl_sync(0xffffffffu, inc, 31);
         }
     }
-    if (lane == 0) R.expert_bounds[e] = run;
+    if (lane == 0) blk_hist[(size_t)gridDim.x * nchunks + e] = run;
 }
 
 // What the plan of a call consists of besides the sorted pairs: expert segment bounds and the tile
@@ -491,7 +491,7 @@ __device__ __forceinline__ void emit_plan(const PlanArgs& a, const RouteDev& R, 
     }
 }
 
-// One CTA: the plan from the row totals that sort_rowscan_kernel (or an expert-parallel plan) left in expert_bounds.
+// One CTA: the plan of an expert-parallel call, from the totals left in expert_bounds.
 __global__ void __launch_bounds__(PLAN_THREADS)
 sort_scan_kernel(const __grid_constant__ PlanArgs a, RouteDev R) {
     grid_dep_sync();
@@ -656,16 +656,48 @@ bool route_single_applicable(const PrefillArgs& a) {
 // a time in order; lanes holding the same expert find each other with match.any, the
 // position inside the expert's segment is the expert's running cursor plus the number
 // of lower lanes with the same expert, so the placement is stable.
-__global__ void __launch_bounds__(256)
-sort_place_kernel(const uint32_t* __restrict__ ids, int T, int K, int E, const int32_t* __restrict__ blk_hist,
-                  int nchunks, RouteDev R) {
+// The segment bounds are a scan of the row totals, which every CTA does for itself, so that the plan (the last CTA) is made beside the
+// placement and not in front of it.
+constexpr int PLACE_CHUNKS = PLAN_THREADS / 32;
+__global__ void __launch_bounds__(PLAN_THREADS)
+sort_place_kernel(const uint32_t* __restrict__ ids, int T, int K, const int32_t* __restrict__ blk_hist, int nchunks, RouteDev R,
+                  const __grid_constant__ PlanArgs plan) {
+    extern __shared__ int cursor[];  // [PLACE_CHUNKS][E]
+    __shared__ int cnt_s[MAX_EXPERTS], bounds_s[MAX_EXPERTS], wsum_s[MAX_EXPERTS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, E = plan.E;
     grid_dep_sync();
-    __shared__ int cursor[8][MAX_EXPERTS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int chunk = blockIdx.x * 8 + warp;
+    int x = 0, inc = 0;
+    if (tid < MAX_EXPERTS) {
+        x = (tid < E) ? blk_hist[(size_t)E * nchunks + tid] : 0;
+        cnt_s[tid] = x;
+    }
+    if (blockIdx.x == gridDim.x - 1) {
+        __syncthreads();
+        emit_plan(plan, R, cnt_s, bounds_s);
+        return;
+    }
+    if (tid < MAX_EXPERTS) {
+        inc = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int w = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += w;
+        }
+        if (lane == 31) wsum_s[warp] = inc;
+    }
+    const int chunk = blockIdx.x * PLACE_CHUNKS + warp;
+    int* cur = cursor + warp * E;
+    if (chunk < nchunks)
+        for (int e = lane; e < E; e += 32) cur[e] = blk_hist[(size_t)e * nchunks + chunk];
+    __syncthreads();
+    if (tid < MAX_EXPERTS) {
+        int base = 0;
+#pragma unroll
+        for (int w = 0; w < MAX_EXPERTS / 32; ++w) base += (w < warp) ? wsum_s[w] : 0;
+        bounds_s[tid] = base + inc - x;
+    }
+    __syncthreads();
     if (chunk >= nchunks) return;
-    for (int e = lane; e < E; e += 32) cursor[warp][e] = R.expert_bounds[e] + blk_hist[(size_t)e * nchunks + chunk];
-    __syncwarp();
     const int t0 = chunk * SORT_TOK;
     const int n = min(SORT_TOK, T - t0) * K;
     for (int p0 = 0; p0 < n; p0 += 32) {
@@ -673,15 +705,15 @@ sort_place_kernel(const uint32_t* __restrict__ ids, int T, int K, int E, const i
         const bool valid = p < n;
         const int e = valid ? (int)ids[(size_t)t0 * K + p] : -1 - lane;  // invalid lanes match nobody
         const unsigned int same = __match_any_sync(0xffffffffu, e);
+        const int rank = __popc(same & ((1u << lane) - 1u));
         if (valid) {
-            const int rank = __popc(same & ((1u << lane) - 1u));
-            const int col = cursor[warp][e] + rank;
+            const int col = bounds_s[e] + cur[e] + rank;
             R.col_expert[col] = e;
             R.col_src_tok[col] = t0 + p / K;
             R.dst_to_col[(size_t)t0 * K + p] = col;
         }
         __syncwarp();
-        if (valid && (same & ((1u << lane) - 1u)) == 0u) cursor[warp][e] += __popc(same);  // one leader per expert
+        if (valid && rank == 0) cur[e] += __popc(same);  // one leader per expert
         __syncwarp();
     }
 }
@@ -942,16 +974,15 @@ cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st) {
     }
     const int nchunks = (T + SORT_TOK - 1) / SORT_TOK;
     const bool one_cta = T * K <= SORT1_MAX;
-    count_launch(one_cta ? 2 : 4);
+    count_launch(one_cta ? 2 : 3);
     if (a.ids_in == nullptr)
         CUDA_RET(launch_topk(a, lg, nparts, one_cta ? nullptr : a.blk_hist, st));
     else if (!one_cta)
         CUDA_RET(launch_dep(sort_hist_kernel, dim3(nchunks), dim3(256), 0, st, a.R.ids, T, K, E, a.blk_hist));
     if (one_cta) return launch_dep(sort_one_kernel, dim3(1), dim3(SORT1_WARPS * 32), 0, st, a.R.ids, C, K, a.R, plan);
-    CUDA_RET(launch_dep(sort_rowscan_kernel, dim3(E), dim3(32), 0, st, a.blk_hist, nchunks, a.R));
-    CUDA_RET(launch_dep(sort_scan_kernel, dim3(1), dim3(PLAN_THREADS), 0, st, plan, a.R));
-    return launch_dep(sort_place_kernel, dim3((nchunks + 7) / 8), dim3(256), 0, st, a.R.ids, T, K, E, a.blk_hist, nchunks,
-                      a.R);
+    CUDA_RET(launch_dep(sort_rowscan_kernel, dim3(E), dim3(32), 0, st, a.blk_hist, nchunks));
+    return launch_dep(sort_place_kernel, dim3((nchunks + PLACE_CHUNKS - 1) / PLACE_CHUNKS + 1), dim3(PLAN_THREADS), (size_t)PLACE_CHUNKS * E * 4, st, a.R.ids, T,
+                      K, a.blk_hist, nchunks, a.R, plan);
 }
 
 cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_cap, int gu_cols, int4* tiles,

@@ -28,12 +28,12 @@ namespace rtc {
 
 using namespace tc;
 
-// Tokens per tile: 128, or 32 for batches whose 128-token tiles would leave most of the chip idle. A logit is
-// the same in both: the tile width only says how many columns one MMA covers. (77 tokens: 11 -> 6 us,
-// with the set-up and the first weight boxes moved ahead of the wait for the kernel before.)
+// Tokens per tile: 32, 64, 128 or 256, whichever moves the fewest bytes through its waves of CTAs (every tile reads the weight
+// planes of its k range). A logit is the same in all of them: the tile width only says how many columns one MMA covers.
+// (77 tokens: 11 us with 128, 6 with 32, the set-up and the first weight boxes ahead of the wait for the kernel before.)
 template <int BN>
 struct Cfg {
-    static constexpr int STAGES = (BN == 128) ? 3 : 5;
+    static constexpr int STAGES = (BN == 256) ? 2 : (BN == 128) ? 3 : (BN == 64) ? 4 : 5;
     static constexpr int X_BYTES = BN * 128;                           // [BN rows x 64 k] f16
     static constexpr int STAGE_BYTES = 2 * SUB_BYTES + 2 * X_BYTES;    // W_hi | W_lo ([128 rows x 64 k] each) | x_hi | x_lo
 };
@@ -261,26 +261,33 @@ split_x16_kernel(const XT* __restrict__ x, size_t n8, const PlaneOut o) {
 // CTA per row, the row held in registers (H <= 8192). The squares are summed in the order of rmsnorm_kernel. At 8192
 // tokens, H = 2048: 72 us as two kernels with the f32 result in between, 26 us (bytes: 128 MB, 20 us at the copy peak).
 constexpr int NORM_MAX_CHUNKS = 4;
-template <int NCH>  // NCH * 2048 >= H
+template <int NCH, int ROWS>  // NCH * 2048 >= H
 __global__ void __launch_bounds__(256)
-norm_split_kernel(const float* __restrict__ x, const float* __restrict__ gamma, float eps, int H, const PlaneOut o) {
+norm_split_kernel(const float* __restrict__ x, const float* __restrict__ gamma, float eps, int T, int H, const PlaneOut o) {
     grid_dep_sync();
-    __shared__ float red[8];
-    const int t = blockIdx.x, tid = threadIdx.x, n8 = H >> 3;
-    const float* xr = x + (size_t)t * H;
-    float4 p[NCH], q[NCH];
-    float ss = 0.0f;
+    __shared__ float red[ROWS][8];
+    const int t0 = blockIdx.x * ROWS, tid = threadIdx.x, n8 = H >> 3;
+    float4 p[ROWS][NCH], q[ROWS][NCH];
 #pragma unroll
-    for (int j = 0; j < NCH; ++j) {
-        const int i = tid + j * 256;
-        if (i < n8) {
-            const int oa = (i >> 2) * 32 + (i & 3) * 4;
-            p[j] = *reinterpret_cast<const float4*>(xr + oa);
-            q[j] = *reinterpret_cast<const float4*>(xr + oa + 16);
-            ss = norm_sq_chunk(ss, p[j], q[j]);
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int j = 0; j < NCH; ++j) {
+            const int i = tid + j * 256;
+            if (i < n8) {
+                const float* xr = x + (size_t)min(t0 + r, T - 1) * H + (i >> 2) * 32 + (i & 3) * 4;
+                p[r][j] = *reinterpret_cast<const float4*>(xr);
+                q[r][j] = *reinterpret_cast<const float4*>(xr + 16);
+            }
         }
+    float sc[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        float ss = 0.0f;
+#pragma unroll
+        for (int j = 0; j < NCH; ++j)
+            if (tid + j * 256 < n8) ss = norm_sq_chunk(ss, p[r][j], q[r][j]);
+        sc[r] = norm_scale(ss, red[r], H, eps);
     }
-    const float sc = norm_scale(ss, red, H, eps);
     unsigned nz = 0u;
 #pragma unroll
     for (int j = 0; j < NCH; ++j) {
@@ -288,9 +295,16 @@ norm_split_kernel(const float* __restrict__ x, const float* __restrict__ gamma, 
         if (i < n8) {
             const int oa = (i >> 2) * 32 + (i & 3) * 4;
             const float4 g = __ldg(reinterpret_cast<const float4*>(gamma + oa)), h = __ldg(reinterpret_cast<const float4*>(gamma + oa + 16));
-            const float4 np = make_float4(p[j].x * sc * g.x, p[j].y * sc * g.y, p[j].z * sc * g.z, p[j].w * sc * g.w);
-            const float4 nq = make_float4(q[j].x * sc * h.x, q[j].y * sc * h.y, q[j].z * sc * h.z, q[j].w * sc * h.w);
-            nz |= store_planes(o, (size_t)t * n8 + i, np, nq);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                // (rounded products: contracted into the subtraction of the high part they would not be the norm's outputs)
+                auto normed = [&](const float4& v, const float4& w) {
+                    return make_float4(__fmul_rn(__fmul_rn(v.x, sc[r]), w.x), __fmul_rn(__fmul_rn(v.y, sc[r]), w.y),
+                                       __fmul_rn(__fmul_rn(v.z, sc[r]), w.z), __fmul_rn(__fmul_rn(v.w, sc[r]), w.w));
+                };
+                const float4 np = normed(p[r][j], g), nq = normed(q[r][j], h);
+                if (t0 + r < T) nz |= store_planes(o, (size_t)(t0 + r) * n8 + i, np, nq);
+            }
         }
     }
     note_low_parts(o, nz);
@@ -349,8 +363,13 @@ cudaError_t launch_norm_split(const float* x, const float* gamma, float eps, int
                               cudaStream_t st) {
     const rtc::PlaneOut o{x16, (size_t)T * H, any_lo, natural};
     count_launch();
-    auto kern = H <= 2048 ? rtc::norm_split_kernel<1> : H <= 4096 ? rtc::norm_split_kernel<2> : rtc::norm_split_kernel<rtc::NORM_MAX_CHUNKS>;
-    return launch_dep(kern, dim3(T), dim3(256), 0, st, x, gamma, eps, H, o);
+    // (two rows a CTA where the batch fills the chip: twice the loads in flight)
+    const int rows = (H <= 2048 && T >= 4096) ? 2 : 1;
+    auto kern = rows == 2 ? rtc::norm_split_kernel<1, 2>
+                : H <= 2048 ? rtc::norm_split_kernel<1, 1>
+                : H <= 4096 ? rtc::norm_split_kernel<2, 1>
+                            : rtc::norm_split_kernel<rtc::NORM_MAX_CHUNKS, 1>;
+    return launch_dep(kern, dim3((T + rows - 1) / rows), dim3(256), 0, st, x, gamma, eps, T, H, o);
 }
 
 template <int BN>
@@ -372,8 +391,17 @@ cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int 
     a.m_tiles = (E + 127) / 128;
     cudaError_t e = make_tmap_f16(w16, (uint64_t)2 * E, (uint64_t)H, 128, &a.tmap_w);
     if (e != cudaSuccess) return e;
-    const bool narrow = (T + 127) / 128 * a.m_tiles * ksplit < sms / 2;  // tiles of 128 tokens would leave half of the SMs idle
-    const int bn = narrow ? 32 : 128;
+    // bytes of a CTA's stage (weights + activations) times the waves of CTAs: 1777 tokens of 128 experts take one wave of tiles
+    // of 64 tokens (two of 32: 15.2 -> 10.3 us), 8192 tokens one of 256 (two of 128: 28.8 -> 28.3 us)
+    int bn = 32;
+    long long least = 0;
+    for (int b = 32; b <= 256; b *= 2) {
+        const long long ctas = (long long)((T + b - 1) / b) * a.m_tiles * ksplit, cost = (ctas + sms - 1) / sms * (2 * tc::SUB_BYTES + 2 * b * 128);
+        if (b == 32 || cost < least) {
+            least = cost;
+            bn = b;
+        }
+    }
     e = make_tmap_f16(x16, (uint64_t)2 * T, (uint64_t)H, bn, &a.tmap_x);
     if (e != cudaSuccess) return e;
     a.part = part;
@@ -385,7 +413,7 @@ cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int 
     a.E = E;
     a.H = H;
     a.ksplit = ksplit;
-    return narrow ? launch_rtc<32>(a, st) : launch_rtc<128>(a, st);
+    return bn == 32 ? launch_rtc<32>(a, st) : bn == 64 ? launch_rtc<64>(a, st) : bn == 128 ? launch_rtc<128>(a, st) : launch_rtc<256>(a, st);
 }
 
 }  // namespace lumen
