@@ -36,35 +36,30 @@ using namespace dcommon;
 
 enum Mode { GATE_UP_1, DOWN_1, GATE_UP_2, DOWN_2, DOWN_2I };
 
-// warps per SM and groups in flight per warp: 131..147 KB on the way per SM (the copy peak times the latency is
-// ~55 KB), the rest of the 256 KB is L1 for the activations
-template <int Q>
-struct Cfg;
-template <>
-struct Cfg<Q4_0> {
-    static constexpr int WARPS = 16, RING_GU = 4, RING_DN = 8;
-};
-template <>
-struct Cfg<Q8_0> {
-    static constexpr int WARPS = 16, RING_GU = 2, RING_DN = 4;
-};
-template <>
-struct Cfg<BF16> {
-    static constexpr int WARPS = 8, RING_GU = 2, RING_DN = 4;
-};
-
-template <int Q, int MODE>
+// Warps per SM and groups in flight per warp: 131..221 KB on the way per SM (the copy peak times the latency is ~55 KB),
+// the rest of the 256 KB is L1 for the activations. An item is a chain (its chunk, its columns, its tiles, its rows out), and
+// the warps of an SM end unevenly; more warps with shorter rings help the down products, whose items are short (16 warps ->
+// now, us a call: 4 tokens of Q8_0, 1408 inputs, 53.1 -> 50.2; 8 tokens of Q4_0, 512 inputs, 40.8 -> 39.1; prompt of 77
+// tokens 124 -> 121.5; with 32 warps 16 tokens of Q4_0 61.7 -> 66.4), not gate/up, which needs the registers (Q8_0 with 20
+// warps: 13 tokens, H = 4096, 190 -> 194).
+template <int Q, int MODE, int WARPS>
 struct Shape {
     static constexpr bool down = (MODE == DOWN_1 || MODE == DOWN_2 || MODE == DOWN_2I), int8 = (MODE == DOWN_2I);
     static constexpr int terms = (MODE == GATE_UP_1 || MODE == DOWN_1) ? 1 : 2;
     static constexpr int nm = down ? 1 : 2;  // matrices of an item: down | gate and up
     static constexpr int grp = (Q == Q4_0) ? 2 : 1;  // 128-input groups of a ring slot
-    static constexpr int warps = Cfg<Q>::WARPS, ring = (down ? Cfg<Q>::RING_DN : Cfg<Q>::RING_GU) / grp;
+    static constexpr int warps = WARPS, ring = (down ? (Q == Q4_0 ? 6 : Q == Q8_0 ? 3 : 4) : (Q == Q4_0 ? 4 : 2)) / grp;
     static constexpr uint32_t q_bytes = QTraits<Q>::NQ * 512, s_bytes = (Q == BF16 ? 0 : 128);  // of a tile: quants, scales
     static constexpr uint32_t tile = grp * (q_bytes + s_bytes);
     static constexpr uint32_t slot = nm * tile;
     static constexpr size_t smem = (size_t)warps * ring * slot;
 };
+template <int Q, int MODE>
+constexpr int default_warps() {
+    if (MODE == DOWN_1) return 24;
+    if (MODE == DOWN_2 || MODE == DOWN_2I) return Q == BF16 ? 12 : 20;
+    return Q == BF16 ? 8 : 16;
+}
 
 struct Args {
     LayerDev L;
@@ -144,12 +139,12 @@ __device__ __forceinline__ int perm32(int e) {
     return t * 8 + ((m & 1) ? 4 : 0) + (hi ? 2 : 0) + ((m >> 1) & 1);
 }
 
-template <int Q, int MODE>
-__global__ void __launch_bounds__(Cfg<Q>::WARPS * 32, 1)
+template <int Q, int MODE, int WARPS = default_warps<Q, MODE>()>
+__global__ void __launch_bounds__(WARPS * 32, 1)
 stream_kernel(const __grid_constant__ Args a) {
-    using S = Shape<Q, MODE>;
+    using S = Shape<Q, MODE, WARPS>;
     constexpr bool DOWN = S::down, I8 = S::int8;
-    constexpr int WARPS = S::warps, RING = S::ring, NM = S::nm, TERMS = S::terms, NQ = QTraits<Q>::NQ, GRP = S::grp;
+    constexpr int RING = S::ring, NM = S::nm, TERMS = S::terms, NQ = QTraits<Q>::NQ, GRP = S::grp;
     static_assert(!I8 || Q == Q4_0, "the integer form is for Q4_0 nibbles");
     static_assert(Q != BF16 || TERMS == 2, "prompts of BF16 layers take the tcgen05 kernels");
     extern __shared__ __align__(128) uint8_t ring_smem[];  // [WARPS][RING][NM][quants of GRP groups | their scales]
@@ -179,6 +174,15 @@ stream_kernel(const __grid_constant__ Args a) {
         i1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
     }
 
+    // Warps that take part: for Q4_0, and for the down product of BF16, as many as give each the same number of items, so that
+    // the last round is as full as the others (a prompt of 30 tokens 104 -> 100 us). Not for the other heavy tiles,
+    // of which a warp less on the way costs more than the uneven round (90 tokens of Q8_0 155 -> 163).
+    int nw = WARPS;
+    if ((Q == Q4_0 || (Q == BF16 && DOWN)) && i1 > i0) {
+        const int n = i1 - i0, rounds = (n + WARPS - 1) / WARPS;
+        nw = (n + rounds - 1) / rounds;
+        if (warp >= nw) i1 = i0;
+    }
     // request cursor: the next groups (of item pi, from group pkg on) to copy, into ring slot wslot
     int pi = i0 + warp, pkg = 0, wslot = 0, rslot = 0;
     uint32_t rphase = 0;
@@ -215,7 +219,7 @@ stream_kernel(const __grid_constant__ Args a) {
         if (++wslot == RING) wslot = 0;
         if ((pkg += GRP) >= kg_n) {
             pkg = 0;
-            pi += WARPS;
+            pi += nw;
         }
     };
     if (a.debug_extra_tx != 0 && warp == 0) {
@@ -412,7 +416,7 @@ stream_kernel(const __grid_constant__ Args a) {
             }
         }
     };
-    for (int i = i0 + warp; i < i1; i += WARPS) {
+    for (int i = i0 + warp; i < i1; i += nw) {
         const int c = i / rt_n;
         const int4 ch = __ldg(&a.chunks[c * a.chunk_stride]);
         const int rt = i - c * rt_n;
@@ -464,17 +468,19 @@ combine_f32_kernel(const float* __restrict__ d32, RouteDev R, const float* resid
 }
 
 // chained: the kernel in front in the stream waits for the routing kernels before it lets this one start (see above)
-template <int Q, int MODE>
+template <int Q, int MODE, int WARPS = default_warps<Q, MODE>()>
 cudaError_t launch_t(const Args& a, int sms, cudaStream_t st, bool chained = true) {
+    auto* kern = stream_kernel<Q, MODE, WARPS>;
+    constexpr size_t smem = Shape<Q, MODE, WARPS>::smem;
     static SmemOptIn optin;
-    const cudaError_t e = ensure_dyn_smem(stream_kernel<Q, MODE>, Shape<Q, MODE>::smem, optin);
+    const cudaError_t e = ensure_dyn_smem(kern, smem, optin);
     if (e != cudaSuccess) return e;
     count_launch();
     if (!chained) {
-        stream_kernel<Q, MODE><<<sms, Cfg<Q>::WARPS * 32, Shape<Q, MODE>::smem, st>>>(a);
+        kern<<<sms, WARPS * 32, smem, st>>>(a);
         return cudaGetLastError();
     }
-    return launch_dep(stream_kernel<Q, MODE>, dim3(sms), dim3(Cfg<Q>::WARPS * 32), Shape<Q, MODE>::smem, st, a);
+    return launch_dep(kern, dim3(sms), dim3(WARPS * 32), smem, st, a);
 }
 
 template <int MODE>
@@ -513,6 +519,9 @@ cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st) {
     g.b_row = (size_t)p.L.kg_h * 16;
     g.sf = p.sf;
     g.debug_extra_tx = p.debug_expire;
+    // BF16: two warps more while the activations still fit into the L1 that their rings leave (H = 2048: 5 tokens 56.9 -> 53.3 us,
+    // 8 tokens 77.4 -> 80.4)
+    if (p.L.quant == BF16 && (size_t)p.T * p.L.kg_h * 512 <= 48 * 1024) return stream::launch_t<BF16, stream::GATE_UP_2, 10>(g, p.sms, st);
     return stream::launch_q<stream::GATE_UP_2>(g, p.sms, st);
 }
 
@@ -524,8 +533,12 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_u
     d.b_row = (size_t)p.L.kg_i * 16;
     d.d32 = p.d32;
     d.debug_extra_tx = int8 ? p.debug_expire : 0;  // (the chain's first streaming kernel)
-    const cudaError_t e = int8 ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st, after_gate_up)
-                               : stream::launch_q<stream::DOWN_2>(d, p.sms, st, after_gate_up);
+    // BF16: the longer rings of twelve warps leave little L1 for the SwiGLU fragments (12 tokens, H = 4096, I = 1536: 279 us with eight
+    // warps, 285 with twelve; 3 tokens 120 and 116)
+    const bool wide_fragments = p.L.quant == BF16 && (size_t)p.T * p.K * p.L.kg_i * 512 > 256 * 1024;
+    const cudaError_t e = int8             ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st, after_gate_up)
+                          : wide_fragments ? stream::launch_t<BF16, stream::DOWN_2, 8>(d, p.sms, st, after_gate_up)
+                                           : stream::launch_q<stream::DOWN_2>(d, p.sms, st, after_gate_up);
     if (e != cudaSuccess) return e;
     count_launch();
     // (H is a multiple of 32, so every row lies on the boundary that the first one does)
