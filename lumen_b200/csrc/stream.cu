@@ -38,17 +38,16 @@ enum Mode { GATE_UP_1, DOWN_1, GATE_UP_2, DOWN_2, DOWN_2I };
 
 // Warps per SM and groups in flight per warp: 131..221 KB on the way per SM (the copy peak times the latency is ~55 KB),
 // the rest of the 256 KB is L1 for the activations. An item is a chain (its chunk, its columns, its tiles, its rows out), and
-// the warps of an SM end unevenly; more warps with shorter rings help the down products, whose items are short (16 warps ->
-// now, us a call: 4 tokens of Q8_0, 1408 inputs, 53.1 -> 50.2; 8 tokens of Q4_0, 512 inputs, 40.8 -> 39.1; prompt of 77
-// tokens 124 -> 121.5; with 32 warps 16 tokens of Q4_0 61.7 -> 66.4), not gate/up, which needs the registers (Q8_0 with 20
-// warps: 13 tokens, H = 4096, 190 -> 194).
+// the warps of an SM end unevenly; more warps with shorter rings help the decode down products, whose items are short (16 warps
+// -> now, us a call: 4 tokens of Q8_0, 1408 inputs, 53.1 -> 50.2; 8 tokens of Q4_0, 512 inputs, 40.8 -> 39.1; with 32 warps
+// 16 tokens of Q4_0 61.7 -> 66.4), not gate/up, which needs the registers (Q8_0 with 20 warps: 13 tokens, H = 4096, 190 -> 194).
 template <int Q, int MODE, int WARPS>
 struct Shape {
     static constexpr bool down = (MODE == DOWN_1 || MODE == DOWN_2 || MODE == DOWN_2I), int8 = (MODE == DOWN_2I);
     static constexpr int terms = (MODE == GATE_UP_1 || MODE == DOWN_1) ? 1 : 2;
     static constexpr int nm = down ? 1 : 2;  // matrices of an item: down | gate and up
     static constexpr int grp = (Q == Q4_0) ? 2 : 1;  // 128-input groups of a ring slot
-    static constexpr int warps = WARPS, ring = (down ? (Q == Q4_0 ? 6 : Q == Q8_0 ? 3 : 4) : (Q == Q4_0 ? 4 : 2)) / grp;
+    static constexpr int warps = WARPS, ring = (!down ? (Q == Q4_0 ? 4 : 2) : warps > 16 ? (Q == Q4_0 ? 6 : 3) : (Q == Q4_0 ? 8 : 4)) / grp;
     static constexpr uint32_t q_bytes = QTraits<Q>::NQ * 512, s_bytes = (Q == BF16 ? 0 : 128);  // of a tile: quants, scales
     static constexpr uint32_t tile = grp * (q_bytes + s_bytes);
     static constexpr uint32_t slot = nm * tile;
@@ -56,7 +55,6 @@ struct Shape {
 };
 template <int Q, int MODE>
 constexpr int default_warps() {
-    if (MODE == DOWN_1) return 24;
     if (MODE == DOWN_2 || MODE == DOWN_2I) return Q == BF16 ? 12 : 20;
     return Q == BF16 ? 8 : 16;
 }
@@ -174,11 +172,11 @@ stream_kernel(const __grid_constant__ Args a) {
         i1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
     }
 
-    // Warps that take part: for Q4_0, and for the down product of BF16, as many as give each the same number of items, so that
-    // the last round is as full as the others (a prompt of 30 tokens 104 -> 100 us). Not for the other heavy tiles,
-    // of which a warp less on the way costs more than the uneven round (90 tokens of Q8_0 155 -> 163).
+    // Warps that take part: in a decode batch of Q4_0, and in the down product of BF16, as many as give each the same number of
+    // items, so that the last round is as full as the others (16 tokens of Q4_0 61.1 -> 60.8 us, 2 tokens of BF16 41.4 -> 39.3).
+    // Elsewhere a warp less on the way costs more than the uneven round (90 tokens of Q8_0 155 -> 163, 110 of Q4_0 129 -> 132).
     int nw = WARPS;
-    if ((Q == Q4_0 || (Q == BF16 && DOWN)) && i1 > i0) {
+    if (((Q == Q4_0 && TERMS == 2) || (Q == BF16 && DOWN)) && i1 > i0) {
         const int n = i1 - i0, rounds = (n + WARPS - 1) / WARPS;
         nw = (n + rounds - 1) / rounds;
         if (warp >= nw) i1 = i0;
@@ -574,6 +572,8 @@ cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __hal
     d.out16 = out16_rows ? out16_rows : p.d16;
     d.out_row_map = out16_rows ? p.R.col_src_tok : nullptr;
     if (peer) d.peer = *peer;
+    // Q4_0: more warps once there are columns enough to keep them busy (E = 128: 77 tokens 125.8 -> 121.0 us, 18 tokens 83.3 and 85.5)
+    if (p.L.quant == Q4_0 && 2 * p.T * p.K > 5 * p.L.E) return stream::launch_t<Q4_0, stream::DOWN_1, 24>(d, p.sms, st);
     return stream::launch_q<stream::DOWN_1>(d, p.sms, st);
 }
 

@@ -117,6 +117,21 @@ def test_decode_chain_wide_layer(cuda_lib, quant, T):
     assert rel_l2((out - x).cpu().numpy(), o_out - x.cpu().numpy()) < TOL_REL_L2
 
 
+# BF16 batches: ten and eight gate/up warps, twelve and eight down warps (by what their activations leave of the L1)
+@pytest.mark.parametrize("H,I,T", [(2048, 512, 6), (2048, 512, 7), (512, 2048, 4), (512, 2048, 5)])
+def test_decode_chain_bf16_warp_rules(cuda_lib, H, I, T):
+    E, K = 16, 8 if H < I else 4
+    lay, meta, blob_np, sc, layer = make_layer(H, I, E, K, 2, seed=T)
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=g, device="cuda")
+    res = torch.randn((T, H), generator=g, device="cuda")
+    out = sc.decode(layer, x, res)
+    r = sc.get_routing(T)
+    o_out, _, _ = oracle.moe_layer(blob_np, 0, meta.expert_gate_offs, meta.expert_up_offs, meta.expert_down_offs, 2, H, I, E, K,
+                                   x.cpu().numpy(), res.cpu().numpy(), ids=r["ids"], weights=r["weights"], threads=8)
+    assert rel_l2((out - res).cpu().numpy(), o_out - res.cpu().numpy()) < TOL_REL_L2
+
+
 # the small router with one and with two rows of experts a warp, at widths with a remainder
 @pytest.mark.parametrize("E,H,T", [(256, 1024, 5), (256, 2080, 16), (128, 4096, 7), (8, 320, 16)])
 def test_small_router_rows(cuda_lib, E, H, T):
@@ -157,6 +172,35 @@ def test_router_tiles_of_32_and_128_tokens_agree(cuda_lib, E):
     for lo, hi in ((0, 31), (33, 98), (6000, 6100)):
         _, _, lg = sc.route_only(layer, x[lo:hi].contiguous(), want_logits=True)
         assert torch.equal(lg, big[lo:hi])
+
+
+# every width of a router tile (64, 128 and 256 tokens beside the 32 of a few rows)
+@pytest.mark.parametrize("E", [128, 256])
+def test_router_tiles_of_every_width_agree(cuda_lib, E):
+    H, T = 256, 4600
+    lay = synth.LayerLayout(H, 128, E, 1)
+    sc = moe.allocate_moe_scratch(H, 128, E, 8, T)
+    layer = sc.prepare_router_only(synth.make_layer_blob(lay, 9), lay.meta().router_weight_off)
+    x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(1), device="cuda")
+    parts = [sc.route_only(layer, x[t:t + 23].contiguous(), want_logits=True)[2].clone() for t in range(0, T, 23)]
+    ref = torch.cat(parts)
+    for n in (1000, 1700, 2300, T):
+        assert torch.equal(sc.route_only(layer, x[:n].contiguous(), want_logits=True)[2], ref[:n])
+
+
+# two rows a CTA: an odd number of them
+@pytest.mark.parametrize("H", [256, 2048])
+def test_norm_folded_into_the_planes_of_a_large_batch(cuda_lib, H):
+    T, E, K = 4097, 16, 2
+    lay = synth.LayerLayout(H, 128, E, 1)
+    sc = moe.allocate_moe_scratch(H, 128, E, K, T)
+    layer = sc.prepare_layer(synth.make_layer_blob(lay, 1), lay.meta())
+    g = torch.Generator("cuda").manual_seed(H)
+    gamma = 1 + 0.1 * torch.randn(H, generator=g, device="cuda")
+    x = torch.randn((T, H), generator=g, device="cuda")
+    y = sc.prefill(layer, moe.rmsnorm(x, gamma, 1e-6), x)
+    sc.stack_prefill([layer, layer], [gamma, gamma], x, 1e-6)
+    assert torch.equal(x, sc.prefill(layer, moe.rmsnorm(y, gamma, 1e-6), y))
 
 
 # the norm that is folded into the operand planes: one to four register chunks a row, whole and partial
