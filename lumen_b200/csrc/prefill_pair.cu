@@ -20,17 +20,22 @@
 //
 // One CTA pair per two SMs, persistent; tiles are claimed from a device-wide counter by the first CTA of the pair.
 // Warps of a CTA: 0-7 epilogue (16 of them for gate/up when the weights come by TMA), then 16 weight producers (with
-// TMA-fed weights a copy warp instead), two copy warps for the columns, one for each set, one warp for the MMAs (idle in the
+// TMA-fed weights a copy warp instead), two copy warps for the columns, every second unit each, one thread for the MMAs (idle in the
 // second CTA), one thread for the tiles (idle in the second CTA).
 //
 // Operands come through two rings: weights in stages of 128 rows x 128 inputs, columns in units of up to 128 rows x 128
-// inputs, of which a stage takes one per set. A pass multiplies one unit with its stage. What a pass costs the MMA warp
-// besides its products bounds narrow tiles, hence 128 inputs, ONE barrier to wait for (the unit's bytes and, in a stage's
+// inputs, of which a stage takes one per set. A pass multiplies one unit with its stage. What a pass costs the issuing thread
+// besides its products (~450 cycles, in order) bounds narrow tiles, hence 128 inputs, ONE barrier to wait for (the unit's bytes and, in a stage's
 // first pass, its weights) and ONE commit (unit free, and the stage with its last pass): with two barriers and two commits
 // for every 64 inputs a tile of 60 columns took ~1200 cycles a pass (1000 tokens, 279 us a call).
 // The columns of gate/up are gathered by the copies themselves (tile::gather4 on the token rows): the plane of the tokens
-// stays in L2, where the gathered rows (268 MB at 8192 tokens of 2048, K = 8, 54 us to write) did not. Every wait is bounded; on expiry the kernel raises the status word, lets its copies and
-// MMAs end, frees its TMEM and returns.
+// stays in L2, where the gathered rows (268 MB at 8192 tokens of 2048, K = 8, 54 us to write) did not.
+//
+// Measured against the one-CTA kernels, gate/up + down in a short run: 4096 Zipf-loaded tokens (H = 2048, I = 768, E = 128, K = 8, Q4_0)
+// 235 + 146 -> 200 + 115 us (1032 and 897 TFLOP/s, 0.64 and 0.56 of the measured burst peak), 8192 tokens 380 + 237 -> 321 + 184;
+// narrow tiles: 300 tokens, a whole call 192 -> 148 us.
+//
+// Every wait is bounded; on expiry the kernel raises the status word, lets its copies and MMAs end, frees its TMEM and returns.
 #include "mma_frag.cuh"
 #include "tc_common.cuh"
 
@@ -381,7 +386,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
     };
     // How many tiles are claimed ahead of the MMAs, and at which stage of a tile they allow the next claim. Long tiles:
     // one ahead, late in a wide tile so that the last tiles go to the pairs that are free first (before the producers need
-    // it: they hold up to `depth` groups and two stages beyond the MMAs), at the start of a narrow one, which
+    // it: they hold up to four groups and two stages beyond the MMAs), at the start of a narrow one, which
     // is over in about the time of a claim. Short ones: two ahead, so that the producers never run dry; four
     // where a tile is one group, because the producers' registers hold more than two of them.
     // (Narrow form: two more stages beyond the MMAs, passes of less than half the time.)

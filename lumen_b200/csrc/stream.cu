@@ -55,7 +55,7 @@ struct Shape {
 };
 template <int Q, int MODE>
 constexpr int default_warps() {
-    if (MODE == DOWN_2 || MODE == DOWN_2I) return Q == BF16 ? 12 : 20;
+    if (MODE == DOWN_2I) return 20;
     return Q == BF16 ? 8 : 16;
 }
 
@@ -172,11 +172,11 @@ stream_kernel(const __grid_constant__ Args a) {
         i1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
     }
 
-    // Warps that take part: in a decode batch of Q4_0, and in the down product of BF16, as many as give each the same number of
+    // Warps that take part: in a decode batch of Q4_0, and in the BF16 down product of twelve warps, as many as give each the same number of
     // items, so that the last round is as full as the others (16 tokens of Q4_0 61.1 -> 60.8 us, 2 tokens of BF16 41.4 -> 39.3).
     // Elsewhere a warp less on the way costs more than the uneven round (90 tokens of Q8_0 155 -> 163, 110 of Q4_0 129 -> 132).
     int nw = WARPS;
-    if (((Q == Q4_0 && TERMS == 2) || (Q == BF16 && DOWN)) && i1 > i0) {
+    if (((Q == Q4_0 && TERMS == 2) || (Q == BF16 && DOWN && WARPS > 8)) && i1 > i0) {
         const int n = i1 - i0, rounds = (n + WARPS - 1) / WARPS;
         nw = (n + rounds - 1) / rounds;
         if (warp >= nw) i1 = i0;
@@ -531,12 +531,17 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_u
     d.b_row = (size_t)p.L.kg_i * 16;
     d.d32 = p.d32;
     d.debug_extra_tx = int8 ? p.debug_expire : 0;  // (the chain's first streaming kernel)
-    // BF16: the longer rings of twelve warps leave little L1 for the SwiGLU fragments (12 tokens, H = 4096, I = 1536: 279 us with eight
-    // warps, 285 with twelve; 3 tokens 120 and 116)
-    const bool wide_fragments = p.L.quant == BF16 && (size_t)p.T * p.K * p.L.kg_i * 512 > 256 * 1024;
-    const cudaError_t e = int8             ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st, after_gate_up)
-                          : wide_fragments ? stream::launch_t<BF16, stream::DOWN_2, 8>(d, p.sms, st, after_gate_up)
-                                           : stream::launch_q<stream::DOWN_2>(d, p.sms, st, after_gate_up);
+    // More warps where an SM's items (at most: of every expert that T * K pairs can reach) are one to four rounds of the usual
+    // ones: below they idle, above the rounds even out by themselves (Q8_0, 16 and 20 warps: 21 items an SM 53.1 and 50.2 us, 35 items
+    // 50.0 and 49.0; 4 items 30.5 and 31.0, 110 items 189.3 and 189.6. BF16, 8 and 12: 35 items 54.3 and 53.3, 14 items 38.9 and
+    // 39.3). BF16: not either where their longer rings leave too little L1 for the SwiGLU fragments (12 tokens, H = 4096,
+    // I = 1536: 279 and 285 us).
+    const long long pairs_max = (long long)p.T * p.K, items = (pairs_max < p.L.E ? pairs_max : p.L.E) * p.L.rt_h;
+    const bool more = items > 16ll * p.sms && (p.L.quant == BF16 ? (size_t)pairs_max * p.L.kg_i * 512 <= 256 * 1024 : items <= 64ll * p.sms);
+    const cudaError_t e = int8                             ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st, after_gate_up)
+                          : more && p.L.quant == BF16      ? stream::launch_t<BF16, stream::DOWN_2, 12>(d, p.sms, st, after_gate_up)
+                          : more && p.L.quant == Q8_0      ? stream::launch_t<Q8_0, stream::DOWN_2, 20>(d, p.sms, st, after_gate_up)
+                                                           : stream::launch_q<stream::DOWN_2>(d, p.sms, st, after_gate_up);
     if (e != cudaSuccess) return e;
     count_launch();
     // (H is a multiple of 32, so every row lies on the boundary that the first one does)
