@@ -535,9 +535,9 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_u
     // ones: below they idle, above the rounds even out by themselves (Q8_0, 16 and 20 warps: 21 items an SM 53.1 and 50.2 us, 35 items
     // 50.0 and 49.0; 4 items 30.5 and 31.0, 110 items 189.3 and 189.6. BF16, 8 and 12: 35 items 54.3 and 53.3, 14 items 38.9 and
     // 39.3). BF16: not either where their longer rings leave too little L1 for the SwiGLU fragments (12 tokens, H = 4096,
-    // I = 1536: 279 and 285 us).
+    // I = 1536: 279 and 285 us; 16 tokens, I = 512: 120.7 and 121.9).
     const long long pairs_max = (long long)p.T * p.K, items = (pairs_max < p.L.E ? pairs_max : p.L.E) * p.L.rt_h;
-    const bool more = items > 16ll * p.sms && (p.L.quant == BF16 ? (size_t)pairs_max * p.L.kg_i * 512 <= 256 * 1024 : items <= 64ll * p.sms);
+    const bool more = items > 16ll * p.sms && (p.L.quant == BF16 ? (size_t)pairs_max * p.L.kg_i * 512 < 256 * 1024 : items <= 64ll * p.sms);
     const cudaError_t e = int8                             ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st, after_gate_up)
                           : more && p.L.quant == BF16      ? stream::launch_t<BF16, stream::DOWN_2, 12>(d, p.sms, st, after_gate_up)
                           : more && p.L.quant == Q8_0      ? stream::launch_t<Q8_0, stream::DOWN_2, 20>(d, p.sms, st, after_gate_up)

@@ -118,7 +118,7 @@ def test_decode_chain_wide_layer(cuda_lib, quant, T):
 
 
 # BF16 batches: ten and eight gate/up warps, twelve and eight down warps (by what their activations leave of the L1)
-@pytest.mark.parametrize("H,I,T", [(2048, 512, 6), (2048, 512, 7), (512, 2048, 4), (512, 2048, 5)])
+@pytest.mark.parametrize("H,I,T", [(2048, 512, 6), (2048, 512, 7), (512, 2048, 3), (512, 2048, 4)])
 def test_decode_chain_bf16_warp_rules(cuda_lib, H, I, T):
     E, K = 16, 8 if H < I else 4
     lay, meta, blob_np, sc, layer = make_layer(H, I, E, K, 2, seed=T)
