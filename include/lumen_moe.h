@@ -89,7 +89,8 @@ typedef struct {
  *   and prefill feeds the tensor cores from them with TMA instead of dequantising in shared
  *   memory: memory traded for prefill speed. BF16 layers always work that way (nothing to
  *   dequantise). Decode is not affected.
- * TC_CTAS(n): cap of the persistent tcgen05 grid, n CTAs (one per SM), 0 = every SM. */
+ * TC_CTAS(n): cap of the persistent tcgen05 grid, n CTAs (one per SM), 0 = every SM. (Pairs of CTAs share a tile:
+ *   an odd n above one runs on n - 1.) */
 #define LUMEN_MOE_FLAG_DECODE_SPLIT 0x1
 #define LUMEN_MOE_FLAG_PREFILL_MMA 0x2
 #define LUMEN_MOE_FLAG_SHORT_WAITS 0x4
