@@ -577,8 +577,10 @@ cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __hal
     d.out16 = out16_rows ? out16_rows : p.d16;
     d.out_row_map = out16_rows ? p.R.col_src_tok : nullptr;
     if (peer) d.peer = *peer;
-    // Q4_0: more warps once there are columns enough to keep them busy (E = 128: 77 tokens 125.8 -> 121.0 us, 18 tokens 83.3 and 85.5)
-    if (p.L.quant == Q4_0 && 2 * p.T * p.K > 5 * p.L.E) return stream::launch_t<Q4_0, stream::DOWN_1, 24>(d, p.sms, st);
+    // Q4_0: more warps once there are columns enough to keep them busy, with long rows earlier (16 and 24 warps, us from the host:
+    // I = 768, E = 128: 3.5 columns an expert 112.1 and 112.3, 4.3 columns 117.0 and 118.0, 4.8 columns 126.2 and 121.6, 5.5
+    // columns 125.9 and 122.9; I = 1536, E = 64: 2.8 columns 194.5 and 191.6, 5.6 columns 227.9 and 218.8)
+    if (p.L.quant == Q4_0 && 2 * p.T * p.K > (p.L.kg_i >= 8 ? 5 : 9) * p.L.E) return stream::launch_t<Q4_0, stream::DOWN_1, 24>(d, p.sms, st);
     return stream::launch_q<stream::DOWN_1>(d, p.sms, st);
 }
 
