@@ -1,5 +1,6 @@
 """Helpers shared by the GPU parity tests."""
 import numpy as np
+import pytest
 import torch
 
 from lumen_b200 import moe, synth
@@ -33,3 +34,16 @@ def oracle_layer(blob_np, meta, lay, K, x, residual, logits=None, gating=0, thre
     threads = threads or oracle.hardware_threads()
     return oracle.moe_layer(blob_np, 0, meta.expert_gate_offs, meta.expert_up_offs, meta.expert_down_offs, lay.quant,
                             lay.H, lay.I, lay.E, K, x, residual, gating=gating, logits=logits, threads=threads)
+
+
+def kernels_of(call):
+    """Names of the kernels that a call launches, in order."""
+    call()  # (one-time set-up inside the library)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if "lumen::" in e.name]
+    if not names:
+        pytest.skip("the profiler records no kernels on this machine")
+    return names
