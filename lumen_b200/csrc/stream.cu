@@ -551,7 +551,7 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_u
 }
 
 // Expert products of a short prompt: x16 rows by token (planes' element order), s16 by column.
-cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __half* out16_rows, cudaStream_t st,
+cudaError_t launch_stream_prefill(const PrefillArgs& p, int columns, const __half* x16, __half* out16_rows, cudaStream_t st,
                                   const TcPeerOut* peer) {
     stream::Args g{};
     g.L = p.L;
@@ -584,8 +584,9 @@ cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __hal
     // 125 and 123, 7 131 and 131, 8 150 and 154; E = 256, 2048 x 512: 3 143 and 141, 5 163 and 161, 6.3 175 and 181, 8 202 and
     // 211. Fewer items: E = 64, 2048 x 1024, K = 4: 4 88 and 90; E = 64, 1024 x 256, K = 4: 6 34.8 and 35.5; a lone expert of
     // 2048 x 4096: 8 49 and 51.)
-    const int C = p.T * p.K, E = p.L.E;
-    const bool wide = p.L.quant == Q4_0 && (long long)E * p.L.rt_h >= 96ll * p.sms && (p.L.kg_i >= 8 ? C > 2 * E : 2 * C > 9 * E && C <= 6 * E);
+    const int E = p.L.E;
+    const bool wide = p.L.quant == Q4_0 && (long long)E * p.L.rt_h >= 96ll * p.sms &&
+                      (p.L.kg_i >= 8 ? columns > 2 * E : 2 * columns > 9 * E && columns <= 6 * E);
     if (wide) return stream::launch_t<Q4_0, stream::DOWN_1, 24>(d, p.sms, st);
     return stream::launch_q<stream::DOWN_1>(d, p.sms, st);
 }

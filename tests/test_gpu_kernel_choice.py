@@ -32,3 +32,17 @@ def test_warps_of_a_prompts_streaming_down_product(cuda_lib, H, I, E, K, T, warp
     ref, ref_layer = context(H, I, E, K, 1, T, _lib.FLAG_PREFILL_MMA)
     want = ref.prefill(ref_layer, x, x)
     assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2
+
+
+# an expert-parallel call: by its own columns, not by what its window could take
+@pytest.mark.parametrize("T,warps", [(2, 16), (256, 16), (257, 24)])
+def test_warps_of_an_expert_parallel_streaming_down_product(cuda_lib, T, warps):
+    from lumen_b200 import ep
+    H, I, E, K = 1024, 1024, 256, 2
+    lay = synth.LayerLayout(H, I, E, 1)
+    pe = ep.PushExpertParallel(H, I, E, K, 1024, 0, 1, 0)
+    layer = pe.prepare_layer(synth.make_layer_blob(lay, 5), lay.meta())
+    x = rows(T, H)
+    names = kernels_of(lambda: pe.forward(layer, x, x))
+    assert [k for k in names if f"stream_kernel<1, 1, {warps}>" in k] and sum("stream_kernel<1, 1," in k for k in names) == 1, names
+    pe.close()
