@@ -282,12 +282,27 @@ struct TcPlan {
 cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_cap, int gu_cols, int4* tiles,
                              int32_t* n_tiles, cudaStream_t st, const int32_t* stream_mode, int4* chunks, int32_t* starts,
                              int sms);
-// Most columns of a prompt that the streaming kernels take. The line lies where the CTA-pair kernels overtake them (E = 128,
-// I = 768, us from the host, streaming and pairs): Q4_0 7.2 columns an expert 132 and 144, 8.1 columns 147 and 146; Q8_0,
-// whose rows cost twice the bytes, 7.2 columns 162 and 174, 8.1 columns 175 and 176, 9 columns 197 and 184; a lone expert of
-// 2048 x 512 with 8 columns 35 and 36, with 12 columns 38 and 35. The same line for an expert-parallel call, whose results
-// are one GPU's to the bit (its one-CTA tiles would overtake later, Q4_0 at 12 columns).
-inline int stream_max_columns(int quant, int experts) { return (quant == Q4_0 ? 16 : 17) * experts / 2; }
+// Most columns of a prompt that the streaming kernels take (experts: of the whole call, an expert-parallel rank's layer has
+// a share of them). The line lies where the CTA-pair kernels overtake them, us replayed, streaming and pairs:
+//   planes           E = 128, 2048 x 768: Q4_0 7 columns an expert 131 and 144, 8 columns 150 and 146, 10 columns 170 and 147; Q8_0 7 columns
+//                    162 and 163, 8 columns 183 and 164; E = 32, 1024 x 512: 8 columns 33.9 and 39.0 (Q4_0), 38.7 and 41.8 (Q8_0), 9
+//                    columns 37.7 and 39.1, 42.5 and 41.9. A lone expert of 2048 x 512: 8 columns 32.9 and 34.9, 9 columns 38.0 and 34.8
+//   narrow planes    rows of up to 512 inputs are a short chain of copies for a streaming warp, while the pairs' set-up stays: 16 experts of
+//                    512 x 256 at 8 columns 25.7 and 28.7, at 12 columns 27.7 and 28.7; 128 of them at 12 columns 42.4 and 44.2 (Q4_0), at 9
+//                    columns 45.5 and 46.8, at 10 columns 49.0 and 46.7 (Q8_0); a lone one at 13 columns 24.7 and 26.6
+//   f16 matrices     the pairs multiply these, four (Q4_0) or two times the bytes that the streaming kernels read from the planes: E = 128,
+//                    2048 x 768: Q4_0 8.1 columns 158 and 212, 12 columns 195 and 215, 14 columns 223 and 217; Q8_0 10 columns 204 and 213, 11
+//                    columns 219 and 214; E = 32, 1024 x 512: Q4_0 12 columns 43.6 and 44.2, Q8_0 10 columns 45.0 and 45.2. With few experts the
+//                    bytes are not what counts (eight of 2048 x 512 at 6 columns 38.9 and 37.3): as planes
+// The same line for an expert-parallel call, whose results are one GPU's to the bit. There it costs time: its one-CTA tiles overtake
+// later (2048 x 768, E = 128, one rank: Q4_0 8.1 columns 199 streaming and 222 on tiles, 10 columns 220 and 223, 11 columns 236 and 224).
+inline int stream_max_columns(const LayerDev& L, int experts) {
+    const bool q4 = L.quant == Q4_0;
+    if (L.gu16 != nullptr && experts >= 32) return (q4 ? 12 : 10) * experts;
+    if (L.H <= 512) return experts == 1 ? 16 : (q4 ? 12 : 9) * experts;
+    return 8 * experts;
+}
+inline int stream_max_columns_of_any(int experts) { return 12 * experts > 16 ? 12 * experts : 16; }
 // gate/up of a decode batch, expert products of short prompts (stream.cu)
 cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st);
 cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_up, cudaStream_t st);

@@ -577,16 +577,16 @@ cudaError_t launch_stream_prefill(const PrefillArgs& p, int columns, const __hal
     d.out16 = out16_rows ? out16_rows : p.d16;
     d.out_row_map = out16_rows ? p.R.col_src_tok : nullptr;
     if (peer) d.peer = *peer;
-    // Q4_0: 24 warps where an SM has four rounds of items for them and more than two columns an expert, rows of 1024 inputs and more; shorter
+    // Q4_0: 24 warps where an SM has four rounds of items for them and two to nine columns an expert, rows of 1024 inputs and more; shorter
     // ones between 4.5 and 6 columns. Beyond, where many experts have more than one operand of eight columns, their registers (80, spills)
     // cost more than they hide. (16 and 24 warps, us replayed, by columns an expert. E = 64, 4096 x 1536: 2.3 186 and 185, 4.5 212 and 206, 7.5 256 and
-    // 245; E = 128, 2048 x 1024: 3 139 and 138, 5 151 and 146, 8 174 and 171; E = 128, 2048 x 768: 4 112.5 and 112.8, 5 120 and 117, 6
+    // 245, 9 262 and 254, 11 352 and 386; E = 128, 2048 x 1024: 3 139 and 138, 5 151 and 146, 8 174 and 171; E = 128, 2048 x 768: 4 112.5 and 112.8, 5 120 and 117, 6
     // 125 and 123, 7 131 and 131, 8 150 and 154; E = 256, 2048 x 512: 3 143 and 141, 5 163 and 161, 6.3 175 and 181, 8 202 and
     // 211. Fewer items: E = 64, 2048 x 1024, K = 4: 4 88 and 90; E = 64, 1024 x 256, K = 4: 6 34.8 and 35.5; a lone expert of
     // 2048 x 4096: 8 49 and 51.)
     const int E = p.L.E;
     const bool wide = p.L.quant == Q4_0 && (long long)E * p.L.rt_h >= 96ll * p.sms &&
-                      (p.L.kg_i >= 8 ? columns > 2 * E : 2 * columns > 9 * E && columns <= 6 * E);
+                      (p.L.kg_i >= 8 ? columns > 2 * E && columns <= 9 * E : 2 * columns > 9 * E && columns <= 6 * E);
     if (wide) return stream::launch_t<Q4_0, stream::DOWN_1, 24>(d, p.sms, st);
     return stream::launch_q<stream::DOWN_1>(d, p.sms, st);
 }

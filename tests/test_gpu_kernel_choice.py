@@ -7,6 +7,8 @@ from tests.gpu_util import TOL_REL_L2, kernels_of, rel_l2
 
 pytestmark = pytest.mark.gpu
 
+F16 = _lib.FLAG_PREFILL_F16_WEIGHTS
+
 
 def context(H, I, E, K, quant, T, flags=0):
     lay = synth.LayerLayout(H, I, E, quant)
@@ -18,13 +20,15 @@ def rows(T, H):
     return torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(T), device="cuda")
 
 
-# streaming down product of Q4_0 prompts: 24 warps for enough items (E * H / 16 rows of tiles) and more than two columns of long rows, 4.5
-# to 6 columns of short ones; 16 elsewhere
-@pytest.mark.parametrize("H,I,E,K,T,warps", [(1024, 1024, 256, 2, 256, 16), (1024, 1024, 256, 2, 257, 24), (1024, 1024, 256, 2, 1024, 24),
-                                             (1024, 1024, 128, 2, 300, 16), (1024, 128, 256, 2, 576, 16), (1024, 128, 256, 2, 577, 24),
-                                             (1024, 128, 256, 2, 768, 24), (1024, 128, 256, 2, 769, 16), (1024, 2048, 1, 1, 8, 16)])
-def test_warps_of_a_prompts_streaming_down_product(cuda_lib, H, I, E, K, T, warps):
-    sc, layer = context(H, I, E, K, 1, T)
+# streaming down product of Q4_0 prompts: 24 warps for enough items (E * H / 16 rows of tiles) and more than two, up to nine columns of long rows,
+# 4.5 to 6 columns of short ones; 16 elsewhere
+@pytest.mark.parametrize("I,E,K,T,flags,warps", [(1024, 256, 2, 256, 0, 16), (1024, 256, 2, 257, 0, 24), (1024, 256, 2, 1024, 0, 24),
+                                                 (1024, 256, 2, 1152, F16, 24), (1024, 256, 2, 1153, F16, 16), (1024, 128, 2, 300, 0, 16),
+                                                 (128, 256, 2, 576, 0, 16), (128, 256, 2, 577, 0, 24), (128, 256, 2, 768, 0, 24),
+                                                 (128, 256, 2, 769, 0, 16), (2048, 1, 1, 8, 0, 16)])
+def test_warps_of_a_prompts_streaming_down_product(cuda_lib, I, E, K, T, flags, warps):
+    H = 1024
+    sc, layer = context(H, I, E, K, 1, T, flags)
     x = rows(T, H)
     out = torch.empty_like(x)
     names = kernels_of(lambda: sc.prefill(layer, x, x, out))
@@ -46,3 +50,22 @@ def test_warps_of_an_expert_parallel_streaming_down_product(cuda_lib, T, warps):
     names = kernels_of(lambda: pe.forward(layer, x, x))
     assert [k for k in names if f"stream_kernel<1, 1, {warps}>" in k] and sum("stream_kernel<1, 1," in k for k in names) == 1, names
     pe.close()
+
+
+# the longest prompt on the streaming kernels: planes (8 columns an expert), narrow ones (12 | 9, a lone expert 16), layers kept as
+# f16 matrices (12 | 10, with few experts as planes)
+@pytest.mark.parametrize("quant,flags,H,E,K,T", [(1, 0, 1024, 16, 4, 32), (0, 0, 1024, 16, 4, 32), (1, 0, 512, 16, 4, 48), (0, 0, 512, 16, 4, 36),
+                                                 (1, F16, 1024, 32, 4, 96), (0, F16, 1024, 32, 4, 80), (1, F16, 1024, 16, 4, 32),
+                                                 (1, 0, 1024, 1, 1, 8), (0, 0, 512, 1, 1, 16)])
+def test_longest_prompt_on_the_streaming_kernels(cuda_lib, quant, flags, H, E, K, T):
+    I = 256
+    sc, layer = context(H, I, E, K, quant, T + 1, flags)
+    ref, ref_layer = context(H, I, E, K, quant, T + 1, _lib.FLAG_PREFILL_MMA)
+    for n, name in ((T, "stream_kernel"), (T + 1, "grouped_gemm_pair_kernel")):
+        x = rows(n, H)
+        out = torch.empty_like(x)
+        names = kernels_of(lambda: sc.prefill(layer, x, x, out))
+        assert [k for k in names if "stream_kernel" in k or "grouped_gemm" in k or "down" in k] and all(
+            name in k for k in names if "stream_kernel" in k or "grouped_gemm" in k), names
+        want = ref.prefill(ref_layer, x, x)
+        assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2

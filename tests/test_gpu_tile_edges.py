@@ -48,7 +48,7 @@ def test_streaming_prefill_chunk_edges(cuda_lib, quant, H, I):
     check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1))
 
 
-# the last batch on the streaming kernels and the first on the tcgen05 ones (8.5 | 8 columns an expert), and batches beyond
+# the last batch on the streaming kernels and the first on the tcgen05 ones (12 | 9 columns an expert of such narrow rows), and others
 @pytest.mark.parametrize("quant,T", [(1, 32), (1, 33), (0, 34), (0, 35), (0, 36), (0, 37), (1, 40), (1, 41), (1, 48), (1, 49)])
 def test_prefill_on_both_sides_of_the_streaming_limit(cuda_lib, quant, T):
     check_prefill(384, 256, 16, 4, quant, synth.zipf_logits(T, 16, 3), torch.bfloat16)
