@@ -507,6 +507,14 @@ static Args decode_args(const DecodeArgs& p) {
     return g;
 }
 
+// Items of an SM in a decode batch: rt rows of tiles of every expert that the tokens' choices hit, as many as under near-uniform routing.
+static int items_per_sm(const DecodeArgs& p, int rt) {
+    float miss = 1.0f;
+    for (int t = 0; t < p.T; ++t) miss *= 1.0f - (float)p.K / (float)p.L.E;
+    return (int)ceilf((float)p.L.E * (1.0f - miss) * (float)rt / (float)p.sms);
+}
+static bool rounds_less(int items, int few, int many) { return (items + many - 1) / many < (items + few - 1) / few; }
+
 }  // namespace stream
 
 // gate/up of a decode batch: hi + lo activation fragments by token, SwiGLU fragments for the down product
@@ -517,9 +525,12 @@ cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st) {
     g.b_row = (size_t)p.L.kg_h * 16;
     g.sf = p.sf;
     g.debug_extra_tx = p.debug_expire;
-    // BF16: two warps more while the activations still fit into the L1 that their rings leave (H = 2048: 5 tokens 56.9 -> 53.3 us,
-    // 8 tokens 77.4 -> 80.4)
-    if (p.L.quant == BF16 && (size_t)p.T * p.L.kg_h * 512 <= 48 * 1024) return stream::launch_t<BF16, stream::GATE_UP_2, 10>(g, p.sms, st);
+    // BF16: ten warps where they take a round less than eight, up to three rounds (eight and ten, us replayed, by items an SM. H = 2048, I = 768, E = 128: 10
+    // 65.2 and 60.2, 12 70.7 and 72.9, 14 79.2 and 80.4, 17 98.5 and 94.6, 23 119.9 and 122.6, 25 137.2 and 136.1; I = 512, E = 256: 7 48.7
+    // and 48.7, 9 63.1 and 56.6, 13 80.5 and 81.5, 18 105.8 and 103.5; H = 3072, I = 1024, E = 32: 10 93 and 80; H = 4096, I = 1536, E = 64: 11 123.7
+    // and 126.5, 14 146 and 150, 19 184 and 178, 31 295 and 303)
+    const int n = stream::items_per_sm(p, p.L.rt_i);
+    if (p.L.quant == BF16 && n <= 30 && stream::rounds_less(n, 8, 10)) return stream::launch_t<BF16, stream::GATE_UP_2, 10>(g, p.sms, st);
     return stream::launch_q<stream::GATE_UP_2>(g, p.sms, st);
 }
 
@@ -531,13 +542,15 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_u
     d.b_row = (size_t)p.L.kg_i * 16;
     d.d32 = p.d32;
     d.debug_extra_tx = int8 ? p.debug_expire : 0;  // (the chain's first streaming kernel)
-    // More warps where an SM's items (at most: of every expert that T * K pairs can reach) are one to four rounds of the usual
-    // ones: below they idle, above the rounds even out by themselves (Q8_0, 16 and 20 warps: 21 items an SM 53.1 and 50.2 us, 35 items
-    // 50.0 and 49.0; 4 items 30.5 and 31.0, 110 items 189.3 and 189.6. BF16, 8 and 12: 35 items 54.3 and 53.3, 14 items 38.9 and
-    // 39.3). BF16: not either where their longer rings leave too little L1 for the SwiGLU fragments (12 tokens, H = 4096,
-    // I = 1536: 279 and 285 us; 16 tokens, I = 512: 120.7 and 121.9).
-    const long long pairs_max = (long long)p.T * p.K, items = (pairs_max < p.L.E ? pairs_max : p.L.E) * p.L.rt_h;
-    const bool more = items > 16ll * p.sms && (p.L.quant == BF16 ? (size_t)pairs_max * p.L.kg_i * 512 < 256 * 1024 : items <= 64ll * p.sms);
+    // More warps where they take a round less. Q8_0, whose rings get shorter for it: up to two rounds (16 and 20 warps, us replayed, by items an SM.
+    // H = 2048, I = 768, E = 128: 20 40.2 and 38.9, 26 44.1 and 44.8, 31 47.7 and 48.2, 36 53.5 and 51.6, 45 71.4 and 72.5, 60 85.1 and 85.9;
+    // H = 2048, I = 1408, E = 64: 19 53.4 and 50.4, 23 63.5 and 65.7, 27 74 and 75.5; H = 3072, I = 1024, E = 32: 18 45.1 and 43.6, 23 49.7
+    // and 51.6, 34 71.4 and 69.5). BF16: any number, while the batch's fragments are not too many (8 and 12 warps. H = 2048, I = 768, E = 128: 14 39.0
+    // and 39.0, 36 79.2 and 77.2; H = 1024, I = 384, E = 64: 8 21.8 and 22.2, 9 24.1 and 23.1, 15 29.1 and 29.4; 256 KB: 16 tokens of I = 512
+    // 125.0 and 124.5, of H = 3072, I = 1024, E = 32 113 and 111; beyond: H = 4096, I = 1536, E = 64 8 tokens, 288 KB, 211 and 215, 16 tokens 295 and 322).
+    const int n = stream::items_per_sm(p, p.L.rt_h);
+    const bool more = p.L.quant == BF16 ? (size_t)p.T * p.K * p.L.kg_i * 512 <= 256 * 1024 && stream::rounds_less(n, 8, 12)
+                                        : n <= 40 && stream::rounds_less(n, 16, 20);
     const cudaError_t e = int8                             ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st, after_gate_up)
                           : more && p.L.quant == BF16      ? stream::launch_t<BF16, stream::DOWN_2, 12>(d, p.sms, st, after_gate_up)
                           : more && p.L.quant == Q8_0      ? stream::launch_t<Q8_0, stream::DOWN_2, 20>(d, p.sms, st, after_gate_up)

@@ -69,3 +69,20 @@ def test_longest_prompt_on_the_streaming_kernels(cuda_lib, quant, flags, H, E, K
             name in k for k in names if "stream_kernel" in k or "grouped_gemm" in k), names
         want = ref.prefill(ref_layer, x, x)
         assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2
+
+
+# decode batches: more warps where an SM's items take a round less with them (gate/up of BF16 8 | 10, down of Q8_0 16 | 20, of BF16 8 | 12)
+@pytest.mark.parametrize("quant,H,I,E,K,T,gate_up,down", [(2, 2048, 768, 128, 8, 4, 10, 12), (2, 2048, 768, 128, 8, 5, 8, 12), (2, 2048, 512, 256, 8, 5, 10, 12),
+                                                          (2, 2048, 512, 256, 8, 16, 8, 12), (2, 2048, 768, 128, 8, 16, 10, 8), (2, 1024, 384, 64, 4, 12, 8, 8),
+                                                          (0, 2048, 768, 128, 8, 3, 16, 20), (0, 2048, 768, 128, 8, 4, 16, 16),
+                                                          (0, 2048, 768, 128, 8, 6, 16, 20), (0, 2048, 768, 128, 8, 16, 16, 16)])
+def test_warps_of_a_decode_batch(cuda_lib, quant, H, I, E, K, T, gate_up, down):
+    sc, layer = context(H, I, E, K, quant, T, _lib.FLAG_DECODE_SPLIT)
+    x = rows(T, H)
+    out = torch.empty_like(x)
+    names = kernels_of(lambda: sc.decode(layer, x, x, out))
+    for mode, warps in ((2, gate_up), (3, down)):
+        assert [k for k in names if f"stream_kernel<{quant}, {mode}, {warps}>" in k], names
+    ref, ref_layer = context(H, I, E, K, quant, T, _lib.FLAG_PREFILL_MMA)
+    want = ref.prefill(ref_layer, x, x)
+    assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2

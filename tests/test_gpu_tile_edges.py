@@ -117,7 +117,7 @@ def test_decode_chain_wide_layer(cuda_lib, quant, T):
     assert rel_l2((out - x).cpu().numpy(), o_out - x.cpu().numpy()) < TOL_REL_L2
 
 
-# BF16 batches: ten and eight gate/up warps, twelve and eight down warps (by what their activations leave of the L1)
+# BF16 batches of few experts (warps by the rounds of items: test_gpu_kernel_choice.py)
 @pytest.mark.parametrize("H,I,T", [(2048, 512, 6), (2048, 512, 7), (512, 2048, 3), (512, 2048, 4)])
 def test_decode_chain_bf16_warp_rules(cuda_lib, H, I, T):
     E, K = 16, 8 if H < I else 4
