@@ -172,11 +172,13 @@ stream_kernel(const __grid_constant__ Args a) {
         i1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
     }
 
-    // Warps that take part: in a decode batch of Q4_0, and in the BF16 down product of twelve warps, as many as give each the same number of
-    // items, so that the last round is as full as the others (16 tokens of Q4_0 61.1 -> 60.8 us, 2 tokens of BF16 41.4 -> 39.3).
-    // Elsewhere a warp less on the way costs more than the uneven round (90 tokens of Q8_0 155 -> 163, 110 of Q4_0 129 -> 132).
+    // Warps that take part where there are more items than warps: in a decode batch of Q4_0, and in the BF16 down product of twelve warps, as many
+    // as give each the same number of items, so that the last round is as full as the others (16 tokens of Q4_0 61.1 -> 60.8 us, 8 tokens of
+    // H = 4096, I = 1536 108.7 -> 103.5). Elsewhere a warp less on the way costs more than the uneven round (90 tokens of Q8_0 155 -> 163, 110
+    // of Q4_0 129 -> 132). With a round or less there is nothing to even out, and the two divisions stand in front of the first request (4 tokens
+    // of 512 x 256 15.3 -> 14.5 us, 2 of 3072 x 1024 35.7 -> 35.1).
     int nw = WARPS;
-    if (((Q == Q4_0 && TERMS == 2) || (Q == BF16 && DOWN && WARPS > 8)) && i1 > i0) {
+    if (((Q == Q4_0 && TERMS == 2) || (Q == BF16 && DOWN && WARPS > 8)) && i1 - i0 > WARPS) {
         const int n = i1 - i0, rounds = (n + WARPS - 1) / WARPS;
         nw = (n + rounds - 1) / rounds;
         if (warp >= nw) i1 = i0;
