@@ -17,7 +17,7 @@ cudaError_t launch_build_xf(const void* x, int act_dtype, int T, int H, int nblk
                             uint4* xf, cudaStream_t st);
 cudaError_t launch_gather_rows(const __half* plane, const int32_t* col_src_tok, int C, int H, void* out, cudaStream_t st);
 cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, cudaStream_t st, __half* out16_rows,
-                              const TcPlan* plan = nullptr, const TcPeerOut* peer = nullptr);
+                              const TcPlan& plan, const TcPeerOut* peer = nullptr);
 cudaError_t launch_rows_from_cols(const __half* d16, const int32_t* dst_to_col, __half* out16, int T, int H, cudaStream_t st);
 
 static std::atomic<long long> g_launches{0};
@@ -620,13 +620,15 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
         if (out16_rows) return Status::Ok();
     } else if (p.impl == 0) {
         const TcForm form = tc_form(layer.dev, batch * s->K, s->sms, s->tc_ctas);
-        if (!single && !form.pairs)  // (pairs gather by themselves)
-             CUDA_TRY(launch_gather_rows(s->xr16, s->R.col_src_tok, batch * s->K, s->H, s->x16, st));
         // persistent grid, one CTA per SM; LUMEN_MOE_FLAG_TC_CTAS leaves some SMs to kernels that run beside it
         int sms = s->sms;
         if (s->tc_ctas > 0 && s->tc_ctas < sms) sms = s->tc_ctas;
-        if (form.pairs) CUDA_TRY(launch_grouped_pair(p, single ? s->xr16 : nullptr, form.cols, sms, st, out16_rows));
-        else CUDA_TRY(launch_grouped_tc(p, single ? s->xr16 : s->x16, sms, st, out16_rows));
+        if (form.pairs) {  // (these gather their columns by themselves)
+            CUDA_TRY(launch_grouped_pair(p, single ? s->xr16 : nullptr, form.cols, sms, st, out16_rows));
+        } else {
+            if (!single) CUDA_TRY(launch_gather_rows(s->xr16, s->R.col_src_tok, batch * s->K, s->H, s->x16, st));
+            CUDA_TRY(launch_grouped_tc(p, single ? s->xr16 : s->x16, sms, st, out16_rows, TcPlan{batch * s->K, form.cols}));
+        }
     } else {
         CUDA_TRY(launch_build_xf(normed, act_dtype, batch, s->H, layer.dev.kg_h * 4, bf16_mode, s->xf, st));
         DecodeArgs a = make_decode_args(s, layer, batch);

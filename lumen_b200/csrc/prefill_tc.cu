@@ -875,9 +875,8 @@ static cudaError_t launch_tc_one(const tc::Args& a, int grid, cudaStream_t st) {
 
 // gate/up + SwiGLU then down, both on tcgen05. x16: permuted 16-bit activations [T,H].
 cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, cudaStream_t st, __half* out16_rows,
-                              const TcPlan* plan, const TcPeerOut* peer) {
-    const int C = plan ? plan->rows : p.T * p.K;
-    const int gu_cols = plan ? plan->gu_cols : 128;  // as the tile lists were built
+                              const TcPlan& plan, const TcPeerOut* peer) {
+    const int C = plan.rows, gu_cols = plan.gu_cols;
     const int max_ct = C / gu_cols + p.L.E;
     // rows that go to other ranks' return buffers leave through the staged epilogue (bulk copies)
     const bool stg = peer != nullptr;

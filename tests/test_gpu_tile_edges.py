@@ -85,15 +85,15 @@ def test_prefill_on_both_sides_of_the_wide_tiles(cuda_lib, quant, E, I, T):
 
 
 @pytest.mark.parametrize("quant", [0, 1, 2])
-@pytest.mark.parametrize("ctas,T", [(1, 300), (3, 300), (3, 1100)])
-def test_prefill_on_a_capped_grid(cuda_lib, quant, ctas, T):
-    H, I, E, K = 512, 384, 16, 2
+@pytest.mark.parametrize("ctas,T,E,K", [(1, 300, 16, 2), (1, 1024, 16, 2), (1, 1025, 16, 2), (1, 400, 1, 1), (3, 300, 16, 2), (3, 1100, 16, 2)])
+def test_prefill_on_a_capped_grid(cuda_lib, quant, ctas, T, E, K):
+    H, I = 512, 384
     lay = synth.LayerLayout(H, I, E, quant)
     blob = synth.make_layer_blob(lay, 3)
     x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(T), device="cuda")
     outs = []
     for flags in (0, _lib.flag_tc_ctas(ctas)):
-        sc = moe.allocate_moe_scratch(H, I, E, K, T, flags=flags)
+        sc = moe.allocate_moe_scratch(H, I, E, K, T, moe.SIGMOID_GATE if E == 1 else moe.SOFTMAX_RENORM, flags=flags)
         outs.append(sc.prefill(sc.prepare_layer(blob, lay.meta()), x, x))
         assert sc.poll_status() == _lib.OK
     assert torch.equal(*outs)
