@@ -156,7 +156,8 @@ static size_t tok_arena_bytes(const CudaMoeScratch& s, int cap, size_t* offs) {
         (size_t)cap * s.E * 4, C * 4, C * 4, C * 4, C * 4, C * 4,
         (size_t)((cap + 7) / 8 + 1) * s.E * 4,  // one histogram per chunk of 8 tokens (SORT_TOK in route_large.cu), the totals
         n_tile_entries * sizeof(int4),
-        C * s.I * 2, C * s.H * 2, C * s.H * 2,
+        C * s.I * 2, C * s.H * 2,
+        s.tc_ctas == 1 ? C * s.H * 2 : 0,  // (gathered rows: only one CTA on its own needs them, 268 MB for 8192 tokens of 2048, K = 8)
         (size_t)cap * 2 * nblk_h_pad * 64, C * 2 * nblk_i_pad * 64,
         (size_t)s.E * s.H * 4,
         (size_t)DECODE_MAX_TOKENS * (18 * nblk_h_pad + 16) * 4,  // xq_tok_words(nblk_h_pad) words per token
@@ -194,7 +195,7 @@ static Status alloc_tok_arena(CudaMoeScratch* s, int cap) {
     s->tiles = reinterpret_cast<int4*>(b + offs[7]);
     s->s16 = reinterpret_cast<__half*>(b + offs[8]);
     s->d16 = reinterpret_cast<__half*>(b + offs[9]);
-    s->x16 = reinterpret_cast<__half*>(b + offs[10]);
+    s->x16 = s->tc_ctas == 1 ? reinterpret_cast<__half*>(b + offs[10]) : nullptr;
     s->xf = reinterpret_cast<uint4*>(b + offs[11]);
     s->sf = reinterpret_cast<uint4*>(b + offs[12]);
     s->w16 = reinterpret_cast<__half*>(b + offs[13]);

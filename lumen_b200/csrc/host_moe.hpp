@@ -110,7 +110,7 @@ struct CudaMoeScratch {
     __half* w16 = nullptr;
     __half* s16 = nullptr;
     __half* d16 = nullptr;
-    __half* x16 = nullptr;  // permuted 16-bit activations for the tcgen05 path
+    __half* x16 = nullptr;  // f16 activation rows by compact column, where the tcgen05 grid is capped at one CTA
     __half* xr16 = nullptr; // f16 high / low planes of the batch for the tcgen05 router
     float* rpart = nullptr; // partial logits of the tcgen05 router
     int32_t* any_lo = nullptr;

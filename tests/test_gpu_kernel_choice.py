@@ -95,3 +95,17 @@ def test_gate_up_tiles_of_one_cta(cuda_lib, quant, flags, T, cols):
     x = rows(T, 512)
     names = kernels_of(lambda: sc.prefill(layer, x, x))
     assert [k for k in names if "grouped_gemm_tc_kernel" in k and f", 0, {cols}," in k], names
+
+
+# rows gathered by column are kept only where a kernel reads them: a grid capped at one CTA
+def test_device_memory_of_a_prefill_context(cuda_lib):
+    H, K, T = 2048, 8, 8192
+    taken = {}
+    for ctas in (1, 0, 2):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        sc = moe.allocate_moe_scratch(H, 128, 16, K, T, flags=_lib.flag_tc_ctas(ctas))
+        taken[ctas] = free - torch.cuda.mem_get_info()[0]
+        sc.close()
+    # (the driver maps device memory in pages of 2 MB)
+    assert abs(taken[1] - taken[0] - T * K * H * 2) <= 4 << 20 and abs(taken[0] - taken[2]) <= 4 << 20, taken
