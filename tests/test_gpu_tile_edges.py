@@ -99,6 +99,25 @@ def test_prefill_on_a_capped_grid(cuda_lib, quant, ctas, T, E, K):
     assert torch.equal(*outs)
 
 
+# f16 rows in the caller's order (top_k = 1): down products by row map on CTA pairs (tiles of 128 and of 512 columns), one CTA, the
+# streaming kernels. With a weight of one and no residual the weighted sum is the same f16 row.
+@pytest.mark.parametrize("quant", [0, 1, 2])
+@pytest.mark.parametrize("T,ctas", [(60, 0), (700, 0), (2500, 0), (2500, 1)])
+def test_routed_rows_leave_by_row_map(cuda_lib, quant, T, ctas):
+    H, I, E = 512, 384, 16
+    lay = synth.LayerLayout(H, I, E, quant)
+    sc = moe.allocate_moe_scratch(H, I, E, 1, T, flags=_lib.flag_tc_ctas(ctas))
+    layer = sc.prepare_layer(synth.make_layer_blob(lay, 3), lay.meta())
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=g, device="cuda")
+    ids = torch.randint(0, E - 3, (T,), generator=g, device="cuda", dtype=torch.int32)  # two experts get no row
+    ids[:1], ids[1:32] = E - 3, 2
+    rows16 = sc.experts_routed_f16(layer, x, ids)
+    want = sc.prefill_routed(layer, x, ids, None, torch.zeros_like(x))
+    assert sc.poll_status() == _lib.OK
+    assert want.abs().sum(1).min() > 0 and torch.equal(rows16.float(), want)
+
+
 # batches of the decode chain for each format, at contractions with a remainder against the ring's chunk
 @pytest.mark.parametrize("quant,T", [(0, 3), (0, 16), (1, 5), (1, 16), (2, 5), (2, 9), (2, 16)])
 def test_decode_chain_wide_layer(cuda_lib, quant, T):
@@ -221,11 +240,11 @@ def test_norm_folded_into_the_planes_matches_the_norm_kernel(cuda_lib, H):
     assert torch.equal(x, y)
 
 
-# a context of one expert: routing, operand plane and plan in one kernel of 8 tokens a CTA, then streaming up to 16
-# columns, tiles of 128 in one wave, CTA pairs beyond
+# a context of one expert: routing, operand plane and plan in one kernel of 8 tokens a CTA, then streaming up to 8 columns (BF16
+# none), CTA pairs beyond (9728: tiles of 512 columns)
 @pytest.mark.parametrize("quant", [0, 1, 2])
-@pytest.mark.parametrize("T,act,gating", [(1, torch.float32, 2), (9, torch.bfloat16, 2), (16, torch.float32, 3), (17, torch.bfloat16, 2),
-                                          (129, torch.float32, 3), (9500, torch.bfloat16, 2)])
+@pytest.mark.parametrize("T,act,gating", [(1, torch.float32, 2), (8, torch.float32, 2), (9, torch.bfloat16, 2), (16, torch.float32, 3), (17, torch.bfloat16, 2),
+                                          (129, torch.float32, 3), (9500, torch.bfloat16, 2), (9728, torch.float32, 2)])
 def test_single_expert_prefill(cuda_lib, quant, T, act, gating):
     H, I = 768, 256
     lay, meta, blob_np, sc, layer = make_layer(H, I, 1, 1, quant, seed=T, max_tokens=T, gating=gating)
