@@ -36,8 +36,7 @@
 // narrow tiles: 300 tokens, a whole call 192 -> 148 us.
 //
 // Every wait is bounded; on expiry the kernel raises the status word, lets its copies and MMAs end, frees its TMEM and returns.
-#include "mma_frag.cuh"
-#include "tc_common.cuh"
+#include "tc_weights.cuh"
 
 namespace lumen {
 
@@ -259,14 +258,6 @@ struct Place {
     }
 };
 
-__device__ __forceinline__ uint32_t scale_f16x2(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-__device__ __forceinline__ void store16(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
 // half a tile (16 rows x 64 inputs): q words of blocks 2 sub, 2 sub + 1, the blocks' f16 scales of rows g and g + 8
 template <int Q, int MODE>
 __device__ __forceinline__ void dequant(const uint4& q0, const uint4& q1, uint32_t s_g, uint32_t s_g8, uint32_t a_base, const Place<MODE>& pl,
@@ -278,33 +269,15 @@ __device__ __forceinline__ void dequant(const uint4& q0, const uint4& q1, uint32
             // (gate/up never swaps: the selections below fold away)
             const bool second = (MODE == 0) ? (p == 1) : ((p == 1) != pl.swap);
             const uint32_t sc = prmt(r ? s_g8 : s_g, 0u, second ? 0x3232u : 0x1010u);
-            uint32_t l0, l1, h0, h1;
+            uint32_t w0, w1 = 0u;
             if constexpr (Q == Q4_0) {
-                const uint32_t a = r ? q0.y : q0.x, b = r ? q0.w : q0.z;
-                const uint32_t x = second ? b : a, y = x >> 8;
-                l0 = hsub2_u32(lop_and_or(x, 0x000F000Fu, k.or_a), k.sub_a);
-                h0 = hsub2_u32(lop_and_or(x, 0x00F000F0u, k.or_b), k.sub_b);
-                l1 = hsub2_u32(lop_and_or(y, 0x000F000Fu, k.or_a), k.sub_a);
-                h1 = hsub2_u32(lop_and_or(y, 0x00F000F0u, k.or_b), k.sub_b);
+                w0 = second ? (r ? q0.w : q0.z) : (r ? q0.y : q0.x);
             } else {
-                const uint32_t a0 = r ? q0.z : q0.x, a1 = r ? q0.w : q0.y;
-                const uint32_t b0 = r ? q1.z : q1.x, b1 = r ? q1.w : q1.y;
-                const uint32_t x = (second ? b0 : a0) ^ k.or_b, y = (second ? b1 : a1) ^ k.or_b;
-                l0 = hsub2_u32(prmt(x, k.or_a, 0x4240u), k.sub_a);
-                l1 = hsub2_u32(prmt(x, k.or_a, 0x4341u), k.sub_a);
-                h0 = hsub2_u32(prmt(y, k.or_a, 0x4240u), k.sub_a);
-                h1 = hsub2_u32(prmt(y, k.or_a, 0x4341u), k.sub_a);
+                w0 = second ? (r ? q1.z : q1.x) : (r ? q0.z : q0.x);
+                w1 = second ? (r ? q1.w : q1.y) : (r ? q0.w : q0.y);
             }
-            store16(a_base + pl.off[p] + r * Place<MODE>::row8, scale_f16x2(l0, sc), scale_f16x2(h0, sc), scale_f16x2(l1, sc), scale_f16x2(h1, sc));
+            store_weights<Q>(a_base + pl.off[p] + r * Place<MODE>::row8, w0, w1, sc, k);
         }
-}
-
-// SwiGLU (cuda/shaders/moe_expert.cu:47-50) as in prefill_tc.cu
-__device__ __forceinline__ float swiglu(float g, float u) {
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-    return g * r * u;
 }
 
 // columns of set h of a tile, rounded up to what an MMA of the pair takes
@@ -423,8 +396,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                         uint32_t o[4];
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-                            o[j] = pack_f16(swiglu(__uint_as_float(x[4 * j]), __uint_as_float(x[4 * j + 2])),
-                                            swiglu(__uint_as_float(x[4 * j + 1]), __uint_as_float(x[4 * j + 3])));
+                            o[j] = pack_f16(swiglu_fast(__uint_as_float(x[4 * j]), __uint_as_float(x[4 * j + 2])),
+                                            swiglu_fast(__uint_as_float(x[4 * j + 1]), __uint_as_float(x[4 * j + 3])));
                         stmatrix4_t(buf + piece(lane, half), o);
                     } else {
 #pragma unroll

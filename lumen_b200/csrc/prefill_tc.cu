@@ -36,8 +36,7 @@
 // pre-permuted within each 32-block to the order the dequantiser emits (route_tc.cu; natural order for TMA-fed
 // weights), gathered into compact-column order (gather_rows_kernel); the SwiGLU output is
 // written in the same order so the down product reads it back without any shuffle.
-#include "mma_frag.cuh"
-#include "tc_common.cuh"
+#include "tc_weights.cuh"
 #include <type_traits>
 
 namespace lumen {
@@ -51,25 +50,6 @@ constexpr int THREADS = (SCHED_WARP + 1) * 32;
 // rows of an activation box: 32 where tiles are narrow (no more of the operand is copied than the tile has)
 __host__ __device__ constexpr int bbox_rows(int bn) { return bn == 256 ? 128 : 32; }
 constexpr int SCHED_RING = 4;             // tile descriptors in flight between the scheduler and the roles
-
-__device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-// SwiGLU (cuda/shaders/moe_expert.cu:47-50), g / (1 + e^-g) * u, on the approximate exp2 and reciprocal units: their error
-// (~2^-21) is far below the f16 rounding of the result that follows. The epilogue of a wide tile is exposed, so its
-// instructions count; the range fix-ups of the library forms are not needed here (e^-g = inf gives 0, as it should; a
-// reciprocal below 2^-126 may flush to 0).
-__device__ __forceinline__ float swiglu_fast(float g, float u) {
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-    return g * r * u;
-}
-__device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
 
 // Position of element e (0..31) of a block in the permuted 16-bit layout:
 // chunk t = (e mod 16) / 4, slot order (4t, 4t+2, 16+4t, 16+4t+2, 4t+1, 4t+3, 16+4t+1, 16+4t+3).
@@ -121,15 +101,13 @@ struct DequantLane {
 };
 
 // Dequantise one lane's share of half a weight tile (16 rows x 64 k: blocks 2*sub and 2*sub+1) into the
-// operand tile at a_base: 4 chunks of 16 bytes (rows g, g+8). The kernel issues this for every weight of a call, so its
-// instructions are counted: per 8 weights 1 shift, 4 logic, 4 subtract, 4 multiply, 1 select, 1 scale
-// permute, 1 store with a constant offset.
+// operand tile at a_base: 4 chunks of 16 bytes (rows g, g+8). (Beside store_weights: 1 select, 1 scale permute per 8 weights.)
 template <int Q>
 __device__ __forceinline__ void dequant_store(const WTile<Q>& w, int sub, uint32_t a_base, const DequantLane<Q>& dl) {
     if constexpr (Q == BF16) return;  // BF16 layers feed this path from plain f16 matrices (ATMA): no producers
     const uint32_t s_g = (sub == 0) ? w.s.x : w.s.y;   // f16 scales of blocks 2 sub, 2 sub + 1: row g
     const uint32_t s_g8 = (sub == 0) ? w.s.z : w.s.w;  // row g + 8
-    uint32_t v0[2][2], v1[2][2];  // [pass][row g | g + 8]: the block's words (Q8_0: elements 0..15 | 16..31)
+    uint32_t v0[2][2], v1[2][2] = {};  // [pass][row g | g + 8]: the block's words (Q8_0: elements 0..15 | 16..31)
     if (Q == Q4_0) {
         const uint4 v = w.q[sub];
         v0[0][0] = dl.odd ? v.z : v.x;
@@ -152,22 +130,7 @@ __device__ __forceinline__ void dequant_store(const WTile<Q>& w, int sub, uint32
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint32_t sc = prmt(r ? s_g8 : s_g, 0u, dl.bsel[p]);
-            uint32_t l0, l1, h0, h1;
-            if (Q == Q4_0) {
-                const uint32_t x = v0[p][r], y = x >> 8;
-                l0 = hsub2_u32(lop_and_or(x, 0x000F000Fu, dl.k.or_a), dl.k.sub_a);
-                h0 = hsub2_u32(lop_and_or(x, 0x00F000F0u, dl.k.or_b), dl.k.sub_b);
-                l1 = hsub2_u32(lop_and_or(y, 0x000F000Fu, dl.k.or_a), dl.k.sub_a);
-                h1 = hsub2_u32(lop_and_or(y, 0x00F000F0u, dl.k.or_b), dl.k.sub_b);
-            } else {
-                // bytes biased by 128 -> unsigned; 0x64xx = 1024 + xx; subtract 1152.
-                const uint32_t x = v0[p][r] ^ dl.k.or_b, y = v1[p][r] ^ dl.k.or_b;
-                l0 = hsub2_u32(prmt(x, dl.k.or_a, 0x4240u), dl.k.sub_a);
-                l1 = hsub2_u32(prmt(x, dl.k.or_a, 0x4341u), dl.k.sub_a);
-                h0 = hsub2_u32(prmt(y, dl.k.or_a, 0x4240u), dl.k.sub_a);
-                h1 = hsub2_u32(prmt(y, dl.k.or_a, 0x4341u), dl.k.sub_a);
-            }
-            sts128(a_base + dl.off[p] + r * 1024, hmul2_u32(l0, sc), hmul2_u32(h0, sc), hmul2_u32(l1, sc), hmul2_u32(h1, sc));
+            store_weights<Q>(a_base + dl.off[p] + r * 1024, v0[p][r], v1[p][r], sc, dl.k);
         }
 }
 
