@@ -547,7 +547,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
         const uint32_t units0 = stage0 + STAGES * STAGE_BYTES;
         const bool gather = (MODE == 0) && a.gather != nullptr;
         int tn = 0;
-        uint32_t u0 = 0;  // the tile's first unit
+        uint32_t u0 = 0;     // the tile's first unit
+        uint32_t asked = 0;  // behind this warp's last unit on its way
         bool ok = true;
         // this CTA's rows of the warp's set of a tile that begins at unit u: `half` of them from the returned column on
         auto rows_of = [&](const int4& t, uint32_t u, int& half) -> int {
@@ -618,15 +619,17 @@ grouped_gemm_pair_kernel(const __grid_constant__ Args a) {
                     }
                 }
                 __syncwarp();
+                asked = unit + 1;
             }
-            if (ok && !fetched) fetch_next();
+            if (!ok) break;
+            if (!fetched) fetch_next();
             u0 = u_next;
             tile = tile_n;
         }
-        // the copies land before the shared memory goes away. The second CTA cannot watch the first one's barriers: it
-        // waits as long as the first one does at most
+        // the copies land before the shared memory goes away (this warp's: every second unit up to the last one it asked for). The
+        // second CTA cannot watch the first one's barriers: it waits longer than the first one does at most
         if (lane == 0 && *abort_flag.flag) {
-            if (rank == 0) let_land(smem_u32(&full_bar[0]), UNITS, u0 + 2 * kgs);
+            if (rank == 0) let_land(smem_u32(&full_bar[0]), UNITS, asked, 2);
             else pause_ns(UNITS * 1000000ull);
         }
         __syncwarp();

@@ -54,12 +54,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const A
     }
 }
 
-// A role that gives up does not leave while its copies are on their way into shared memory: the last `stages` of the n
-// phases it has asked for on the ring of barriers at bar0, each complete or the limit over (a phase that other roles
-// have a part in may stay incomplete for good).
-__device__ __forceinline__ void let_land(uint32_t bar0, int stages, int n) {
+// A role that gives up does not leave while its copies are on their way into shared memory: of the phases up to number n - 1
+// that it has asked for on the ring of barriers at bar0, every step-th, those that the ring can still hold, each complete or the
+// limit over (a phase that other roles have a part in may stay incomplete for good).
+__host__ __device__ constexpr int first_to_land(int n, int stages, int step) {
+    return n <= 0 ? n : n > stages ? n - stages + step - 1 : (n - 1) % step;
+}
+static_assert(first_to_land(0, 4, 2) == 0 && first_to_land(1, 4, 2) == 0 && first_to_land(2, 4, 2) == 1 && first_to_land(3, 4, 2) == 0, "");
+static_assert(first_to_land(4, 4, 2) == 1 && first_to_land(5, 4, 2) == 2 && first_to_land(48, 4, 2) == 45, "");  // 45 and 47
+static_assert(first_to_land(0, 4, 1) == 0 && first_to_land(3, 4, 1) == 0 && first_to_land(9, 4, 1) == 5, "");
+__device__ __forceinline__ void let_land(uint32_t bar0, int stages, int n, int step = 1) {
     const uint64_t t0 = globaltimer_ns();
-    for (int q = n > stages ? n - stages : 0; q < n; ++q)
+    for (int q = first_to_land(n, stages, step); q < n; q += step)
         while (!mbar_try(bar0 + (q % stages) * 8, (q / stages) & 1) && globaltimer_ns() - t0 < 1000000ull) {
         }
 }

@@ -47,3 +47,8 @@ def kernels_of(call):
     if not names:
         pytest.skip("the profiler records no kernels on this machine")
     return names
+
+
+def pair_kernel(quant, mode, narrow):
+    """Name of the CTA-pair kernel of a layer (BF16: weights by TMA); mode 0 gate/up, 1 down; narrow: tiles of 128 columns, else 512."""
+    return f"grouped_gemm_pair_kernel<{quant}, {mode}, {str(quant == 2).lower()}, {str(narrow).lower()}>"

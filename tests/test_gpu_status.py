@@ -10,6 +10,7 @@ import torch
 
 from lumen_b200 import _lib, moe, synth
 from oracle import oracle
+from tests.gpu_util import kernels_of, pair_kernel
 
 pytestmark = pytest.mark.gpu
 
@@ -69,16 +70,18 @@ def test_grouped_gemm_stage_barrier_that_runs_out_is_reported_and_recoverable(cu
     assert torch.equal(again, good)
 
 
-# the same on CTA pairs (both CTAs give up), dequantised and TMA-fed weights
+# the same on CTA pairs (both CTAs give up), tiles of 128 columns (I = 256: too few of 512) and of 512, dequantised and TMA-fed weights
 @pytest.mark.parametrize("quant", [0, 1, 2])
-def test_pair_stage_barrier_that_runs_out_is_reported_and_recoverable(cuda_lib, quant):
-    H, I, E, K, T = 2048, 256, 8, 2, 1500
+@pytest.mark.parametrize("I,narrow", [(256, True), (640, False)])
+def test_pair_stage_barrier_that_runs_out_is_reported_and_recoverable(cuda_lib, quant, I, narrow):
+    H, E, K, T = 2048, 8, 2, 1500
     lay = synth.LayerLayout(H, I, E, quant)
     sc = moe.allocate_moe_scratch(H, I, E, K, T, flags=_lib.FLAG_SHORT_WAITS)
     layer = sc.prepare_layer(synth.make_layer_blob(lay, 0), lay.meta())
     x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(4), device="cuda")
     good = sc.prefill(layer, x, x).clone()
-    torch.cuda.synchronize()
+    names = kernels_of(lambda: sc.prefill(layer, x, x))
+    assert sum(pair_kernel(quant, mode, narrow) in k for k in names for mode in (0, 1)) == 2, names
     assert sc.poll_status() == _lib.OK
     sc.debug_expire_next_wait(1)
     sc.prefill(layer, x, x)
