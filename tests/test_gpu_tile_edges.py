@@ -6,7 +6,7 @@ import torch
 
 from lumen_b200 import _lib, moe, synth
 from oracle import oracle
-from tests.gpu_util import TOL_REL_L2, make_layer, oracle_layer, rel_l2
+from tests.gpu_util import TOL_REL_L2, kernels_of, make_layer, oracle_layer, pair_kernel, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -25,7 +25,8 @@ def logits_for_counts(counts, K):
     return torch.from_numpy(np.stack(rows)).cuda()
 
 
-def check_prefill(H, I, E, K, quant, lg, act=torch.float32):
+def check_prefill(H, I, E, K, quant, lg, act=torch.float32, kernels=False):
+    """kernels: the names of the call's kernels are returned."""
     T = lg.shape[0]
     lay, meta, blob_np, sc, layer = make_layer(H, I, E, K, quant, seed=T, max_tokens=T)
     g = torch.Generator("cuda").manual_seed(T + 1)
@@ -38,6 +39,7 @@ def check_prefill(H, I, E, K, quant, lg, act=torch.float32):
     assert np.array_equal(r["ids"], o_ids)
     assert rel_l2((out - res).cpu().numpy(), o_out - res.cpu().numpy()) < TOL_REL_L2
     assert torch.equal(out, sc.prefill(layer, x, res))
+    return kernels_of(lambda: sc.prefill(layer, x, res)) if kernels else None
 
 
 # streaming kernels: chunks of 32 columns, operands of 8; experts with none, one, one more than an operand or a chunk
@@ -62,12 +64,16 @@ def test_tcgen05_tiles_of_short_contractions(cuda_lib, quant, H, I, E, T):
 
 
 # products on CTA pairs, tiles of up to 512 columns: sets of 32..256 columns and what is left of them, one and two sets a
-# tile, contractions of one, two, three and many 128-input groups (tiles claimed four, two and one ahead)
+# tile, contractions of one, two, three and many 128-input groups (tiles claimed four, two and one ahead). Rows of 128
+# inputs (down products of one group) are one tile of 128 an expert: 64 experts, so that half of the pairs have one
+WIDE_COUNTS = [0, 1, 16, 31, 33, 64, 255, 256, 257, 288, 511, 512, 513, 1025, 7, 95]
+
+
 @pytest.mark.parametrize("quant", [0, 1, 2])
-@pytest.mark.parametrize("H,I", [(256, 1024), (2048, 384), (1536, 384), (3072, 512), (768, 640)])
-def test_pair_products_wide_tile_edges(cuda_lib, quant, H, I):
-    counts = [0, 1, 16, 31, 33, 64, 255, 256, 257, 288, 511, 512, 513, 1025, 7, 95]
-    check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1), torch.bfloat16)
+@pytest.mark.parametrize("H,I,E", [(256, 1024, 16), (2048, 384, 16), (1536, 384, 16), (3072, 512, 16), (768, 640, 16), (256, 128, 64), (512, 128, 64)])
+def test_pair_products_wide_tile_edges(cuda_lib, quant, H, I, E):
+    form = check_prefill(H, I, E, 1, quant, logits_for_counts(WIDE_COUNTS * (E // 16), 1), torch.bfloat16, kernels=True)
+    assert sum(pair_kernel(quant, mode, False) in k for k in form for mode in (0, 1)) == 2, form
 
 
 # tiles of up to 128 columns: operands of 32..128 columns, several tiles an expert, contractions of one group and more
@@ -75,7 +81,8 @@ def test_pair_products_wide_tile_edges(cuda_lib, quant, H, I):
 @pytest.mark.parametrize("H,I", [(256, 1024), (2048, 128), (1536, 384), (3072, 256), (768, 640)])
 def test_pair_products_narrow_tile_edges(cuda_lib, quant, H, I):
     counts = [0, 1, 16, 31, 32, 33, 63, 65, 96, 97, 127, 128, 129, 257, 7, 400]
-    check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1), torch.bfloat16)
+    form = check_prefill(H, I, 16, 1, quant, logits_for_counts(counts, 1), torch.bfloat16, kernels=True)
+    assert sum(pair_kernel(quant, mode, True) in k for k in form for mode in (0, 1)) == 2, form
 
 
 # tiles of 128 | 512: the last batch of the one and the first of the other; few experts; a grid capped at one CTA and at three
@@ -258,6 +265,9 @@ def test_single_expert_prefill(cuda_lib, quant, T, act, gating):
     assert rel_l2((out - res).cpu().numpy(), o_out - res.cpu().numpy()) < TOL_REL_L2
     r = sc.get_routing(T)
     assert (r["ids"] == 0).all() and np.array_equal(r["dst_to_col"].ravel(), np.arange(T))
+    if T > 16:
+        names = kernels_of(lambda: sc.prefill(layer, x, res))
+        assert sum(pair_kernel(quant, mode, T < 9728) in k for k in names for mode in (0, 1)) == 2, names
 
 
 # the fused decode kernel on one expert: no router exchange; items on some CTAs, on all, more than one each, ragged groups
