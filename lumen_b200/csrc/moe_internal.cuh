@@ -61,24 +61,23 @@ struct LayerDev {
 };
 
 // Form of the tcgen05 products of a one-GPU call: columns per tile, and whether CTA pairs work them (prefill_pair.cu: 512 or
-// 128 columns) or single CTAs (prefill_tc.cu, only where the grid is capped at one: gate/up 256 or 128, down 128).
+// 128 columns) or single CTAs (prefill_tc.cu, only where the grid is capped at one: 256 or 128).
 // Pairs, 512: once the experts average so many columns that tiles of 128 would be cut often (E = 128, I = 768, us from the host, tiles of
 // 128 and of 512: Q4_0 112 columns 249 and 261, 128 columns 301 and 275; f16 matrices, whose weights come through the
 // ring as they are, 128 columns 320 and 332, 144 columns 360 and 345), and its tiles give half of the pairs work (a lone expert of
 // 2048 x 512: 2048 tokens 65 and 80, 4096 90 and 90; four experts of 1024 x 512 with 200 columns 37 and 41, sixteen with
 // 150 48 and 44).
-// One CTA, 256: above 128 columns an expert (16 experts of 1024 x 512, K = 4, ms a call, tiles of 128 and of 256: Q4_0 700 tokens 1.88
-// and 1.56, 2000 4.20 and 3.60; Q8_0 2000 4.37 and 3.74; BF16 540 1.22 and 1.03, 2000 3.15 and 2.79).
+// One CTA, 256: above 128 columns an expert (16 experts of 1024 x 512, K = 4, ms a call, gate/up and down tiles of 128 and of 256: Q4_0 700
+// tokens 1.88 and 1.37, 2000 4.20 and 3.34; Q8_0 2000 4.37 and 3.49; BF16 2000 3.15 and 2.86).
 // ctas: cap of the persistent grid (0 = every SM).
 struct TcForm {
-    int cols, down_cols;
+    int cols;
     bool pairs;
 };
 inline TcForm tc_form(const LayerDev& L, int columns, int sms, int ctas) {
-    if (ctas == 1) return TcForm{columns > 128 * L.E ? 256 : 128, 128, false};
+    if (ctas == 1) return TcForm{columns > 128 * L.E ? 256 : 128, false};
     const int least = L.gu16 != nullptr ? 136 : 120, tiles = (columns / 512 > L.E ? columns / 512 : L.E) * (L.I / 128);
-    const int cols = columns > least * L.E && 4 * tiles >= sms ? 512 : 128;
-    return TcForm{cols, cols, true};
+    return TcForm{columns > least * L.E && 4 * tiles >= sms ? 512 : 128, true};
 }
 
 // Routing tables of one call (device pointers into the context's scratch).

@@ -12,7 +12,8 @@
 // (Zipf-skewed loads) without padding M. Down ("tokens are the M operand"): for up to 128
 // columns,  D[128 tokens, 256 output rows] += S[128, k] W[256, k]^T, one MMA per 16 inputs
 // whose N operand is the stage's two adjacent 128-row weight tiles, so that an epilogue
-// thread owns one token and stores 32 bytes at a time.
+// thread owns one token and stores 32 bytes at a time; a tile of up to 256 columns (a grid capped at one CTA) is two such
+// products against the same weight stage, into the two accumulator sets.
 //
 // One CTA per SM, persistent over a device-built tile list, warp-specialised (27 warps):
 //   warps 0-7   epilogue: tcgen05.ld of the accumulators, SwiGLU (gate/up), f16 stores
@@ -182,12 +183,11 @@ __device__ unsigned long long g_tc_trace[2][160][8];
 template <int Q, int MODE, int BN, bool ATMA = false, bool STG = false>
 __global__ void __launch_bounds__(THREADS, 1)
 grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
-    static_assert(!STG || MODE == 1, "the staged epilogue belongs to the down product");
-    static_assert(MODE == 0 || BN == 128, "down tiles are 128 tokens");
+    static_assert(!STG || (MODE == 1 && BN == 128), "the staged epilogue belongs to the 128-token down product");
     // Two 128-row weight operands share every activation stage (gate and up rows of the
     // same I range; two adjacent row tiles of the down matrix): the activation operand,
     // which comes from L2 at 2 bytes per element, is then read at half the rate.
-    // 256-column tiles (gate/up of expert-parallel calls whose experts average more than 128 columns): each dequantised
+    // 256-column tiles (experts of more than 128 columns on average; down: not in an expert-parallel call): each dequantised
     // weight tile serves 256 columns, and with K = H the main loop is long; the two 256-column f32
     // accumulators of a full tile fill TMEM (512 columns), so its epilogue is not overlapped with
     // the next tile's MMAs (its producers do run ahead).
@@ -197,7 +197,9 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
     constexpr int NA = 2;
     // BN: columns per tile
     // Accumulator sets in TMEM (512 columns), always two.
-    // Down: a set is 256 columns (the output rows of an m-tile) for 128 tokens.
+    // Down: a set is 256 columns (the output rows of an m-tile) for 128 tokens; a 256-token tile of
+    // the BN = 256 form takes both at once (its two token halves, one weight stage serving both),
+    // a tile of up to 128 tokens takes one, and the epilogue works through the halves one by one.
     // Gate/up, BN = 128: a set is the gate and the up accumulator side by side (2 x 128 columns).
     // Gate/up, BN = 256: the gate accumulator lives in TMEM columns 0..255 and the up accumulator in
     // 256..511; a tile of up to 128 columns (the last chunk of most experts under skewed loads) takes
@@ -302,7 +304,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
 
     // Epilogue of one tile by one warp: the warp's TMEM lanes are 32 (warp % 4).. (hardware rule);
     // of the tile's 16-column TMEM chunks it takes those with chunk % nparts == part.
-    auto epilogue_part = [&](const int4& tile, int ab, int part, int nparts) {
+    auto epilogue_part = [&](const int4& tile, int ab, int h, int part, int nparts) {
         const int row = (warp & 3) * 32 + lane;
         const int ncols = tile.z;
         const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + ab * ACC_COLS;
@@ -312,7 +314,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
             // output rows per load: its stores are 32 bytes wide and each token's 512 bytes are
             // contiguous (a whole NVLink packet when the row lives on another rank).
             {
-                const int tcol = row;  // token column of the tile
+                const int tcol = h * 128 + row;  // token column of the tile (h: its half of a 256-token tile)
                 bool live = tcol < ncols;
                 __half* dst = a.out16;
                 if (live) {
@@ -432,18 +434,22 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
     };
     constexpr int EPI_PARTS = EPI_WARPS / 4 + (HELP ? A_WARPS / 4 : 0);  // groups of four warps sharing a tile's epilogue
     // A warp's share of one tile's epilogue. v: accumulator sets handed over so far (set v % NACC, used v / NACC times
-    // before). A gate/up tile of more than 128 columns holds both sets.
+    // before). A tile of more than 128 columns holds both sets: the down product works
+    // through them one after the other (its two token halves), gate/up reads them as one tile.
     auto epilogue_tile = [&](const int4& tile, int& v, int part) -> bool {
         const int nsets = (tile.z > 128) ? 2 : 1;
-        for (int j = 0; j < nsets; ++j)
-            if (!mbar_wait(smem_u32(&acc_full_bar[(v + j) % NACC]), ((v + j) / NACC) & 1, abort_flag)) return false;
-        tc_fence_after();
-        epilogue_part(tile, nsets == 2 ? 0 : v % NACC, part, EPI_PARTS);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0)
-            for (int j = 0; j < nsets; ++j) mbar_arrive(smem_u32(&acc_empty_bar[(v + j) % NACC]));
-        v += nsets;
+        const int passes = (MODE == 1) ? nsets : 1, per_pass = (MODE == 1) ? 1 : nsets;
+        for (int h = 0; h < passes; ++h) {
+            for (int j = 0; j < per_pass; ++j)
+                if (!mbar_wait(smem_u32(&acc_full_bar[(v + j) % NACC]), ((v + j) / NACC) & 1, abort_flag)) return false;
+            tc_fence_after();
+            epilogue_part(tile, per_pass == 2 ? 0 : v % NACC, h, part, EPI_PARTS);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                for (int j = 0; j < per_pass; ++j) mbar_arrive(smem_u32(&acc_empty_bar[(v + j) % NACC]));
+            v += per_pass;
+        }
         return true;
     };
 
@@ -672,7 +678,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
             for (; ok && next_tile_warp(tn, tile); ++tl) {
                 const int n16 = (tile.z + 15) & ~15;
                 // down: D[128 tokens, 256 output rows] = X[128, k] W[256, k]^T, the two adjacent 128-row
-                // weight operands of a stage forming one 256-row N operand
+                // weight operands of a stage forming one 256-row N operand; a tile of more than 128
+                // tokens is two such products per 16 inputs, into two accumulator sets
                 const uint32_t idesc = make_idesc(MODE == 1 ? 256 : n16, false);  // (every operand is f16)
                 const int nh = (tile.z > 128) ? 2 : 1;  // accumulator sets of the tile
                 for (int h = 0; ok && h < nh; ++h) {
@@ -682,7 +689,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t acc0 = tmem_base + (v % NACC) * ACC_COLS;
+                const uint32_t acc0 = tmem_base + (v % NACC) * ACC_COLS, acc1 = tmem_base + ((v + 1) % NACC) * ACC_COLS;
                 for (int kh = 0; kh < khs; ++kh) {
                     if (kh == go_kh && lane == 0) mbar_arrive(smem_u32(&sched_go_bar[tl % ahead]));  // the CTA's next tile may be claimed now
                     ok = __all_sync(0xffffffffu, TRACE_WAIT(tr_wf, mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag)));
@@ -695,6 +702,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ Args a) {
                             const uint32_t acc = (kh > 0 || j > 0) ? 1u : 0u;
                             if (MODE == 1) {
                                 umma(acc0, b0 + j * 2, w0 + j * 2, idesc, acc);
+                                if (BN == 256 && nh == 2) umma(acc1, b0 + (SUB_BYTES >> 4) + j * 2, w0 + j * 2, idesc, acc);
                             } else {
 #pragma unroll
                                 for (int op = 0; op < NA; ++op)
@@ -843,6 +851,9 @@ cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, c
     const int max_ct = C / gu_cols + p.L.E;
     // rows that go to other ranks' return buffers leave through the staged epilogue (bulk copies)
     const bool stg = peer != nullptr;
+    // down tiles as wide as the gate/up ones, except there: its epilogue stores into other GPUs' memory, and with two
+    // independent accumulator sets those stores always run under the next tile's MMAs
+    const bool dn256 = gu_cols == 256 && !stg;
     const int mt_gu = p.L.I / 128;
     tc::Args gu{};
     cudaError_t te = make_tmap_f16(x16, (uint64_t)C, (uint64_t)p.L.H, tc::bbox_rows(gu_cols), &gu.tmap);
@@ -858,7 +869,7 @@ cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, c
     gu.kdim = p.L.H;
     gu.out_ld = p.L.I;
     tc::Args dn = gu;
-    te = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, tc::bbox_rows(128), &dn.tmap);
+    te = make_tmap_f16(p.s16, (uint64_t)C, (uint64_t)p.L.I, tc::bbox_rows(dn256 ? 256 : 128), &dn.tmap);
     if (te != cudaSuccess) return te;
     dn.debug_extra_tx = 0;  // the hook applies to the first kernel of the pair
     dn.tiles = p.tiles + (size_t)max_ct * (mt_gu > 0 ? mt_gu : 1);  // as laid out by launch_route_large
@@ -882,19 +893,19 @@ cudaError_t launch_grouped_tc(const PrefillArgs& p, const void* x16, int grid, c
         e = (gu_cols == 256) ? launch_tc_one<BF16, 0, 256, true>(gu, grid, st) : launch_tc_one<BF16, 0, 128, true>(gu, grid, st);
         if (e != cudaSuccess) return e;
         if (stg) return launch_tc_one<BF16, 1, 128, true, true>(dn, grid, st);
-        return launch_tc_one<BF16, 1, 128, true>(dn, grid, st);
+        return dn256 ? launch_tc_one<BF16, 1, 256, true>(dn, grid, st) : launch_tc_one<BF16, 1, 128, true>(dn, grid, st);
     }
     switch (p.L.quant) {
         case Q4_0:
             e = (gu_cols == 256) ? launch_tc_one<Q4_0, 0, 256>(gu, grid, st) : launch_tc_one<Q4_0, 0, 128>(gu, grid, st);
             if (e != cudaSuccess) return e;
             if (stg) return launch_tc_one<Q4_0, 1, 128, false, true>(dn, grid, st);
-            return launch_tc_one<Q4_0, 1, 128>(dn, grid, st);
+            return dn256 ? launch_tc_one<Q4_0, 1, 256>(dn, grid, st) : launch_tc_one<Q4_0, 1, 128>(dn, grid, st);
         case Q8_0:
             e = (gu_cols == 256) ? launch_tc_one<Q8_0, 0, 256>(gu, grid, st) : launch_tc_one<Q8_0, 0, 128>(gu, grid, st);
             if (e != cudaSuccess) return e;
             if (stg) return launch_tc_one<Q8_0, 1, 128, false, true>(dn, grid, st);
-            return launch_tc_one<Q8_0, 1, 128>(dn, grid, st);
+            return dn256 ? launch_tc_one<Q8_0, 1, 256>(dn, grid, st) : launch_tc_one<Q8_0, 1, 128>(dn, grid, st);
         default:
             // BF16 layers always carry their plain f16 matrices on this path (see above)
             return cudaErrorInvalidValue;

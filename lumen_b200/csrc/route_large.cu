@@ -905,10 +905,9 @@ cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st) {
     const int T = a.T, E = a.L.E, H = a.L.H, K = a.K;
     const float* lg = a.logits_override;
     const int C = T * K;
-    // columns per grouped-GEMM tile (the streaming kernels share one list of column chunks and cut the rows themselves)
+    // columns per grouped-GEMM tile, the same for gate/up and down (the streaming kernels share one list of column chunks and cut the rows themselves)
     const bool stream = (a.impl == 2);
-    const TcForm form = tc_form(a.L, C, a.sms, a.tc_ctas);
-    const int tile_cols = stream ? STREAM_CHUNK : form.cols, tile_cols_dn = stream ? STREAM_CHUNK : form.down_cols;
+    const int tile_cols = stream ? STREAM_CHUNK : tc_form(a.L, C, a.sms, a.tc_ctas).cols, tile_cols_dn = tile_cols;
     const int max_ct = C / tile_cols + E, max_ct_dn = C / tile_cols_dn + E;
     const int mt_gu = stream ? 1 : a.L.I / 128, mt_dn = a.L.H / 256;  // m-tiles: 128 gate + 128 up rows | 256 down rows
     int4* tiles_gu = a.tiles;

@@ -88,13 +88,14 @@ def test_warps_of_a_decode_batch(cuda_lib, quant, H, I, E, K, T, gate_up, down):
     assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2
 
 
-# tcgen05 products on a grid capped at one CTA: gate/up in tiles of 256 columns above 128 columns an expert
+# tcgen05 products on a grid capped at one CTA: tiles of 256 columns above 128 columns an expert
 @pytest.mark.parametrize("quant,flags,T,cols", [(2, 0, 1025, 256), (2, 0, 1024, 128), (1, F16, 1025, 256), (1, 0, 1025, 256), (0, 0, 1024, 128)])
 def test_gate_up_tiles_of_one_cta(cuda_lib, quant, flags, T, cols):
     sc, layer = context(512, 384, 16, 2, quant, T, flags | _lib.flag_tc_ctas(1))
     x = rows(T, 512)
     names = kernels_of(lambda: sc.prefill(layer, x, x))
-    assert [k for k in names if "grouped_gemm_tc_kernel" in k and f", 0, {cols}," in k], names
+    for mode in (0, 1):
+        assert [k for k in names if "grouped_gemm_tc_kernel" in k and f", {mode}, {cols}," in k], names
 
 
 # rows gathered by column are kept only where a kernel reads them: a grid capped at one CTA
