@@ -617,7 +617,7 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
         s->expire_next[1] = 0;
     }
     if (p.impl == 2) {
-        CUDA_TRY(launch_stream_prefill(p, batch * s->K, s->xr16, out16_rows, st));
+        CUDA_TRY(launch_stream_prefill(p, s->xr16, out16_rows, st));
         if (out16_rows) return Status::Ok();
     } else if (p.impl == 0) {
         const TcForm form = tc_form(layer.dev, batch * s->K, s->sms, s->tc_ctas);

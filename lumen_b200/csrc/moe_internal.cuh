@@ -308,9 +308,7 @@ inline int stream_max_columns_of_any(int experts) { return 12 * experts > 16 ? 1
 // gate/up of a decode batch, expert products of short prompts (stream.cu)
 cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st);
 cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_up, cudaStream_t st);
-// (columns: of the layer's experts in all, as far as the host knows them)
-cudaError_t launch_stream_prefill(const PrefillArgs& p, int columns, const __half* x16, __half* out16_rows, cudaStream_t st,
-                                  const TcPeerOut* peer = nullptr);
+cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __half* out16_rows, cudaStream_t st, const TcPeerOut* peer = nullptr);
 constexpr int STREAM_SHIFT = 5;
 constexpr int STREAM_CHUNK = 1 << STREAM_SHIFT;  // columns of an expert that one item of the streaming kernels multiplies
 

@@ -36,7 +36,7 @@ using namespace dcommon;
 
 enum Mode { GATE_UP_1, DOWN_1, GATE_UP_2, DOWN_2, DOWN_2I };
 
-// Warps per SM and groups in flight per warp: 131..221 KB on the way per SM (the copy peak times the latency is ~55 KB),
+// Warps per SM and groups in flight per warp: 131..197 KB on the way per SM (the copy peak times the latency is ~55 KB),
 // the rest of the 256 KB is L1 for the activations. An item is a chain (its chunk, its columns, its tiles, its rows out), and
 // the warps of an SM end unevenly; more warps with shorter rings help the decode down products, whose items are short (16 warps
 // -> now, us a call: 4 tokens of Q8_0, 1408 inputs, 53.1 -> 50.2; 8 tokens of Q4_0, 512 inputs, 40.8 -> 39.1; with 32 warps
@@ -566,7 +566,7 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_u
 }
 
 // Expert products of a short prompt: x16 rows by token (planes' element order), s16 by column.
-cudaError_t launch_stream_prefill(const PrefillArgs& p, int columns, const __half* x16, __half* out16_rows, cudaStream_t st,
+cudaError_t launch_stream_prefill(const PrefillArgs& p, const __half* x16, __half* out16_rows, cudaStream_t st,
                                   const TcPeerOut* peer) {
     stream::Args g{};
     g.L = p.L;
@@ -592,17 +592,9 @@ cudaError_t launch_stream_prefill(const PrefillArgs& p, int columns, const __hal
     d.out16 = out16_rows ? out16_rows : p.d16;
     d.out_row_map = out16_rows ? p.R.col_src_tok : nullptr;
     if (peer) d.peer = *peer;
-    // Q4_0: 24 warps where an SM has four rounds of items for them and two to nine columns an expert, rows of 1024 inputs and more; shorter
-    // ones between 4.5 and 6 columns. Beyond, where many experts have more than one operand of eight columns, their registers (80, spills)
-    // cost more than they hide. (16 and 24 warps, us replayed, by columns an expert. E = 64, 4096 x 1536: 2.3 186 and 185, 4.5 212 and 206, 7.5 256 and
-    // 245, 9 262 and 254, 11 352 and 386; E = 128, 2048 x 1024: 3 139 and 138, 5 151 and 146, 8 174 and 171; E = 128, 2048 x 768: 4 112.5 and 112.8, 5 120 and 117, 6
-    // 125 and 123, 7 131 and 131, 8 150 and 154; E = 256, 2048 x 512: 3 143 and 141, 5 163 and 161, 6.3 175 and 181, 8 202 and
-    // 211. Fewer items: E = 64, 2048 x 1024, K = 4: 4 88 and 90; E = 64, 1024 x 256, K = 4: 6 34.8 and 35.5; a lone expert of
-    // 2048 x 4096: 8 49 and 51.)
-    const int E = p.L.E;
-    const bool wide = p.L.quant == Q4_0 && (long long)E * p.L.rt_h >= 96ll * p.sms &&
-                      (p.L.kg_i >= 8 ? columns > 2 * E && columns <= 9 * E : 2 * columns > 9 * E && columns <= 6 * E);
-    if (wide) return stream::launch_t<Q4_0, stream::DOWN_1, 24>(d, p.sms, st);
+    // (24 warps of Q4_0, with the 80 registers that they leave, gain up to 4 % under even loads and lose 6-14 % where some experts have several
+    // operands of eight columns, which the host cannot see: 83 tokens of 2048 x 768, E = 128, 121 and 117 us, with Zipf loads 144 and
+    // 158; 64 tokens of 4096 x 1536, E = 64, 222 and 212, 280 and 299)
     return stream::launch_q<stream::DOWN_1>(d, p.sms, st);
 }
 

@@ -20,36 +20,19 @@ def rows(T, H):
     return torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(T), device="cuda")
 
 
-# streaming down product of Q4_0 prompts: 24 warps for enough items (E * H / 16 rows of tiles) and more than two, up to nine columns of long rows,
-# 4.5 to 6 columns of short ones; 16 elsewhere
-@pytest.mark.parametrize("I,E,K,T,flags,warps", [(1024, 256, 2, 256, 0, 16), (1024, 256, 2, 257, 0, 24), (1024, 256, 2, 1024, 0, 24),
-                                                 (1024, 256, 2, 1152, F16, 24), (1024, 256, 2, 1153, F16, 16), (1024, 128, 2, 300, 0, 16),
-                                                 (128, 256, 2, 576, 0, 16), (128, 256, 2, 577, 0, 24), (128, 256, 2, 768, 0, 24),
-                                                 (128, 256, 2, 769, 0, 16), (2048, 1, 1, 8, 0, 16)])
-def test_warps_of_a_prompts_streaming_down_product(cuda_lib, I, E, K, T, flags, warps):
+# streaming down product of Q4_0 prompts: 16 warps whatever the columns, whose distribution over the experts the host does not know
+@pytest.mark.parametrize("I,E,K,T,flags", [(1024, 256, 2, 256, 0), (1024, 256, 2, 257, 0), (1024, 256, 2, 1024, 0), (1024, 256, 2, 1152, F16),
+                                           (128, 256, 2, 577, 0), (128, 256, 2, 768, 0), (2048, 1, 1, 8, 0)])
+def test_warps_of_a_prompts_streaming_down_product(cuda_lib, I, E, K, T, flags):
     H = 1024
     sc, layer = context(H, I, E, K, 1, T, flags)
     x = rows(T, H)
     out = torch.empty_like(x)
     names = kernels_of(lambda: sc.prefill(layer, x, x, out))
-    assert [k for k in names if f"stream_kernel<1, 1, {warps}>" in k] and sum("stream_kernel<1, 1," in k for k in names) == 1, names
+    assert [k for k in names if "stream_kernel<1, 1, 16>" in k] and sum("stream_kernel<1, 1," in k for k in names) == 1, names
     ref, ref_layer = context(H, I, E, K, 1, T, _lib.FLAG_PREFILL_MMA)
     want = ref.prefill(ref_layer, x, x)
     assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2
-
-
-# an expert-parallel call: by its own columns, not by what its window could take
-@pytest.mark.parametrize("T,warps", [(2, 16), (256, 16), (257, 24)])
-def test_warps_of_an_expert_parallel_streaming_down_product(cuda_lib, T, warps):
-    from lumen_b200 import ep
-    H, I, E, K = 1024, 1024, 256, 2
-    lay = synth.LayerLayout(H, I, E, 1)
-    pe = ep.PushExpertParallel(H, I, E, K, 1024, 0, 1, 0)
-    layer = pe.prepare_layer(synth.make_layer_blob(lay, 5), lay.meta())
-    x = rows(T, H)
-    names = kernels_of(lambda: pe.forward(layer, x, x))
-    assert [k for k in names if f"stream_kernel<1, 1, {warps}>" in k] and sum("stream_kernel<1, 1," in k for k in names) == 1, names
-    pe.close()
 
 
 # the longest prompt on the streaming kernels: planes (8 columns an expert), narrow ones (12 | 9, a lone expert 16), layers kept as
