@@ -529,8 +529,8 @@ Status encode_route_only(CudaMoeScratch* s, const MoeLayer* layer, const float* 
 // Which prompts take the streaming kernels: those whose experts have so few columns on average that
 // the call is bound by reading the weights, not by multiplying. (BF16 layers have their f16 matrices copied by
 // TMA on the tcgen05 path, which then is bound by HBM as well: 240 against 224 us at 64 tokens.)
-static bool prefill_streams(int columns, const LayerDev& L, const void* normed) {
-    return L.quant != BF16 && L.H % 128 == 0 && L.I % 128 == 0 && L.H >= 256 && columns <= stream_max_columns(L, L.E) &&
+static bool prefill_streams(const CudaMoeScratch* s, int columns, const LayerDev& L, const void* normed) {
+    return L.quant != BF16 && L.H % 128 == 0 && L.I % 128 == 0 && L.H >= 256 && columns <= stream_max_columns(L, L.E, s->sms, s->tc_ctas) &&
            reinterpret_cast<uintptr_t>(normed) % 16 == 0;
 }
 
@@ -584,7 +584,7 @@ Status encode_moe_ffn_prefill_grouped(CudaMoeScratch* s, const MoeLayer& layer, 
     const bool tc_ok = (s->H % 256 == 0) && (s->I % 128 == 0) && (reinterpret_cast<uintptr_t>(normed) % 16 == 0) &&
                        (reinterpret_cast<uintptr_t>(out16_rows) % 32 == 0);
     p.impl = (s->prefill_impl == 1 || !tc_ok) ? 1 : 0;
-    if (s->prefill_impl == 0 && prefill_streams(batch * s->K, layer.dev, normed)) {
+    if (s->prefill_impl == 0 && prefill_streams(s, batch * s->K, layer.dev, normed)) {
         p.impl = 2;
         p.stream_starts = reinterpret_cast<int32_t*>(s->R.work);  // (decode's work records: 8 KB, unused by a prefill)
     }

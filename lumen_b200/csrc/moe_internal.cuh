@@ -298,11 +298,20 @@ cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_ca
 //                    bytes are not what counts (eight of 2048 x 512 at 6 columns 38.9 and 37.3): as planes
 // The same line for an expert-parallel call, whose results are one GPU's to the bit. There it costs time: its one-CTA tiles overtake
 // later (2048 x 768, E = 128, one rank: Q4_0 8.1 columns 199 streaming and 222 on tiles, 10 columns 220 and 223, 11 columns 236 and 224).
-inline int stream_max_columns(const LayerDev& L, int experts) {
+// ctas: cap of the tcgen05 grid, which the streaming kernels do not have (0 = none). The line rises with the waves of gate/up tiles that the cap
+// adds, up to 12 columns (Q8_0 9, a lone expert 16). 2048 x 768, E = 128, Q4_0, streaming and tiles: 9 columns on 120 CTAs 163 and 168, 12 columns on 100
+// 193 and 196, on 48 194 and 359, 9 columns on one CTA 164 and 19393; a lone expert of few tiles keeps its line down to a few CTAs.
+inline int stream_max_columns(const LayerDev& L, int experts, int sms, int ctas) {
     const bool q4 = L.quant == Q4_0;
-    if (L.gu16 != nullptr && experts >= 32) return (q4 ? 12 : 10) * experts;
-    if (L.H <= 512) return experts == 1 ? 16 : (q4 ? 12 : 9) * experts;
-    return 8 * experts;
+    int most = 8 * experts;
+    if (L.gu16 != nullptr && experts >= 32) most = (q4 ? 12 : 10) * experts;
+    else if (L.H <= 512) most = experts == 1 ? 16 : (q4 ? 12 : 9) * experts;
+    if (ctas > 0 && ctas < sms) {
+        const int tiles = 2 * experts * ((L.I + 127) / 128), ceiling = experts == 1 ? 16 : (q4 ? 12 : 9) * experts;  // (a tile of 128 rows occupies a pair)
+        const int capped = most * ((tiles + ctas - 1) / ctas) / ((tiles + sms - 1) / sms);
+        if (capped > most && most < ceiling) most = capped < ceiling ? capped : ceiling;
+    }
+    return most;
 }
 inline int stream_max_columns_of_any(int experts) { return 12 * experts > 16 ? 12 * experts : 16; }
 // gate/up of a decode batch, expert products of short prompts (stream.cu)

@@ -54,6 +54,38 @@ def test_longest_prompt_on_the_streaming_kernels(cuda_lib, quant, flags, H, E, K
         assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2
 
 
+# ... where the tcgen05 grid is capped: 12 | 9 columns and a lone expert 16 on a few CTAs, 8 columns on nearly all
+@pytest.mark.parametrize("ctas,quant,flags,E,K,T,tiles", [(1, 1, 0, 16, 4, 48, "tc"), (1, 0, 0, 16, 4, 36, "tc"), (1, 1, F16, 16, 4, 48, "tc"), (1, 1, 0, 1, 1, 16, "tc"),
+                                                          (2, 1, 0, 16, 4, 48, "pair"), (24, 1, 0, 16, 4, 48, "pair"), (146, 1, 0, 16, 4, 32, "pair"),
+                                                          (48, 1, 0, 1, 1, 8, "pair")])
+def test_longest_prompt_on_the_streaming_kernels_beside_a_capped_grid(cuda_lib, ctas, quant, flags, E, K, T, tiles):
+    H, I = 1024, 256
+    sc, layer = context(H, I, E, K, quant, T + 1, flags | _lib.flag_tc_ctas(ctas))
+    ref, ref_layer = context(H, I, E, K, quant, T + 1, _lib.FLAG_PREFILL_MMA)
+    for n, name in ((T, "stream_kernel"), (T + 1, f"grouped_gemm_{tiles}_kernel")):
+        x = rows(n, H)
+        out = torch.empty_like(x)
+        names = kernels_of(lambda: sc.prefill(layer, x, x, out))
+        assert sum(name in k for k in names if "stream_kernel" in k or "grouped_gemm" in k) == 2, names
+        want = ref.prefill(ref_layer, x, x)
+        assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2
+
+
+# an expert-parallel call on a capped grid draws the one-GPU line of its planes: the same bits on both sides of it
+@pytest.mark.parametrize("T", [40, 48, 49])
+def test_expert_parallel_call_beside_a_capped_grid(cuda_lib, T):
+    from lumen_b200 import ep
+    H, I, E, K, flags = 1024, 256, 16, 4, _lib.flag_tc_ctas(1)
+    sc, layer = context(H, I, E, K, 1, T, flags)
+    lay = synth.LayerLayout(H, I, E, 1)
+    pe = ep.PushExpertParallel(H, I, E, K, 64, 0, 1, 0, flags=flags)
+    pe_layer = pe.prepare_layer(synth.make_layer_blob(lay, 5), lay.meta())
+    x = rows(T, H)
+    want, got = sc.prefill(layer, x, x), pe.forward(pe_layer, x, x)
+    assert pe.sc.poll_status() == _lib.OK and torch.equal(got, want)
+    pe.close()
+
+
 # decode batches: more warps where an SM's items take a round less with them (gate/up of BF16 8 | 10, down of Q8_0 16 | 20, of BF16 8 | 12)
 @pytest.mark.parametrize("quant,H,I,E,K,T,gate_up,down", [(2, 2048, 768, 128, 8, 4, 10, 12), (2, 2048, 768, 128, 8, 5, 8, 12), (2, 2048, 512, 256, 8, 5, 10, 12),
                                                           (2, 2048, 512, 256, 8, 16, 8, 12), (2, 2048, 768, 128, 8, 16, 10, 8), (2, 1024, 384, 64, 4, 12, 8, 8),
