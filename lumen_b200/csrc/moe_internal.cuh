@@ -286,16 +286,20 @@ cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_ca
                              int sms);
 // Most columns of a prompt that the streaming kernels take (experts: of the whole call, an expert-parallel rank's layer has
 // a share of them). The line lies where the CTA-pair kernels overtake them, us replayed, streaming and pairs:
-//   planes           E = 128, 2048 x 768: Q4_0 7 columns an expert 131 and 144, 8 columns 150 and 146, 10 columns 170 and 147; Q8_0 7 columns
-//                    162 and 163, 8 columns 183 and 164; E = 32, 1024 x 512: 8 columns 33.9 and 39.0 (Q4_0), 38.7 and 41.8 (Q8_0), 9
-//                    columns 37.7 and 39.1, 42.5 and 41.9. A lone expert of 2048 x 512: 8 columns 32.9 and 34.9, 9 columns 38.0 and 34.8
+//   planes           E = 128, 2048 x 768: Q4_0 7 columns an expert 131 and 143, 8 columns 144 and 144, 10 columns 168 and 147; Q8_0 7 columns
+//                    161 and 164, 8 columns 174 and 164. A lone expert of 2048 x 512: 8 columns 32.9 and 34.9, 9 columns 38.0 and 34.8
+//   small planes     with up to 1536 inputs and no more items than the SMs have warps, one item's chain is the kernel's time, and it grows when
+//                    some expert has a third operand of columns: 9 columns of E = 32, 1024 x 512 35.8 and 39.2 (Q4_0), 39.0 and 42.2 (Q8_0), of
+//                    E = 16, 1024 x 1024 35.8 and 38.9; 11 columns of the former 43.3 and 39.0; E = 64, 1024 x 512 at 8 columns 49.3 and 51.8, at 9
+//                    55.9 and 52.3; E = 64, 768 x 512 at 9 45.0 and 46.5
 //   narrow planes    rows of up to 512 inputs are a short chain of copies for a streaming warp, while the pairs' set-up stays: 16 experts of
 //                    512 x 256 at 8 columns 25.7 and 28.7, at 12 columns 27.7 and 28.7; 128 of them at 12 columns 42.4 and 44.2 (Q4_0), at 9
 //                    columns 45.5 and 46.8, at 10 columns 49.0 and 46.7 (Q8_0); a lone one at 13 columns 24.7 and 26.6
-//   f16 matrices     the pairs multiply these, four (Q4_0) or two times the bytes that the streaming kernels read from the planes: E = 128,
-//                    2048 x 768: Q4_0 8.1 columns 158 and 212, 12 columns 195 and 215, 14 columns 223 and 217; Q8_0 10 columns 204 and 213, 11
-//                    columns 219 and 214; E = 32, 1024 x 512: Q4_0 12 columns 43.6 and 44.2, Q8_0 10 columns 45.0 and 45.2. With few experts the
-//                    bytes are not what counts (eight of 2048 x 512 at 6 columns 38.9 and 37.3): as planes
+//   f16 matrices     the pairs multiply these, four (Q4_0) or two times the bytes that the streaming kernels read from the planes, which counts
+//                    where the matrices are more than 100 MB: E = 128, 2048 x 768: Q4_0 8 columns 146 and 209, 12 columns 196 and 214; Q8_0 10 columns
+//                    202 and 212, 11 columns 217 and 213; E = 16, 2048 x 1408 at 11 columns 61 and 73; E = 8, 1024 x 2816 at 10 columns 48 and 52; but
+//                    100 MB of E = 32, 2048 x 256 at 7 columns 47.0 and 46.0, at 8 columns 61.3 and 46.1, of E = 8, 2048 x 1024 at 9 columns 45.5 and 45.2.
+//                    Many short rows again have the longer line: E = 32, 1024 x 512 at 10 columns 37.1 and 44.6, at 12 columns 45.0 and 44.7
 // The same line for an expert-parallel call, whose results are one GPU's to the bit. There it costs time: its one-CTA tiles overtake
 // later (2048 x 768, E = 128, one rank: Q4_0 8.1 columns 199 streaming and 222 on tiles, 10 columns 220 and 223, 11 columns 236 and 224).
 // ctas: cap of the tcgen05 grid, which the streaming kernels do not have (0 = none). The line rises with the waves of gate/up tiles that the cap
@@ -304,8 +308,9 @@ cudaError_t launch_tile_plan(const RouteDev& R, int E, int H, int I, int rows_ca
 inline int stream_max_columns(const LayerDev& L, int experts, int sms, int ctas) {
     const bool q4 = L.quant == Q4_0;
     int most = 8 * experts;
-    if (L.gu16 != nullptr && experts >= 32) most = (q4 ? 12 : 10) * experts;
+    if (L.gu16 != nullptr && ((long long)experts * L.H * L.I > (1 << 24) ? experts >= 8 : experts >= 32 && L.H <= 1536)) most = (q4 ? 12 : 10) * experts;
     else if (L.H <= 512) most = experts == 1 ? 16 : (q4 ? 12 : 9) * experts;
+    else if (L.H <= 1536 && experts > 1 && (long long)experts * L.I <= 256ll * sms) most = 9 * experts;  // (16 warps, items of 16 rows)
     if (ctas > 0 && ctas < sms) {
         const int tiles = 2 * experts * ((L.I + 127) / 128), ceiling = experts == 1 ? 16 : (q4 ? 12 : 9) * experts;  // (a tile of 128 rows occupies a pair)
         const int capped = most * ((tiles + ctas - 1) / ctas) / ((tiles + sms - 1) / sms);

@@ -35,11 +35,12 @@ def test_warps_of_a_prompts_streaming_down_product(cuda_lib, I, E, K, T, flags):
     assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2
 
 
-# the longest prompt on the streaming kernels: planes (8 columns an expert), narrow ones (12 | 9, a lone expert 16), layers kept as
-# f16 matrices (12 | 10, with few experts as planes)
-@pytest.mark.parametrize("quant,flags,H,E,K,T", [(1, 0, 1024, 16, 4, 32), (0, 0, 1024, 16, 4, 32), (1, 0, 512, 16, 4, 48), (0, 0, 512, 16, 4, 36),
-                                                 (1, F16, 1024, 32, 4, 96), (0, F16, 1024, 32, 4, 80), (1, F16, 1024, 16, 4, 32),
-                                                 (1, 0, 1024, 1, 1, 8), (0, 0, 512, 1, 1, 16)])
+# the longest prompt on the streaming kernels: planes (8 columns an expert), small ones (9), narrow ones (12 | 9, a lone expert 16), layers
+# kept as f16 matrices (12 | 10 where these are many bytes or many short rows, else as planes)
+@pytest.mark.parametrize("quant,flags,H,E,K,T", [(1, 0, 2048, 16, 4, 32), (0, 0, 2048, 16, 4, 32), (1, 0, 1024, 16, 4, 36), (0, 0, 1024, 16, 4, 36),
+                                                 (1, 0, 1024, 256, 4, 512), (1, 0, 512, 16, 4, 48), (0, 0, 512, 16, 4, 36),
+                                                 (1, F16, 1024, 32, 4, 96), (0, F16, 1024, 32, 4, 80), (1, F16, 1024, 16, 4, 36), (1, F16, 2048, 64, 4, 192),
+                                                 (0, F16, 2048, 64, 4, 160), (1, F16, 2048, 32, 4, 64), (1, 0, 1024, 1, 1, 8), (0, 0, 512, 1, 1, 16)])
 def test_longest_prompt_on_the_streaming_kernels(cuda_lib, quant, flags, H, E, K, T):
     I = 256
     sc, layer = context(H, I, E, K, quant, T + 1, flags)
@@ -54,9 +55,9 @@ def test_longest_prompt_on_the_streaming_kernels(cuda_lib, quant, flags, H, E, K
         assert rel_l2((out - x).cpu(), (want - x).cpu()) < TOL_REL_L2
 
 
-# ... where the tcgen05 grid is capped: 12 | 9 columns and a lone expert 16 on a few CTAs, 8 columns on nearly all
+# ... where the tcgen05 grid is capped: 12 | 9 columns and a lone expert 16 on a few CTAs, 9 columns on nearly all
 @pytest.mark.parametrize("ctas,quant,flags,E,K,T,tiles", [(1, 1, 0, 16, 4, 48, "tc"), (1, 0, 0, 16, 4, 36, "tc"), (1, 1, F16, 16, 4, 48, "tc"), (1, 1, 0, 1, 1, 16, "tc"),
-                                                          (2, 1, 0, 16, 4, 48, "pair"), (24, 1, 0, 16, 4, 48, "pair"), (146, 1, 0, 16, 4, 32, "pair"),
+                                                          (2, 1, 0, 16, 4, 48, "pair"), (24, 1, 0, 16, 4, 48, "pair"), (146, 1, 0, 16, 4, 36, "pair"),
                                                           (48, 1, 0, 1, 1, 8, "pair")])
 def test_longest_prompt_on_the_streaming_kernels_beside_a_capped_grid(cuda_lib, ctas, quant, flags, E, K, T, tiles):
     H, I = 1024, 256
