@@ -55,7 +55,6 @@ struct Shape {
 };
 template <int Q, int MODE>
 constexpr int default_warps() {
-    if (MODE == DOWN_2I) return 20;
     return Q == BF16 ? 8 : 16;
 }
 
@@ -553,7 +552,12 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_u
     const int n = stream::items_per_sm(p, p.L.rt_h);
     const bool more = p.L.quant == BF16 ? (size_t)p.T * p.K * p.L.kg_i * 512 <= 256 * 1024 && stream::rounds_less(n, 8, 12)
                                         : n <= 40 && stream::rounds_less(n, 16, 20);
-    const cudaError_t e = int8                             ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st, after_gate_up)
+    // Q4_0: 20 warps from 10 items an SM on. Fewer are one round of 16 warps with room for their longer rings (16 and 20 warps, us replayed, by items an
+    // SM: a lone expert of 1024 x 2816, 0.4, 11 tokens 35.9 and 40.3; 1024 x 2816, E = 8, 3.4 41.1 and 46.5; 1024 x 512, E = 32, 11.7 20.3 and 19.7; 1024 x
+    // 768, E = 128, 17.8 27.6 and 25.9; 2048 x 1408, E = 64, 21.5 39.8 and 35.2, 38 59.1 and 55.2; 2048 x 768, E = 128, 25 29.4 and 30.1, 35.5 37.2 and 35.1,
+    // 71 61.5 and 60.6; the worst 4096 x 512, E = 64, 25 40.6 and 41.7)
+    const cudaError_t e = int8 && n > 10                   ? stream::launch_t<Q4_0, stream::DOWN_2I, 20>(d, p.sms, st, after_gate_up)
+                          : int8                           ? stream::launch_t<Q4_0, stream::DOWN_2I>(d, p.sms, st, after_gate_up)
                           : more && p.L.quant == BF16      ? stream::launch_t<BF16, stream::DOWN_2, 12>(d, p.sms, st, after_gate_up)
                           : more && p.L.quant == Q8_0      ? stream::launch_t<Q8_0, stream::DOWN_2, 20>(d, p.sms, st, after_gate_up)
                                                            : stream::launch_q<stream::DOWN_2>(d, p.sms, st, after_gate_up);

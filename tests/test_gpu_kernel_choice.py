@@ -87,17 +87,20 @@ def test_expert_parallel_call_beside_a_capped_grid(cuda_lib, T):
     pe.close()
 
 
-# decode batches: more warps where an SM's items take a round less with them (gate/up of BF16 8 | 10, down of Q8_0 16 | 20, of BF16 8 | 12)
+# decode batches: more warps where an SM's items take a round less with them (gate/up of BF16 8 | 10, down of Q8_0 16 | 20, of BF16 8 | 12), of
+# Q4_0 (down on int8, its gate/up kernel has one form) from ten items on
 @pytest.mark.parametrize("quant,H,I,E,K,T,gate_up,down", [(2, 2048, 768, 128, 8, 4, 10, 12), (2, 2048, 768, 128, 8, 5, 8, 12), (2, 2048, 512, 256, 8, 5, 10, 12),
                                                           (2, 2048, 512, 256, 8, 16, 8, 12), (2, 2048, 768, 128, 8, 16, 10, 8), (2, 1024, 384, 64, 4, 12, 8, 8),
                                                           (0, 2048, 768, 128, 8, 3, 16, 20), (0, 2048, 768, 128, 8, 4, 16, 16),
-                                                          (0, 2048, 768, 128, 8, 6, 16, 20), (0, 2048, 768, 128, 8, 16, 16, 16)])
+                                                          (0, 2048, 768, 128, 8, 6, 16, 20), (0, 2048, 768, 128, 8, 16, 16, 16),
+                                                          (1, 1024, 2816, 1, 1, 11, 0, 16), (1, 1024, 2816, 8, 2, 15, 0, 16), (1, 1024, 512, 32, 4, 9, 0, 16),
+                                                          (1, 1024, 512, 32, 4, 14, 0, 20), (1, 2048, 768, 128, 8, 16, 0, 20)])
 def test_warps_of_a_decode_batch(cuda_lib, quant, H, I, E, K, T, gate_up, down):
     sc, layer = context(H, I, E, K, quant, T, _lib.FLAG_DECODE_SPLIT)
     x = rows(T, H)
     out = torch.empty_like(x)
     names = kernels_of(lambda: sc.decode(layer, x, x, out))
-    for mode, warps in ((2, gate_up), (3, down)):
+    for mode, warps in ((4, down),) if quant == 1 else ((2, gate_up), (3, down)):
         assert [k for k in names if f"stream_kernel<{quant}, {mode}, {warps}>" in k], names
     ref, ref_layer = context(H, I, E, K, quant, T, _lib.FLAG_PREFILL_MMA)
     want = ref.prefill(ref_layer, x, x)
