@@ -509,12 +509,13 @@ static Args decode_args(const DecodeArgs& p) {
 }
 
 // Items of an SM in a decode batch: rt rows of tiles of every expert that the tokens' choices hit, as many as under near-uniform routing.
-static int items_per_sm(const DecodeArgs& p, int rt) {
+// margin: so many more, for a choice that loses where the tokens hit more experts than that.
+static int items_per_sm(const DecodeArgs& p, int rt, float margin = 0.0f) {
     float miss = 1.0f;
     for (int t = 0; t < p.T; ++t) miss *= 1.0f - (float)p.K / (float)p.L.E;
-    return (int)ceilf((float)p.L.E * (1.0f - miss) * (float)rt / (float)p.sms);
+    return (int)ceilf((float)p.L.E * (1.0f - miss) * (float)rt / (float)p.sms + margin);
 }
-static bool rounds_less(int items, int few, int many) { return (items + many - 1) / many < (items + few - 1) / few; }
+static int rounds(int items, int warps) { return (items + warps - 1) / warps; }
 
 }  // namespace stream
 
@@ -531,7 +532,7 @@ cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st) {
     // and 48.7, 9 63.1 and 56.6, 13 80.5 and 81.5, 18 105.8 and 103.5; H = 3072, I = 1024, E = 32: 10 93 and 80; H = 4096, I = 1536, E = 64: 11 123.7
     // and 126.5, 14 146 and 150, 19 184 and 178, 31 295 and 303)
     const int n = stream::items_per_sm(p, p.L.rt_i);
-    if (p.L.quant == BF16 && n <= 30 && stream::rounds_less(n, 8, 10)) return stream::launch_t<BF16, stream::GATE_UP_2, 10>(g, p.sms, st);
+    if (p.L.quant == BF16 && n <= 30 && stream::rounds(n, 10) < stream::rounds(n, 8)) return stream::launch_t<BF16, stream::GATE_UP_2, 10>(g, p.sms, st);
     return stream::launch_q<stream::GATE_UP_2>(g, p.sms, st);
 }
 
@@ -546,12 +547,15 @@ cudaError_t launch_stream_down(const DecodeArgs& p, bool int8, bool after_gate_u
     // More warps where they take a round less. Q8_0, whose rings get shorter for it: up to two rounds (16 and 20 warps, us replayed, by items an SM.
     // H = 2048, I = 768, E = 128: 20 40.2 and 38.9, 26 44.1 and 44.8, 31 47.7 and 48.2, 36 53.5 and 51.6, 45 71.4 and 72.5, 60 85.1 and 85.9;
     // H = 2048, I = 1408, E = 64: 19 53.4 and 50.4, 23 63.5 and 65.7, 27 74 and 75.5; H = 3072, I = 1024, E = 32: 18 45.1 and 43.6, 23 49.7
-    // and 51.6, 34 71.4 and 69.5). BF16: any number, while the batch's fragments are not too many (8 and 12 warps. H = 2048, I = 768, E = 128: 14 39.0
-    // and 39.0, 36 79.2 and 77.2; H = 1024, I = 384, E = 64: 8 21.8 and 22.2, 9 24.1 and 23.1, 15 29.1 and 29.4; 256 KB: 16 tokens of I = 512
+    // and 51.6, 34 71.4 and 69.5), with half an item to spare: at the brink the tokens often hit an expert more, and a round more it is (H = 2048,
+    // I = 1408, E = 64: 40.0 105.7 and 114.0; H = 4096, I = 1536, E = 64: 19.8 62.3 and 65.9; H = 4096, I = 512, E = 64: 19.54 46.3 and 47.6).
+    // BF16: any number, while the batch's fragments are not too many (8 and 12 warps. H = 2048, I = 768, E = 128: 14 39.0 and 39.0, 36 79.2 and 77.2;
+    // H = 1024, I = 384, E = 64: 8 21.8 and 22.2, 9 24.1 and 23.1, 15 29.1 and 29.4; 256 KB: 16 tokens of I = 512
     // 125.0 and 124.5, of H = 3072, I = 1024, E = 32 113 and 111; beyond: H = 4096, I = 1536, E = 64 8 tokens, 288 KB, 211 and 215, 16 tokens 295 and 322).
     const int n = stream::items_per_sm(p, p.L.rt_h);
-    const bool more = p.L.quant == BF16 ? (size_t)p.T * p.K * p.L.kg_i * 512 <= 256 * 1024 && stream::rounds_less(n, 8, 12)
-                                        : n <= 40 && stream::rounds_less(n, 16, 20);
+    const int spare = stream::items_per_sm(p, p.L.rt_h, 0.5f);
+    const bool more = p.L.quant == BF16 ? (size_t)p.T * p.K * p.L.kg_i * 512 <= 256 * 1024 && stream::rounds(n, 12) < stream::rounds(n, 8)
+                                        : spare <= 40 && stream::rounds(spare, 20) < stream::rounds(n, 16);
     // Q4_0: 20 warps from 10 items an SM on. Fewer are one round of 16 warps with room for their longer rings (16 and 20 warps, us replayed, by items an
     // SM: a lone expert of 1024 x 2816, 0.4, 11 tokens 35.9 and 40.3; 1024 x 2816, E = 8, 3.4 41.1 and 46.5; 1024 x 512, E = 32, 11.7 20.3 and 19.7; 1024 x
     // 768, E = 128, 17.8 27.6 and 25.9; 2048 x 1408, E = 64, 21.5 39.8 and 35.2, 38 59.1 and 55.2; 2048 x 768, E = 128, 25 29.4 and 30.1, 35.5 37.2 and 35.1,

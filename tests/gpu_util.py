@@ -1,4 +1,6 @@
 """Helpers shared by the GPU parity tests."""
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -37,20 +39,22 @@ def oracle_layer(blob_np, meta, lay, K, x, residual, logits=None, gating=0, thre
 
 
 def kernels_of(call):
-    """Names of the kernels that a call launches, in the order of their start. Of a short recording the profiler now and then drops the first events, so
-    two calls are recorded, until they show the same kernels."""
+    """Names of the kernels that a call launches, in the order of their start. The profiler drops kernels that its clocks place before
+    the recording's start, hence the pause, and two calls that have to show the same kernels."""
     call()  # (one-time set-up inside the library)
     for _ in range(5):
         torch.cuda.synchronize()
         with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+            time.sleep(0.02)
             for _ in range(2):
                 call()
                 torch.cuda.synchronize()
+            time.sleep(0.02)
         names = [e.name for e in sorted(prof.events(), key=lambda e: e.time_range.start) if "lumen::" in e.name]
         half = len(names) // 2
         if names and sorted(names[:half]) == sorted(names[half:]):  # (kernels that overlap may start in either order)
             return names[:half]
-    pytest.skip("the profiler records no kernels on this machine" if not names else "the profiler drops kernels")
+    pytest.skip(f"the profiler does not record every kernel: {names}")
 
 
 def pair_kernel(quant, mode, narrow):

@@ -93,6 +93,7 @@ def test_expert_parallel_call_beside_a_capped_grid(cuda_lib, T):
                                                           (2, 2048, 512, 256, 8, 16, 8, 12), (2, 2048, 768, 128, 8, 16, 10, 8), (2, 1024, 384, 64, 4, 12, 8, 8),
                                                           (0, 2048, 768, 128, 8, 3, 16, 20), (0, 2048, 768, 128, 8, 4, 16, 16),
                                                           (0, 2048, 768, 128, 8, 6, 16, 20), (0, 2048, 768, 128, 8, 16, 16, 16),
+                                                          (0, 2048, 1408, 64, 6, 12, 16, 20), (0, 2048, 1408, 64, 6, 13, 16, 16), (0, 4096, 1536, 64, 6, 2, 16, 16),
                                                           (1, 1024, 2816, 1, 1, 11, 0, 16), (1, 1024, 2816, 8, 2, 15, 0, 16), (1, 1024, 512, 32, 4, 9, 0, 16),
                                                           (1, 1024, 512, 32, 4, 14, 0, 20), (1, 2048, 768, 128, 8, 16, 0, 20)])
 def test_warps_of_a_decode_batch(cuda_lib, quant, H, I, E, K, T, gate_up, down):
