@@ -657,12 +657,13 @@ bool route_single_applicable(const PrefillArgs& a) {
 // position inside the expert's segment is the expert's running cursor plus the number
 // of lower lanes with the same expert, so the placement is stable.
 // The segment bounds are a scan of the row totals, which every CTA does for itself, so that the plan (the last CTA) is made beside the
-// placement and not in front of it.
+// placement and not in front of it. The rows of the histogram are read by expert, a lane per chunk (a warp reading its own
+// chunk's column made as many requests as there are counts: 4096 tokens of 256 experts, the whole chain 24.5 -> 19.9 us).
 constexpr int PLACE_CHUNKS = PLAN_THREADS / 32;
 __global__ void __launch_bounds__(PLAN_THREADS)
 sort_place_kernel(const uint32_t* __restrict__ ids, int T, int K, const int32_t* __restrict__ blk_hist, int nchunks, RouteDev R,
                   const __grid_constant__ PlanArgs plan) {
-    extern __shared__ int cursor[];  // [PLACE_CHUNKS][E]
+    extern __shared__ int cursor[];  // [PLACE_CHUNKS][E | 1]
     __shared__ int cnt_s[MAX_EXPERTS], bounds_s[MAX_EXPERTS], wsum_s[MAX_EXPERTS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, E = plan.E;
     grid_dep_sync();
@@ -685,10 +686,10 @@ sort_place_kernel(const uint32_t* __restrict__ ids, int T, int K, const int32_t*
         }
         if (lane == 31) wsum_s[warp] = inc;
     }
-    const int chunk = blockIdx.x * PLACE_CHUNKS + warp;
-    int* cur = cursor + warp * E;
-    if (chunk < nchunks)
-        for (int e = lane; e < E; e += 32) cur[e] = blk_hist[(size_t)e * nchunks + chunk];
+    const int chunk0 = blockIdx.x * PLACE_CHUNKS, chunk = chunk0 + warp;
+    int* cur = cursor + warp * (E | 1);  // (an odd stride: the lanes below hit 32 banks)
+    if (chunk0 + lane < nchunks)
+        for (int e = warp; e < E; e += PLACE_CHUNKS) cursor[lane * (E | 1) + e] = blk_hist[(size_t)e * nchunks + chunk0 + lane];
     __syncthreads();
     if (tid < MAX_EXPERTS) {
         int base = 0;
@@ -980,7 +981,7 @@ cudaError_t launch_route_large(const PrefillArgs& a, cudaStream_t st) {
         CUDA_RET(launch_dep(sort_hist_kernel, dim3(nchunks), dim3(256), 0, st, a.R.ids, T, K, E, a.blk_hist));
     if (one_cta) return launch_dep(sort_one_kernel, dim3(1), dim3(SORT1_WARPS * 32), 0, st, a.R.ids, C, K, a.R, plan);
     CUDA_RET(launch_dep(sort_rowscan_kernel, dim3(E), dim3(32), 0, st, a.blk_hist, nchunks));
-    return launch_dep(sort_place_kernel, dim3((nchunks + PLACE_CHUNKS - 1) / PLACE_CHUNKS + 1), dim3(PLAN_THREADS), (size_t)PLACE_CHUNKS * E * 4, st, a.R.ids, T,
+    return launch_dep(sort_place_kernel, dim3((nchunks + PLACE_CHUNKS - 1) / PLACE_CHUNKS + 1), dim3(PLAN_THREADS), (size_t)PLACE_CHUNKS * (E | 1) * 4, st, a.R.ids, T,
                       K, a.blk_hist, nchunks, a.R, plan);
 }
 

@@ -173,7 +173,7 @@ def test_small_router_rows(cuda_lib, E, H, T):
 
 
 # one CTA sorts up to 2048 pairs, the general chain more; experts beyond one warp's 128
-@pytest.mark.parametrize("T,E,K", [(256, 128, 8), (257, 128, 8), (2048, 16, 1), (2049, 16, 1), (129, 256, 16), (700, 33, 5)])
+@pytest.mark.parametrize("T,E,K", [(256, 128, 8), (257, 128, 8), (2048, 16, 1), (2049, 16, 1), (129, 256, 16), (700, 33, 5), (512, 256, 8), (2050, 255, 2)])
 def test_sorting_on_both_sides_of_one_cta(cuda_lib, T, E, K):
     lg = synth.zipf_logits(T, E, T)
     sc = moe.allocate_moe_scratch(256, 128, E, K, T)
