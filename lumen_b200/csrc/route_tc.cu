@@ -391,16 +391,21 @@ cudaError_t launch_router_logits_tc(const __half* w16, int T, int E, int H, int 
     a.m_tiles = (E + 127) / 128;
     cudaError_t e = make_tmap_f16(w16, (uint64_t)2 * E, (uint64_t)H, 128, &a.tmap_w);
     if (e != cudaSuccess) return e;
-    // bytes of a CTA's stage (weights + activations) times the waves of CTAs: 1777 tokens of 128 experts take one wave of tiles
-    // of 64 tokens (two of 32: 15.2 -> 10.3 us), 8192 tokens one of 256 (two of 128: 28.8 -> 28.3 us)
+    // The least bytes of a CTA's stage (weights + activations) times the waves of CTAs. Two measured exceptions: tiles of 64 tokens lose to
+    // half as many of 128 from 5/7 of the SMs on, and tiles of 256 to a second wave of 128 that is short (the whole routing, us, f32 and bf16-valued rows,
+    // H = 2048, by tile width. E = 128: 1200 tokens 32 39.7 and 29.5, 64 37.2 and 26.6; 1800 tokens 32 46.5 and 33.4, 64 (116 CTAs) 47.5 and 35.3, 128 46.6
+    // and 29.9; 8192 tokens 128 87.7 and 68.3, 256 84.5 and 65.3. E = 256: 832 tokens 64 (104 CTAs) 37.7 and 29.4, 128 39.7 and 30.6; 896 tokens 64 (112)
+    // 44.2 and 36.3, 128 39.6 and 31.7; 2500 tokens 128 (160) 60.3 and 45.7, 256 67.2 and 49.3; 3000 tokens 128 (192) 66.8 and 52.3, 256 64.4 and 49.5)
     int bn = 32;
-    long long least = 0;
+    long long least = 0, before = 0;  // before: CTAs of the width before
     for (int b = 32; b <= 256; b *= 2) {
-        const long long ctas = (long long)((T + b - 1) / b) * a.m_tiles * ksplit, cost = (ctas + sms - 1) / sms * (2 * tc::SUB_BYTES + 2 * b * 128);
-        if (b == 32 || cost < least) {
+        const long long ctas = (long long)((T + b - 1) / b) * a.m_tiles * ksplit, room = b == 64 ? sms * 5 / 7 : sms;
+        const long long cost = (ctas + room - 1) / room * (2 * tc::SUB_BYTES + 2 * b * 128);
+        if (b == 32 || (cost <= least && !(b == 256 && 4 * before < 5 * sms))) {
             least = cost;
             bn = b;
         }
+        before = ctas;
     }
     e = make_tmap_f16(x16, (uint64_t)2 * T, (uint64_t)H, bn, &a.tmap_x);
     if (e != cudaSuccess) return e;

@@ -118,6 +118,18 @@ def test_gate_up_tiles_of_one_cta(cuda_lib, quant, flags, T, cols):
         assert [k for k in names if "grouped_gemm_tc_kernel" in k and f", {mode}, {cols}," in k], names
 
 
+# tokens per tile of the tcgen05 router: by bytes and waves of CTAs, 128 instead of 64 where these fill most SMs, instead of 256 where its second wave is short
+@pytest.mark.parametrize("E,T,width", [(128, 100, 32), (128, 1000, 32), (128, 1500, 64), (128, 1800, 128), (128, 4096, 128), (128, 6000, 256),
+                                       (256, 832, 64), (256, 1000, 128), (256, 2500, 128), (256, 3000, 256)])
+def test_router_tile_width(cuda_lib, E, T, width):
+    lay = synth.LayerLayout(2048, 128, E, 1)
+    sc = moe.allocate_moe_scratch(2048, 128, E, 8, T)
+    layer = sc.prepare_router_only(synth.make_layer_blob(lay, 9), lay.meta().router_weight_off)
+    x = rows(T, 2048)
+    names = kernels_of(lambda: sc.route_only(layer, x))
+    assert [k for k in names if f"router_logits_tc_kernel<{width}>" in k], names
+
+
 # rows gathered by column are kept only where a kernel reads them: a grid capped at one CTA
 def test_device_memory_of_a_prefill_context(cuda_lib):
     H, K, T = 2048, 8, 8192

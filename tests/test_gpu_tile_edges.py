@@ -210,7 +210,7 @@ def test_router_tiles_of_every_width_agree(cuda_lib, E):
     x = torch.randn((T, H), generator=torch.Generator("cuda").manual_seed(1), device="cuda")
     parts = [sc.route_only(layer, x[t:t + 23].contiguous(), want_logits=True)[2].clone() for t in range(0, T, 23)]
     ref = torch.cat(parts)
-    for n in (1000, 1700, 2300, T):
+    for n in (700, 1000, 1400, 1700, 2300, T):
         assert torch.equal(sc.route_only(layer, x[:n].contiguous(), want_logits=True)[2], ref[:n])
 
 
