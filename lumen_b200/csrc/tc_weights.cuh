@@ -1,5 +1,6 @@
 // Arithmetic that the tcgen05 prefill kernels on CTA pairs (prefill_pair.cu) and on single CTAs (prefill_tc.cu) share: the results of an
-// expert-parallel call are one GPU's to the bit because both take their weights and SwiGLU from here.
+// expert-parallel call are one GPU's to the bit because both take their SwiGLU from here and unpack weights as here
+// (prefill_tc.cu has store_weights written out, see dequant_store there; tests compare the two forms' outputs).
 #pragma once
 #include "mma_frag.cuh"
 #include "tc_common.cuh"
