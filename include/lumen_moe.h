@@ -90,7 +90,8 @@ typedef struct {
  *   memory: memory traded for prefill speed. BF16 layers always work that way (nothing to
  *   dequantise). Decode is not affected.
  * TC_CTAS(n): cap of the persistent tcgen05 grid, n CTAs (one per SM), 0 = every SM. (Pairs of CTAs share a tile:
- *   an odd n above one runs on n - 1.) */
+ *   an odd n above one runs on n - 1.) The fewer CTAs, the longer prompts stay on kernels that the cap does not concern; around that
+ *   line a capped and an uncapped context's results differ in the rounding of sums. */
 #define LUMEN_MOE_FLAG_DECODE_SPLIT 0x1
 #define LUMEN_MOE_FLAG_PREFILL_MMA 0x2
 #define LUMEN_MOE_FLAG_SHORT_WAITS 0x4
@@ -326,7 +327,8 @@ LUMEN_MOE_API lumen_moe_status_t lumen_moe_ep_prepare(lumen_moe_ctx* ctx, const 
  * calls, each on its own tokens; tokens may differ per rank, 1 <= tokens <= max_tokens):
  *   lumen_moe_prefill_ep  out[t] = residual[t] + sum_k w[t,k] * FFN_{e(t,k)}(normed[t]) for this
  *                         rank's tokens; bit-identical to lumen_moe_prefill on one GPU for the
- *                         same tokens. d_normed [T,H] f32 or bf16, 16-byte aligned.
+ *                         same tokens (contexts of the same flags; layers kept as f16 matrices: of
+ *                         an uncapped tcgen05 grid). d_normed [T,H] f32 or bf16, 16-byte aligned.
  *   lumen_moe_stack_prefill_ep   the layer stack of lumen_moe_stack_prefill in this form.
  * Every cross-rank wait is bounded (2 s; 2 ms with LUMEN_MOE_FLAG_SHORT_WAITS): a rank whose
  * peer does not show up gets LUMEN_MOE_TIMEOUT through lumen_moe_poll_status, and an overflow
