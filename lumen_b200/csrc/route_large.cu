@@ -658,7 +658,7 @@ bool route_single_applicable(const PrefillArgs& a) {
 // of lower lanes with the same expert, so the placement is stable.
 // The segment bounds are a scan of the row totals, which every CTA does for itself, so that the plan (the last CTA) is made beside the
 // placement and not in front of it. The rows of the histogram are read by expert, a lane per chunk (a warp reading its own
-// chunk's column made as many requests as there are counts: 4096 tokens of 256 experts, the whole chain 24.5 -> 19.9 us).
+// chunk's column made as many requests as there are counts: 4096 tokens of 256 experts, top-k and sort 24.5 -> 20.8 us).
 constexpr int PLACE_CHUNKS = PLAN_THREADS / 32;
 __global__ void __launch_bounds__(PLAN_THREADS)
 sort_place_kernel(const uint32_t* __restrict__ ids, int T, int K, const int32_t* __restrict__ blk_hist, int nchunks, RouteDev R,
