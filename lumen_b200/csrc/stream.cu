@@ -177,7 +177,8 @@ stream_kernel(const __grid_constant__ Args a) {
     // of Q4_0 129 -> 132). With a round or less there is nothing to even out, and the two divisions stand in front of the first request (4 tokens
     // of 512 x 256 15.3 -> 14.5 us, 2 of 3072 x 1024 35.7 -> 35.1).
     int nw = WARPS;
-    if (((Q == Q4_0 && TERMS == 2) || (Q == BF16 && DOWN && WARPS > 8)) && i1 - i0 > WARPS) {
+    // (16 warps on int8 are for batches of fewer items, and pay for the code: a lone expert of 1024 x 2816 with 16 tokens 39.3 -> 42.0)
+    if (((Q == Q4_0 && TERMS == 2 && !(I8 && WARPS == 16)) || (Q == BF16 && DOWN && WARPS > 8)) && i1 - i0 > WARPS) {
         const int n = i1 - i0, rounds = (n + WARPS - 1) / WARPS;
         nw = (n + rounds - 1) / rounds;
         if (warp >= nw) i1 = i0;
