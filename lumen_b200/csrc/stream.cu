@@ -528,12 +528,13 @@ cudaError_t launch_stream_gate_up(const DecodeArgs& p, cudaStream_t st) {
     g.b_row = (size_t)p.L.kg_h * 16;
     g.sf = p.sf;
     g.debug_extra_tx = p.debug_expire;
-    // BF16: ten warps where they take a round less than eight, up to three rounds (eight and ten, us replayed, by items an SM. H = 2048, I = 768, E = 128: 10
+    // BF16: ten warps where they take a round less than eight, up to two rounds (eight and ten, us replayed, by items an SM. H = 2048, I = 768, E = 128: 10
     // 65.2 and 60.2, 12 70.7 and 72.9, 14 79.2 and 80.4, 17 98.5 and 94.6, 23 119.9 and 122.6, 25 137.2 and 136.1; I = 512, E = 256: 7 48.7
     // and 48.7, 9 63.1 and 56.6, 13 80.5 and 81.5, 18 105.8 and 103.5; H = 3072, I = 1024, E = 32: 10 93 and 80; H = 4096, I = 1536, E = 64: 11 123.7
-    // and 126.5, 14 146 and 150, 19 184 and 178, 31 295 and 303)
+    // and 126.5, 14 146 and 150, 19 184 and 178, 31 295 and 303. Three rounds for four gain 2 % at most, as 25 above, and one call loses by them: H = 4096, I = 1536,
+    // E = 64: 24.4 222 and 242)
     const int n = stream::items_per_sm(p, p.L.rt_i);
-    if (p.L.quant == BF16 && n <= 30 && stream::rounds(n, 10) < stream::rounds(n, 8)) return stream::launch_t<BF16, stream::GATE_UP_2, 10>(g, p.sms, st);
+    if (p.L.quant == BF16 && n <= 20 && stream::rounds(n, 10) < stream::rounds(n, 8)) return stream::launch_t<BF16, stream::GATE_UP_2, 10>(g, p.sms, st);
     return stream::launch_q<stream::GATE_UP_2>(g, p.sms, st);
 }
 

@@ -90,7 +90,7 @@ def test_expert_parallel_call_beside_a_capped_grid(cuda_lib, T):
 # decode batches: more warps where an SM's items take a round less with them (gate/up of BF16 8 | 10, down of Q8_0 16 | 20, of BF16 8 | 12), of
 # Q4_0 (down on int8, its gate/up kernel has one form) from ten items on
 @pytest.mark.parametrize("quant,H,I,E,K,T,gate_up,down", [(2, 2048, 768, 128, 8, 4, 10, 12), (2, 2048, 768, 128, 8, 5, 8, 12), (2, 2048, 512, 256, 8, 5, 10, 12),
-                                                          (2, 2048, 512, 256, 8, 16, 8, 12), (2, 2048, 768, 128, 8, 16, 10, 8), (2, 1024, 384, 64, 4, 12, 8, 8),
+                                                          (2, 2048, 512, 256, 8, 16, 8, 12), (2, 2048, 768, 128, 8, 16, 8, 8), (2, 4096, 1536, 64, 6, 9, 8, 8), (2, 1024, 384, 64, 4, 12, 8, 8),
                                                           (0, 2048, 768, 128, 8, 3, 16, 20), (0, 2048, 768, 128, 8, 4, 16, 16),
                                                           (0, 2048, 768, 128, 8, 6, 16, 20), (0, 2048, 768, 128, 8, 16, 16, 16),
                                                           (0, 2048, 1408, 64, 6, 12, 16, 20), (0, 2048, 1408, 64, 6, 13, 16, 16), (0, 4096, 1536, 64, 6, 2, 16, 16),
